@@ -714,14 +714,6 @@ int build_tasks(Ctx& c, int depth) {
   if ((int64_t)tasks.size() > c.ntasks_cap) return set_err(HF_EARG, "task depth below the minimum");
   c.ntasks = (int64_t)tasks.size();
   c.A.ntasks = c.ntasks;
-  std::vector<int32_t> large;
-  for (int64_t i = 0; i < c.ninst; ++i)
-    if (c.h_inst[i].ntask > kWarpSumMax) large.push_back((int32_t)i);
-  c.A.nlarge = (int64_t)large.size();
-  c.A.nsmall = c.ninst - c.A.nlarge;
-  if (!large.empty())
-    CU(cudaMemcpyAsync(const_cast<int32_t*>(c.A.large), large.data(), sizeof(int32_t) * large.size(),
-                       cudaMemcpyHostToDevice, c.stream));
   CU(cudaMemcpyAsync(const_cast<int4*>(c.A.tasks), tasks.data(), sizeof(int4) * tasks.size(),
                      cudaMemcpyHostToDevice, c.stream));
   CU(cudaMemcpyAsync(const_cast<InstDesc*>(c.A.inst), c.h_inst.data(), sizeof(InstDesc) * c.ninst,
@@ -865,13 +857,15 @@ int create_impl(const hf_problem* probs, int64_t count, const hf_solver_opts* op
   A.task_heat = d_task_heat;
   A.tasks = d_tasks;
   A.ntasks = c.ntasks;
-  ALLOC(A.partials, (size_t)c.ntasks * kNR);
-  ALLOC(c.d_sctl, (size_t)1);
+  A.pcap = c.ntasks;
+  ALLOC(A.partials, (size_t)A.pcap * kNR * 2);   // two tables (the one-grid solve alternates)
+  {
+    char* sctl;                 // the control block and, behind it, the instances' queue entries
+    ALLOC(sctl, solve_ctl_bytes(count));
+    c.d_sctl = reinterpret_cast<SolveCtl*>(sctl);
+  }
   ALLOC(A.counters, (size_t)count);
   ALLOC(c.d_bc, (size_t)count);
-  int32_t* d_large;
-  ALLOC(d_large, (size_t)count);
-  A.large = d_large;
   A.inst = d_inst; A.scal = d_scal; A.tile_inst = d_tile_inst;
   ALLOC(A.diag, N); ALLOC(A.cx, N); ALLOC(A.cy, N); ALLOC(A.cz, N); ALLOC(A.sinv, N);
   ALLOC(A.rsum, N); ALLOC(A.sinv32, N);
@@ -899,7 +893,7 @@ int create_impl(const hf_problem* probs, int64_t count, const hf_solver_opts* op
 #define CK(call) do { cudaError_t e_ = (call); if (e_ != cudaSuccess) return fail(set_err(HF_ECUDA, std::string(#call) + ": " + cudaGetErrorString(e_))); } while (0)
   CK(cudaMemsetAsync(A.counters, 0, sizeof(unsigned) * count, c.stream));
   CK(cudaMemsetAsync(d_scal, 0, sizeof(InstScal) * count, c.stream));
-  CK(cudaMemsetAsync(c.d_sctl, 0, sizeof(SolveCtl), c.stream));
+  CK(cudaMemsetAsync(c.d_sctl, 0, solve_ctl_bytes(count), c.stream));
   CK(cudaMemsetAsync(A.stamps, 0, sizeof(unsigned long long) * kStamps, c.stream));
   CK(cudaMemsetAsync(A.check, 0, sizeof(unsigned long long) * 4, c.stream));
   for (void* p : {(void*)A.diag, (void*)A.cx, (void*)A.cy, (void*)A.cz, (void*)c.asm_.kappa,

@@ -35,9 +35,6 @@ constexpr int kNR = 8;
 // depth (InstDesc::zc planes, an option; kZC by default) along z.  (kXC > 1 trades occupancy for
 // per-thread parallelism; on GB300 kXC = 1 is faster.)
 constexpr int kXC = 1, kTX = 32 * kXC, kTY = 8, kZC = 32;
-// Instances with more tasks than this have their task partials summed by a whole block, the
-// others by one warp.
-constexpr int kWarpSumMax = 512;
 constexpr int kMinTaskDepth = 4;   // task buffers are sized for the shallowest task depth
 // InstScal::status bit: some S was NaN; the failing vector is found by the diagnosis kernel.
 constexpr int kStatusRhsNan = 1 << 16;                       // reduction slots per tile
@@ -145,18 +142,33 @@ enum : int32_t {
 // Control block of one launch of the persistent solve kernel (zeroed before every launch).
 constexpr int kRoundLog = 512;                     // rounds whose end time is recorded
 struct SolveCtl {
-  unsigned count;          // blocks arrived at the current grid barrier
-  unsigned gen;            // barrier generation (release/acquire)
-  unsigned result[2];      // "some instance has work", published by barrier parity
-  int32_t err;             // a barrier wait gave up (time limit): the launch was abandoned
+  int32_t err;             // a wait gave up (time limit): the launch was abandoned
   int32_t guard_hit;       // the round bound was reached
-  int32_t pad;
-  unsigned next_task[2];   // tasks handed out in the current round (by round parity)
+  // one grid
+  alignas(128) unsigned long long arrived;   // blocks arrived at all grid barriers so far
+  alignas(128) unsigned next_task[4];        // tasks handed out in a round (by round mod 4)
+  // several grids
+  alignas(128) unsigned long long ticket;    // tickets handed out
+  alignas(128) unsigned long long tail;      // tickets published beyond the first phase's
+  unsigned long long phases;                 // phases published
+  unsigned finished;                         // instances without work left
   int64_t rounds;          // rounds run
   unsigned long long t_start;                 // %globaltimer at kernel start (ns)
   unsigned long long t_round[kRoundLog];      // %globaltimer when round r's barrier opened
   int32_t phase_log[kRoundLog];               // phase instance 0 ran in round r
 };
+
+// Several grids: behind the control block, each instance's published ticket range, then its count
+// of finished tasks.
+__host__ __device__ inline size_t solve_ctl_bytes(int64_t ninst) {
+  return sizeof(SolveCtl) + (size_t)ninst * (sizeof(unsigned long long) + sizeof(unsigned));
+}
+__device__ __forceinline__ unsigned long long* solve_slots(SolveCtl* ctl) {
+  return reinterpret_cast<unsigned long long*>(ctl + 1);
+}
+__device__ __forceinline__ unsigned* solve_done(SolveCtl* ctl, int64_t ninst) {
+  return reinterpret_cast<unsigned*>(solve_slots(ctl) + ninst);
+}
 
 // Options mirrored on the device.
 struct DevOpts {
@@ -172,7 +184,8 @@ struct DevArrays {
   const InstDesc* inst;
   InstScal* scal;
   const int32_t* tile_inst;
-  double* partials;       // ntasks * kNR partial sums, one fixed slot range per task
+  double* partials;       // partial sums of the tasks: value k of task t at [k * pcap + t]; two such
+                          // tables of kNR values, used by alternate rounds of the one-grid solve
   unsigned int* counters; // per instance, last-block detection
   DevOpts opts;
   // static
@@ -199,9 +212,7 @@ struct DevArrays {
   const int8_t* task_heat;  // per task: some cell holds a heater
   const int4* tasks;        // (instance, x0, y0, z0) per task
   int64_t ncells, ntiles, ninst, ntasks;
-  int64_t nsmall;           // instances with at most kWarpSumMax tasks (their partials: one warp)
-  const int32_t* large;     // the other instances (block sums), nlarge of them
-  int64_t nlarge;
+  int64_t pcap;             // tasks that a table of partial sums holds
   // index-check record of the checked build (HF_CHECKED): [0] failed checks, [1] site of the
   // first, [2] its index, [3] the extent it was checked against
   unsigned long long* check;
@@ -390,20 +401,22 @@ __device__ __forceinline__ void block_sum(double (&v)[NRV], double* smem /* [32*
   __syncthreads();
 }
 
-// Write this tile's partial sums (fixed slot per tile; summed by a finalize kernel).
-// FP64 values go through shared memory and only warp 0 adds them (8 + 5 adds per value per
-// block): on GB300 every FP64 warp instruction costs the slow FP64 pipe, so a shuffle tree in
-// all eight warps would cost more than the kernel's own arithmetic.
-template <int NRV>
-__device__ __forceinline__ void tile_store(double* dst, const double (&v)[NRV]);
-template <int NRV>
-__device__ __forceinline__ void tile_store(const DevArrays& A, int64_t tile, const double (&v)[NRV]) {
-  tile_store<NRV>(A.partials + tile * kNR, v);
+// Sum of 256 values, one per thread, by the first warp of the block: the values of the threads
+// with the same lane as a tree over the eight warps, then a shuffle tree over the lanes.  This is
+// the order of every sum over a task's threads and over an instance's tasks: three and five adds
+// deep, because an FP64 add's latency is paid at each level.
+__device__ __forceinline__ double tree8(const double (&t)[8]) {
+  return ((t[0] + t[1]) + (t[2] + t[3])) + ((t[4] + t[5]) + (t[6] + t[7]));
 }
-// dst: the kNR partial slots of one task
+
+// Write a task's partial sums (a fixed place per task; summed by instance_sum): value k to
+// dst[k * stride].  FP64 values go through shared memory and only warp 0 adds them (8 + 5 adds per
+// value per block): on GB300 every FP64 warp instruction costs the slow FP64 pipe, so a shuffle
+// tree in all eight warps would cost more than the kernel's own arithmetic.
 template <int NRV>
-__device__ __forceinline__ void tile_store(double* dst, const double (&v)[NRV]) {
+__device__ __forceinline__ void tile_store(double* dst, int64_t stride, const double (&v)[NRV]) {
   static_assert(NRV <= kNR, "reduction slots");
+  static_assert(kBlock == 256, "eight warps");
   __shared__ double stage[NRV][kBlock];
   __syncthreads();   // the previous tile of this block has finished reading the stage
 #pragma unroll
@@ -411,15 +424,28 @@ __device__ __forceinline__ void tile_store(double* dst, const double (&v)[NRV]) 
   __syncthreads();
   if (threadIdx.x < 32) {
     const int lane = threadIdx.x;
+    double t[NRV];
 #pragma unroll
     for (int k = 0; k < NRV; ++k) {
-      double t = stage[k][lane];
+      double u[8];
 #pragma unroll
-      for (int w = 1; w < kBlock / 32; ++w) t += stage[k][lane + 32 * w];
-      t = warp_sum(t);
-      if (lane == 0) dst[k] = t;
+      for (int w = 0; w < 8; ++w) u[w] = stage[k][lane + 32 * w];
+      t[k] = tree8(u);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+      for (int k = 0; k < NRV; ++k) t[k] += __shfl_xor_sync(0xffffffffu, t[k], o);
+    }
+    if (lane == 0) {
+#pragma unroll
+      for (int k = 0; k < NRV; ++k) dst[k * stride] = t[k];
     }
   }
+}
+template <int NRV>
+__device__ __forceinline__ void tile_store(const DevArrays& A, int64_t task, const double (&v)[NRV]) {
+  tile_store<NRV>(A.partials + task, A.pcap, v);
 }
 
 // The columns of a task that this thread owns.

@@ -185,7 +185,7 @@ __device__ __forceinline__ void rhs4_fast_task(const DevArrays& A, int64_t task,
     }
   }
   const double bb = sq.value();
-  if (threadIdx.x == 0) A.partials[task * kNR + 1] = 0.0;   // no x0 - T < TINY test here
+  if (threadIdx.x == 0) A.partials[A.pcap + task] = 0.0;   // no x0 - T < TINY test here
   const double v[1] = {bb};
   tile_store<1>(A, task, v);
 }
@@ -253,7 +253,7 @@ __device__ __noinline__ void rhs4_task(const DevArrays& A, int64_t task, const I
   }
   bb = sq.value();
   const int any_flag = __syncthreads_or(flag);
-  if (threadIdx.x == 0) A.partials[task * kNR + 1] = any_flag ? 1.0 : 0.0;
+  if (threadIdx.x == 0) A.partials[A.pcap + task] = any_flag ? 1.0 : 0.0;
   const double v[1] = {bb};
   tile_store<1>(A, task, v);
 }
@@ -384,13 +384,13 @@ __global__ void __launch_bounds__(kBlock, 4) k_rhs(DevArrays A, double* oB, doub
     const int c1 = __syncthreads_count(nan_q), c2 = __syncthreads_count(nan_qd);
     const int c3 = __syncthreads_count(nan_sc), c4 = __syncthreads_count(nan_s);
     if (threadIdx.x == 0) {
-      A.partials[task * kNR + 1] = (double)c1;
-      A.partials[task * kNR + 2] = (double)c2;
-      A.partials[task * kNR + 3] = (double)c3;
-      A.partials[task * kNR + 4] = (double)c4;
+      A.partials[A.pcap + task] = (double)c1;
+      A.partials[2 * A.pcap + task] = (double)c2;
+      A.partials[3 * A.pcap + task] = (double)c3;
+      A.partials[4 * A.pcap + task] = (double)c4;
     }
   } else if (threadIdx.x == 0) {
-    A.partials[task * kNR + 1] = any_flag ? 1.0 : 0.0;
+    A.partials[A.pcap + task] = any_flag ? 1.0 : 0.0;
   }
   const double v[1] = {bb};
   tile_store<1>(A, task, v);
@@ -694,7 +694,7 @@ __global__ void k_sumsq_partial(DevArrays A, const double* b, int64_t n) {
 
 __global__ void k_sumsq_final(DevArrays A, int nparts) {
   double acc = 0.0;
-  for (int t = threadIdx.x; t < nparts; t += blockDim.x) acc += A.partials[(int64_t)t * kNR];
+  for (int t = threadIdx.x; t < nparts; t += blockDim.x) acc += A.partials[t];
   __shared__ double red[32];
   double v[1] = {acc};
   block_sum<1>(v, red);

@@ -142,8 +142,8 @@ __device__ __forceinline__ T plane_above(const TCell& c, int j, V v, int z) {
   return T(0);
 }
 
-// FP32 block sum of one value into partial slot k of a task (one conversion per block).
-__device__ __forceinline__ void task_store_f(double* dst, int k, float v) {
+// FP32 block sum of one value into *dst, a partial sum of a task (one conversion per block).
+__device__ __forceinline__ void task_store_f(double* dst, float v) {
   __shared__ float red[kBlock / 32];
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -155,7 +155,7 @@ __device__ __forceinline__ void task_store_f(double* dst, int k, float v) {
     v = lane < kBlock / 32 ? red[lane] : 0.f;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
-    if (lane == 0) dst[k] = (double)v;
+    if (lane == 0) *dst = (double)v;
   }
 }
 
@@ -254,12 +254,12 @@ __device__ __forceinline__ void res_hx_task(const DevArrays& A, double* part, in
   }
   if (sizeof(TR) == 4) rr = rq.value();
   if (sizeof(TR) == 4) {
-    task_store_f(part + task * kNR, 1, gg);
+    task_store_f(part + A.pcap + task, gg);
     const double v[1] = {rr};
-    tile_store<1>(part + task * kNR, v);
+    tile_store<1>(part + task, A.pcap, v);
   } else {
     const double v[2] = {rr, gg64};
-    tile_store<2>(part + task * kNR, v);
+    tile_store<2>(part + task, A.pcap, v);
   }
 }
 
@@ -375,12 +375,12 @@ __device__ __forceinline__ void res_task(const DevArrays& A, double* part, int64
   }
   if (sizeof(TR) == 4) rr = rq.value();
   if (sizeof(TR) == 4) {
-    task_store_f(part + task * kNR, 1, gg);
+    task_store_f(part + A.pcap + task, gg);
     const double v[1] = {rr};
-    tile_store<1>(part + task * kNR, v);
+    tile_store<1>(part + task, A.pcap, v);
   } else {
     const double v[2] = {rr, gg64};
-    tile_store<2>(part + task * kNR, v);
+    tile_store<2>(part + task, A.pcap, v);
   }
 }
 
@@ -562,10 +562,10 @@ __device__ __forceinline__ void spmv_task(const DevArrays& A, double* part, int6
     cur = nxt;
   }
   if (sizeof(T) == 4) {
-    task_store_f(part + task * kNR, 0, (float)pq);
+    task_store_f(part + task, (float)pq);
   } else {
     const double v[1] = {(double)pq};
-    tile_store<1>(part + task * kNR, v);
+    tile_store<1>(part + task, A.pcap, v);
   }
 }
 
@@ -616,10 +616,10 @@ __device__ __forceinline__ void upd_task(const DevArrays& A, double* part, int64
     }
   }
   if (sizeof(T) == 4 && !weighted) {
-    task_store_f(part + task * kNR, 0, (float)rr);
+    task_store_f(part + task, (float)rr);
   } else {
     const double v[2] = {(double)rr, rw};
-    tile_store<2>(part + task * kNR, v);
+    tile_store<2>(part + task, A.pcap, v);
   }
 }
 
@@ -801,7 +801,7 @@ __device__ __forceinline__ void spmv4_task(const DevArrays& A, double* part, int
       poc = pou;
     }
   }
-  task_store_f(part + task * kNR, 0, pq);
+  task_store_f(part + task, pq);
 }
 
 // ---- element-wise passes on 4-cell vectors (rows of 4k cells) --------------------------------
@@ -962,10 +962,10 @@ __device__ __forceinline__ void upd4_task(const DevArrays& A, double* part, int6
     }
   }
   if (sizeof(T) == 4 && !weighted) {
-    task_store_f(part + task * kNR, 0, (float)rr);
+    task_store_f(part + task, (float)rr);
   } else {
     const double v[2] = {(double)rr, rw};
-    tile_store<2>(part + task * kNR, v);
+    tile_store<2>(part + task, A.pcap, v);
   }
 }
 
@@ -1107,12 +1107,12 @@ __device__ __forceinline__ void res_hx4_task(const DevArrays& A, double* part, i
   }
   if (f32) rr = rq.value();
   if (sizeof(TR) == 4) {
-    task_store_f(part + task * kNR, 1, gg);
+    task_store_f(part + A.pcap + task, gg);
     const double v[1] = {rr};
-    tile_store<1>(part + task * kNR, v);
+    tile_store<1>(part + task, A.pcap, v);
   } else {
     const double v[2] = {rr, gg64};
-    tile_store<2>(part + task * kNR, v);
+    tile_store<2>(part + task, A.pcap, v);
   }
 }
 
@@ -1189,56 +1189,55 @@ __global__ void __launch_bounds__(kBlock) k_cg_upd(DevArrays A) {
 }
 
 // ---- summation of an instance's task partials ------------------------------------------------
-// The order depends only on the instance's task count, so every path (finalize kernels, the
-// persistent solve's barrier epilogue) and every batch composition obtains the same bits: above
-// kWarpSumMax tasks the whole block sums (thread-strided, then block_sum), otherwise warp 0 sums
-// (lane-strided, then a shuffle tree).  The result is valid in thread 0.  Partials are read
-// through L2 (written by other blocks of the same persistent launch).
-// acc += the partials of tasks first, first + step, ... (< ntask) of an instance, in that order.
-// The loads of kSumBatch tasks are issued before their adds (the same adds in the same order, so
-// the same bits): a grid barrier's epilogue waits on this sum, and one L2 round trip per task
-// made it several microseconds per round.
-constexpr int kSumBatch = 8;
+// One order for every path (finalize kernels, both persistent solves) and every batch composition:
+// thread c adds the partials of tasks c, c + kBlock, ... in turn, the eight threads of a lane are
+// added as tree8, the lanes as a shuffle tree.  The result is valid in thread 0.  Partials are read
+// through L2 (written by other blocks of the same persistent launch); the loads of a pass are
+// issued together, because a round of the persistent solve waits for this sum.
+constexpr int kSumBatch = 4;
 template <int NRV>
-__device__ __forceinline__ void strided_sum(const double* part, int64_t task0, int64_t ntask,
-                                            int64_t first, int step, double (&acc)[NRV]) {
-  for (int64_t t0 = first; t0 < ntask; t0 += (int64_t)kSumBatch * step) {
+__device__ __forceinline__ void strided_sum(const double* part, int64_t stride, int64_t task0,
+                                            int64_t ntask, int64_t first, double (&acc)[NRV]) {
+  for (int64_t t0 = first; t0 < ntask; t0 += (int64_t)kSumBatch * kBlock) {
     double v[kSumBatch][NRV];
 #pragma unroll
     for (int u = 0; u < kSumBatch; ++u) {
-      const int64_t t = t0 + (int64_t)u * step;
+      const int64_t t = t0 + (int64_t)u * kBlock;
 #pragma unroll
-      for (int k = 0; k < NRV; ++k) v[u][k] = t < ntask ? __ldcg(&part[(task0 + t) * kNR + k]) : 0.0;
+      for (int k = 0; k < NRV; ++k) v[u][k] = t < ntask ? __ldcg(&part[k * stride + task0 + t]) : 0.0;
     }
 #pragma unroll
     for (int u = 0; u < kSumBatch; ++u) {
-      if (t0 + (int64_t)u * step >= ntask) break;
+      if (t0 + (int64_t)u * kBlock >= ntask) break;
 #pragma unroll
       for (int k = 0; k < NRV; ++k) acc[k] += v[u][k];
     }
   }
 }
 
+// Block-uniform call (all threads of the block); red: NRV * kBlock values of shared memory.
 template <int NRV>
-__device__ __forceinline__ void warp_instance_sum(const double* part, const InstDesc& d, int lane,
-                                                  double (&acc)[NRV]) {
+__device__ __forceinline__ void instance_sum(const double* part, int64_t stride, const InstDesc& d,
+                                             double (&acc)[NRV], double* red) {
 #pragma unroll
   for (int k = 0; k < NRV; ++k) acc[k] = 0.0;
-  strided_sum<NRV>(part, d.task0, d.ntask, lane, 32, acc);
+  strided_sum<NRV>(part, stride, d.task0, d.ntask, threadIdx.x, acc);
 #pragma unroll
-  for (int k = 0; k < NRV; ++k) acc[k] = warp_sum(acc[k]);
-}
-// Block-uniform call (all threads of the block).
-template <int NRV>
-__device__ __forceinline__ void instance_sum(const double* part, const InstDesc& d,
-                                             double (&acc)[NRV], double* red) {
-  if (d.ntask > kWarpSumMax) {
+  for (int k = 0; k < NRV; ++k) red[k * kBlock + threadIdx.x] = acc[k];
+  __syncthreads();
+  if (threadIdx.x < 32) {
 #pragma unroll
-    for (int k = 0; k < NRV; ++k) acc[k] = 0.0;
-    strided_sum<NRV>(part, d.task0, d.ntask, threadIdx.x, (int)blockDim.x, acc);
-    block_sum<NRV>(acc, red);
-  } else if (threadIdx.x < 32) {
-    warp_instance_sum<NRV>(part, d, (int)threadIdx.x, acc);
+    for (int k = 0; k < NRV; ++k) {
+      double u[8];
+#pragma unroll
+      for (int w = 0; w < 8; ++w) u[w] = red[k * kBlock + threadIdx.x + 32 * w];
+      acc[k] = tree8(u);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+      for (int k = 0; k < NRV; ++k) acc[k] += __shfl_xor_sync(kFull, acc[k], o);
+    }
   }
 }
 
@@ -1411,7 +1410,7 @@ __device__ __forceinline__ bool took_part(const InstScal& s) {
 }
 
 template <int KIND, bool FP32>
-__global__ void __launch_bounds__(256) k_finalize(DevArrays A, CtrlState* ctrl,
+__global__ void __launch_bounds__(kBlock) k_finalize(DevArrays A, CtrlState* ctrl,
                                                   cudaGraphConditionalHandle hw, int graph) {
   constexpr int NR = (KIND == FIN_RHS_DIAG) ? 5 : (KIND == FIN_SPMV ? 1 : 2);
   const int inst = blockIdx.x;
@@ -1419,8 +1418,8 @@ __global__ void __launch_bounds__(256) k_finalize(DevArrays A, CtrlState* ctrl,
   const InstDesc& d = A.inst[inst];
   if (took_part<KIND>(A.scal[inst])) {
     double acc[NR];
-    __shared__ double red[32 * NR];
-    instance_sum<NR>(A.partials, d, acc, red);
+    __shared__ double red[kBlock * NR];
+    instance_sum<NR>(A.partials, A.pcap, d, acc, red);
     if (threadIdx.x == 0) {
       switch (KIND) {
         case FIN_RHS: epi_rhs(A, inst, acc); break;
@@ -1504,29 +1503,34 @@ __global__ void k_ctrl_select(DevArrays A, CtrlState* ctrl, cudaGraphConditional
 }
 
 // ---- persistent solve ------------------------------------------------------------------------
-// One cooperative launch runs a step's whole refinement loop.  Work proceeds in grid-wide rounds:
-// in round r every task does the work of its instance's current phase (PH_*), writing its partial
-// sums to its fixed slot; then every block arrives at a grid barrier.  The last block to arrive
-// runs the epilogue of every instance -- it sums each instance's task partials in the fixed order
-// of instance_sum (the order the finalize kernels use, so every path obtains the same bits) and
-// updates the instance's scalars (alpha, beta, convergence test, next phase) in device memory --
-// and only then opens the barrier.  Blocks read the scalars of the instances they work on through
-// L2 at the start of each round.  Tasks are handed out one at a time from a per-round counter
-// (SolveCtl::next_task), so blocks on busier SMs take fewer of them.  The kernel returns when the
-// last epilogue reports that no instance has work left.
+// One cooperative launch runs a step's whole refinement loop.  An instance goes through phases
+// (PH_*); in a phase every one of its tasks does the phase's work, writing its partial sums to its
+// fixed slot; then an epilogue sums the partials in the fixed order of instance_sum (the order the
+// finalize kernels use, so every path obtains the same bits) and updates the instance's scalars
+// (alpha, beta, convergence test, next phase).  One grid runs its phases in grid-wide rounds
+// (k_solve_one); the grids of a batch each at their own pace (k_solve_batch).
 //
-// Termination: every barrier wait is bounded in time (wait_ns, 4 s by default) and in polls; a block that
+// Termination: every wait is bounded in time (wait_ns, 4 s by default) and in polls; a block that
 // gives up records SolveCtl::err and returns, and the blocks still waiting see the flag and return
-// too.  The number of rounds is bounded by `limit`.  Co-residency of all blocks, which the barrier
-// needs, is guaranteed by the cooperative launch (the grid never exceeds the occupancy bound).
+// too.  The number of phases is bounded by `limit`.  Co-residency of all blocks, which the grid-wide
+// barrier needs, is guaranteed by the cooperative launch (the grid never exceeds the occupancy
+// bound).
 
-__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
-  unsigned v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+__device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return v;
 }
-__device__ __forceinline__ void st_release_u32(unsigned* p, unsigned v) {
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+__device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_release_u64(unsigned long long* p, unsigned long long v) {
+  asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ void red_release_add_u64(unsigned long long* p, unsigned long long v) {
+  asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
 template <typename T>
@@ -1544,22 +1548,18 @@ __device__ __forceinline__ int phase_partials(int32_t ph) {
 constexpr int kScalWords = (int)(sizeof(InstScal) / 8);
 static_assert(sizeof(InstScal) % 8 == 0 && kScalWords < kBlock, "scalar copy");
 
-// Epilogue of one instance after a round (one thread): scalars read through L2, updated, stored.
-// Returns whether the instance has work in the next round.
+// Scalar epilogue of an instance after a round: its sums update the scalars and name its next phase.
+// Out of line: inlined, its scalars took registers from the passes of the solve kernels.
 template <typename T>
-__device__ int instance_epilogue(const DevArrays& A, int64_t inst, const double (&acc)[2]) {
-  InstScal sc;
-  const unsigned long long* src = reinterpret_cast<const unsigned long long*>(A.scal + inst);
-  unsigned long long* w = reinterpret_cast<unsigned long long*>(&sc);
-  for (int k = 0; k < kScalWords; ++k) w[k] = __ldcg(src + k);
-  const InstDesc& d = A.inst[inst];
+__device__ __noinline__ void phase_epilogue(InstScal& sc, const InstDesc& d, const DevOpts& o,
+                                            const double (&acc)[2]) {
   switch (sc.phase) {
     case PH_RES_INIT:
-      epi_residual_s<true>(sc, d, A.opts, acc);
+      epi_residual_s<true>(sc, d, o, acc);
       sc.phase = phase_after<T>(sc);
       break;
     case PH_RES:
-      epi_residual_s<false>(sc, d, A.opts, acc);
+      epi_residual_s<false>(sc, d, o, acc);
       sc.phase = phase_after<T>(sc);
       break;
     case PH_CG_P: sc.phase = PH_CG_Q; break;
@@ -1569,136 +1569,12 @@ __device__ int instance_epilogue(const DevArrays& A, int64_t inst, const double 
       sc.phase = sc.inner_active ? PH_CG_B : phase_after<T>(sc);
       break;
     case PH_CG_B:
-      epi_upd_s<T>(sc, A.opts, acc);
+      epi_upd_s<T>(sc, o, acc);
       sc.phase = phase_after<T>(sc);
       break;
     case PH_XUPD: sc.phase = PH_RES; break;
     default: sc.phase = PH_IDLE; break;
   }
-  unsigned long long* dst = reinterpret_cast<unsigned long long*>(A.scal + inst);
-  for (int k = 0; k < kScalWords; ++k) dst[k] = w[k];
-  return sc.phase != PH_IDLE ? 1 : 0;
-}
-
-// Epilogues of all instances (the whole last-arriving block).  Large instances (block sums) one
-// after the other.  Small ones kBlock at a time: each warp sums the partials of its instances
-// (per instance exactly warp_instance_sum's order, as in the finalize kernels), kEpiUnroll
-// instances' loads in flight at once, into shared memory; then one thread per instance runs the
-// epilogues side by side (with many instances, one lane running them in turn set the round's
-// length).  Returns (in every thread) whether any instance has work left.
-constexpr int kEpiUnroll = 4;
-constexpr int kPhaseCache = 1024;   // instances whose phases a solve block keeps in shared memory
-template <typename T>
-__device__ int all_epilogues(const DevArrays& A, double* red) {
-  __shared__ double s_acc[kBlock][2];
-  __shared__ int32_t s_ph[kBlock];
-  int act = 0;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int64_t k = 0; k < A.nlarge; ++k) {     // a list: no serial walk over every instance
-    const int64_t i = A.large[k];
-    const InstDesc& d = A.inst[i];
-    const int32_t ph = __ldcg(&A.scal[i].phase);
-    double acc[2] = {0.0, 0.0};
-    if (phase_partials(ph) > 0) instance_sum<2>(A.partials, d, acc, red);
-    if (threadIdx.x == 0) act |= instance_epilogue<T>(A, i, acc);
-    __syncthreads();
-  }
-  for (int64_t base = 0; A.nsmall > 0 && base < A.ninst; base += kBlock) {
-    const int nb = (int)(A.ninst - base < kBlock ? A.ninst - base : kBlock);
-    if ((int)threadIdx.x < nb) s_ph[threadIdx.x] = __ldcg(&A.scal[base + threadIdx.x].phase);
-    __syncthreads();
-    for (int j0 = warp * kEpiUnroll; j0 < nb; j0 += (kBlock / 32) * kEpiUnroll) {
-      double acc[kEpiUnroll][2];
-#pragma unroll
-      for (int u = 0; u < kEpiUnroll; ++u) {
-        acc[u][0] = 0.0;
-        acc[u][1] = 0.0;
-        const int j = j0 + u;
-        if (j >= nb) continue;
-        const InstDesc& d = A.inst[base + j];
-        if (d.ntask > kWarpSumMax || phase_partials(s_ph[j]) == 0) continue;
-        strided_sum<2>(A.partials, d.task0, d.ntask, lane, 32, acc[u]);
-      }
-#pragma unroll
-      for (int u = 0; u < kEpiUnroll; ++u) {
-        const double v0 = warp_sum(acc[u][0]), v1 = warp_sum(acc[u][1]);
-        if (lane == 0 && j0 + u < nb) {
-          s_acc[j0 + u][0] = v0;
-          s_acc[j0 + u][1] = v1;
-        }
-      }
-    }
-    __syncthreads();
-    if ((int)threadIdx.x < nb && A.inst[base + threadIdx.x].ntask <= kWarpSumMax) {
-      const double acc[2] = {s_acc[threadIdx.x][0], s_acc[threadIdx.x][1]};
-      act |= instance_epilogue<T>(A, base + threadIdx.x, acc);
-    }
-    __syncthreads();
-  }
-  return __syncthreads_or(act);
-}
-
-// Grid barrier whose last arriving block runs all epilogues before opening it.  Returns false if
-// the wait gave up; `any` = some instance has work in the next round.
-template <typename T>
-__device__ bool grid_barrier_epilogue(const DevArrays& A, SolveCtl* ctl, unsigned nblocks,
-                                      int64_t round, double* red, unsigned long long wait_ns,
-                                      unsigned& any) {
-  __shared__ unsigned s_gen, s_any;
-  __shared__ int s_last, s_ok;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const unsigned g = ld_acquire_u32(&ctl->gen);   // cannot advance before this block arrives
-    __threadfence();
-    const unsigned arrived = atomicAdd(&ctl->count, 1u);
-    s_gen = g;
-    s_last = (arrived == nblocks - 1) ? 1 : 0;
-    if (s_last) __threadfence();                   // every block's partials are visible now
-  }
-  __syncthreads();
-  const unsigned g = s_gen;
-  if (s_last) {
-    if (threadIdx.x == 0 && round < kRoundLog) {
-      int32_t ph = __ldcg(&A.scal[0].phase);
-      if (ph == PH_RES_INIT && __ldcg(&A.scal[0].hx_ok) >= 2) ph = HF_PHASE_RES_INIT_HX;
-      if (ph == PH_CG_B && (__ldcg(&A.scal[0].xw) & kXwThis)) ph = HF_PHASE_CG_BX;
-      ctl->phase_log[round] = ph;
-    }
-    const int act = all_epilogues<T>(A, red);
-    if (threadIdx.x == 0) {
-      ctl->next_task[round & 1] = 0u;     // every block is done taking this round's tasks
-      ctl->result[(g + 1) & 1] = act ? 1u : 0u;
-      const unsigned long long t = gtimer();
-      if (round < kRoundLog) ctl->t_round[round] = t;
-      A.stamps[kStampSolveEnd] = t;
-      ctl->rounds = round + 1;
-      ctl->count = 0u;
-      __threadfence();
-      st_release_u32(&ctl->gen, g + 1);
-      s_ok = 1;
-    }
-  } else if (threadIdx.x == 0) {
-    int ok = 1;
-    const unsigned long long t0 = gtimer();
-    unsigned polls = 0;
-    while (ld_acquire_u32(&ctl->gen) == g) {
-      if (*(volatile int*)&ctl->err) { ok = 0; break; }
-      if ((++polls & 255u) == 0u && (gtimer() - t0 > wait_ns || polls > (1u << 27))) {
-        atomicExch(&ctl->err, 1);
-        ok = 0;
-        break;
-      }
-      __nanosleep(32);
-    }
-    s_ok = ok;
-  }
-  if (threadIdx.x == 0) {
-    __threadfence();
-    s_any = s_ok ? *(volatile unsigned*)&ctl->result[(g + 1) & 1] : 0u;
-  }
-  __syncthreads();
-  any = s_any;
-  return s_ok != 0;
 }
 
 template <typename T, bool XOUT>
@@ -1724,70 +1600,269 @@ __device__ __forceinline__ void round_task(const DevArrays& A, double* part, int
   }
 }
 
+// The phase as the round log names it.
+__device__ __forceinline__ int32_t logged_phase(const InstScal& s) {
+  if (s.phase == PH_RES_INIT && s.hx_ok >= 2) return HF_PHASE_RES_INIT_HX;
+  if (s.phase == PH_CG_B && (s.xw & kXwThis)) return HF_PHASE_CG_BX;
+  return s.phase;
+}
+
+// ---- persistent solve of several grids ---------------------------------------------------------
+// Tasks come from one queue of tickets (SolveCtl::ticket).  A phase of an instance is a range of
+// tickets, published in the instance's slot; the first ntasks tickets are all instances' first
+// phase, in task-table order.  A block takes a ticket, finds the instance whose published range
+// holds it (its threads look at all slots at once), does that task and counts it in the instance's
+// done counter.  The block that finishes an instance's last task of a phase runs its epilogue and
+// publishes its next phase at the end of the queue.  So no instance waits for another: with a
+// grid-wide barrier after every phase, each round lasted as long as its slowest instance and the
+// epilogues of all instances ran in one block while the others waited (64 grids of 16..96 cells an
+// edge: 88 us a round for about 40 us of traffic; 20 steps 125 -> 88 ms).
+// Tickets are handed out in order and a phase is published only after its predecessor's tickets
+// were all done, so every published ticket is held by a block that is running it or will be handed
+// out next: a block that waits for its ticket's range to be published never holds up the others.
+// An instance's old range stays in its slot until the next replaces it; only blocks that hold one
+// of its tickets match it.
 // Blocks per SM: 3 (85 registers: the FP64 stencil and the FP32 vector pass need about that).
 // XOUT: the instance used by the graphs of host-buffer steps, whose residual sweeps also store x
 // into A.xout (a variant of its own, so the other solves carry none of it).
+constexpr int kSlotShift = 24;      // slot: first ticket << 24 | tasks << 1 | walk the tasks backwards
 template <typename T, bool XOUT>
 __global__ void __launch_bounds__(kBlock, 3)
-    k_solve(DevArrays A, SolveCtl* ctl, int64_t limit, unsigned long long wait_ns, int leaver) {
+    k_solve_batch(DevArrays A, SolveCtl* ctl, int64_t limit, unsigned long long wait_ns, int leaver) {
   __shared__ InstScal sh;
-  __shared__ double red[32 * 2];
-  __shared__ int32_t s_phase[kPhaseCache];
+  __shared__ double red[kBlock * 2];
+  __shared__ unsigned long long s_ticket, s_slot;
+  __shared__ int s_inst, s_last, s_stop;
+  const int ninst = (int)A.ninst;
+  const unsigned long long first = (unsigned long long)A.ntasks;
+  unsigned long long* slots = solve_slots(ctl);
+  unsigned* done = solve_done(ctl, A.ninst);
+  if (blockIdx.x == 0 && threadIdx.x == 0) A.stamps[kStampSolve] = ctl->t_start = gtimer();
+  if (threadIdx.x == 0) s_ticket = atomicAdd(&ctl->ticket, 1ull);
+  // failure-path check only (leaver >= 0): that block leaves with a ticket, so its instance never
+  // finishes and the others' waits run out and record SolveCtl::err
+  if ((int)blockIdx.x == leaver) return;
+  for (;;) {
+    __syncthreads();
+    const unsigned long long t = s_ticket;
+    int inst = -1;
+    unsigned n = 0, local = 0;
+    bool back = false;
+    if (t < first) {
+      inst = A.tasks[t].x;
+      local = (unsigned)(t - (unsigned long long)A.inst[inst].task0);
+      n = (unsigned)A.inst[inst].ntask;
+      __syncthreads();                       // every thread has read s_ticket
+    } else {
+      unsigned long long t0 = 0;
+      for (unsigned polls = 0;; ++polls) {
+        bool hit = false;
+        for (int i = threadIdx.x; i < ninst; i += kBlock) {
+          const unsigned long long v = ld_relaxed_u64(slots + i);
+          const unsigned long long s0 = v >> kSlotShift;
+          if (t >= s0 && t - s0 < ((v >> 1) & ((1ull << (kSlotShift - 1)) - 1ull))) {
+            hit = true;
+            s_inst = i;
+            s_slot = v;
+          }
+        }
+        if (hit) __threadfence();            // what the epilogue before this phase wrote is visible
+        if (__syncthreads_or(hit)) break;
+        if (threadIdx.x == 0) {
+          int stop = *(volatile unsigned*)&ctl->finished >= (unsigned)ninst || *(volatile int*)&ctl->err ||
+                     *(volatile int*)&ctl->guard_hit;
+          if (!stop && (polls & 63u) == 0u) {
+            const unsigned long long now = gtimer();
+            if (t0 == 0) t0 = now;
+            if (now - t0 > wait_ns || polls > (1u << 26)) {
+              atomicExch(&ctl->err, 1);
+              stop = 1;
+            }
+          }
+          s_stop = stop;
+          if (!stop) __nanosleep(64);
+        }
+        __syncthreads();
+        if (s_stop) return;
+      }
+      inst = s_inst;
+      const unsigned long long v = s_slot;
+      n = (unsigned)((v >> 1) & ((1ull << (kSlotShift - 1)) - 1ull));
+      local = (unsigned)(t - (v >> kSlotShift));
+      back = v & 1ull;
+    }
+    const InstDesc& d = A.inst[inst];
+    if ((int)threadIdx.x < kScalWords)       // this instance's scalars, through L2
+      reinterpret_cast<unsigned long long*>(&sh)[threadIdx.x] =
+          __ldcg(reinterpret_cast<const unsigned long long*>(A.scal + inst) + threadIdx.x);
+    if (threadIdx.x == kBlock - 1) s_ticket = atomicAdd(&ctl->ticket, 1ull);   // the block's next one
+    __syncthreads();
+    const int32_t ph = sh.phase;             // read before any thread can run the epilogue
+    round_task<T, XOUT>(A, A.partials, d.task0 + (back ? n - 1 - local : local), sh);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      __threadfence();
+      s_last = atomicAdd(done + inst, 1u) == n - 1u;
+      if (s_last) __threadfence();           // every block's work of this phase is visible now
+    }
+    __syncthreads();
+    if (!s_last) continue;
+    double acc[2] = {0.0, 0.0};
+    if (phase_partials(ph) > 0) instance_sum<2>(A.partials, A.pcap, d, acc, red);
+    if (threadIdx.x == 0) {
+      if (inst == 0) {
+        const int64_t r = ctl->rounds;
+        if (r < kRoundLog) {
+          ctl->phase_log[r] = logged_phase(sh);
+          ctl->t_round[r] = gtimer();
+        }
+        ctl->rounds = r + 1;
+      }
+      if (ph != PH_IDLE) phase_epilogue<T>(sh, d, A.opts, acc);
+    }
+    __syncthreads();
+    if ((int)threadIdx.x < kScalWords)
+      reinterpret_cast<unsigned long long*>(A.scal + inst)[threadIdx.x] =
+          reinterpret_cast<const unsigned long long*>(&sh)[threadIdx.x];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      done[inst] = 0u;
+      __threadfence();
+      if (sh.phase == PH_IDLE) {
+        A.stamps[kStampSolveEnd] = gtimer();
+        atomicAdd(&ctl->finished, 1u);
+      } else if (atomicAdd(&ctl->phases, 1ull) >= (unsigned long long)limit * (unsigned long long)ninst) {
+        atomicExch(&ctl->guard_hit, 1);
+      } else {
+        const unsigned long long m = (unsigned long long)d.ntask;
+        const unsigned long long s0 = first + atomicAdd(&ctl->tail, m);
+        st_release_u64(slots + inst, s0 << kSlotShift | m << 1 | (back ? 0ull : 1ull));
+      }
+    }
+  }
+}
+
+// ---- persistent solve of one grid ------------------------------------------------------------
+// With one grid every block can keep its scalars itself: after each grid barrier every block sums
+// all the tasks' partials (the same adds in the same order, so all blocks obtain the same bits) and
+// runs the scalar epilogue on its own copy in shared memory.  The barrier is then one arrival and
+// one wait.  Where the last block to arrive reads the scalars, sums, runs the epilogue, writes them
+// back and opens the barrier, and every block reads them again, each round holds six dependent
+// trips through L2, which was most of a small grid's round (a CG iteration of its three rounds took
+// 29 us on 625 cells and 34 us on 64^3, 15 and 17 with the epilogue in every block).
+// Partial sums alternate between two tables by round: a block may write round r + 1's while another
+// still sums round r's, and none writes round r + 2's before all have arrived at the barrier of
+// round r + 1.
+// Tasks: one each where the blocks suffice, else handed out one at a time from a per-round counter,
+// so blocks on busier SMs take fewer of them (counter r mod 4; block 0 clears the one of round
+// r + 2, which every block has left behind and none has reached).
+// Measured: the layered slab at 64^3, mixed, 20 steps 11.7 -> 6.1 ms; a 25 x 25 x 1 grid under the
+// reference's rule, 10 steps 17.3 -> 9.1 ms; 128^3 1.17 times as fast, 256^3 1.03 times.
+template <typename T, bool XOUT>
+__global__ void __launch_bounds__(kBlock, 3)
+    k_solve_one(DevArrays A, SolveCtl* ctl, int64_t limit, unsigned long long wait_ns, int leaver) {
+  __shared__ InstScal sh;
+  __shared__ InstDesc sd;
+  __shared__ double red[kBlock * 2];
   __shared__ unsigned s_next;
+  __shared__ int s_ok;
+  static_assert(sizeof(InstDesc) % 8 == 0 && sizeof(InstDesc) / 8 <= kBlock, "descriptor copy");
   const unsigned G = gridDim.x;
   const unsigned nt = (unsigned)A.ntasks;
-  // several instances: every round starts with all their phases in shared memory, so tasks of
-  // instances without work this round are passed over without reading their scalars
-  const bool cache = A.ninst > 1 && A.ninst <= kPhaseCache;
-  const bool single = A.ninst == 1;
+  const bool hand_out = nt > G;
+  if ((int)threadIdx.x < kScalWords)
+    reinterpret_cast<unsigned long long*>(&sh)[threadIdx.x] =
+        reinterpret_cast<const unsigned long long*>(A.scal)[threadIdx.x];
+  if (threadIdx.x < sizeof(InstDesc) / 8)
+    reinterpret_cast<unsigned long long*>(&sd)[threadIdx.x] =
+        reinterpret_cast<const unsigned long long*>(A.inst)[threadIdx.x];
   if (blockIdx.x == 0 && threadIdx.x == 0) A.stamps[kStampSolve] = ctl->t_start = gtimer();
-  for (int64_t r = 0;; ++r) {
+  __syncthreads();
+  int64_t r = 0;
+  for (; sh.phase != PH_IDLE; ++r) {
     if (r >= limit) {
       if (blockIdx.x == 0 && threadIdx.x == 0) ctl->guard_hit = 1;
-      return;
+      break;
     }
     // odd rounds walk the tasks backwards, so a round starts on the data the previous round wrote
     // last, which is still in L2 (the partial sums have fixed slots: the order changes no bits)
-    int cur = single ? 0 : -1;
-    if (cache) {
-      for (int i = threadIdx.x; i < (int)A.ninst; i += kBlock) s_phase[i] = __ldcg(&A.scal[i].phase);
+    double* part = A.partials + (r & 1) * (kNR * A.pcap);
+    const int32_t ph = sh.phase;             // read before any thread can run the epilogue
+    unsigned k = blockIdx.x;
+    if (hand_out) {
+      if (threadIdx.x == 0) s_next = atomicAdd(&ctl->next_task[r & 3], 1u);
+      if (blockIdx.x == 0 && threadIdx.x == 32) ctl->next_task[(r + 2) & 3] = 0u;
+      __syncthreads();
+      k = s_next;
     }
-    // tasks are handed out one at a time from a counter, so a block on a busier SM takes fewer
-    // (every SM holds the same number of blocks, but a round lasts as long as its slowest SM);
-    // each block asks for its next task while it runs the current one.  With one instance its
-    // scalars are loaded beside the first request (threads 1..kScalWords), not after it.
-    if (threadIdx.x == 0) s_next = atomicAdd(&ctl->next_task[r & 1], 1u);
-    if (single && threadIdx.x >= 1 && (int)threadIdx.x <= kScalWords)
-      reinterpret_cast<unsigned long long*>(&sh)[threadIdx.x - 1] =
-          __ldcg(reinterpret_cast<const unsigned long long*>(A.scal) + threadIdx.x - 1);
-    __syncthreads();
-    for (unsigned k = s_next; k < nt;) {
-      __syncthreads();                       // every thread has read s_next
-      if (threadIdx.x == 0) s_next = atomicAdd(&ctl->next_task[r & 1], 1u);
-      const unsigned t = (r & 1) ? nt - 1 - k : k;
-      const int inst = A.tasks[t].x;
-      const bool skip = cache && s_phase[inst] == PH_IDLE;
-      if (!skip) {
-        if (inst != cur) {                   // this instance's scalars, through L2
-          __syncthreads();
-          if ((int)threadIdx.x < kScalWords)
-            reinterpret_cast<unsigned long long*>(&sh)[threadIdx.x] =
-                __ldcg(reinterpret_cast<const unsigned long long*>(A.scal + inst) + threadIdx.x);
-          __syncthreads();
-          cur = inst;
-        }
-        if (sh.phase != PH_IDLE) round_task<T, XOUT>(A, A.partials, t, sh);
+    while (k < nt) {
+      if (hand_out) {
+        __syncthreads();                     // every thread has read s_next
+        if (threadIdx.x == 0) s_next = atomicAdd(&ctl->next_task[r & 3], 1u);
       }
+      round_task<T, XOUT>(A, part, (r & 1) ? nt - 1 - k : k, sh);
+      if (!hand_out) break;
       __syncthreads();                       // s_next holds the block's next task
       k = s_next;
     }
-    unsigned any = 0;
     // failure-path check only (leaver >= 0): that block leaves without arriving, so the others'
     // waits run out and record SolveCtl::err
     if ((int)blockIdx.x == leaver) return;
-    if (!grid_barrier_epilogue<T>(A, ctl, G, r, red, wait_ns, any)) return;
-    if (!any) return;
+    __syncthreads();                         // the block's work is done
+    if (threadIdx.x == 0) {
+      __threadfence();
+      red_release_add_u64(&ctl->arrived, 1ull);
+      const unsigned long long want = (unsigned long long)G * (unsigned long long)(r + 1);
+      int ok = 1;
+      unsigned long long t0 = 0;
+      for (unsigned polls = 0; ld_acquire_u64(&ctl->arrived) < want; ++polls) {
+        if (polls < 64u) continue;           // a round of a small grid is a few microseconds
+        if (*(volatile int*)&ctl->err) { ok = 0; break; }
+        if ((polls & 255u) == 64u) {
+          const unsigned long long t = gtimer();
+          if (t0 == 0) t0 = t;
+          if (t - t0 > wait_ns || polls > (1u << 27)) {
+            atomicExch(&ctl->err, 1);
+            ok = 0;
+            break;
+          }
+        }
+        __nanosleep(32);
+      }
+      __threadfence();
+      s_ok = ok;
+    }
+    __syncthreads();
+    if (!s_ok) return;
+    double acc[2] = {0.0, 0.0};
+    if (phase_partials(ph) > 0) instance_sum<2>(part, A.pcap, sd, acc, red);
+    if (threadIdx.x == 0) {
+      if (blockIdx.x == 0 && r < kRoundLog) {
+        ctl->phase_log[r] = logged_phase(sh);
+        ctl->t_round[r] = gtimer();
+      }
+      phase_epilogue<T>(sh, sd, A.opts, acc);
+    }
+    __syncthreads();
   }
+  if (blockIdx.x != 0) return;
+  if ((int)threadIdx.x < kScalWords)
+    reinterpret_cast<unsigned long long*>(A.scal)[threadIdx.x] =
+        reinterpret_cast<const unsigned long long*>(&sh)[threadIdx.x];
+  if (threadIdx.x == 0) {
+    A.stamps[kStampSolveEnd] = gtimer();
+    ctl->rounds = r;
+  }
+}
+
+typedef void (*SolveKernel)(DevArrays, SolveCtl*, int64_t, unsigned long long, int);
+static SolveKernel solve_kernel(const Ctx& c, int fp32, bool xout) {
+  if (c.ninst == 1) {
+    if (fp32) return xout ? k_solve_one<float, true> : k_solve_one<float, false>;
+    return xout ? k_solve_one<double, true> : k_solve_one<double, false>;
+  }
+  if (fp32) return xout ? k_solve_batch<float, true> : k_solve_batch<float, false>;
+  return xout ? k_solve_batch<double, true> : k_solve_batch<double, false>;
 }
 
 // Largest co-resident grid of the persistent solve (cooperative launch bound), capped by tasks.
@@ -1795,12 +1870,11 @@ int solve_grid_blocks(Ctx& c, int fp32) {
   int& cached = c.solve_blocks[fp32 ? 1 : 0];
   if (cached > 0) return cached;
   int per_sm = 0, per_sm_x = 0, nsm = 0;
-  cudaError_t e = fp32 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_solve<float, false>, kBlock, 0)
-                       : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_solve<double, false>, kBlock, 0);
-  if (e != cudaSuccess) return -1;
-  e = fp32 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_x, k_solve<float, true>, kBlock, 0)
-           : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_x, k_solve<double, true>, kBlock, 0);
-  if (e != cudaSuccess) return -1;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, solve_kernel(c, fp32, false), kBlock, 0) !=
+          cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_x, solve_kernel(c, fp32, true), kBlock, 0) !=
+          cudaSuccess)
+    return -1;
   if (per_sm_x < per_sm) per_sm = per_sm_x;    // one grid size for both variants
   if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c.device) != cudaSuccess) return -1;
   // every SM holds the same number of blocks; tasks are handed out one at a time, so the blocks
@@ -1817,7 +1891,7 @@ cudaError_t launch_solve(Ctx& c, unsigned long long wait_ns, int leaver) {
   const bool fp32 = c.opts.precision == HF_PREC_MIXED;
   const int g = solve_grid_blocks(c, fp32 ? 1 : 0);
   if (g < 1) return cudaErrorInvalidConfiguration;
-  cudaError_t e = cudaMemsetAsync(c.d_sctl, 0, sizeof(SolveCtl), c.stream);
+  cudaError_t e = cudaMemsetAsync(c.d_sctl, 0, solve_ctl_bytes(c.ninst), c.stream);
   if (e != cudaSuccess) return e;
   const int64_t per = fp32 ? c.opts.inner_itmax : c.opts.itmax;
   const int64_t limit = (int64_t)(c.opts.max_refine + 3) * (3 * per + 6) + 8;
@@ -1831,12 +1905,8 @@ cudaError_t launch_solve(Ctx& c, unsigned long long wait_ns, int leaver) {
   at[0].val.cooperative = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  if (c.A.xout) {
-    if (fp32) return cudaLaunchKernelEx(&cfg, k_solve<float, true>, c.A, c.d_sctl, limit, wait_ns, leaver);
-    return cudaLaunchKernelEx(&cfg, k_solve<double, true>, c.A, c.d_sctl, limit, wait_ns, leaver);
-  }
-  if (fp32) return cudaLaunchKernelEx(&cfg, k_solve<float, false>, c.A, c.d_sctl, limit, wait_ns, leaver);
-  return cudaLaunchKernelEx(&cfg, k_solve<double, false>, c.A, c.d_sctl, limit, wait_ns, leaver);
+  return cudaLaunchKernelEx(&cfg, solve_kernel(c, fp32 ? 1 : 0, c.A.xout != nullptr), c.A, c.d_sctl, limit,
+                            wait_ns, leaver);
 }
 
 #ifdef HF_CHECKED
