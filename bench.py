@@ -52,15 +52,12 @@ BYTES_PER_CELL = {
     "residual_init_hx_mixed": 3 * 8 + 4 + 4,
     # FP64: x, diag, cx, cy, cz, S, 1/sqrt|H_II| (8 B) read; g, H x (8 B) written
     "residual_fp64": 7 * 8 + 8 + 8,
-    # direction update: r, p_old read, p written; SpMV: p, ax, ay, az read, q written
-    "cg_p_fp32": 3 * 4, "cg_spmv_fp32": 5 * 4, "cg_update_fp32": 6 * 4,
-    # fused direction update + SpMV: r, p_old, ax, ay, az read, p, q written
-    "cg_pq_fp32": 7 * 4,
-    # x read (8) + y (4) + sinv (4) read, x written (8)
-    "xupdate_mixed": 8 + 4 + 4 + 8,
-    # x, y, sinv read and x written (8 B each)
-    "xupdate_fp64": 4 * 8,
-    "cg_p_fp64": 3 * 8, "cg_spmv_fp64": 5 * 8, "cg_update_fp64": 6 * 8,
+    # CG pass: r, p_old, y, ax, ay, az read, p, y, q written; update: r, q read, r written
+    "cg_pq_fp32": 9 * 4, "cg_update_fp32": 3 * 4, "cg_pq_fp64": 9 * 8, "cg_update_fp64": 3 * 8,
+    # x read (8) + y, p (the last direction) and sinv (4 each) read, x written (8)
+    "xupdate_mixed": 8 + 4 + 4 + 4 + 8,
+    # x, y, p, sinv read and x written (8 B each)
+    "xupdate_fp64": 5 * 8,
 }
 # FP64 floating-point operations per cell (an FMA counts 2) of the FP64-pipe kernels: the mixed
 # residual does 7 FMA for S - Hx and 1 sub for H x = S - r (||r||^2 in FP32), the FP64 one also
@@ -71,8 +68,8 @@ BYTES_PER_CELL = {
 FP64_FLOPS_PER_CELL = {"residual_mixed": 15, "residual_fp64": 20, "residual_init_hx_mixed": 3,
                        "rhs": 5}
 
-# Algorithmic bytes per cell of each round of the persistent solve kernel (k_solve), by phase:
-# (bytes, bytes of the first inner iteration / of an update without a correction).  Under the
+# Algorithmic bytes per cell of each round of the solve, by phase: (bytes, bytes of the first inner
+# iteration / of an update without a correction; the second iteration's CG pass reads no y).  Under the
 # true-residual criterion the reference's +TINY on x0 is not applied (it moves only the starting
 # point), so the first residual does not read H*1.  A CG update that also forms x ("cg_bx", the
 # iteration predicted to end the inner solve) counts the CG update's bytes plus, if its x is the
@@ -80,12 +77,13 @@ FP64_FLOPS_PER_CELL = {"residual_mixed": 15, "residual_fp64": 20, "residual_init
 # on after it, the x it formed was not used and is not counted.
 PHASE_BYTES = {
     "mixed": {"res_init": (56, 56), "res_init_hx": (32, 32), "res": (64, 64), "cg_p": (12, 12),
-              "cg_q": (20, 20), "cg_pq": (28, 24), "cg_b": (24, 20), "cg_bx": (24, 20),
-              "xupd": (24, 16)},
+              "cg_q": (20, 20), "cg_pq": (36, 24), "cg_b": (12, 12), "cg_bx": (12, 12),
+              "xupd": (28, 16)},
     "fp64": {"res_init": (64, 64), "res_init_hx": (40, 40), "res": (72, 72), "cg_p": (24, 24),
-             "cg_q": (40, 40), "cg_b": (48, 40), "cg_bx": (48, 40), "xupd": (32, 16)},
+             "cg_q": (40, 40), "cg_pq": (72, 48), "cg_b": (24, 24), "cg_bx": (24, 24),
+             "xupd": (40, 16)},
 }
-XB = {"mixed": 8 + 4 + 8, "fp64": 3 * 8}
+XB = {"mixed": 8 + 4 + 4 + 4 + 8, "fp64": 5 * 8}
 
 
 def rhs_bytes(prob):
@@ -106,7 +104,7 @@ def rhs_bytes(prob):
 def round_bytes_per_cell(rounds, precision):
     """Algorithmic bytes per cell of each round of one persistent-solve launch (its round log)."""
     table = PHASE_BYTES[precision]
-    out, first_cg, first_b, have_y, bx = [], True, True, False, None
+    out, first_cg, first_b, have_y, bx, passes = [], True, True, False, None, 0
     for ph, _ in rounds:
         full, alt = table.get(ph, (0, 0))
         b = 0
@@ -117,12 +115,14 @@ def round_bytes_per_cell(rounds, precision):
             first_cg = first_b = True
             have_y = False
             bx = None
+            passes = 0
         elif ph == "cg_p":                        # iteration 0 has no direction round (p_0 = r)
             b = full
             first_cg = False
         elif ph == "cg_pq":
-            b = alt if first_cg else full
+            b = alt if first_cg else full - (4 if precision == "mixed" else 8) * (passes == 1)
             first_cg = False
+            passes += 1
         elif ph == "cg_q":
             b = full
         elif ph in ("cg_b", "cg_bx"):
@@ -148,8 +148,8 @@ def solve_bytes_per_cell(rounds, precision):
 # forms x).
 PHASE_FP64_INSTR = {
     "mixed": {"res_init_hx": 2, "res_init": 7, "res": 8, "xupd": 1, "cg_bx": 1},
-    "fp64": {"res_init_hx": 5, "res_init": 10, "res": 11, "xupd": 1, "cg_p": 1, "cg_q": 7,
-             "cg_b": 3, "cg_bx": 4},
+    "fp64": {"res_init_hx": 5, "res_init": 10, "res": 11, "xupd": 2, "cg_p": 1, "cg_q": 7,
+             "cg_pq": 9, "cg_b": 2, "cg_bx": 4},
 }
 
 
@@ -559,10 +559,9 @@ def main():
     cell_iters = N * (st["inner_iterations"] + st["iterations"] + st["refinements"])
     cell_iters_per_s = world * cell_iters / (ms / 1000.0)
 
-    # ---- kernel roofline.  The dominant kernel is the persistent solve (k_solve: the whole
-    # refinement loop of a step in one cooperative launch); it is timed alone with CUDA events on
-    # the library's stream.  Its algorithmic bytes come from the phase of every grid-wide round of
-    # the timed launches (the kernel's own round log).
+    # ---- roofline of the solve: the refinement loop of a step (residual sweeps and the persistent
+    # kernel of the inner CG), timed alone with CUDA events on the library's stream.  Its algorithmic
+    # bytes come from the phase of every grid-wide round of the timed solves (their own round log).
     peak, peak_kind = measured_peak()
     prec = "mixed"
     solve_ms = hf.time_kernel(abi.HF_KERNEL_SOLVE, reps=10)
@@ -574,7 +573,7 @@ def main():
     fp_rates = {"fp64_tflops": f64.value, "fp32_tflops": f32.value} if rc == 0 else None
     achieved = solve_bpc * N / (solve_ms / 1000.0) / 1e9
     ratio = ncu_traffic().get("solve_mixed_ratio")     # DRAM bytes per algorithmic byte (ncu)
-    roofline = {"kernel": "k_solve<float> (persistent cooperative solve, one launch per step)",
+    roofline = {"kernel": "the solve of a step: residual sweeps and k_solve_one<float> (persistent inner CG)",
                 "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "peak_kind": f"of {peak_kind}",
                 "traffic": ratio * solve_bpc * N if ratio else None,
@@ -596,8 +595,7 @@ def main():
                                         "measured FP64 rate); by_phase: [us, frac, bound]"}
     if args.detail:
         # standalone kernels (timed repeatedly on the same data, partly L2-resident)
-        kernels = {"cg_p_fp32": abi.HF_KERNEL_CG_P, "cg_spmv_fp32": abi.HF_KERNEL_CG_SPMV,
-                   "cg_pq_fp32": abi.HF_KERNEL_CG_PQ, "cg_update_fp32": abi.HF_KERNEL_CG_UPDATE,
+        kernels = {"cg_pq_fp32": abi.HF_KERNEL_CG_PQ, "cg_update_fp32": abi.HF_KERNEL_CG_UPDATE,
                    "xupdate_mixed": abi.HF_KERNEL_XUPDATE,
                    "residual_init_hx_mixed": abi.HF_KERNEL_RESIDUAL_INIT,   # before the sweep
                    "residual_mixed": abi.HF_KERNEL_RESIDUAL}                # that rewrites H x
@@ -632,9 +630,8 @@ def main():
         if args.detail:
             k64 = {"residual_fp64": h2.time_kernel(abi.HF_KERNEL_RESIDUAL, 10),
                    "xupdate_fp64": h2.time_kernel(abi.HF_KERNEL_XUPDATE, 10),
-                   "cg_spmv_fp64": h2.time_kernel(abi.HF_KERNEL_CG_SPMV, 10),
-                   "cg_update_fp64": h2.time_kernel(abi.HF_KERNEL_CG_UPDATE, 10),
-                   "cg_p_fp64": h2.time_kernel(abi.HF_KERNEL_CG_P, 10)}
+                   "cg_pq_fp64": h2.time_kernel(abi.HF_KERNEL_CG_PQ, 10),
+                   "cg_update_fp64": h2.time_kernel(abi.HF_KERNEL_CG_UPDATE, 10)}
             detail["fp64_kernels"] = kernel_table(k64, N, peak, fp_rates)
             detail["fp64_phases"] = phase_table(r64, "fp64", N)
         h2.close()

@@ -111,6 +111,10 @@ void drop_graph(Ctx& c) {
   if (c.loop_graph) cudaGraphDestroy(c.loop_graph);
   c.loop_exec = nullptr;
   c.loop_graph = nullptr;
+  if (c.solve_exec) cudaGraphExecDestroy(c.solve_exec);
+  if (c.solve_graph) cudaGraphDestroy(c.solve_graph);
+  c.solve_exec = nullptr;
+  c.solve_graph = nullptr;
   for (int j = 0; j < 2; ++j) {
     if (c.post_exec[j]) cudaGraphExecDestroy(c.post_exec[j]);
     if (c.post_graph[j]) cudaGraphDestroy(c.post_graph[j]);
@@ -257,7 +261,7 @@ int solve_loop(Ctx& c) {
     if (!any_outer) return HF_OK;
     if (any_inner) {
       for (int k = 0; k < c.opts.check_every; ++k) CU(launch_inner_iteration(c, fp32 ? 1 : 0));
-      c.launches += 5 * c.opts.check_every;
+      c.launches += 4 * c.opts.check_every;
     } else {
       CU(launch_residual(c, 1));
       c.launches += 3;
@@ -378,16 +382,96 @@ int build_graph_cond(Ctx& c) {
   return HF_OK;
 }
 
-// Capture one step with the persistent solve: step begin, RHS and its finalize, the cooperative
-// solve kernel (zeroing its control block first), step end.  Five kernels per step.
-int build_graph_persistent(Ctx& c) {
+// The solve of a captured step, on the capturing stream c.stream.  Whole: one cooperative kernel.
+// Split: the first residual, then a WHILE node around [the inner solves that are due as one
+// cooperative kernel, x update, residual], as kernels of their own (split_solve says where).
+int capture_solve(Ctx& c, std::string& err) {
+  auto chk = [&](cudaError_t e, const char* what) {
+    if (e != cudaSuccess && err.empty()) err = std::string(what) + ": " + cudaGetErrorString(e);
+    return e == cudaSuccess;
+  };
+  if (!c.split) return chk(launch_solve(c), "persistent solve") ? HF_OK : HF_ECUDA;
+  cudaStream_t cs = c.stream, cb = nullptr;
+  cudaStreamCaptureStatus st;
+  cudaGraph_t g = nullptr, tmp = nullptr;
+  const cudaGraphNode_t* deps = nullptr;
+  size_t nd = 0;
+  cudaGraphConditionalHandle hw;
+  if (!chk(cudaMemsetAsync(c.d_sctl, 0, solve_ctl_bytes(c.ninst), cs), "control block")) return HF_ECUDA;
+  if (!chk(cudaStreamGetCaptureInfo(cs, &st, nullptr, &g, &deps, nullptr, &nd), "capture info")) return HF_ECUDA;
+  if (!chk(cudaGraphConditionalHandleCreate(&hw, g, 0, cudaGraphCondAssignDefault), "handle(solve)")) return HF_ECUDA;
+  if (!chk(launch_residual(c, 0, c.d_ctrl, hw, 2), "first residual")) return HF_ECUDA;
+  if (!chk(cudaStreamGetCaptureInfo(cs, &st, nullptr, &g, &deps, nullptr, &nd), "capture info")) return HF_ECUDA;
+  cudaGraphNodeParams wp = {};
+  wp.type = cudaGraphNodeTypeConditional;
+  wp.conditional.handle = hw;
+  wp.conditional.type = cudaGraphCondTypeWhile;
+  wp.conditional.size = 1;
+  cudaGraphNode_t wnode = nullptr;
+  if (!chk(cudaGraphAddNode(&wnode, g, deps, nullptr, nd, &wp), "while(solve)")) return HF_ECUDA;
+  if (!chk(cudaStreamUpdateCaptureDependencies(cs, &wnode, nullptr, 1, cudaStreamSetCaptureDependencies), "deps"))
+    return HF_ECUDA;
+  if (!chk(cudaStreamCreateWithFlags(&cb, cudaStreamNonBlocking), "stream")) return HF_ECUDA;
+  if (chk(cudaStreamBeginCaptureToGraph(cb, wp.conditional.phGraph_out[0], nullptr, nullptr, 0,
+                                        cudaStreamCaptureModeRelaxed), "capture solve")) {
+    c.stream = cb;
+    chk(launch_solve(c, false), "inner solves");
+    chk(launch_residual(c, 1, c.d_ctrl, hw, 2), "residual");
+    chk(cudaStreamEndCapture(cb, &tmp), "end solve");
+    c.stream = cs;
+  }
+  cudaStreamDestroy(cb);
+  return err.empty() ? HF_OK : HF_ECUDA;
+}
+
+int solve_grids(Ctx& c) {
+  const int fp32 = c.opts.precision == HF_PREC_MIXED ? 1 : 0;
+  if (solve_grid_blocks(c, fp32, true) < 1 || solve_grid_blocks(c, fp32, false) < 1)
+    return set_err(HF_ECUDA, "no co-resident grid for the persistent solve kernel");
   if (!c.d_ctrl) {
     int r = dalloc(c, &c.d_ctrl, 1);
     if (r) return r;
     CU(cudaMemset(c.d_ctrl, 0, sizeof(CtrlState)));
   }
-  if (solve_grid_blocks(c, c.opts.precision == HF_PREC_MIXED ? 1 : 0) < 1)
-    return set_err(HF_ECUDA, "no co-resident grid for the persistent solve kernel");
+  return HF_OK;
+}
+
+// One solve on the context stream, outside a captured step.
+int run_solve(Ctx& c) {
+  if (int r = solve_grids(c)) return r;
+  if (!c.split) {
+    CU(launch_solve(c));
+    return HF_OK;
+  }
+  if (!c.solve_exec) {
+    cudaStream_t cs = nullptr, saved = c.stream;
+    CU(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
+    std::string err;
+    cudaGraph_t g = nullptr;
+    cudaError_t e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeRelaxed);
+    if (e == cudaSuccess) {
+      c.stream = cs;
+      capture_solve(c, err);
+      c.stream = saved;
+      e = cudaStreamEndCapture(cs, &g);
+    }
+    cudaStreamDestroy(cs);
+    if (e == cudaSuccess && err.empty()) e = cudaGraphInstantiate(&c.solve_exec, g, 0);
+    if (e != cudaSuccess || !err.empty()) {
+      if (g) cudaGraphDestroy(g);
+      cudaGetLastError();
+      return set_err(HF_ECUDA, "solve graph: " + (err.empty() ? std::string(cudaGetErrorString(e)) : err));
+    }
+    c.solve_graph = g;
+  }
+  CU(cudaGraphLaunch(c.solve_exec, c.stream));
+  return HF_OK;
+}
+
+// Capture one step with the persistent solve: step begin, RHS and its finalize, the cooperative
+// solve kernel (zeroing its control block first), step end.  Five kernels per step.
+int build_graph_persistent(Ctx& c) {
+  if (int r = solve_grids(c)) return r;
   cudaStream_t cs = nullptr;
   CU(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
   cudaStream_t saved = c.stream;
@@ -399,10 +483,10 @@ int build_graph_persistent(Ctx& c) {
   };
   if (chk(cudaStreamBeginCapture(cs, cudaStreamCaptureModeRelaxed), "capture")) {
     c.stream = cs;
-    chk(launch_graph_step_begin(c, c.d_ctrl, c.tempdep ? 9 : 5), "step begin");
+    chk(launch_graph_step_begin(c, c.d_ctrl, (c.split ? 6 : 5) + (c.tempdep ? 4 : 0)), "step begin");
     chk(launch_rhs(c), "rhs");
     chk(launch_finalize(c, FIN_RHS, nullptr, 0, 0), "rhs finalize");
-    chk(launch_solve(c), "persistent solve");
+    capture_solve(c, err);
     chk(launch_graph_step_end(c, c.d_ctrl, c.d_sctl), "step end");
     if (c.tempdep) chk(launch_tempdep(c), "properties");
     chk(cudaStreamEndCapture(cs, &g), "end capture");
@@ -430,13 +514,7 @@ int build_graph_persistent(Ctx& c) {
 int build_loop_graph(Ctx& c) {
   if (c.loop_exec) return HF_OK;
   if (c.loop_unsupported) return HF_EARG;
-  if (!c.d_ctrl) {
-    int r = dalloc(c, &c.d_ctrl, 1);
-    if (r) return r;
-    CU(cudaMemset(c.d_ctrl, 0, sizeof(CtrlState)));
-  }
-  if (solve_grid_blocks(c, c.opts.precision == HF_PREC_MIXED ? 1 : 0) < 1)
-    return set_err(HF_ECUDA, "no co-resident grid for the persistent solve kernel");
+  if (int r = solve_grids(c)) return r;
   cudaStream_t cs = nullptr;
   CU(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
   cudaStream_t saved = c.stream;
@@ -461,10 +539,10 @@ int build_loop_graph(Ctx& c) {
     if (!chk(cudaStreamBeginCaptureToGraph(cs, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed),
              "capture body")) break;
     c.stream = cs;
-    chk(launch_graph_step_begin(c, c.d_ctrl, c.tempdep ? 9 : 5), "step begin");
+    chk(launch_graph_step_begin(c, c.d_ctrl, (c.split ? 6 : 5) + (c.tempdep ? 4 : 0)), "step begin");
     chk(launch_rhs(c), "rhs");
     chk(launch_finalize(c, FIN_RHS, nullptr, 0, 0), "rhs finalize");
-    chk(launch_solve(c), "persistent solve");
+    capture_solve(c, err);
     chk(launch_graph_step_end(c, c.d_ctrl, c.d_sctl, hl, 1), "step end");
     if (c.tempdep) chk(launch_tempdep(c), "properties");
     cudaGraph_t tmp = nullptr;
@@ -510,13 +588,7 @@ int build_post_graph(Ctx& c) {
     c.post_exec[j] = nullptr;
     c.post_graph[j] = nullptr;
   }
-  if (!c.d_ctrl) {
-    int r = dalloc(c, &c.d_ctrl, 1);
-    if (r) return r;
-    CU(cudaMemset(c.d_ctrl, 0, sizeof(CtrlState)));
-  }
-  if (solve_grid_blocks(c, c.opts.precision == HF_PREC_MIXED ? 1 : 0) < 1)
-    return set_err(HF_ECUDA, "no co-resident grid for the persistent solve kernel");
+  if (int r = solve_grids(c)) return r;
   cudaStream_t cs = nullptr;
   CU(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
   cudaStream_t saved = c.stream;
@@ -532,7 +604,7 @@ int build_post_graph(Ctx& c) {
       c.stream = cs;
       c.A.xout = c.d_stage_x[j];
       chk(launch_finalize(c, FIN_RHS, nullptr, 0, 0), "rhs finalize");
-      chk(launch_solve(c), "persistent solve");
+      capture_solve(c, err);
       chk(launch_stage_fallback(c), "result fallback");
       chk(launch_graph_step_end(c, c.d_ctrl, c.d_sctl), "step end");
       if (c.tempdep) chk(launch_tempdep(c), "properties");
@@ -694,6 +766,109 @@ int effective_depth(const Ctx& c, const hf_solver_opts& o) {
   return kMinTaskDepth;
 }
 
+// Cells of the inner solve's layout.
+int64_t inner_cells(const Ctx& c) {
+  const InstDesc& d = c.h_inst.back();
+  const int64_t n4 = (int64_t)d.sx * d.ny * d.nz;
+  return d.off4 + (n4 + kTile - 1) / kTile * kTile;
+}
+
+// The tasks of the inner solve's passes.  A tile is 2^cqx 16-byte vectors (4 FP32 or 2 FP64 cells)
+// wide and kBlock / 2^cqx rows high, of the shapes the one that covers the grid's plane with the
+// fewest tiles (of equals the one of 16 vectors: its halo rows and the sectors that its row ends
+// read beside it are fewest).  Along z a tile is cut into parts, whose ends read a plane of their
+// neighbours.  One grid: as many parts as make its longest chain of planes per block, over waves of
+// kSolveBlocks blocks, shortest, the halo counted as one plane per part; a count above one wave
+// pays only where a wave could not be filled.  Several grids: parts of one length for all, such
+// that there are about kBatchWaves tasks per block -- they are handed out one at a time, and each
+// costs a few trips through L2.  Small grids get one plane per part either way, so a grid's bits
+// do not depend on the batch it is in there.
+constexpr int64_t kBatchWaves = 4;
+int cg_plan(Ctx& c) {
+  const int64_t kSolveBlocks = 2 * 152;
+  const int vec = c.opts.precision == HF_PREC_MIXED ? 4 : 2;
+  int64_t planes = 0;                 // tile planes of all grids
+  for (InstDesc& d : c.h_inst) {
+    int64_t best = 0;
+    for (int q : {4, 5, 3}) {
+      const int w = vec << q, h = kBlock >> q;
+      const int64_t nbx = (d.nx + w - 1) / w, nby = (d.ny + h - 1) / h;
+      if (best != 0 && nbx * nby >= best) continue;
+      best = nbx * nby;
+      d.cqx = q;
+      d.cgnx = (int32_t)nbx;
+      d.cgny = (int32_t)nby;
+    }
+    planes += best * d.nz;
+  }
+  int64_t total = 0;
+  for (InstDesc& d : c.h_inst) {
+    const int64_t tiles = (int64_t)d.cgnx * d.cgny;
+    int64_t parts = 1;
+    if (c.ninst == 1) {
+      int64_t best = INT64_MAX;
+      for (int64_t n = 1; n <= d.nz && (n == 1 || n * tiles <= 16 * kSolveBlocks); ++n) {
+        const int64_t waves = (n * tiles + kSolveBlocks - 1) / kSolveBlocks;
+        const int64_t cost = waves * ((d.nz + n - 1) / n + 1);
+        if (cost < best) {
+          best = cost;
+          parts = n;
+        }
+      }
+    } else {
+      const int64_t deep = std::max<int64_t>(1, std::min<int64_t>(32, planes / (kBatchWaves * kSolveBlocks)));
+      parts = (d.nz + deep - 1) / deep;
+    }
+    d.cgnz = (int32_t)parts;
+    d.cgn = (int32_t)(tiles * parts);
+    d.cg0 = total;
+    total += tiles * parts;
+  }
+  c.ncg = c.A.ncg = total;
+  c.cg_precision = c.opts.precision;
+  std::vector<int32_t> inst((size_t)total);
+  for (int64_t i = 0; i < c.ninst; ++i)
+    std::fill_n(inst.begin() + c.h_inst[i].cg0, c.h_inst[i].cgn, (int32_t)i);
+  auto regrow = [&](void* old) {
+    if (!old) return;
+    cudaFree(old);
+    c.allocs.erase(std::remove(c.allocs.begin(), c.allocs.end(), old), c.allocs.end());
+  };
+  if (total > c.ncg_cap) {
+    regrow(const_cast<int32_t*>(c.A.cg_inst));
+    c.A.cg_inst = nullptr;
+    int32_t* p = nullptr;
+    if (int r = dalloc(c, &p, (size_t)total)) return r;
+    c.A.cg_inst = p;
+    c.ncg_cap = total;
+  }
+  if (std::max(c.ntasks, total) > c.A.pcap) {   // two tables (the one-grid solve alternates)
+    regrow(c.A.partials);
+    c.A.partials = nullptr;
+    c.A.pcap = 0;
+    const int64_t cap = std::max(c.ntasks_cap, total);
+    if (int r = dalloc(c, &c.A.partials, (size_t)cap * kNR * 2)) return r;
+    c.A.pcap = cap;
+  }
+  CU(cudaMemcpyAsync(const_cast<int32_t*>(c.A.cg_inst), inst.data(), sizeof(int32_t) * inst.size(),
+                     cudaMemcpyHostToDevice, c.stream));
+  CU(cudaStreamSynchronize(c.stream));
+  return HF_OK;
+}
+
+// Whether the solve runs as several kernels (capture_solve).  The FP64 sweeps and the inner solve's
+// passes want different registers and blocks per SM, and in one kernel the passes spill: at 256^3 the
+// SpMV pass took 242 us in the whole form and 115 in the split, the residual 407 and 274.  The split
+// costs about 10 us of launches per refinement; one grid still gains by it on 625 cells (0.86
+// against 0.92 ms a step), a batch of uneven grids only once its solve is longer than that.
+constexpr int64_t kSplitCells = 1000000;
+bool split_solve(const Ctx& c) {
+  if (c.ninst == 1) return true;
+  int64_t cells = 0;
+  for (const InstDesc& d : c.h_inst) cells += d.n;
+  return cells >= kSplitCells;
+}
+
 // (Re)build the task table for a task depth: per instance, kTX x kTY column tiles x `depth`
 // planes, ordered (z, y, x); uploads the table and the instance descriptors, recomputes the
 // per-task heater flags and forgets what depended on the old table (captured graph, grid size).
@@ -714,6 +889,7 @@ int build_tasks(Ctx& c, int depth) {
   if ((int64_t)tasks.size() > c.ntasks_cap) return set_err(HF_EARG, "task depth below the minimum");
   c.ntasks = (int64_t)tasks.size();
   c.A.ntasks = c.ntasks;
+  if (int r = cg_plan(c)) return r;
   CU(cudaMemcpyAsync(const_cast<int4*>(c.A.tasks), tasks.data(), sizeof(int4) * tasks.size(),
                      cudaMemcpyHostToDevice, c.stream));
   CU(cudaMemcpyAsync(const_cast<InstDesc*>(c.A.inst), c.h_inst.data(), sizeof(InstDesc) * c.ninst,
@@ -721,7 +897,8 @@ int build_tasks(Ctx& c, int depth) {
   CU(launch_task_heat(c));
   CU(cudaStreamSynchronize(c.stream));
   c.depth = depth;
-  c.solve_blocks[0] = c.solve_blocks[1] = 0;
+  for (auto& b : c.solve_blocks) b[0] = b[1] = 0;
+  c.split = split_solve(c);
   drop_graph(c);
   return HF_OK;
 }
@@ -839,7 +1016,7 @@ int create_impl(const hf_problem* probs, int64_t count, const hf_solver_opts* op
   }
   c.ntasks = c.ntasks_cap;
   const size_t N = (size_t)c.ncells;
-  const size_t N4 = (size_t)off4;   // cells of the FP32 inner-solve layout
+  const size_t N4 = (size_t)off4;   // cells of the inner solve's layout
   // ---- device memory
   DevArrays& A = c.A;
   std::memset(&A, 0, sizeof(A));
@@ -857,19 +1034,17 @@ int create_impl(const hf_problem* probs, int64_t count, const hf_solver_opts* op
   A.task_heat = d_task_heat;
   A.tasks = d_tasks;
   A.ntasks = c.ntasks;
-  A.pcap = c.ntasks;
-  ALLOC(A.partials, (size_t)A.pcap * kNR * 2);   // two tables (the one-grid solve alternates)
   {
     char* sctl;                 // the control block and, behind it, the instances' queue entries
     ALLOC(sctl, solve_ctl_bytes(count));
-    c.d_sctl = reinterpret_cast<SolveCtl*>(sctl);
+    c.d_sctl = A.sctl = reinterpret_cast<SolveCtl*>(sctl);
   }
   ALLOC(A.counters, (size_t)count);
   ALLOC(c.d_bc, (size_t)count);
   A.inst = d_inst; A.scal = d_scal; A.tile_inst = d_tile_inst;
   ALLOC(A.diag, N); ALLOC(A.cx, N); ALLOC(A.cy, N); ALLOC(A.cz, N); ALLOC(A.sinv, N);
   ALLOC(A.rsum, N); ALLOC(A.sinv32, N);
-  ALLOC(A.a64x, N); ALLOC(A.a64y, N); ALLOC(A.a64z, N);
+  ALLOC(A.a64x, N4); ALLOC(A.a64y, N4); ALLOC(A.a64z, N4);
   ALLOC(A.a32x, N4); ALLOC(A.a32y, N4); ALLOC(A.a32z, N4);
   ALLOC(A.rhoc, N); ALLOC(A.ccat, N); ALLOC(A.bvec, N); ALLOC(A.tau_s, N); ALLOC(A.scoef, N);
   ALLOC(c.asm_.kappa, N);
@@ -880,7 +1055,7 @@ int create_impl(const hf_problem* probs, int64_t count, const hf_solver_opts* op
   ALLOC(A.hx[0], N); ALLOC(A.hx[1], N);
   ALLOC(A.stamps, (size_t)kStamps);
   ALLOC(A.check, (size_t)4);
-  ALLOC(A.b, N); ALLOC(A.y, N); ALLOC(A.r, N); ALLOC(A.p, N); ALLOC(A.q, N); ALLOC(A.p2, N);
+  ALLOC(A.b, N); ALLOC(A.y, N4); ALLOC(A.r, N4); ALLOC(A.p, N4); ALLOC(A.q, N4); ALLOC(A.p2, N4);
   ALLOC(A.y32, N4); ALLOC(A.r32, N4); ALLOC(A.p32, N4); ALLOC(A.q32, N4); ALLOC(A.p232, N4);
   double *d_rho, *d_hc, *d_tau, *d_em = nullptr;
   ALLOC(d_rho, N); ALLOC(d_hc, N); ALLOC(d_tau, N);
@@ -898,11 +1073,14 @@ int create_impl(const hf_problem* probs, int64_t count, const hf_solver_opts* op
   CK(cudaMemsetAsync(A.check, 0, sizeof(unsigned long long) * 4, c.stream));
   for (void* p : {(void*)A.diag, (void*)A.cx, (void*)A.cy, (void*)A.cz, (void*)c.asm_.kappa,
                   (void*)d_rho, (void*)d_hc, (void*)d_tau, (void*)A.rhoc, (void*)A.ccat, (void*)A.scoef,
-                  (void*)A.bvec, (void*)A.tau_s, (void*)A.a64x, (void*)A.a64y, (void*)A.a64z,
-                  (void*)A.b, (void*)A.y, (void*)A.r, (void*)A.p, (void*)A.q, (void*)A.rsum,
-                  (void*)A.p2, (void*)A.hx[0], (void*)A.hx[1]})
+                  (void*)A.bvec, (void*)A.tau_s, (void*)A.b, (void*)A.rsum, (void*)A.hx[0],
+                  (void*)A.hx[1]})
     CK(cudaMemsetAsync(p, 0, N * sizeof(double), c.stream));
-  // the padding cells of the FP32 layout stay zero: no kernel writes them anything else
+  // the padding cells of the inner solve's layout stay zero: no kernel of a step writes them
+  // anything else
+  for (void* p : {(void*)A.a64x, (void*)A.a64y, (void*)A.a64z, (void*)A.y, (void*)A.r, (void*)A.p,
+                  (void*)A.q, (void*)A.p2})
+    CK(cudaMemsetAsync(p, 0, N4 * sizeof(double), c.stream));
   for (void* p : {(void*)A.a32x, (void*)A.a32y, (void*)A.a32z, (void*)A.y32, (void*)A.r32,
                   (void*)A.p32, (void*)A.q32, (void*)A.p232})
     CK(cudaMemsetAsync(p, 0, N4 * sizeof(float), c.stream));
@@ -1024,7 +1202,8 @@ int hf_set_opts(hf_ctx* h, const hf_solver_opts* opts) {
   h->c.opts = *opts;
   h->c.A.opts = dev_opts(*opts);
   drop_graph(h->c);   // captured kernels hold the options by value
-  if (effective_depth(h->c, *opts) != h->c.depth) return build_tasks(h->c, effective_depth(h->c, *opts));
+  if (effective_depth(h->c, *opts) != h->c.depth || opts->precision != h->c.cg_precision)
+    return build_tasks(h->c, effective_depth(h->c, *opts));
   return HF_OK;
 }
 
@@ -1240,7 +1419,7 @@ int hf_step_host_async(hf_ctx* h, int64_t itime, const double* tp, const double*
   if (early) {
     // begin the step from the device's copy of the inputs; the whole RHS as one launch
     CU(launch_ctrl_init(c, itime, 2 * (int64_t)(c.opts.max_refine + 3) * (per + 3)));
-    CU(launch_graph_step_begin(c, c.d_ctrl, 1 + 5 + (c.tempdep ? 4 : 0)));
+    CU(launch_graph_step_begin(c, c.d_ctrl, 1 + (c.split ? 6 : 5) + (c.tempdep ? 4 : 0)));
     CU(launch_rhs(c));
     c.async_host_kernels += 1;                    // control reset
   } else {
@@ -1251,7 +1430,7 @@ int hf_step_host_async(hf_ctx* h, int64_t itime, const double* tp, const double*
     CU(launch_ctrl_init(c, itime, 2 * (int64_t)(c.opts.max_refine + 3) * (per + 3)));
     // kernels of the step outside the host copies: begin, RHS per chunk, finalize, solve, result
     // fallback, end
-    CU(launch_graph_step_begin(c, c.d_ctrl, nch + 5 + (c.tempdep ? 4 : 0)));
+    CU(launch_graph_step_begin(c, c.d_ctrl, nch + (c.split ? 6 : 5) + (c.tempdep ? 4 : 0)));
     for (int k = 0; k < nch; ++k) {
       CU(cudaStreamWaitEvent(c.stream, st.in_chunk[k], 0));
       CU(launch_host_in_range(c, st.p, 0, ch[k].glo, ch[k].ghi, c.stream));
@@ -1662,7 +1841,7 @@ int time_solve(Ctx& c, int reps, double* ms) {
     CU(launch_rhs(c));
     CU(launch_finalize(c, FIN_RHS, nullptr, 0, 0));
     CU(cudaEventRecord(e0, c.stream));
-    CU(launch_solve(c));
+    if ((rc = run_solve(c))) return rc;
     CU(cudaEventRecord(e1, c.stream));
     CU(cudaEventSynchronize(e1));
     float t = 0.f;
@@ -1704,7 +1883,9 @@ int hf_check_barrier_timeout(hf_ctx* h, int32_t wait_ms, int32_t* status, double
   CU(cudaEventCreate(&e0));
   CU(cudaEventCreate(&e1));
   CU(cudaEventRecord(e0, c.stream));
-  CU(launch_solve(c, (unsigned long long)wait_ms * 1000000ull, 0));
+  CU(cudaMemsetAsync(c.d_sctl, 0, solve_ctl_bytes(c.ninst), c.stream));
+  if (c.split) CU(launch_residual(c, 0));
+  CU(launch_solve(c, !c.split, (unsigned long long)wait_ms * 1000000ull, 0));
   CU(cudaEventRecord(e1, c.stream));
   CU(cudaEventSynchronize(e1));
   float ms = 0.f;
@@ -1792,8 +1973,8 @@ int hf_time_kernel(hf_ctx* h, int which, int reps, double* ms) {
     const bool cg = (which >= HF_KERNEL_CG_P && which <= HF_KERNEL_CG_UPDATE) || which == HF_KERNEL_CG_PQ;
     s.inner_active = cg ? 1 : 0;
     s.refine = which == HF_KERNEL_RESIDUAL_INIT ? 0 : 1;
-    s.iter = (which == HF_KERNEL_CG_P || which == HF_KERNEL_CG_UPDATE || which == HF_KERNEL_CG_PQ ||
-              which == HF_KERNEL_RESIDUAL) ? 1 : 0;
+    s.iter = cg || which == HF_KERNEL_XUPDATE ? 2 : (which == HF_KERNEL_RESIDUAL ? 1 : 0);
+    s.ypend = which == HF_KERNEL_XUPDATE ? 1 : 0;   // the solve ended on a CG update
     s.status = 0;
     s.rho = 1.0; s.gg0 = 1.0; s.beta = 0.5; s.alpha = 0.5; s.eta = 0.0;
     s.sigma = 1.0; s.sigma_prev = 1.0;
@@ -1845,6 +2026,8 @@ int hf_apply_operator(hf_ctx* h, const double* x, double* y) {
   if ((rc = upload_padded(c, c.A.p, x))) return rc;   // p and q are free outside a step
   CU(launch_apply(c, c.A.p, c.A.q));
   if ((rc = download_padded(c, y, c.A.q))) return rc;
+  const size_t n4 = (size_t)inner_cells(c);
+  for (double* p : {c.A.p, c.A.q}) CU(cudaMemsetAsync(p, 0, n4 * sizeof(double), c.stream));
   CU(cudaStreamSynchronize(c.stream));
   return HF_OK;
 }
@@ -1854,7 +2037,8 @@ int hf_get_rhs(hf_ctx* h, int64_t itime, double* B, double* Q, double* Qd, doubl
   if (!h) return set_err(HF_EARG, "null context");
   Ctx& c = h->c;
   if (!c.state_set) return set_err(HF_ESTATE, "hf_set_state must be called first");
-  // scratch: the FP64 CG vectors are free outside a step
+  // scratch: the FP64 CG vectors are free outside a step (they start a solve as zeros in their
+  // padding cells, so they are cleared afterwards)
   CU(launch_step_begin(c, itime, 0));
   CU(launch_rhs_parts(c, c.A.y, c.A.r, c.A.p, c.A.q));
   CU(launch_finalize(c, FIN_RHS, nullptr, 0, 0));
@@ -1873,6 +2057,8 @@ int hf_get_rhs(hf_ctx* h, int64_t itime, double* B, double* Q, double* Qd, doubl
     if (x0) CU(cudaMemcpyAsync(x0 + pos, c.A.tbuf[s.role[2]] + d.off, 8 * d.n, cudaMemcpyDeviceToHost, c.stream));
     pos += d.n;
   }
+  const size_t n4 = (size_t)inner_cells(c);
+  for (double* p : {c.A.y, c.A.r, c.A.p, c.A.q}) CU(cudaMemsetAsync(p, 0, n4 * sizeof(double), c.stream));
   CU(cudaStreamSynchronize(c.stream));
   if (x0) {
     pos = 0;
@@ -1895,9 +2081,7 @@ namespace {
 // (use_graph = 1) or the host-polled kernels.
 int device_solve(Ctx& c) {
   if (c.opts.use_graph == 1 || c.opts.use_graph == 3) {
-    if (solve_grid_blocks(c, c.opts.precision == HF_PREC_MIXED ? 1 : 0) < 1)
-      return set_err(HF_ECUDA, "no co-resident grid for the persistent solve kernel");
-    CU(launch_solve(c));
+    if (int r = run_solve(c)) return r;
     SolveCtl sc;
     CU(cudaMemcpyAsync(&sc, c.d_sctl, sizeof(sc), cudaMemcpyDeviceToHost, c.stream));
     CU(cudaStreamSynchronize(c.stream));
@@ -1939,6 +2123,7 @@ int hf_solve(hf_ctx* h, const double* b, double* x, hf_stats* stats) {
   s.sigma = (c.opts.precision == HF_PREC_MIXED && rms > 0.0 && std::isfinite(rms))
                 ? std::exp2(std::rint(std::log2(rms))) : 1.0;
   s.xw = 0;
+  s.ypend = 0;
   s.phase = PH_RES_INIT;
   if ((rc = push_scal(c))) return rc;
   if ((rc = device_solve(c))) return rc;
@@ -1996,6 +2181,7 @@ int hf_solve_device(hf_ctx* h, const double* b, double* x, hf_stats* stats) {
   s.tiny_pending = 0;
   s.status = 0;
   s.xw = 0;
+  s.ypend = 0;
   s.phase = PH_RES_INIT;
   if ((rc = push_scal(c))) return rc;
   CU(cudaMemcpyAsync(c.A.b + d.off, b, 8 * d.n, cudaMemcpyDeviceToDevice, c.stream));

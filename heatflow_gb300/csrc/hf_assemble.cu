@@ -222,7 +222,8 @@ __global__ void k_assemble(DevArrays A, const InstBC* bcs, const double* kappa) 
 // Interior face P|Q (Q the + neighbour): calculate_conductivity(P->Q) (kin = kappa_P) is both the
 // stored slot of P (hmatrixfunc(Q,P)) and the - face term of Q's diagonal; (Q->P) is P's + face
 // term.  The products (L+L)*kin*kout round differently in the two orders, so both are evaluated.
-// Pass 1 writes P->Q per axis into the a64 arrays (k_scale rewrites them afterwards); on the last
+// Pass 1 writes P->Q per axis into the a64 arrays, by cell (k_scale rewrites them afterwards, in the
+// inner solve's layout); on the last
 // cell of a periodic axis it writes last->first, the - face term of the first cell.  Pass 2 forms
 // the + face terms, the diagonal in hmatrixfunc's summation order, the wrap slots (the + face term
 // of the last cell), the boundary vector and 1/sqrt|H_II|.  k_assemble instead evaluates
@@ -351,9 +352,11 @@ __global__ void k_scale(DevArrays A) {
   double ax = -A.cx[g] * si * A.sinv[ex];
   double ay = -A.cy[g] * si * A.sinv[ey];
   double az = -A.cz[g] * si * A.sinv[ez];
-  A.a64x[g] = ax; A.a64y[g] = ay; A.a64z[g] = az;
-  const int64_t g4 = d.off4 + (z * ny + y) * d.sx + x;   // the FP32 layout (rows of sx cells)
+  const int64_t g4 = d.off4 + (z * ny + y) * d.sx + x;   // the inner solve's layout (rows of sx cells)
+  A.a64x[g4] = ax; A.a64y[g4] = ay; A.a64z[g4] = az;
   A.a32x[g4] = (float)ax; A.a32y[g4] = (float)ay; A.a32z[g4] = (float)az;
+  if (x == nx - 1)                       // padding cells: a rebuild used them as scratch
+    for (int64_t k = 1; k < d.sx - x; ++k) A.a64x[g4 + k] = A.a64y[g4 + k] = A.a64z[g4 + k] = 0.0;
   // H*1: the diagonal plus every face of the row
   double rs = A.diag[g];
   if (nx > 1 && (x + 1 < nx || d.px)) rs += A.cx[g];

@@ -27,6 +27,9 @@ struct Ctx {
   int64_t ntasks = 0;            // blocks of the step kernels
   int64_t ntasks_cap = 0;        // task buffers' capacity (shallowest task depth)
   int depth = 0;                 // task depth of the current table
+  int64_t ncg = 0;               // tasks of the inner solve's passes, planned for a precision
+  int cg_precision = -1;
+  int64_t ncg_cap = 0;           // entries of cg_inst
   std::vector<InstDesc> h_inst;
   std::vector<InstBC> h_bc;
   std::vector<int64_t> h_tile0;
@@ -43,7 +46,10 @@ struct Ctx {
   cudaGraph_t graph = nullptr;
   CtrlState* d_ctrl = nullptr;
   SolveCtl* d_sctl = nullptr;    // control block of the persistent solve kernel
-  int solve_blocks[2] = {0, 0};  // co-resident grid of the persistent solve (FP64, FP32)
+  int solve_blocks[2][2] = {{0, 0}, {0, 0}};  // its co-resident grid: [full][FP64, FP32]
+  bool split = false;            // the solve as several kernels (split_solve)
+  cudaGraphExec_t solve_exec = nullptr;   // the split solve on its own (hf_solve, timing)
+  cudaGraph_t solve_graph = nullptr;
   int graph_mode = 0;            // use_graph value the graph was captured for
   // use_graph = 1: the whole time loop as one graph (WHILE node around one step)
   cudaGraphExec_t loop_exec = nullptr;

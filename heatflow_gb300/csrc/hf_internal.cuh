@@ -61,12 +61,16 @@ struct InstDesc {
   int32_t ntask;      // tasks of this instance
   int32_t zc;         // planes per task (the task depth)
   int64_t hoff;       // first cell in the compact host layout (instances back to back, no padding)
-  // The FP32 vectors of the inner solve (a32x/y/z, y32, r32, p32, p232, q32) use their own layout:
-  // rows of sx = nx rounded up to 4 cells (the padding cells hold zeros), so every grid takes the
-  // 16-byte vector passes; instance at off4, a multiple of kTile cells.  sx = nx: the FP64 layout.
+  // The vectors of the inner solve (a32x/y/z, y32, r32, p32, p232, q32 and their FP64 twins) use
+  // their own layout: rows of sx = nx rounded up to 4 cells (the padding cells hold zeros), so every
+  // grid takes 16-byte vector passes; instance at off4, a multiple of kTile cells.  sx = nx: the
+  // layout of the other FP64 arrays.
   int64_t off4;
   int32_t sx;
-  int32_t pad4;
+  // Tasks of the inner solve's passes (cg_plan): tiles of 2^cqx 16-byte vectors x kBlock / 2^cqx rows,
+  // cgnx x cgny of them, each cut into cgnz parts along z; cgn in all, the first at cg0.
+  int32_t cqx, cgnx, cgny, cgnz, cgn;
+  int64_t cg0;
 };
 
 // Per-instance mutable scalars (device memory).
@@ -106,6 +110,8 @@ struct InstScal {
   double sigma_prev;    // scale used by the previous residual sweep
   double last_err, last_relres;   // of the last finished step
   int64_t last_iter;
+  int32_t ypend;        // y still lacks the last direction of the inner solve (YEnd)
+  int32_t pad;
 };
 
 // InstScal::xw.  kXwAllowed: the inner CG update may form x itself (true-residual criterion, rows
@@ -131,31 +137,30 @@ enum : int32_t {
   PH_IDLE = HF_PHASE_IDLE,          // step finished (or failed): nothing to do
   PH_START = HF_PHASE_START,        // reserved
   PH_RES_INIT = HF_PHASE_RES_INIT,  // r = S - H x0 (x0 + TINY), g, norms
-  PH_CG_P = HF_PHASE_CG_P,          // p = r + beta p                      (FP64 inner solve)
-  PH_CG_Q = HF_PHASE_CG_Q,          // q = Ah p, p.q                        (FP64 inner solve)
-  PH_CG_PQ = HF_PHASE_CG_PQ,        // p = r + beta p and q = Ah p fused    (FP32 inner solve)
-  PH_CG_B = HF_PHASE_CG_B,          // y += alpha p, r -= alpha q, r.r
+  PH_CG_PQ = HF_PHASE_CG_PQ,        // y += alpha p, p = r + beta p, q = Ah p, p.q
+  PH_CG_B = HF_PHASE_CG_B,          // r -= alpha q, r.r
   PH_XUPD = HF_PHASE_XUPD,          // x += sigma S^-1 y (+ TINY once)
   PH_RES = HF_PHASE_RES             // true residual of the updated x
 };
 
-// Control block of one launch of the persistent solve kernel (zeroed before every launch).
+// Control block of the persistent solve (zeroed before every solve; the counters before every launch
+// of its kernel).
 constexpr int kRoundLog = 512;                     // rounds whose end time is recorded
 struct SolveCtl {
   int32_t err;             // a wait gave up (time limit): the launch was abandoned
   int32_t guard_hit;       // the round bound was reached
-  // one grid
+  int64_t rounds;          // rounds run
+  unsigned long long t_start;                 // %globaltimer at kernel start (ns)
+  unsigned long long t_round[kRoundLog];      // %globaltimer when round r ended
+  int32_t phase_log[kRoundLog];               // phase instance 0 ran in round r
+  // counters, one grid
   alignas(128) unsigned long long arrived;   // blocks arrived at all grid barriers so far
   alignas(128) unsigned next_task[4];        // tasks handed out in a round (by round mod 4)
-  // several grids
+  // counters, several grids
   alignas(128) unsigned long long ticket;    // tickets handed out
   alignas(128) unsigned long long tail;      // tickets published beyond the first phase's
   unsigned long long phases;                 // phases published
   unsigned finished;                         // instances without work left
-  int64_t rounds;          // rounds run
-  unsigned long long t_start;                 // %globaltimer at kernel start (ns)
-  unsigned long long t_round[kRoundLog];      // %globaltimer when round r's barrier opened
-  int32_t phase_log[kRoundLog];               // phase instance 0 ran in round r
 };
 
 // Several grids: behind the control block, each instance's published ticket range, then its count
@@ -185,7 +190,8 @@ struct DevArrays {
   InstScal* scal;
   const int32_t* tile_inst;
   double* partials;       // partial sums of the tasks: value k of task t at [k * pcap + t]; two such
-                          // tables of kNR values, used by alternate rounds of the one-grid solve
+                          // tables of kNR values: the persistent solve of one grid uses them in
+                          // alternate rounds, that of several for the two kinds of tasks
   unsigned int* counters; // per instance, last-block detection
   DevOpts opts;
   // static
@@ -211,11 +217,13 @@ struct DevArrays {
   float *y32, *r32, *p32, *q32, *p232;   // p / p2: search directions, ping-pong by iteration
   const int8_t* task_heat;  // per task: some cell holds a heater
   const int4* tasks;        // (instance, x0, y0, z0) per task
-  int64_t ncells, ntiles, ninst, ntasks;
+  const int32_t* cg_inst;   // instance per task of the inner solve's passes
+  int64_t ncells, ntiles, ninst, ntasks, ncg;   // ncg: tasks of the inner solve's passes
   int64_t pcap;             // tasks that a table of partial sums holds
   // index-check record of the checked build (HF_CHECKED): [0] failed checks, [1] site of the
   // first, [2] its index, [3] the extent it was checked against
   unsigned long long* check;
+  SolveCtl* sctl;           // control block of the persistent solve
   // host-buffer steps (the graphs of hf_step_host_async only, null elsewhere): the residual
   // sweeps after an update also store x here, in the compact layout (InstDesc::hoff), so the
   // step's result needs no gather for its download
@@ -224,9 +232,9 @@ struct DevArrays {
 
 // ---- index checks of the checked build ----------------------------------------------------------
 // Compiled with -DHF_CHECKED (build_library(checked=True): a separate library for tests), every
-// global load and store of the step kernels takes its index through HF_IX (one cell) or HF_IX4 (a
+// global load and store of the step kernels takes its index through HF_IX (one cell), HF_IX4 (a
 // 4-cell vector, which must also start on a multiple of 4 cells: a 16-byte boundary for FP32, two
-// for FP64).  An index outside [0, n) -- n the extent of that array in the instance's layout -- is
+// for FP64) or HF_IXV (a vector of v = 2 or 4 cells).  An index outside [0, n) -- n the extent of that array in the instance's layout -- is
 // recorded in DevArrays::check and replaced by 0, so the access stays inside the array and the
 // kernel goes on: no trap, no fault.  The host reports a record as HF_EDEVICE (the site is
 // 100000 * file + line).  In the normal build both macros are the index itself.
@@ -248,9 +256,11 @@ __device__ __noinline__ inline long long hf_check_ix(unsigned long long* rec, in
 #define HF_SITE (HF_FILE_ID * 100000 + __LINE__)
 #define HF_IX(A, i, n) ((int)hf_check_ix((A).check, HF_SITE, (long long)(i), (long long)(n), 1))
 #define HF_IX4(A, i, n) ((int)hf_check_ix((A).check, HF_SITE, (long long)(i), (long long)(n), 4))
+#define HF_IXV(A, i, n, v) ((int)hf_check_ix((A).check, HF_SITE, (long long)(i), (long long)(n), (v)))
 #else
 #define HF_IX(A, i, n) (i)
 #define HF_IX4(A, i, n) (i)
+#define HF_IXV(A, i, n, v) (i)
 #endif
 
 // Slots of DevArrays::stamps: step begin, RHS start, RHS finalize start, solve start, end of the
@@ -522,9 +532,11 @@ cudaError_t launch_residual(Ctx& c, int mode, CtrlState* ctrl = nullptr,
 cudaError_t launch_inner_iteration(Ctx& c, int fp32, CtrlState* ctrl = nullptr,
                                    cudaGraphConditionalHandle hw = 0, int graph = 0);
 cudaError_t launch_step_end(Ctx& c);
-// Persistent solve: one cooperative launch runs the whole refinement loop of a step.
-cudaError_t launch_solve(Ctx& c, unsigned long long wait_ns = 4000000000ull, int leaver = -1);
-int solve_grid_blocks(Ctx& c, int fp32);
+// Persistent solve: one cooperative launch runs the whole refinement loop of a step, or (full =
+// false) the inner solves that are due.
+cudaError_t launch_solve(Ctx& c, bool full = true, unsigned long long wait_ns = 4000000000ull,
+                         int leaver = -1);
+int solve_grid_blocks(Ctx& c, int fp32, bool full = true);
 cudaError_t launch_apply(Ctx& c, const double* x, double* y);
 cudaError_t launch_single(Ctx& c, int which);
 cudaError_t launch_graph_step_begin(Ctx& c, CtrlState* ctrl, int launches_per_step);
@@ -533,7 +545,8 @@ cudaError_t launch_graph_step_end(Ctx& c, CtrlState* ctrl, const SolveCtl* sctl,
 cudaError_t launch_ctrl_select(Ctx& c, CtrlState* ctrl, cudaGraphConditionalHandle hs,
                                cudaGraphConditionalHandle hw);
 // Finalize kernels: sum the tile partials of each instance and run the scalar epilogue of the
-// kernel that produced them.  With graph != 0 the last block also sets the loop condition hw.
+// kernel that produced them.  With graph != 0 the last block also sets the loop condition hw; graph
+// = 2: the split solve's loop, whose rounds are logged.
 enum { FIN_RHS = 0, FIN_RHS_DIAG, FIN_RES_INIT, FIN_RES, FIN_SPMV, FIN_UPD };
 cudaError_t launch_finalize(Ctx& c, int kind, CtrlState* ctrl, cudaGraphConditionalHandle hw,
                             int graph);

@@ -22,6 +22,8 @@
 // All solver state is per instance in device memory; tiles of instances that are not in the
 // phase a kernel serves return at once (per-instance convergence masks).
 #include <algorithm>
+#include <climits>
+#include <cstddef>
 
 #include "hf_ctx.cuh"
 
@@ -218,8 +220,7 @@ __device__ __forceinline__ void res_hx_task(const DevArrays& A, double* part, in
   const double* __restrict__ rsum = A.rsum + off;
   const float* __restrict__ sinv32 = A.sinv32 + off;
   const double* __restrict__ sinv = A.sinv + off;
-  const bool f32 = sizeof(TR) == 4;           // FP32 g goes into the FP32 layout
-  TR* R = Vec<TR>::r(A) + (f32 ? c.off4 : off);
+  TR* R = Vec<TR>::r(A) + c.off4;             // the inner solve's layout
   const float isig = (float)(1.0 / s.sigma);
   const bool tiny = tiny_applies(A, s);       // the residual of x0 + TINY: r(x0) - TINY * H1
   double rr = 0.0, gg64 = 0.0;
@@ -227,7 +228,7 @@ __device__ __forceinline__ void res_hx_task(const DevArrays& A, double* part, in
   SqSum rq;                                    // mixed: ||r||^2 off the FP64 pipe
   if (c.act(0)) {
     const int nxy = c.nxy, base = c.base(0);
-    const int rxy = f32 ? c.nxy4 : nxy, rbase = f32 ? c.base4(0) : base;
+    const int rxy = c.nxy4, rbase = c.base4(0);
 #pragma unroll 4
     for (int z = c.z0; z < c.z1; ++z) {
       const int l = base + z * nxy, lr = rbase + z * rxy;
@@ -247,7 +248,7 @@ __device__ __forceinline__ void res_hx_task(const DevArrays& A, double* part, in
         gg = fmaf(g, g, gg);
       } else {
         const double g = -sinv[lc] * a;
-        R[HF_IX(A, lr, c.n())] = (TR)g;
+        R[HF_IX(A, lr, c.n4())] = (TR)g;
         gg64 = fma(g, g, gg64);
       }
     }
@@ -292,9 +293,8 @@ __device__ __forceinline__ void res_task(const DevArrays& A, double* part, int64
   const double* __restrict__ rsum = A.rsum + off;
   const float* __restrict__ sinv32 = A.sinv32 + off;
   const double* __restrict__ sinv = A.sinv + off;
-  const bool f32 = sizeof(TR) == 4;           // FP32 g goes into the FP32 layout
-  TR* R = Vec<TR>::r(A) + (f32 ? c.off4 : off);
-  const int rxy = f32 ? c.nxy4 : c.nxy, rbase = f32 ? c.base4(0) : c.base(0);
+  TR* R = Vec<TR>::r(A) + c.off4;             // the inner solve's layout
+  const int rxy = c.nxy4, rbase = c.base4(0);
   double* HX = A.hx[1 - s.hx_role] + off;
   // host-buffer steps (the persistent solve of their graphs): x into the result buffer too
   double* XO = (XOUT && !INIT) ? A.xout + A.inst[c.inst].hoff : nullptr;
@@ -310,68 +310,74 @@ __device__ __forceinline__ void res_task(const DevArrays& A, double* part, int64
   const int yn = y_north(c), ys = y_south(c);
   const int n = c.n();
   auto xval = [&](int m) -> double { return X[HF_IX(A, m, n)]; };
+  // the operands of a plane; those of the next are loaded while one is computed
+  struct Plane {
+    double up, diag, b, cx, cy, cz, cys, xn, xs, xw, cxw, xe, rs, si;
+    float si32;
+  };
+  auto load = [&](int z, Plane& o) {
+    o.up = plane_above<double>(c, 0, xval, z);
+    o.xw = o.cxw = o.xe = o.xn = o.xs = o.cys = o.rs = o.si = 0.0;
+    o.cx = o.diag = o.b = o.cy = o.cz = 0.0;
+    o.si32 = 0.f;
+    if (!act) return;
+    const int l = base + z * nxy, lc = HF_IX(A, l, n);
+    o.diag = diag[lc];
+    o.b = b[lc];
+    o.cx = cx[lc];
+    o.cy = cy[lc];
+    o.cz = cz[lc];
+    if (tiny) o.rs = rsum[lc];
+    if (xe.w != kNoNbr) { o.xw = xval(l + xe.w); o.cxw = cx[HF_IX(A, l + xe.w, n)]; }
+    if (xe.e != kNoNbr) o.xe = xval(l + xe.e);
+    if (yn != kNoNbr) o.xn = xval(l + yn);
+    if (ys != kNoNbr) { o.cys = cy[HF_IX(A, l + ys, n)]; o.xs = xval(l + ys); }
+    if (sizeof(TR) == 4) o.si32 = sinv32[lc];
+    else o.si = sinv[lc];
+  };
   double xm, czm;
   plane_below<double>(A, c, 0, xval, cz, xm, czm);
   double xc = act ? xval(base + c.z0 * nxy) : 0.0;
   double rr = 0.0, gg64 = 0.0;
   float gg = 0.f;
+  Plane cur, nxt;
+  load(c.z0, cur);
   for (int z = c.z0; z < c.z1; ++z) {
-    const int l = base + z * nxy;
-    const double xn = plane_above<double>(c, 0, xval, z);
-    double cxc = 0.0, a = 0.0, bl = 0.0, xwl = 0.0, cxwl = 0.0, xel = 0.0;
-    double cyn = 0.0, xyn = 0.0, cys = 0.0, xys = 0.0, czc = 0.0;
-    if (act) {
-      if (z + 2 < c.z1) {                    // the plane after next: x, diag, b, cx, cy, cz
-        const int lp = l + 2 * nxy;
-        prefetch_l2(X + lp);
-        prefetch_l2(diag + lp);
-        prefetch_l2(b + lp);
-        prefetch_l2(cx + lp);
-        prefetch_l2(cy + lp);
-        prefetch_l2(cz + lp);
-      }
-      const int lc = HF_IX(A, l, n);
-      cxc = cx[lc];
-      bl = b[lc];
-      a = fma(-diag[lc], xc, bl);
-      if (tiny) a = fma(-kTiny, rsum[lc], a);
-      if (xe.w != kNoNbr) { xwl = xval(l + xe.w); cxwl = cx[HF_IX(A, l + xe.w, n)]; }
-      if (xe.e != kNoNbr) xel = xval(l + xe.e);
-      if (yn != kNoNbr) { cyn = cy[lc]; xyn = xval(l + yn); }
-      if (ys != kNoNbr) { cys = cy[HF_IX(A, l + ys, n)]; xys = xval(l + ys); }
-      czc = cz[lc];
-    }
-    const double up = __shfl_up_sync(kFull, xc, 1), cup = __shfl_up_sync(kFull, cxc, 1);
+    if (z + 1 < c.z1) load(z + 1, nxt);
+    const double up = __shfl_up_sync(kFull, xc, 1), cup = __shfl_up_sync(kFull, cur.cx, 1);
     const double dn = __shfl_down_sync(kFull, xc, 1);
     if (act) {
-      const double xw = c.lane > 0 ? up : xwl, cxw = c.lane > 0 ? cup : cxwl;
-      const double xeast = (c.x(0) + 1 < c.nx && c.lane < 31) ? dn : xel;
-      a = fma(-cxc, xeast, a);
+      const double xw = c.lane > 0 ? up : cur.xw, cxw = c.lane > 0 ? cup : cur.cxw;
+      const double xeast = (c.x(0) + 1 < c.nx && c.lane < 31) ? dn : cur.xe;
+      double a = fma(-cur.diag, xc, cur.b);
+      if (tiny) a = fma(-kTiny, cur.rs, a);
+      a = fma(-cur.cx, xeast, a);
       a = fma(-cxw, xw, a);
-      if (yn != kNoNbr) a = fma(-cyn, xyn, a);
-      if (ys != kNoNbr) a = fma(-cys, xys, a);
+      if (yn != kNoNbr) a = fma(-cur.cy, cur.xn, a);
+      if (ys != kNoNbr) a = fma(-cur.cys, cur.xs, a);
       if (nz > 1) {
-        a = fma(-czc, xn, a);
+        a = fma(-cur.cz, cur.up, a);
         a = fma(-czm, xm, a);
       }
       if (sizeof(TR) == 8) rr = fma(a, a, rr);
       else rq.add(a);
-      const int lc = HF_IX(A, l, n);
-      if (!INIT) HX[lc] = bl - a;
+      const int lc = HF_IX(A, base + z * nxy, n);
+      if (!INIT) HX[lc] = cur.b - a;
       if (XOUT && !INIT) XO[lc] = xc;
       if (sizeof(TR) == 4) {             // mixed: g in FP32, scaled by 1/sigma
-        const float g = -sinv32[lc] * f64_to_f32_trunc(a) * isig;
+        const float g = -cur.si32 * f64_to_f32_trunc(a) * isig;
         R[HF_IX(A, rbase + z * rxy, c.n4())] = (TR)g;
         gg = fmaf(g, g, gg);
       } else {                           // FP64 path: sigma = 1
-        const double g = -sinv[lc] * a;
-        R[HF_IX(A, rbase + z * rxy, n)] = (TR)g;
+        const double g = -cur.si * a;
+        R[HF_IX(A, rbase + z * rxy, c.n4())] = (TR)g;
         gg64 = fma(g, g, gg64);
       }
     }
-    czm = czc;
+    czm = cur.cz;
     xm = xc;
-    xc = xn;
+    xc = cur.up;
+    cur = nxt;
   }
   if (sizeof(TR) == 4) rr = rq.value();
   if (sizeof(TR) == 4) {
@@ -384,6 +390,20 @@ __device__ __forceinline__ void res_task(const DevArrays& A, double* part, int64
   }
 }
 
+// The inner solution y at the end of an inner solve.  A direction p_k enters y one pass late, in
+// the pass that forms p_(k+1) and reads p_k anyway (pq_task): the last one is still missing where
+// the solve ended on a CG update (InstScal::ypend).  old, last: which of y and p are read.
+template <typename T>
+struct YEnd {
+  T alpha;
+  bool old, last;
+  __device__ __forceinline__ explicit YEnd(const InstScal& s)
+      : alpha((T)s.alpha), old(s.ypend == 0 || s.iter > 1), last(s.ypend != 0) {}
+  __device__ __forceinline__ T operator()(T y, T p) const {
+    return last ? fma(alpha, p, old ? y : T(0)) : y;
+  }
+};
+
 // Solution update of one task: x_new = x + sigma S^-1 y (+ TINY once).
 template <typename TY>
 __device__ __forceinline__ void xupd_task(const DevArrays& A, double* part, int64_t task,
@@ -393,15 +413,16 @@ __device__ __forceinline__ void xupd_task(const DevArrays& A, double* part, int6
   const int64_t off = c.off;
   const double* XR = A.tbuf[s.role[2]] + off;
   double* XW = A.tbuf[s.role[3]] + off;
-  const bool f32 = sizeof(TY) == 4;           // FP32 y is read from the FP32 layout
-  const TY* Y = Vec<TY>::y(A) + (f32 ? c.off4 : off);
+  const TY* Y = Vec<TY>::y(A) + c.off4;       // the inner solve's layout
+  const TY* P = Vec<TY>::pb(A, s.iter - 1) + c.off4;
+  const YEnd<TY> ye(s);
   const double* __restrict__ sinv = A.sinv + off;
   const float* __restrict__ sinv32 = A.sinv32 + off;
   const bool use_y = s.iter > 0;
   const bool tiny = s.tiny_pending != 0;
   const float sig = (float)s.sigma_prev;
   const int nxy = c.nxy, base = c.base(0);
-  const int yxy = f32 ? c.nxy4 : nxy, ybase = f32 ? c.base4(0) : base;
+  const int yxy = c.nxy4, ybase = c.base4(0);
   for (int z0 = c.z0; z0 < c.z1; z0 += 4) {
     double xv[4], sv[4];
     float sv32[4];
@@ -414,7 +435,8 @@ __device__ __forceinline__ void xupd_task(const DevArrays& A, double* part, int6
         const int lc = HF_IX(A, l, c.n());
         xv[u] = XR[lc];
         if (use_y) {
-          yv[u] = Y[HF_IX(A, ybase + (z0 + u) * yxy, f32 ? c.n4() : c.n())];
+          const int ly = HF_IX(A, ybase + (z0 + u) * yxy, c.n4());
+          yv[u] = ye(ye.old ? Y[ly] : TY(0), ye.last ? P[ly] : TY(0));
           if (sizeof(TY) == 8) sv[u] = sinv[lc];
           else sv32[u] = sinv32[lc];
         }
@@ -435,379 +457,12 @@ __device__ __forceinline__ void xupd_task(const DevArrays& A, double* part, int6
   }
 }
 
-// Direction update of one task: p_k = r + beta p_(k-1) (p_0 = r) into the buffer of parity k.
-template <typename T>
-__device__ __forceinline__ void cgp_task(const DevArrays& A, double* part, int64_t task,
-                                          const InstScal& s) {
-  const TCell c = task_cell(A, task);
-  if (!c.act(0)) return;
-  const int64_t k = s.iter;
-  const bool first = (k == 0);
-  const T beta = (T)s.beta;
-  const T* R = Vec<T>::r(A) + c.off;
-  const T* Po = Vec<T>::pb(A, k + 1) + c.off;
-  T* Pn = Vec<T>::pb(A, k) + c.off;
-  const int nxy = c.nxy, base = c.base(0);
-  for (int z0 = c.z0; z0 < c.z1; z0 += 4) {
-    T rv[4], pv[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      rv[u] = T(0); pv[u] = T(0);
-      if (z0 + u < c.z1) {
-        const int l = HF_IX(A, base + (z0 + u) * nxy, c.n());
-        rv[u] = R[l];
-        if (!first) pv[u] = Po[l];
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      if (z0 + u >= c.z1) continue;
-      Pn[HF_IX(A, base + (z0 + u) * nxy, c.n())] = first ? rv[u] : fma(beta, pv[u], rv[u]);
-    }
-  }
-}
-
-// q = Ah p and p.q for one task.  FUSED: p is formed on the fly from r and the previous direction
-// (p = r + beta p_old, the value the direction update would store) and written out beside q, so
-// one pass replaces two.  One column per thread; the operands of plane z+1 (its coefficients, y
-// neighbours, x-edge neighbours and plane z+2) are loaded while plane z is computed.
-template <typename T, bool FUSED>
-__device__ __forceinline__ void spmv_task(const DevArrays& A, double* part, int64_t task,
-                                          const InstScal& s) {
-  static_assert(kXC == 1, "one column per thread");
-  const TCell c = task_cell(A, task);
-  const int64_t off = c.off;
-  const int64_t k = s.iter;
-  const bool first = !FUSED || (k == 0);
-  const T beta = (T)s.beta;
-  // r, or p itself (p_0 = r: the first iteration reads r, its direction update has no round)
-  const T* Src = (FUSED || k == 0) ? Vec<T>::r(A) + off : Vec<T>::pb(A, k) + off;
-  const T* Po = Vec<T>::pb(A, k + 1) + off;
-  T* Pn = Vec<T>::pb(A, k) + off;
-  T* Q = Vec<T>::q(A) + off;
-  const T* __restrict__ ax = Vec<T>::ax(A) + off;
-  const T* __restrict__ ay = Vec<T>::ay(A) + off;
-  const T* __restrict__ az = Vec<T>::az(A) + off;
-  const bool act = c.act(0);
-  const int nx = c.nx, nz = c.nz, nxy = c.nxy, base = c.base(0);
-  const XEdge xe = x_edges(c);
-  const int yn = y_north(c), ys = y_south(c);
-  const bool east_shfl = act && (c.x(0) + 1 < nx) && c.lane < 31;
-  // raw operands of one direction value: p = first ? a : beta * b + a
-  struct RP { T a, b; };
-  const int n = c.n();
-  auto ld = [&](int m) -> RP {
-    const int mc = HF_IX(A, m, n);
-    return RP{Src[mc], first ? T(0) : Po[mc]};
-  };
-  auto pval = [&](const RP& v) -> T { return first ? v.a : fma(beta, v.b, v.a); };
-  struct Plane { RP own, n, s, w, e; T axc, ayc, azc, ays, axw; };
-  const RP z0v{T(0), T(0)};
-  auto load = [&](int z, Plane& o) {
-    o.own = z0v; o.n = z0v; o.s = z0v; o.w = z0v; o.e = z0v;
-    o.axc = T(0); o.ayc = T(0); o.azc = T(0); o.ays = T(0); o.axw = T(0);
-    if (!act) return;
-    if (z >= nz) {                      // above the top plane: the periodic wrap, or nothing
-      if (c.pz && nz > 1) o.own = ld(base);
-      return;
-    }
-    const int l = base + z * nxy, lc = HF_IX(A, l, n);
-    o.own = ld(l);
-    o.axc = ax[lc]; o.ayc = ay[lc]; o.azc = az[lc];
-    if (yn != kNoNbr) o.n = ld(l + yn);
-    if (ys != kNoNbr) { o.s = ld(l + ys); o.ays = ay[HF_IX(A, l + ys, n)]; }
-    if (xe.w != kNoNbr) { o.w = ld(l + xe.w); o.axw = ax[HF_IX(A, l + xe.w, n)]; }
-    if (xe.e != kNoNbr) o.e = ld(l + xe.e);
-  };
-  // plane below the task (z0 - 1, or the periodic wrap to nz - 1)
-  T pm = T(0), azm = T(0);
-  if (act && nz > 1) {
-    int lb = -1;
-    if (c.z0 > 0) lb = base + (c.z0 - 1) * nxy;
-    else if (c.pz) lb = base + (nz - 1) * nxy;
-    if (lb >= 0) { pm = pval(ld(lb)); azm = az[HF_IX(A, lb, n)]; }
-  }
-  Plane cur, nxt;
-  load(c.z0, cur);
-  T pq = T(0);
-  for (int z = c.z0; z < c.z1; ++z) {
-    if (z + 1 < nz) load(z + 1, nxt);
-    else load(nz, nxt);
-    const int l = base + z * nxy;
-    const T pc = pval(cur.own);
-    const T up = __shfl_up_sync(kFull, pc, 1);
-    const T cup = __shfl_up_sync(kFull, cur.axc, 1);
-    const T dn = __shfl_down_sync(kFull, pc, 1);
-    if (act) {
-      const T pw = c.lane > 0 ? up : pval(cur.w);
-      const T axw = c.lane > 0 ? cup : cur.axw;
-      const T pe = east_shfl ? dn : pval(cur.e);
-      T acc = pc;
-      acc = fma(cur.axc, pe, acc);
-      acc = fma(axw, pw, acc);
-      if (c.ny > 1) {
-        acc = fma(cur.ayc, pval(cur.n), acc);
-        acc = fma(cur.ays, pval(cur.s), acc);
-      }
-      if (nz > 1) {
-        acc = fma(cur.azc, pval(nxt.own), acc);
-        acc = fma(azm, pm, acc);
-      }
-      const int lc = HF_IX(A, l, n);
-      if (FUSED) Pn[lc] = pc;
-      Q[lc] = acc;
-      pq = fma(pc, acc, pq);
-    }
-    pm = pc; azm = cur.azc;
-    cur = nxt;
-  }
-  if (sizeof(T) == 4) {
-    task_store_f(part + task, (float)pq);
-  } else {
-    const double v[1] = {(double)pq};
-    tile_store<1>(part + task, A.pcap, v);
-  }
-}
-
-// y += alpha p, r -= alpha q, r.r (and the unscaled ||r||^2 for the reference rule) of one task.
-template <typename T>
-__device__ __forceinline__ void upd_task(const DevArrays& A, double* part, int64_t task,
-                                          const InstScal& s) {
-  const TCell c = task_cell(A, task);
-  const DevOpts& o = A.opts;
-  const bool weighted = (o.criterion == HF_STOP_RECURSIVE);
-  const T alpha = (T)s.alpha;
-  const bool first = (s.iter == 0);
-  const int64_t off = c.off;
-  T* Y = Vec<T>::y(A) + off;
-  T* R = Vec<T>::r(A) + off;
-  const T* P = Vec<T>::pb(A, s.iter) + off;
-  T* P0 = Vec<T>::pb(A, 0) + off;            // p_0 = r, left for p_1 (as in upd4_task)
-  const T* Q = Vec<T>::q(A) + off;
-  const double* __restrict__ diag = A.diag + off;
-  const bool act = c.act(0);
-  const int nxy = c.nxy, base = c.base(0);
-  T rr = T(0);
-  double rw = 0.0;
-  if (act) {
-    for (int z0 = c.z0; z0 < c.z1; z0 += 4) {
-      T pv[4], qv[4], rv[4], yv[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        pv[u] = T(0); qv[u] = T(0); rv[u] = T(0); yv[u] = T(0);
-        if (z0 + u < c.z1) {
-          const int l = HF_IX(A, base + (z0 + u) * nxy, c.n());
-          qv[u] = Q[l]; rv[u] = R[l];
-          pv[u] = first ? rv[u] : P[l];
-          if (!first) yv[u] = Y[l];
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        if (z0 + u >= c.z1) continue;
-        const int l = HF_IX(A, base + (z0 + u) * nxy, c.n());
-        Y[l] = first ? alpha * pv[u] : fma(alpha, pv[u], yv[u]);
-        const T r = fma(-alpha, qv[u], rv[u]);
-        R[l] = r;
-        if (first) P0[l] = rv[u];
-        rr = fma(r, r, rr);
-        if (weighted) rw = fma(-diag[l] * (double)r, (double)r, rw);
-      }
-    }
-  }
-  if (sizeof(T) == 4 && !weighted) {
-    task_store_f(part + task, (float)rr);
-  } else {
-    const double v[2] = {(double)rr, rw};
-    tile_store<2>(part + task, A.pcap, v);
-  }
-}
-
-// ---- FP32 p + SpMV on 16-byte vectors ---------------------------------------------------------
-// The FP32 vectors have rows of sx = nx rounded up to 4 cells (every row starts 16-byte aligned;
-// the instances start at multiples of 1024 cells), so each thread owns 4 consecutive x cells and
-// works on float4 vectors: a quarter of the scalar version's instructions per cell.  In a row's
-// last quad the cells past nx are padding: their coefficients and p are zero, q is kept zero, and
-// the last grid cell takes its east neighbour from a load (the periodic wrap) or has none.  Block layout over a
-// 32 x 8 column tile: four z-groups of 64 threads, each marching its quarter of the task's planes;
-// in a group, thread w owns row w / 8 and cells x0 + 4 (w % 8) .. + 3, so a warp holds 4 rows of
-// 8 quads and the x neighbours across quads are shuffles.  Per plane a thread issues its ten
-// vector loads (own r, p_old, three faces; the y-neighbour rows; the next plane's r, p_old) at
-// once, which keeps ~40 KB per block in flight.  FUSED: p = r + beta p_old is formed on the fly and
-// stored beside q (the persistent solve's pass); otherwise p is read (the standalone SpMV).  The
-// per-cell arithmetic is the scalar version's; the p.q partial is summed per thread over its 4
-// cells plane by plane, the same way in both uses.
 __device__ __forceinline__ bool vec4_ok(const InstDesc& d) { return (d.nx & 3) == 0; }
 
-// The quad (4 consecutive x cells) of thread w (0..63) of a z-group: 8 quads x 8 rows of the
-// task's tile.  west_lane / east_lane: the neighbouring quad of the row is not in the adjacent
-// lane of this warp.
-struct QuadPos {
-  int x, y;
-  bool act, west_lane, east_lane;
-};
-__device__ __forceinline__ QuadPos quad_pos(const int4& tk, const InstDesc& d, int w) {
-  QuadPos p;
-  p.x = tk.y + 4 * (w & 7);
-  p.y = tk.z + (w >> 3);
-  p.act = p.x < d.nx && p.y < d.ny;
-  p.west_lane = (w & 7) == 0;
-  p.east_lane = (w & 7) == 7;
-  return p;
-}
-
-__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
-
-__device__ __forceinline__ void st4(float* p, const float4& v) { *reinterpret_cast<float4*>(p) = v; }
-__device__ __forceinline__ float f4(const float4& v, int i) {
-  return i == 0 ? v.x : (i == 1 ? v.y : (i == 2 ? v.z : v.w));
-}
-
-template <bool FUSED>
-__device__ __forceinline__ void spmv4_task(const DevArrays& A, double* part, int64_t task,
-                                           const InstScal& s) {
-  const int4 tk = A.tasks[task];
-  const InstDesc& d = A.inst[tk.x];
-  const int nx = d.nx, ny = d.ny, nz = d.nz, sx = d.sx, nxy = sx * ny;
-  const int64_t off = d.off4;
-  const int tid = threadIdx.x, grp = tid >> 6, w = tid & 63;
-  const QuadPos qp = quad_pos(tk, d, w);
-  const int x = qp.x, y = qp.y;
-  const int z0 = tk.w, z1 = min(z0 + d.zc, nz);
-  const int per = (z1 - z0 + 3) >> 2;
-  const int za = min(z0 + grp * per, z1), zb = min(za + per, z1);
-  const bool act = qp.act;
-  const int last = min(3, nx - 1 - x);   // the quad's last grid cell; cells past it are padding
-  const int64_t k = s.iter;
-  const bool first = !FUSED || k == 0;
-  const float beta = (float)s.beta;
-  const float* Src = (FUSED || k == 0) ? A.r32 + off : ((k & 1) ? A.p232 : A.p32) + off;
-  const float* Po = (((k + 1) & 1) ? A.p232 : A.p32) + off;
-  float* Pn = ((k & 1) ? A.p232 : A.p32) + off;
-  float* Q = A.q32 + off;
-  const float* __restrict__ ax = A.a32x + off;
-  const float* __restrict__ ay = A.a32y + off;
-  const float* __restrict__ az = A.a32z + off;
-  const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
-  // neighbour offsets (y rows, x edges, z wrap); has_* false: the face is absent (value 0)
-  bool hn = false, hs = false;
-  int dn = 0, ds = 0;
-  if (ny > 1) {
-    if (y + 1 < ny) { dn = sx; hn = true; } else if (d.py) { dn = -(ny - 1) * sx; hn = true; }
-    if (y > 0) { ds = -sx; hs = true; } else if (d.py) { ds = (ny - 1) * sx; hs = true; }
-  }
-  const bool wload = (qp.west_lane || x == 0);     // west of cell 0 is loaded, not shuffled
-  const bool eload = (qp.east_lane || x + 4 >= nx); // east of the last cell is loaded, not shuffled
-  bool hw = false, he = false;
-  int dw = 0, de = 0;
-  if (x > 0) { dw = -1; hw = true; } else if (d.px && nx > 1) { dw = nx - 1; hw = true; }
-  if (x + 4 < nx) { de = 4; he = true; } else if (d.px && nx > 1) { de = -x; he = true; }
-  auto pv = [&](float a, float b) -> float { return first ? a : fmaf(beta, b, a); };
-  auto pv4 = [&](const float4& a, const float4& b) -> float4 {
-    return make_float4(pv(a.x, b.x), pv(a.y, b.y), pv(a.z, b.z), pv(a.w, b.w));
-  };
-  const int n4 = nxy * nz;               // the instance's cells in the FP32 layout
-  auto ldp = [&](int l, float4& r, float4& po) {
-    const int lc = HF_IX4(A, l, n4);
-    r = ld4(Src + lc);
-    po = first ? zero4 : ld4(Po + lc);
-  };
-  const int lxy = y * sx + x;
-  // plane below the group (za - 1, or the periodic wrap to nz - 1), and the group's first plane
-  float4 pm = zero4, azm = zero4, rc = zero4, poc = zero4;
-  if (act && za < zb) {
-    if (nz > 1) {
-      int lb = -1;
-      if (za > 0) lb = lxy + (za - 1) * nxy;
-      else if (d.pz) lb = lxy + (nz - 1) * nxy;
-      if (lb >= 0) {
-        float4 rb, pob;
-        ldp(lb, rb, pob);
-        pm = pv4(rb, pob);
-        azm = ld4(az + HF_IX4(A, lb, n4));
-      }
-    }
-    ldp(lxy + za * nxy, rc, poc);
-  }
-  float pq = 0.f;
-  for (int z = za; z < zb; ++z) {
-    const int l = lxy + z * nxy;
-    float4 ru = zero4, pou = zero4, axv = zero4, ayv = zero4, azv = zero4;
-    float4 rn = zero4, pon = zero4, rs = zero4, pos = zero4, aysv = zero4;
-    float rw = 0.f, pow_ = 0.f, axwl = 0.f, re = 0.f, poe = 0.f;
-    if (act) {
-      if (nz > 1) {
-        if (z + 1 < nz) ldp(l + nxy, ru, pou);
-        else if (d.pz) ldp(lxy, ru, pou);
-      }
-      const int lc = HF_IX4(A, l, n4);
-      axv = ld4(ax + lc); ayv = ld4(ay + lc); azv = ld4(az + lc);
-      if (z + 1 < zb) {
-        prefetch_l2(ax + l + nxy);
-        prefetch_l2(ay + l + nxy);
-        prefetch_l2(az + l + nxy);
-      }
-      if (hn) ldp(l + dn, rn, pon);
-      if (hs) { ldp(l + ds, rs, pos); aysv = ld4(ay + HF_IX4(A, l + ds, n4)); }
-      if (wload && hw) {
-        const int lw = HF_IX(A, l + dw, n4);
-        rw = Src[lw];
-        pow_ = first ? 0.f : Po[lw];
-        axwl = ax[lw];
-      }
-      if (eload && he) {
-        const int le = HF_IX(A, l + de, n4);
-        re = Src[le];
-        poe = first ? 0.f : Po[le];
-      }
-    }
-    const float4 p = pv4(rc, poc);
-    const float pw_sh = __shfl_up_sync(kFull, p.w, 1);
-    const float axw_sh = __shfl_up_sync(kFull, axv.w, 1);
-    const float pe_sh = __shfl_down_sync(kFull, p.x, 1);
-    if (act) {
-      const float pw0 = wload ? (hw ? pv(rw, pow_) : 0.f) : pw_sh;
-      const float axw0 = wload ? (hw ? axwl : 0.f) : axw_sh;
-      const float pe3 = eload ? (he ? pv(re, poe) : 0.f) : pe_sh;
-      const float4 pu = pv4(ru, pou), pn = pv4(rn, pon), ps = pv4(rs, pos);
-      float4 qv;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float pc = f4(p, i);
-        const float pe = i < last ? f4(p, i + 1) : pe3;
-        const float pw = i > 0 ? f4(p, i - 1) : pw0;
-        const float axw = i > 0 ? f4(axv, i - 1) : axw0;
-        float acc = pc;
-        acc = fmaf(f4(axv, i), pe, acc);
-        acc = fmaf(axw, pw, acc);
-        if (ny > 1) {
-          acc = fmaf(f4(ayv, i), f4(pn, i), acc);
-          acc = fmaf(f4(aysv, i), f4(ps, i), acc);
-        }
-        if (nz > 1) {
-          acc = fmaf(f4(azv, i), f4(pu, i), acc);
-          acc = fmaf(f4(azm, i), f4(pm, i), acc);
-        }
-        if (i > last) acc = 0.f;       // padding: q stays 0 (its p is 0)
-        pq = fmaf(pc, acc, pq);
-        if (i == 0) qv.x = acc; else if (i == 1) qv.y = acc; else if (i == 2) qv.z = acc; else qv.w = acc;
-      }
-      const int ls = HF_IX4(A, l, n4);
-      if (FUSED) st4(Pn + ls, p);
-      st4(Q + ls, qv);
-      pm = p;
-      azm = azv;
-      rc = ru;
-      poc = pou;
-    }
-  }
-  task_store_f(part + task, pq);
-}
-
-// ---- element-wise passes on 4-cell vectors (rows of 4k cells) --------------------------------
-// Same thread layout as spmv4_task (four z-groups of 64 threads, 4 consecutive x cells per
-// thread); FP32 vectors are one 16-byte access, FP64 vectors two.  Two planes of loads are issued
-// before they are used.  Reductions are summed per thread plane by plane, cells in x order.
+// ---- passes over the cell tasks on 4-cell vectors (rows of 4k cells) --------------------------
+// Four z-groups of 64 threads, 4 consecutive x cells per thread; FP32 vectors are one 16-byte
+// access, FP64 vectors two.  Two planes of loads are issued before they are used.  Reductions are
+// summed per thread plane by plane, cells in x order.
 template <typename T> struct V4 { T v[4]; };
 __device__ __forceinline__ V4<float> ldv4(const float* p) {
   const float4 t = *reinterpret_cast<const float4*>(p);
@@ -825,190 +480,49 @@ __device__ __forceinline__ void stv4(double* p, const V4<double>& v) {
   reinterpret_cast<double2*>(p)[1] = make_double2(v.v[2], v.v[3]);
 }
 
-// A thread's quad.  F32: the pass's vectors are FP32 and live in the FP32 layout (rows of sx
-// cells; voff, nxy, lxy index them); FP64 arrays beside them use the FP64 layout (off, dxy, dlxy).
-// For FP64 vectors (F32 false) both are the FP64 layout.
+// A thread's quad: 4 consecutive x cells of a quarter of the task's planes.
 struct Quad {
-  int64_t off, voff;
-  int nxy, lxy, dxy, dlxy, za, zb, nx, x;
-  int vn, dn;        // cells of the instance in the vectors' layout and in the FP64 layout
-  bool act, padded;
+  int64_t off;
+  int nxy, lxy, za, zb, n;
+  bool act;
 };
-template <bool F32>
 __device__ __forceinline__ Quad quad_cell(const DevArrays& A, int64_t task) {
   const int4 tk = A.tasks[task];
   const InstDesc& d = A.inst[tk.x];
   const int tid = threadIdx.x, grp = tid >> 6, w = tid & 63;
-  const QuadPos qp = quad_pos(tk, d, w);
-  const int x = qp.x, y = qp.y;
+  const int x = tk.y + 4 * (w & 7), y = tk.z + (w >> 3);
   const int z1 = min(tk.w + d.zc, d.nz);
   const int per = (z1 - tk.w + 3) >> 2;
-  const int sx = F32 ? d.sx : d.nx;
   Quad c;
   c.off = d.off;
-  c.voff = F32 ? d.off4 : d.off;
-  c.nxy = sx * d.ny;
-  c.lxy = y * sx + x;
-  c.dxy = d.nx * d.ny;
-  c.dlxy = y * d.nx + x;
-  c.nx = d.nx;
-  c.x = x;
-  c.padded = sx != d.nx;
+  c.nxy = d.nx * d.ny;
+  c.lxy = y * d.nx + x;
   c.za = min(tk.w + grp * per, z1);
   c.zb = min(c.za + per, z1);
-  c.act = qp.act;
-  c.vn = c.nxy * d.nz;
-  c.dn = c.dxy * d.nz;
+  c.act = x < d.nx && y < d.ny;
+  c.n = c.nxy * d.nz;
   return c;
-}
-
-// The FP64-layout diagonal of a quad's cells (zeros for padding cells).
-__device__ __forceinline__ V4<double> diag4(const DevArrays& A, const double* __restrict__ diag,
-                                            const Quad& c, int z) {
-  const int l = c.dlxy + z * c.dxy;
-  if (!c.padded) return ldv4(diag + HF_IX4(A, l, c.dn));
-  V4<double> v{};
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-    if (c.x + i < c.nx) v.v[i] = diag[HF_IX(A, l + i, c.dn)];
-  return v;
-}
-
-template <typename T>
-__device__ __forceinline__ void upd4_task(const DevArrays& A, double* part, int64_t task,
-                                          const InstScal& s) {
-  const Quad c = quad_cell<sizeof(T) == 4>(A, task);
-  const bool weighted = (A.opts.criterion == HF_STOP_RECURSIVE);
-  const T alpha = (T)s.alpha;
-  const bool first = (s.iter == 0);
-  T* Y = Vec<T>::y(A) + c.voff;
-  T* R = Vec<T>::r(A) + c.voff;
-  // p_0 = r has no round of its own: the first update takes p from r and leaves it in the
-  // direction buffer of iteration 0 (p_1 = r_1 + beta p_0 reads it there)
-  const T* P = Vec<T>::pb(A, s.iter) + c.voff;
-  T* P0 = Vec<T>::pb(A, 0) + c.voff;
-  const T* Q = Vec<T>::q(A) + c.voff;
-  const double* __restrict__ diag = A.diag + c.off;
-  T rr = T(0);
-  double rw = 0.0;
-  if (c.act && (s.xw & kXwThis)) {
-    // The iteration predicted to end the inner solve also forms x_new = x + sigma S^-1 y_new, the
-    // x update's arithmetic on the y it stores (rows of 4k cells: both layouts index alike).
-    const double* XR = A.tbuf[s.role[2]] + c.off;
-    double* XW = A.tbuf[s.role[3]] + c.off;
-    const double* __restrict__ sinv = A.sinv + c.off;
-    const float* __restrict__ sinv32 = A.sinv32 + c.off;
-    const float sig = (float)s.sigma_prev;
-    for (int z = c.za; z < c.zb; ++z) {
-      const int l = HF_IX4(A, c.lxy + z * c.nxy, c.vn);
-      const V4<T> qv = ldv4(Q + l), rv = ldv4(R + l);
-      const V4<T> pv = first ? rv : ldv4(P + l);
-      V4<T> yv{};
-      if (!first) yv = ldv4(Y + l);
-      V4<double> xv = ldv4(XR + l), sv{};
-      V4<float> fv{};
-      if (sizeof(T) == 8) sv = ldv4(sinv + l); else fv = ldv4(sinv32 + l);
-      V4<T> yo, ro;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        yo.v[i] = first ? alpha * pv.v[i] : fma(alpha, pv.v[i], yv.v[i]);
-        const T r = fma(-alpha, qv.v[i], rv.v[i]);
-        ro.v[i] = r;
-        rr = fma(r, r, rr);
-        if (sizeof(T) == 8) xv.v[i] = fma(sv.v[i], (double)yo.v[i], xv.v[i]);
-        else xv.v[i] = xv.v[i] + f32_to_f64(sig * fv.v[i] * (float)yo.v[i]);
-      }
-      stv4(Y + l, yo);
-      stv4(R + l, ro);
-      stv4(XW + l, xv);
-      if (first) stv4(P0 + l, rv);
-    }
-  } else if (c.act) {
-    for (int z = c.za; z < c.zb; z += 2) {
-      const bool two = z + 1 < c.zb;
-      const int l0 = HF_IX4(A, c.lxy + z * c.nxy, c.vn);
-      const int l1 = two ? HF_IX4(A, l0 + c.nxy, c.vn) : 0;
-      V4<T> q0 = ldv4(Q + l0), r0 = ldv4(R + l0), p0{}, y0{}, p1{}, q1{}, r1{}, y1{};
-      p0 = first ? r0 : ldv4(P + l0);
-      if (!first) y0 = ldv4(Y + l0);
-      if (two) {
-        q1 = ldv4(Q + l1); r1 = ldv4(R + l1);
-        p1 = first ? r1 : ldv4(P + l1);
-        if (!first) y1 = ldv4(Y + l1);
-      }
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        if (h == 1 && !two) break;
-        const int l = h ? l1 : l0;
-        const V4<T>& pv = h ? p1 : p0;
-        const V4<T>& qv = h ? q1 : q0;
-        const V4<T>& rv = h ? r1 : r0;
-        const V4<T>& yv = h ? y1 : y0;
-        V4<T> yo, ro;
-        V4<double> dg{};
-        if (weighted) dg = diag4(A, diag, c, z + h);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          yo.v[i] = first ? alpha * pv.v[i] : fma(alpha, pv.v[i], yv.v[i]);
-          const T r = fma(-alpha, qv.v[i], rv.v[i]);
-          ro.v[i] = r;
-          rr = fma(r, r, rr);
-          if (weighted) rw = fma(-dg.v[i] * (double)r, (double)r, rw);
-        }
-        stv4(Y + l, yo);
-        stv4(R + l, ro);
-        if (first) stv4(P0 + l, rv);
-      }
-    }
-  }
-  if (sizeof(T) == 4 && !weighted) {
-    task_store_f(part + task, (float)rr);
-  } else {
-    const double v[2] = {(double)rr, rw};
-    tile_store<2>(part + task, A.pcap, v);
-  }
-}
-
-template <typename T>
-__device__ __forceinline__ void cgp4_task(const DevArrays& A, double* part, int64_t task,
-                                          const InstScal& s) {
-  const Quad c = quad_cell<sizeof(T) == 4>(A, task);
-  if (!c.act) return;
-  const int64_t k = s.iter;
-  const bool first = (k == 0);
-  const T beta = (T)s.beta;
-  const T* R = Vec<T>::r(A) + c.voff;
-  const T* Po = Vec<T>::pb(A, k + 1) + c.voff;
-  T* Pn = Vec<T>::pb(A, k) + c.voff;
-  for (int z = c.za; z < c.zb; z += 2) {
-    const bool two = z + 1 < c.zb;
-    const int l0 = HF_IX4(A, c.lxy + z * c.nxy, c.vn);
-    const int l1 = two ? HF_IX4(A, l0 + c.nxy, c.vn) : 0;
-    V4<T> r0 = ldv4(R + l0), o0{}, r1{}, o1{};
-    if (!first) o0 = ldv4(Po + l0);
-    if (two) {
-      r1 = ldv4(R + l1);
-      if (!first) o1 = ldv4(Po + l1);
-    }
-    V4<T> n0, n1;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      n0.v[i] = first ? r0.v[i] : fma(beta, o0.v[i], r0.v[i]);
-      n1.v[i] = first ? r1.v[i] : fma(beta, o1.v[i], r1.v[i]);
-    }
-    stv4(Pn + l0, n0);
-    if (two) stv4(Pn + l1, n1);
-  }
 }
 
 template <typename TY>
 __device__ __forceinline__ void xupd4_task(const DevArrays& A, double* part, int64_t task,
                                            const InstScal& s) {
-  const Quad c = quad_cell<false>(A, task);   // rows of 4k cells: the two layouts agree in shape
+  const Quad c = quad_cell(A, task);   // rows of 4k cells: the two layouts agree in shape
   if (!c.act) return;
   const double* XR = A.tbuf[s.role[2]] + c.off;
   double* XW = A.tbuf[s.role[3]] + c.off;
-  const TY* Y = Vec<TY>::y(A) + (sizeof(TY) == 4 ? A.inst[A.tasks[task].x].off4 : c.off);
+  const int64_t off4 = A.inst[A.tasks[task].x].off4;
+  const TY* Y = Vec<TY>::y(A) + off4;
+  const TY* P = Vec<TY>::pb(A, s.iter - 1) + off4;
+  const YEnd<TY> ye(s);
+  auto ldy = [&](int l) -> V4<TY> {
+    V4<TY> y{}, p{};
+    if (ye.old) y = ldv4(Y + l);
+    if (ye.last) p = ldv4(P + l);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) y.v[i] = ye(y.v[i], p.v[i]);
+    return y;
+  };
   const double* __restrict__ sinv = A.sinv + c.off;
   const float* __restrict__ sinv32 = A.sinv32 + c.off;
   const bool use_y = s.iter > 0;
@@ -1016,19 +530,19 @@ __device__ __forceinline__ void xupd4_task(const DevArrays& A, double* part, int
   const float sig = (float)s.sigma_prev;
   for (int z = c.za; z < c.zb; z += 2) {
     const bool two = z + 1 < c.zb;
-    const int l0 = HF_IX4(A, c.lxy + z * c.nxy, c.vn);
-    const int l1 = two ? HF_IX4(A, l0 + c.nxy, c.vn) : 0;
+    const int l0 = HF_IX4(A, c.lxy + z * c.nxy, c.n);
+    const int l1 = two ? HF_IX4(A, l0 + c.nxy, c.n) : 0;
     V4<double> x0 = ldv4(XR + l0), x1{}, s0{}, s1{};
     V4<TY> y0{}, y1{};
     V4<float> f0{}, f1{};
     if (use_y) {
-      y0 = ldv4(Y + l0);
+      y0 = ldy(l0);
       if (sizeof(TY) == 8) s0 = ldv4(sinv + l0); else f0 = ldv4(sinv32 + l0);
     }
     if (two) {
       x1 = ldv4(XR + l1);
       if (use_y) {
-        y1 = ldv4(Y + l1);
+        y1 = ldy(l1);
         if (sizeof(TY) == 8) s1 = ldv4(sinv + l1); else f1 = ldv4(sinv32 + l1);
       }
     }
@@ -1061,7 +575,7 @@ __device__ __forceinline__ void xupd4_task(const DevArrays& A, double* part, int
 template <typename TR>
 __device__ __forceinline__ void res_hx4_task(const DevArrays& A, double* part, int64_t task,
                                              const InstScal& s) {
-  const Quad c = quad_cell<false>(A, task);   // rows of 4k cells: the two layouts agree in shape
+  const Quad c = quad_cell(A, task);   // rows of 4k cells: the two layouts agree in shape
   const int64_t off = c.off;
   const double* __restrict__ b = A.b + off;
   const double* __restrict__ yc = A.hx[s.hx_role] + off;
@@ -1070,7 +584,7 @@ __device__ __forceinline__ void res_hx4_task(const DevArrays& A, double* part, i
   const float* __restrict__ sinv32 = A.sinv32 + off;
   const double* __restrict__ sinv = A.sinv + off;
   const bool f32 = sizeof(TR) == 4;
-  TR* R = Vec<TR>::r(A) + (f32 ? A.inst[A.tasks[task].x].off4 : off);
+  TR* R = Vec<TR>::r(A) + A.inst[A.tasks[task].x].off4;
   const float isig = (float)(1.0 / s.sigma);
   const bool tiny = tiny_applies(A, s);       // the residual of x0 + TINY: r(x0) - TINY * H1
   double rr = 0.0, gg64 = 0.0;
@@ -1078,7 +592,7 @@ __device__ __forceinline__ void res_hx4_task(const DevArrays& A, double* part, i
   SqSum rq;                                    // mixed: ||r||^2 off the FP64 pipe
   if (c.act) {
     for (int z = c.za; z < c.zb; ++z) {
-      const int l = HF_IX4(A, c.lxy + z * c.nxy, c.vn);
+      const int l = HF_IX4(A, c.lxy + z * c.nxy, c.n);
       const V4<double> bv = ldv4(b + l), cv = ldv4(yc + l), pv = ldv4(yp + l);
       V4<double> rs{}, s64{};
       V4<float> s32{};
@@ -1116,40 +630,472 @@ __device__ __forceinline__ void res_hx4_task(const DevArrays& A, double* part, i
   }
 }
 
-// Dispatch between the vector and the scalar form of a pass (same choice on every path).  The
-// FP32 vectors are padded to rows of 4k cells, so their passes are always vector passes.
-template <typename T>
-__device__ __forceinline__ void upd_any(const DevArrays& A, double* part, int64_t task, const InstScal& s) {
-  if constexpr (sizeof(T) == 4) upd4_task<T>(A, part, task, s);
-  else if (vec4_ok(A.inst[A.tasks[task].x])) upd4_task<T>(A, part, task, s);
-  else upd_task<T>(A, part, task, s);
-}
-template <typename T>
-__device__ __forceinline__ void cgp_any(const DevArrays& A, double* part, int64_t task, const InstScal& s) {
-  if constexpr (sizeof(T) == 4) cgp4_task<T>(A, part, task, s);
-  else if (vec4_ok(A.inst[A.tasks[task].x])) cgp4_task<T>(A, part, task, s);
-  else cgp_task<T>(A, part, task, s);
-}
+// Dispatch between the vector and the scalar form of the x update (same choice on every path).
 template <typename TY>
 __device__ __forceinline__ void xupd_any(const DevArrays& A, double* part, int64_t task, const InstScal& s) {
   if (vec4_ok(A.inst[A.tasks[task].x])) xupd4_task<TY>(A, part, task, s);
   else xupd_task<TY>(A, part, task, s);
 }
 
-// The FP32 p + SpMV pass of one task (always the vector form: the FP32 layout has rows of 4k).
-template <bool FUSED>
-__device__ __forceinline__ void pq_f32_task(const DevArrays& A, double* part, int64_t task,
-                                            const InstScal& s) {
-  spmv4_task<FUSED>(A, part, task, s);
+// ---- the inner solve's passes ------------------------------------------------------------------
+// An inner CG iteration is two passes over the vectors of type T, each ended by the sum it forms:
+//   pq:   y += alpha p_(k-1), p_k = r + beta p_(k-1), q = Ah p_k, p.q     (9 T per cell)
+//   upd:  r -= alpha q, r.r                                               (3 T per cell)
+// y takes a direction one pass late, where p_(k-1) is read anyway (YEnd adds the last one), and p
+// is formed by the pass that applies Ah to it: 12 T per cell and iteration against 14 with a
+// direction update of its own and y in the second pass, and two grid-wide sums instead of three
+// rounds.  Iteration 0 has p_0 = r and no y.
+//
+// Tasks (InstDesc::cgn of them): a block's thread owns one 16-byte vector (4 FP32 or 2 FP64 cells)
+// of a tile of 2^cqx vectors x kBlock / 2^cqx rows and marches the task's planes along z.  p is
+// formed once per cell, from r and p_(k-1), and shared through shared memory: three planes of the
+// tile, with the cells around it, whose p is formed from their r and p_(k-1) as well (the value that
+// their own tile stores) by threads that take one such vector or cell each.  The operands of the
+// plane after next are loaded into registers while a plane is computed, those beyond the tile into
+// shared memory (cp.async: few threads have any, but registers are the same for all).  The
+// neighbours' p comes from shared memory, so that few registers are live at the same time: spilled,
+// the pass took 1.8 times as long.
+// The rows of the inner solve's layout are padded to 4 cells: in a row's last vector the cells past
+// nx have zero coefficients, and q and r are kept zero there.  A face that does not exist has a
+// zero coefficient or a zero neighbour.
+// Bound by HBM in FP32 and by the FP64 pipe in FP64 (9 instructions per cell).  Measured on the
+// layered slab: 256^3 FP32, pq 115 us (5.2 TB/s) and upd 34 us (5.9 TB/s), where the direction
+// update, the SpMV and the update took 38 + 68 + 75 us; 190 x 192 x 192 FP64, 134 + 31 us against
+// 34 + 111 + 68 us.
+template <typename T>
+struct alignas(16) Vec16 {
+  static constexpr int N = 16 / (int)sizeof(T);
+  T v[N];
+};
+template <typename T>
+__device__ __forceinline__ Vec16<T> ld16(const T* p) {
+  const uint4 u = *reinterpret_cast<const uint4*>(p);
+  return *reinterpret_cast<const Vec16<T>*>(&u);
+}
+template <typename T>
+__device__ __forceinline__ void st16(T* p, const Vec16<T>& v) {
+  *reinterpret_cast<uint4*>(p) = *reinterpret_cast<const uint4*>(&v);
+}
+
+// p of three planes: rows -1..rows of a tile, each of nq vectors with one more at either end (the
+// cell beside the row's first is the last of its vector, the cell beside its last the first of its
+// vector); the y faces of two planes, rows -1..rows-1; the x faces beside the rows' first cells.
+template <typename T>
+struct PqShared {
+  Vec16<T> p[3][340], ay[2][288];
+  Vec16<T> hr[80], hpo[80], hf[80];   // operands of the vectors and cells beyond the tile, by thread
+  T ax[2][32];
+};
+template <typename T>
+constexpr int kPqSmem = (int)sizeof(PqShared<T>);   // (beside at most 11 KB of the kernels' own: below 48 KB)
+static_assert(kBlock == 256 && (8 + 2) * (32 + 2) <= 340 && (16 + 2) * (16 + 2) <= 340 && 8 * (32 + 1) <= 288 &&
+                  16 * (16 + 1) <= 288 && 32 * (8 + 1) <= 288, "tiles of 8, 16 or 32 vectors a row");
+
+__device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+template <typename T>
+__device__ __forceinline__ void cp16(Vec16<T>* dst, const T* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
+template <typename T>
+__device__ __forceinline__ void cp1(T* dst, const T* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_addr(dst)), "l"(src), "n"((int)sizeof(T))
+               : "memory");
+}
+// This thread's copies have arrived.
+__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// Place of a thread in task `local` of the inner solve's passes.
+struct CgPos {
+  int x, y, z0, z1, vx, ry, x0, y0;
+  bool act;
+};
+template <typename T>
+__device__ __forceinline__ CgPos cg_pos(const InstDesc& d, int local) {
+  const int bx = local % d.cgnx, rest = local / d.cgnx, by = rest % d.cgny, bz = rest / d.cgny;
+  CgPos c;
+  c.vx = (int)threadIdx.x & ((1 << d.cqx) - 1);
+  c.ry = (int)threadIdx.x >> d.cqx;
+  c.x0 = (bx << d.cqx) * Vec16<T>::N;
+  c.y0 = by * (kBlock >> d.cqx);
+  c.x = c.x0 + c.vx * Vec16<T>::N;
+  c.y = c.y0 + c.ry;
+  c.z0 = (int)((int64_t)bz * d.nz / d.cgnz);
+  c.z1 = (int)((int64_t)(bz + 1) * d.nz / d.cgnz);
+  c.act = c.x < d.nx && c.y < d.ny;
+  return c;
+}
+
+// off: the instance's first cell (d.off4; a constant 0 where there is one instance keeps the base
+// pointers out of the registers).  pslot: the task's place in the table of partial sums; dyn:
+// kPqSmem<T> bytes of shared memory.
+template <typename T>
+__device__ __forceinline__ void pq_task(const DevArrays& A, const InstDesc& d, int64_t off, int local,
+                                        const InstScal& s, double* pslot, char* dyn) {
+  constexpr int V = Vec16<T>::N;
+  typedef Vec16<T> VT;
+  PqShared<T>& sm = *reinterpret_cast<PqShared<T>*>(dyn);
+  const CgPos c = cg_pos<T>(d, local);
+  const int tid = threadIdx.x, nq = 1 << d.cqx, rows = kBlock >> d.cqx, prow = nq + 2;
+  const int nx = d.nx, ny = d.ny, nz = d.nz, sx = d.sx, nxy = sx * ny, n4 = nxy * nz;
+  const int z0 = c.z0, z1 = c.z1;
+  const bool act = c.act;
+  const int last = min(V - 1, nx - 1 - c.x);   // the vector's last grid cell; cells past it are padding
+  const int64_t k = s.iter;
+  const bool first = k == 0;
+  const T beta = (T)s.beta, alpha = (T)s.alpha;      // alpha: of the previous iteration
+  const T* R = Vec<T>::r(A) + off;
+  const T* Po = Vec<T>::pb(A, k + 1) + off;
+  T* Pn = Vec<T>::pb(A, k) + off;
+  T* Q = Vec<T>::q(A) + off;
+  T* Y = Vec<T>::y(A) + off;
+  const T* __restrict__ ax = Vec<T>::ax(A) + off;
+  const T* __restrict__ ay = Vec<T>::ay(A) + off;
+  const T* __restrict__ az = Vec<T>::az(A) + off;
+  const int lxy = c.y * sx + c.x;
+  const int own = (c.ry + 1) * prow + c.vx + 1, ownay = (c.ry + 1) * nq + c.vx;
+  // the vector or cell beyond the tile that this thread also forms: threads 0..nq-1 the row above
+  // the tile's last one, nq..2nq-1 the row below its first (with that row's y faces), then the
+  // cells beside the first column (with their x faces) and beside the last
+  const int nv = min(nq, (nx - c.x0 + V - 1) / V), nr = min(rows, ny - c.y0);   // vectors, rows in use
+  int hl = -1, hp = 0;                         // its cell in a plane, its place in sm.p
+  bool hvec = true, hc = false;                // a vector; with a face (ay, or ax for a cell)
+  if (tid < 2 * nq) {
+    const int v = tid & (nq - 1), xv = c.x0 + v * V;
+    if (v < nv && ny > 1) {
+      if (tid < nq) {
+        if (c.y0 + nr < ny) hl = (c.y0 + nr) * sx + xv;
+        else if (d.py) hl = xv;
+        hp = (nr + 1) * prow + v + 1;
+      } else {
+        if (c.y0 > 0) hl = (c.y0 - 1) * sx + xv;
+        else if (d.py) hl = (ny - 1) * sx + xv;
+        hp = v + 1;
+        hc = true;
+      }
+    }
+  } else if (tid < 2 * nq + 2 * rows) {
+    const bool west = tid < 2 * nq + rows;
+    const int row = tid - 2 * nq - (west ? 0 : rows);
+    hvec = false;
+    if (row < nr) {
+      const int lr = (c.y0 + row) * sx, xe = c.x0 + nv * V;
+      if (west) {
+        if (c.x0 > 0) hl = lr + c.x0 - 1;
+        else if (d.px && nx > 1) hl = lr + nx - 1;
+        hp = (row + 1) * prow;
+        hc = true;
+      } else {
+        if (xe < nx) hl = lr + xe;
+        else if (d.px && nx > 1) hl = lr;
+        hp = (row + 1) * prow + nv + 1;
+      }
+    }
+  }
+  const VT zero{};
+  auto form = [&](const VT& r, const VT& po) -> VT {
+    VT p;
+#pragma unroll
+    for (int i = 0; i < V; ++i) p.v[i] = first ? r.v[i] : fma(beta, po.v[i], r.v[i]);
+    return p;
+  };
+  auto above = [&](int z) { return z < nz || (d.pz && nz > 1); };   // plane z, or the wrap of z = nz
+  VT r = zero, po = zero, yv = zero;           // of the next plane to form
+  VT cx = zero, cy = zero, cz = zero;          // faces of the plane formed last
+  const bool rdy = act && k > 1;
+  auto load_p = [&](int z) {                  // r, p_(k-1), y and the vector beyond of plane z
+    const int zp = (z < nz ? z : 0) * nxy;
+    if (act) {
+      const int l = HF_IXV(A, lxy + zp, n4, V);
+      r = ld16(R + l);
+      if (!first) po = ld16(Po + l);
+      if (rdy && z < z1) yv = ld16(Y + l);
+    }
+    if (hl >= 0 && z < z1) {
+      if (hvec) {
+        const int l = HF_IXV(A, hl + zp, n4, V);
+        cp16(&sm.hr[tid], R + l);
+        if (!first) cp16(&sm.hpo[tid], Po + l);
+      } else {
+        const int l = HF_IX(A, hl + zp, n4);
+        cp1(&sm.hr[tid].v[0], R + l);
+        if (!first) cp1(&sm.hpo[tid].v[0], Po + l);
+      }
+    }
+  };
+  auto load_c = [&](int z) {                  // the faces of plane z
+    if (act) {
+      const int l = HF_IXV(A, lxy + z * nxy, n4, V);
+      cx = ld16(ax + l);
+      cy = ld16(ay + l);
+      cz = ld16(az + l);
+    }
+    if (hl >= 0 && hc) {
+      if (hvec) cp16(&sm.hf[tid], ay + HF_IXV(A, hl + z * nxy, n4, V));
+      else cp1(&sm.hf[tid].v[0], ax + HF_IX(A, hl + z * nxy, n4));
+    }
+  };
+  // p of plane z into shared memory; the task's own planes are stored, and p_(k-1) goes into y
+  auto put_p = [&](int z, VT* pl) {
+    if (act) {
+      const VT p = above(z) ? form(r, po) : zero;
+      pl[own] = p;
+      if (z < z1) {
+        const int l = HF_IXV(A, lxy + z * nxy, n4, V);
+        st16(Pn + l, p);
+        if (!first) {
+          VT yn;
+#pragma unroll
+          for (int i = 0; i < V; ++i) yn.v[i] = fma(alpha, po.v[i], yv.v[i]);   // y is 0 before p_0
+          st16(Y + l, yn);
+        }
+      }
+    }
+    if (hl >= 0 && z < z1) {
+      if (hvec) {
+        pl[hp] = form(sm.hr[tid], first ? zero : sm.hpo[tid]);
+      } else {
+        const T h = first ? sm.hr[tid].v[0] : fma(beta, sm.hpo[tid].v[0], sm.hr[tid].v[0]);
+        pl[hp].v[hc ? V - 1 : 0] = h;
+      }
+    }
+  };
+  __syncthreads();                            // the block's previous task is done with shared memory
+  load_p(z0);
+  load_c(z0);
+  VT azm = zero, pb = zero;
+  if (act && nz > 1) {                        // the plane below the task
+    int lb = -1;
+    if (z0 > 0) lb = lxy + (z0 - 1) * nxy;
+    else if (d.pz) lb = lxy + (nz - 1) * nxy;
+    if (lb >= 0) {
+      lb = HF_IXV(A, lb, n4, V);
+      pb = form(ld16(R + lb), first ? zero : ld16(Po + lb));
+      azm = ld16(az + lb);
+    }
+  }
+  for (int i = tid; i < 3 * 340; i += kBlock) sm.p[0][i] = zero;
+  for (int i = tid; i < 2 * 288; i += kBlock) sm.ay[0][i] = zero;
+  if (tid < 64) sm.ax[0][tid] = T(0);
+  __syncthreads();
+  sm.p[2][own] = pb;
+  cp_wait();
+  if (hl >= 0 && hc) {                        // the faces beyond the tile of plane z0
+    if (hvec) sm.ay[0][hp - 1] = sm.hf[tid];
+    else sm.ax[0][hp / prow - 1] = sm.hf[tid].v[0];
+  }
+  put_p(z0, sm.p[0]);
+  if (above(z0 + 1)) load_p(z0 + 1);
+  // FP32 sums: per-thread sums of 8 planes, added up, so that no chain is longer than where four
+  // groups of threads marched a quarter of a task's planes each
+  T dot = T(0), dot8 = T(0);
+  VT *pm = sm.p[2], *pc = sm.p[0], *pu = sm.p[1];
+  for (int z = z0; z < z1; ++z) {
+    const int b = (z - z0) & 1;
+    cp_wait();
+    if (hl >= 0 && hc && z > z0) {
+      if (hvec) sm.ay[b][hp - 1] = sm.hf[tid];
+      else sm.ax[b][hp / prow - 1] = sm.hf[tid].v[0];
+    }
+    put_p(z + 1, pu);
+    const VT axv = cx, azv = cz;
+    if (act) sm.ay[b][ownay] = cy;
+    if (z + 1 < z1) {
+      load_c(z + 1);
+      if (above(z + 2)) load_p(z + 2);
+    }
+    __syncthreads();                          // p of planes z and z + 1 and the y faces of z are there
+    T axw = __shfl_up_sync(kFull, axv.v[V - 1], 1);
+    if (c.vx == 0) axw = sm.ax[b][c.ry];
+    if (act) {
+      const VT p = pc[own], pn = pc[own + prow], ps = pc[own - prow], pa = pu[own], pd = pm[own];
+      const VT ayv = sm.ay[b][ownay], ays = sm.ay[b][ownay - nq];
+      const T pw = pc[own - 1].v[V - 1], pe = pc[own + 1].v[0];
+      VT qv;
+#pragma unroll
+      for (int i = 0; i < V; ++i) {
+        const T pi = p.v[i];
+        T acc = pi;
+        acc = fma(axv.v[i], i < last ? p.v[i < V - 1 ? i + 1 : i] : pe, acc);
+        if (i > 0) acc = fma(axv.v[i > 0 ? i - 1 : 0], p.v[i > 0 ? i - 1 : 0], acc);
+        else acc = fma(axw, pw, acc);
+        acc = fma(ayv.v[i], pn.v[i], acc);
+        acc = fma(ays.v[i], ps.v[i], acc);
+        acc = fma(azv.v[i], pa.v[i], acc);
+        acc = fma(azm.v[i], pd.v[i], acc);
+        if (i > last) acc = T(0);             // padding: q stays 0
+        dot8 = fma(pi, acc, dot8);
+        qv.v[i] = acc;
+      }
+      st16(Q + HF_IXV(A, lxy + z * nxy, n4, V), qv);
+    }
+    if (sizeof(T) == 4 && ((z - z0) & 7) == 7) {
+      dot += dot8;
+      dot8 = T(0);
+    }
+    azm = azv;
+    VT* t = pm;
+    pm = pc;
+    pc = pu;
+    pu = t;
+  }
+  dot += dot8;
+  if constexpr (sizeof(T) == 4) {
+    task_store_f(pslot, dot);
+  } else {
+    const double v[1] = {dot};
+    tile_store<1>(pslot, A.pcap, v);
+  }
+}
+
+// r -= alpha q and r.r (and the unscaled ||r||^2 for the reference rule).  The planes are walked
+// downwards: the pass before ended on the task's last ones, which are still in L2.  The iteration
+// predicted to end the inner solve also forms x_new = x + sigma S^-1 y (rows of 4k cells: both
+// layouts index alike).
+// WEIGHTED is a form of its own: as a condition in the loop its FP64 instructions, predicated off,
+// took the FP64 pipe all the same (ncu: pipe 72 % busy for 2 FMAs per cell).
+template <typename T, bool WEIGHTED>
+__device__ __forceinline__ void upd_form(const DevArrays& A, const InstDesc& d, int local, const InstScal& s,
+                                         double* pslot) {
+  constexpr int V = Vec16<T>::N;
+  typedef Vec16<T> VT;
+  const CgPos c = cg_pos<T>(d, local);
+  const T alpha = (T)s.alpha;
+  const int nxy = d.sx * d.ny, n4 = nxy * d.nz, lxy = c.y * d.sx + c.x;
+  const int last = min(V - 1, d.nx - 1 - c.x);
+  T* R = Vec<T>::r(A) + d.off4;
+  const T* Q = Vec<T>::q(A) + d.off4;
+  T rr = T(0), rr8 = T(0);
+  double rw = 0.0;
+  if (!WEIGHTED && c.act && (s.xw & kXwThis)) {   // (never under the reference's rule)
+    const bool first = s.iter == 0;
+    const T* P = Vec<T>::pb(A, s.iter) + d.off4;
+    const T* Y = Vec<T>::y(A) + d.off4;
+    const double* XR = A.tbuf[s.role[2]] + d.off;
+    double* XW = A.tbuf[s.role[3]] + d.off;
+    const double* __restrict__ sinv = A.sinv + d.off;
+    const float* __restrict__ sinv32 = A.sinv32 + d.off;
+    const float sig = (float)s.sigma_prev;
+    for (int z = c.z1 - 1; z >= c.z0; --z) {
+      const int l = HF_IXV(A, lxy + z * nxy, n4, V);
+      const VT qv = ld16(Q + l), pv = ld16(P + l);
+      VT rv = ld16(R + l), yv{};
+      if (!first) yv = ld16(Y + l);
+      double xv[V], sv[V];
+#pragma unroll
+      for (int i = 0; i < V; i += 2) {
+        const double2 t = *reinterpret_cast<const double2*>(XR + l + i);
+        xv[i] = t.x;
+        xv[i + 1] = t.y;
+      }
+      if constexpr (sizeof(T) == 8) {
+        const double2 t = *reinterpret_cast<const double2*>(sinv + l);
+        sv[0] = t.x;
+        sv[1] = t.y;
+      }
+      VT fv{};
+      if constexpr (sizeof(T) == 4) fv = ld16(sinv32 + l);
+#pragma unroll
+      for (int i = 0; i < V; ++i) {
+        const T yo = fma(alpha, pv.v[i], yv.v[i]);
+        rv.v[i] = fma(-alpha, qv.v[i], rv.v[i]);
+        rr8 = fma(rv.v[i], rv.v[i], rr8);
+        if constexpr (sizeof(T) == 8) xv[i] = fma(sv[i], yo, xv[i]);
+        else xv[i] = xv[i] + f32_to_f64(sig * fv.v[i] * yo);
+      }
+      st16(R + l, rv);
+#pragma unroll
+      for (int i = 0; i < V; i += 2) *reinterpret_cast<double2*>(XW + l + i) = make_double2(xv[i], xv[i + 1]);
+      if (sizeof(T) == 4 && ((c.z1 - 1 - z) & 7) == 7) {
+        rr += rr8;
+        rr8 = T(0);
+      }
+    }
+  } else if (c.act) {
+    // U planes of loads are in flight while the U before are computed
+    constexpr int U = 4;
+    VT qn[U], rn[U];
+    auto load = [&](int zt) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (zt - u < c.z0) continue;
+        const int l = HF_IXV(A, lxy + (zt - u) * nxy, n4, V);
+        qn[u] = ld16(Q + l);
+        rn[u] = ld16(R + l);
+      }
+    };
+    load(c.z1 - 1);
+    for (int zt = c.z1 - 1; zt >= c.z0; zt -= U) {
+      VT qv[U], rv[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        qv[u] = qn[u];
+        rv[u] = rn[u];
+      }
+      load(zt - U);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int z = zt - u;
+        if (z < c.z0) continue;
+#pragma unroll
+        for (int i = 0; i < V; ++i) {
+          T r = fma(-alpha, qv[u].v[i], rv[u].v[i]);
+          if (i > last) r = T(0);
+          rv[u].v[i] = r;
+          rr8 = fma(r, r, rr8);
+          if (WEIGHTED && i <= last) {
+            const double dg = A.diag[d.off + HF_IX(A, (z * d.ny + c.y) * d.nx + c.x + i, d.nx * d.ny * d.nz)];
+            rw = fma(-dg * (double)r, (double)r, rw);
+          }
+        }
+        st16(R + HF_IXV(A, lxy + z * nxy, n4, V), rv[u]);
+        if (sizeof(T) == 4 && ((c.z1 - 1 - z) & 7) == 7) {
+          rr += rr8;
+          rr8 = T(0);
+        }
+      }
+    }
+  }
+  rr += rr8;
+  if constexpr (sizeof(T) == 4) {
+    task_store_f(pslot, rr);
+  } else if constexpr (WEIGHTED) {
+    const double v[2] = {rr, rw};
+    tile_store<2>(pslot, A.pcap, v);
+  } else {
+    const double v[1] = {rr};
+    tile_store<1>(pslot, A.pcap, v);
+  }
+}
+template <typename T>
+__device__ __forceinline__ void upd_task(const DevArrays& A, const InstDesc& d, int local, const InstScal& s,
+                                         double* pslot) {
+  if (sizeof(T) == 8 && A.opts.criterion == HF_STOP_RECURSIVE) upd_form<T, sizeof(T) == 8>(A, d, local, s, pslot);
+  else upd_form<T, false>(A, d, local, s, pslot);
 }
 
 // ---- standalone kernels (host-polled loop, conditional-node graph, kernel timing) --------------
-template <bool INIT, typename TR>
-__global__ void __launch_bounds__(kBlock) k_residual(DevArrays A) {
+// A round of the split solve in its log (one thread).
+__device__ __forceinline__ void log_round(SolveCtl* ctl, int32_t phase) {
+  const int64_t r = ctl->rounds;
+  if (r < kRoundLog) {
+    ctl->phase_log[r] = phase;
+    ctl->t_round[r] = gtimer();
+  }
+  ctl->rounds = r + 1;
+}
+
+// log: the split solve's sweeps note their start (the first) and the end of the x update before them.
+template <bool INIT, typename TR, bool XOUT = false>
+__global__ void __launch_bounds__(kBlock) k_residual(DevArrays A, int log) {
+  if (log && blockIdx.x == 0 && threadIdx.x == 0) {
+    if (INIT) A.stamps[kStampSolve] = A.sctl->t_start = gtimer();
+    else if (A.scal[0].outer_active && !A.scal[0].inner_active && !(A.scal[0].xw & kXwDone))
+      log_round(A.sctl, HF_PHASE_XUPD);
+  }
   const InstScal& s = A.scal[A.tasks[blockIdx.x].x];
   if (!s.outer_active || s.inner_active) return;
   if (INIT != (s.refine == 0)) return;
-  res_task<INIT, TR>(A, A.partials, blockIdx.x, s);
+  res_task<INIT, TR, XOUT>(A, A.partials, blockIdx.x, s);
 }
 
 template <typename TY>
@@ -1160,32 +1106,22 @@ __global__ void __launch_bounds__(kBlock) k_xupdate(DevArrays A) {
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kBlock) k_cg_p(DevArrays A) {
-  const InstScal& s = A.scal[A.tasks[blockIdx.x].x];
-  if (!s.inner_active || s.iter == 0) return;   // p_0 = r: the SpMV and the update read r
-  cgp_any<T>(A, A.partials, blockIdx.x, s);
-}
-
-template <typename T>
-__global__ void __launch_bounds__(kBlock) k_cg_spmv(DevArrays A) {
-  const InstScal& s = A.scal[A.tasks[blockIdx.x].x];
+__global__ void __launch_bounds__(kBlock) k_cg_pq(DevArrays A) {
+  extern __shared__ __align__(16) char dyn[];
+  const int inst = A.cg_inst[blockIdx.x];
+  const InstScal& s = A.scal[inst];
   if (!s.inner_active) return;
-  if constexpr (sizeof(T) == 4) pq_f32_task<false>(A, A.partials, blockIdx.x, s);
-  else spmv_task<T, false>(A, A.partials, blockIdx.x, s);
-}
-
-// The persistent solve's fused FP32 pass on its own (timing and profiling).
-__global__ void __launch_bounds__(kBlock) k_cg_pq_f32(DevArrays A) {
-  const InstScal& s = A.scal[A.tasks[blockIdx.x].x];
-  if (!s.inner_active) return;
-  pq_f32_task<true>(A, A.partials, blockIdx.x, s);
+  const InstDesc& d = A.inst[inst];
+  pq_task<T>(A, d, d.off4, (int)(blockIdx.x - d.cg0), s, A.partials + blockIdx.x, dyn);
 }
 
 template <typename T>
 __global__ void __launch_bounds__(kBlock) k_cg_upd(DevArrays A) {
-  const InstScal& s = A.scal[A.tasks[blockIdx.x].x];
+  const int inst = A.cg_inst[blockIdx.x];
+  const InstScal& s = A.scal[inst];
   if (!s.inner_active) return;
-  upd_any<T>(A, A.partials, blockIdx.x, s);
+  const InstDesc& d = A.inst[inst];
+  upd_task<T>(A, d, (int)(blockIdx.x - d.cg0), s, A.partials + blockIdx.x);
 }
 
 // ---- summation of an instance's task partials ------------------------------------------------
@@ -1217,11 +1153,11 @@ __device__ __forceinline__ void strided_sum(const double* part, int64_t stride, 
 
 // Block-uniform call (all threads of the block); red: NRV * kBlock values of shared memory.
 template <int NRV>
-__device__ __forceinline__ void instance_sum(const double* part, int64_t stride, const InstDesc& d,
-                                             double (&acc)[NRV], double* red) {
+__device__ __forceinline__ void instance_sum(const double* part, int64_t stride, int64_t task0,
+                                             int64_t ntask, double (&acc)[NRV], double* red) {
 #pragma unroll
   for (int k = 0; k < NRV; ++k) acc[k] = 0.0;
-  strided_sum<NRV>(part, stride, d.task0, d.ntask, threadIdx.x, acc);
+  strided_sum<NRV>(part, stride, task0, ntask, threadIdx.x, acc);
 #pragma unroll
   for (int k = 0; k < NRV; ++k) red[k * kBlock + threadIdx.x] = acc[k];
   __syncthreads();
@@ -1313,6 +1249,7 @@ __device__ void epi_residual_s(InstScal& s, const InstDesc& G, const DevOpts& o,
     return;
   }
   s.iter = 0;
+  s.ypend = 0;
   if (o.criterion != HF_STOP_RECURSIVE && converged) {   // only the +TINY is left to apply
     s.inner_active = 0;
     return;
@@ -1340,6 +1277,7 @@ __device__ void epi_residual_s(InstScal& s, const InstDesc& G, const DevOpts& o,
 
 __device__ void epi_spmv_s(InstScal& s, const double* tot) {
   s.pq = tot[0];
+  s.ypend = 0;                           // the pass took the previous direction into y
   if (tot[0] > 0.0 && isfinite(tot[0])) {
     s.alpha = s.rho / tot[0];
   } else {            // breakdown (p = 0 or non-finite): stop this inner solve
@@ -1356,6 +1294,7 @@ __device__ void epi_upd_s(InstScal& s, const DevOpts& o, const double* tot) {
   s.beta = rho_new / s.rho;
   s.rho = rho_new;
   s.iter += 1;
+  s.ypend = 1;
   s.step_iters += 1;
   if (sizeof(T) == 8) s.tot_iters += 1; else s.tot_inner += 1;
   bool stop;
@@ -1416,10 +1355,16 @@ __global__ void __launch_bounds__(kBlock) k_finalize(DevArrays A, CtrlState* ctr
   const int inst = blockIdx.x;
   if (KIND == FIN_RHS && inst == 0 && threadIdx.x == 0) A.stamps[kStampFin] = gtimer();
   const InstDesc& d = A.inst[inst];
+  if (graph == 2 && inst == 0 && threadIdx.x == 0 && took_part<KIND>(A.scal[0])) {
+    log_round(A.sctl, KIND == FIN_RES ? (int32_t)HF_PHASE_RES
+                                      : A.scal[0].hx_ok >= 2 ? (int32_t)HF_PHASE_RES_INIT_HX : (int32_t)HF_PHASE_RES_INIT);
+    A.stamps[kStampSolveEnd] = gtimer();
+  }
   if (took_part<KIND>(A.scal[inst])) {
     double acc[NR];
     __shared__ double red[kBlock * NR];
-    instance_sum<NR>(A.partials, A.pcap, d, acc, red);
+    constexpr bool cg = KIND == FIN_SPMV || KIND == FIN_UPD;
+    instance_sum<NR>(A.partials, A.pcap, cg ? d.cg0 : d.task0, cg ? d.cgn : d.ntask, acc, red);
     if (threadIdx.x == 0) {
       switch (KIND) {
         case FIN_RHS: epi_rhs(A, inst, acc); break;
@@ -1447,6 +1392,11 @@ __global__ void __launch_bounds__(kBlock) k_finalize(DevArrays A, CtrlState* ctr
       int any_outer = 0;
       for (int64_t i = 0; i < A.ninst; ++i) any_outer |= __ldcg(&A.scal[i].outer_active);
       ctrl->fin_count = 0u;
+      if (graph == 2) {
+        // a split solve's kernel that gave up leaves its instance as it was: the loop ends there
+        if (A.sctl->err || A.sctl->guard_hit) any_outer = 0;
+        ctrl->launches += KIND == FIN_RES ? 4 : 0;
+      }
       cudaGraphSetConditional(hw, any_outer ? 1u : 0u);
     }
   }
@@ -1497,7 +1447,7 @@ __global__ void k_ctrl_select(DevArrays A, CtrlState* ctrl, cudaGraphConditional
     ctrl->guard_hit = 1;
     branch = 2u;
   }
-  ctrl->launches += 1 + (branch == 0u ? 5 : (branch == 1u ? 3 : 0));
+  ctrl->launches += 1 + (branch == 0u ? 4 : (branch == 1u ? 3 : 0));
   if (branch == 2u) cudaGraphSetConditional(hw, 0u);
   cudaGraphSetConditional(hs, branch);
 }
@@ -1536,13 +1486,21 @@ __device__ __forceinline__ void red_release_add_u64(unsigned long long* p, unsig
 template <typename T>
 __device__ __forceinline__ int32_t phase_after(const InstScal& s) {
   if (!s.outer_active) return PH_IDLE;
-  // the fused FP32 pass (PH_CG_PQ) measured slower; iteration 0 needs no direction update (p_0 = r)
-  if (s.inner_active) return s.iter == 0 ? PH_CG_Q : PH_CG_P;
+  if (s.inner_active) return PH_CG_PQ;
   return (s.xw & kXwDone) ? PH_RES : PH_XUPD;   // the last CG update may have formed x already
 }
 __device__ __forceinline__ int phase_partials(int32_t ph) {
   return (ph == PH_RES_INIT || ph == PH_RES || ph == PH_CG_B) ? 2
-         : ((ph == PH_CG_Q || ph == PH_CG_PQ) ? 1 : 0);
+         : (ph == PH_CG_PQ ? 1 : 0);
+}
+// The tasks of a phase: the inner solve's passes have their own (InstDesc::cgn), all others the
+// cell tasks.
+__device__ __forceinline__ bool cg_phase(int32_t ph) { return ph == PH_CG_PQ || ph == PH_CG_B; }
+__device__ __forceinline__ unsigned phase_ntask(const InstDesc& d, int32_t ph) {
+  return (unsigned)(cg_phase(ph) ? d.cgn : d.ntask);
+}
+__device__ __forceinline__ int64_t phase_task0(const InstDesc& d, int32_t ph) {
+  return cg_phase(ph) ? d.cg0 : d.task0;
 }
 
 constexpr int kScalWords = (int)(sizeof(InstScal) / 8);
@@ -1562,8 +1520,6 @@ __device__ __noinline__ void phase_epilogue(InstScal& sc, const InstDesc& d, con
       epi_residual_s<false>(sc, d, o, acc);
       sc.phase = phase_after<T>(sc);
       break;
-    case PH_CG_P: sc.phase = PH_CG_Q; break;
-    case PH_CG_Q:
     case PH_CG_PQ:
       epi_spmv_s(sc, acc);
       sc.phase = sc.inner_active ? PH_CG_B : phase_after<T>(sc);
@@ -1577,26 +1533,20 @@ __device__ __noinline__ void phase_epilogue(InstScal& sc, const InstDesc& d, con
   }
 }
 
-template <typename T, bool XOUT>
-__device__ __forceinline__ void round_task(const DevArrays& A, double* part, int64_t task,
-                                           const InstScal& s) {
-  if constexpr (sizeof(T) == 4) {
-    if (s.phase == PH_CG_PQ || s.phase == PH_CG_Q) {
-      if (s.phase == PH_CG_PQ) pq_f32_task<true>(A, part, task, s);
-      else pq_f32_task<false>(A, part, task, s);
-      return;
+// Task `local` of an instance's current phase.
+template <typename T, bool XOUT, bool FULL, bool WEIGHTED>
+__device__ __forceinline__ void round_task(const DevArrays& A, const InstDesc& d, double* part, int local,
+                                           const InstScal& s, char* dyn) {
+  if (s.phase == PH_CG_PQ) pq_task<T>(A, d, d.off4, local, s, part + d.cg0 + local, dyn);
+  else if (s.phase == PH_CG_B) upd_form<T, WEIGHTED>(A, d, local, s, part + d.cg0 + local);
+  if constexpr (FULL) {
+    const int64_t task = d.task0 + local;
+    switch (s.phase) {
+      case PH_RES_INIT: res_task<true, T>(A, part, task, s); break;
+      case PH_RES: res_task<false, T, XOUT>(A, part, task, s); break;
+      case PH_XUPD: xupd_any<T>(A, part, task, s); break;
+      default: break;
     }
-  } else {
-    if (s.phase == PH_CG_Q) { spmv_task<T, false>(A, part, task, s); return; }
-    if (s.phase == PH_CG_PQ) { spmv_task<T, true>(A, part, task, s); return; }
-  }
-  switch (s.phase) {
-    case PH_RES_INIT: res_task<true, T>(A, part, task, s); break;
-    case PH_RES: res_task<false, T, XOUT>(A, part, task, s); break;
-    case PH_CG_P: cgp_any<T>(A, part, task, s); break;
-    case PH_CG_B: upd_any<T>(A, part, task, s); break;
-    case PH_XUPD: xupd_any<T>(A, part, task, s); break;
-    default: break;
   }
 }
 
@@ -1626,18 +1576,20 @@ __device__ __forceinline__ int32_t logged_phase(const InstScal& s) {
 // XOUT: the instance used by the graphs of host-buffer steps, whose residual sweeps also store x
 // into A.xout (a variant of its own, so the other solves carry none of it).
 constexpr int kSlotShift = 24;      // slot: first ticket << 24 | tasks << 1 | walk the tasks backwards
-template <typename T, bool XOUT>
-__global__ void __launch_bounds__(kBlock, 3)
+template <typename T, bool XOUT, bool FULL, bool WEIGHTED>
+__global__ void __launch_bounds__(kBlock, 2)
     k_solve_batch(DevArrays A, SolveCtl* ctl, int64_t limit, unsigned long long wait_ns, int leaver) {
   __shared__ InstScal sh;
   __shared__ double red[kBlock * 2];
   __shared__ unsigned long long s_ticket, s_slot;
   __shared__ int s_inst, s_last, s_stop;
+  extern __shared__ __align__(16) char dyn[];
   const int ninst = (int)A.ninst;
-  const unsigned long long first = (unsigned long long)A.ntasks;
+  // the first phase's tickets: all instances' cell tasks, or those of the inner solve's passes
+  const unsigned long long first = (unsigned long long)(FULL ? A.ntasks : A.ncg);
   unsigned long long* slots = solve_slots(ctl);
   unsigned* done = solve_done(ctl, A.ninst);
-  if (blockIdx.x == 0 && threadIdx.x == 0) A.stamps[kStampSolve] = ctl->t_start = gtimer();
+  if (FULL && blockIdx.x == 0 && threadIdx.x == 0) A.stamps[kStampSolve] = ctl->t_start = gtimer();
   if (threadIdx.x == 0) s_ticket = atomicAdd(&ctl->ticket, 1ull);
   // failure-path check only (leaver >= 0): that block leaves with a ticket, so its instance never
   // finishes and the others' waits run out and record SolveCtl::err
@@ -1649,9 +1601,9 @@ __global__ void __launch_bounds__(kBlock, 3)
     unsigned n = 0, local = 0;
     bool back = false;
     if (t < first) {
-      inst = A.tasks[t].x;
-      local = (unsigned)(t - (unsigned long long)A.inst[inst].task0);
-      n = (unsigned)A.inst[inst].ntask;
+      inst = FULL ? A.tasks[t].x : A.cg_inst[t];
+      local = (unsigned)(t - (unsigned long long)(FULL ? A.inst[inst].task0 : A.inst[inst].cg0));
+      n = (unsigned)(FULL ? A.inst[inst].ntask : A.inst[inst].cgn);
       __syncthreads();                       // every thread has read s_ticket
     } else {
       unsigned long long t0 = 0;
@@ -1697,8 +1649,15 @@ __global__ void __launch_bounds__(kBlock, 3)
           __ldcg(reinterpret_cast<const unsigned long long*>(A.scal + inst) + threadIdx.x);
     if (threadIdx.x == kBlock - 1) s_ticket = atomicAdd(&ctl->ticket, 1ull);   // the block's next one
     __syncthreads();
+    if (!FULL && t < first) {                // the inner solves that are due
+      if (threadIdx.x == 0) sh.phase = sh.inner_active ? PH_CG_PQ : PH_IDLE;
+      __syncthreads();
+    }
     const int32_t ph = sh.phase;             // read before any thread can run the epilogue
-    round_task<T, XOUT>(A, A.partials, d.task0 + (back ? n - 1 - local : local), sh);
+    // the two kinds of tasks are numbered apart, and instances in phases of either kind run at once:
+    // the inner solve's passes use the second table of partial sums
+    double* part = A.partials + (cg_phase(ph) ? kNR * A.pcap : 0);
+    round_task<T, XOUT, FULL, WEIGHTED>(A, d, part, (int)(back ? n - 1 - local : local), sh, dyn);
     __syncthreads();
     if (threadIdx.x == 0) {
       __threadfence();
@@ -1708,16 +1667,9 @@ __global__ void __launch_bounds__(kBlock, 3)
     __syncthreads();
     if (!s_last) continue;
     double acc[2] = {0.0, 0.0};
-    if (phase_partials(ph) > 0) instance_sum<2>(A.partials, A.pcap, d, acc, red);
+    if (phase_partials(ph) > 0) instance_sum<2>(part, A.pcap, phase_task0(d, ph), n, acc, red);
     if (threadIdx.x == 0) {
-      if (inst == 0) {
-        const int64_t r = ctl->rounds;
-        if (r < kRoundLog) {
-          ctl->phase_log[r] = logged_phase(sh);
-          ctl->t_round[r] = gtimer();
-        }
-        ctl->rounds = r + 1;
-      }
+      if (inst == 0 && ph != PH_IDLE) log_round(ctl, logged_phase(sh));
       if (ph != PH_IDLE) phase_epilogue<T>(sh, d, A.opts, acc);
     }
     __syncthreads();
@@ -1728,13 +1680,13 @@ __global__ void __launch_bounds__(kBlock, 3)
     if (threadIdx.x == 0) {
       done[inst] = 0u;
       __threadfence();
-      if (sh.phase == PH_IDLE) {
+      if (FULL ? sh.phase == PH_IDLE : !cg_phase(sh.phase)) {
         A.stamps[kStampSolveEnd] = gtimer();
         atomicAdd(&ctl->finished, 1u);
       } else if (atomicAdd(&ctl->phases, 1ull) >= (unsigned long long)limit * (unsigned long long)ninst) {
         atomicExch(&ctl->guard_hit, 1);
       } else {
-        const unsigned long long m = (unsigned long long)d.ntask;
+        const unsigned long long m = phase_ntask(d, sh.phase);
         const unsigned long long s0 = first + atomicAdd(&ctl->tail, m);
         st_release_u64(slots + inst, s0 << kSlotShift | m << 1 | (back ? 0ull : 1ull));
       }
@@ -1758,40 +1710,45 @@ __global__ void __launch_bounds__(kBlock, 3)
 // r + 2, which every block has left behind and none has reached).
 // Measured: the layered slab at 64^3, mixed, 20 steps 11.7 -> 6.1 ms; a 25 x 25 x 1 grid under the
 // reference's rule, 10 steps 17.3 -> 9.1 ms; 128^3 1.17 times as fast, 256^3 1.03 times.
-template <typename T, bool XOUT>
-__global__ void __launch_bounds__(kBlock, 3)
+// WEIGHTED: the reference's stopping rule (upd_form).
+template <typename T, bool WEIGHTED>
+__global__ void __launch_bounds__(kBlock, 2)
     k_solve_one(DevArrays A, SolveCtl* ctl, int64_t limit, unsigned long long wait_ns, int leaver) {
   __shared__ InstScal sh;
   __shared__ InstDesc sd;
   __shared__ double red[kBlock * 2];
   __shared__ unsigned s_next;
   __shared__ int s_ok;
+  extern __shared__ __align__(16) char dyn[];
   static_assert(sizeof(InstDesc) % 8 == 0 && sizeof(InstDesc) / 8 <= kBlock, "descriptor copy");
   const unsigned G = gridDim.x;
-  const unsigned nt = (unsigned)A.ntasks;
-  const bool hand_out = nt > G;
   if ((int)threadIdx.x < kScalWords)
     reinterpret_cast<unsigned long long*>(&sh)[threadIdx.x] =
         reinterpret_cast<const unsigned long long*>(A.scal)[threadIdx.x];
   if (threadIdx.x < sizeof(InstDesc) / 8)
     reinterpret_cast<unsigned long long*>(&sd)[threadIdx.x] =
         reinterpret_cast<const unsigned long long*>(A.inst)[threadIdx.x];
-  if (blockIdx.x == 0 && threadIdx.x == 0) A.stamps[kStampSolve] = ctl->t_start = gtimer();
+  __syncthreads();
+  if (!sh.inner_active) return;              // no inner solve is due
+  __syncthreads();
+  if (threadIdx.x == 0) sh.phase = PH_CG_PQ;
   __syncthreads();
   int64_t r = 0;
-  for (; sh.phase != PH_IDLE; ++r) {
+  for (; cg_phase(sh.phase); ++r) {
     if (r >= limit) {
       if (blockIdx.x == 0 && threadIdx.x == 0) ctl->guard_hit = 1;
       break;
     }
-    // odd rounds walk the tasks backwards, so a round starts on the data the previous round wrote
+    // odd rounds hand the tasks out backwards, so a round starts on the data the previous round wrote
     // last, which is still in L2 (the partial sums have fixed slots: the order changes no bits)
     double* part = A.partials + (r & 1) * (kNR * A.pcap);
     const int32_t ph = sh.phase;             // read before any thread can run the epilogue
+    const unsigned nt = (unsigned)sd.cgn;
+    const bool hand_out = nt > G;
     unsigned k = blockIdx.x;
+    if (blockIdx.x == 0 && threadIdx.x == 32) ctl->next_task[(r + 2) & 3] = 0u;
     if (hand_out) {
       if (threadIdx.x == 0) s_next = atomicAdd(&ctl->next_task[r & 3], 1u);
-      if (blockIdx.x == 0 && threadIdx.x == 32) ctl->next_task[(r + 2) & 3] = 0u;
       __syncthreads();
       k = s_next;
     }
@@ -1800,7 +1757,9 @@ __global__ void __launch_bounds__(kBlock, 3)
         __syncthreads();                     // every thread has read s_next
         if (threadIdx.x == 0) s_next = atomicAdd(&ctl->next_task[r & 3], 1u);
       }
-      round_task<T, XOUT>(A, part, (r & 1) ? nt - 1 - k : k, sh);
+      const int local = (int)(hand_out && (r & 1) ? nt - 1 - k : k);
+      if (ph == PH_CG_PQ) pq_task<T>(A, sd, 0, local, sh, part + local, dyn);
+      else upd_form<T, WEIGHTED>(A, sd, local, sh, part + local);
       if (!hand_out) break;
       __syncthreads();                       // s_next holds the block's next task
       k = s_next;
@@ -1810,8 +1769,7 @@ __global__ void __launch_bounds__(kBlock, 3)
     if ((int)blockIdx.x == leaver) return;
     __syncthreads();                         // the block's work is done
     if (threadIdx.x == 0) {
-      __threadfence();
-      red_release_add_u64(&ctl->arrived, 1ull);
+      red_release_add_u64(&ctl->arrived, 1ull);   // releases what the block wrote before the barrier
       const unsigned long long want = (unsigned long long)G * (unsigned long long)(r + 1);
       int ok = 1;
       unsigned long long t0 = 0;
@@ -1829,18 +1787,14 @@ __global__ void __launch_bounds__(kBlock, 3)
         }
         __nanosleep(32);
       }
-      __threadfence();
       s_ok = ok;
     }
     __syncthreads();
     if (!s_ok) return;
     double acc[2] = {0.0, 0.0};
-    if (phase_partials(ph) > 0) instance_sum<2>(part, A.pcap, sd, acc, red);
+    if (phase_partials(ph) > 0) instance_sum<2>(part, A.pcap, 0, nt, acc, red);
     if (threadIdx.x == 0) {
-      if (blockIdx.x == 0 && r < kRoundLog) {
-        ctl->phase_log[r] = logged_phase(sh);
-        ctl->t_round[r] = gtimer();
-      }
+      if (blockIdx.x == 0) log_round(ctl, logged_phase(sh));
       phase_epilogue<T>(sh, sd, A.opts, acc);
     }
     __syncthreads();
@@ -1849,63 +1803,67 @@ __global__ void __launch_bounds__(kBlock, 3)
   if ((int)threadIdx.x < kScalWords)
     reinterpret_cast<unsigned long long*>(A.scal)[threadIdx.x] =
         reinterpret_cast<const unsigned long long*>(&sh)[threadIdx.x];
-  if (threadIdx.x == 0) {
-    A.stamps[kStampSolveEnd] = gtimer();
-    ctl->rounds = r;
-  }
+  if (threadIdx.x == 0) A.stamps[kStampSolveEnd] = gtimer();
 }
 
 typedef void (*SolveKernel)(DevArrays, SolveCtl*, int64_t, unsigned long long, int);
-static SolveKernel solve_kernel(const Ctx& c, int fp32, bool xout) {
-  if (c.ninst == 1) {
-    if (fp32) return xout ? k_solve_one<float, true> : k_solve_one<float, false>;
-    return xout ? k_solve_one<double, true> : k_solve_one<double, false>;
-  }
-  if (fp32) return xout ? k_solve_batch<float, true> : k_solve_batch<float, false>;
-  return xout ? k_solve_batch<double, true> : k_solve_batch<double, false>;
+template <typename T, bool FULL, bool WEIGHTED>
+static SolveKernel solve_kernel_of(const Ctx& c, bool xout) {
+  if (c.ninst == 1) return k_solve_one<T, WEIGHTED>;
+  return FULL && xout ? k_solve_batch<T, FULL, FULL, WEIGHTED> : k_solve_batch<T, false, FULL, WEIGHTED>;
+}
+static SolveKernel solve_kernel(const Ctx& c, int fp32, bool xout, bool full) {
+  if (fp32) return full ? solve_kernel_of<float, true, false>(c, xout) : solve_kernel_of<float, false, false>(c, xout);
+  if (c.opts.criterion == HF_STOP_RECURSIVE)
+    return full ? solve_kernel_of<double, true, true>(c, xout) : solve_kernel_of<double, false, true>(c, xout);
+  return full ? solve_kernel_of<double, true, false>(c, xout) : solve_kernel_of<double, false, false>(c, xout);
 }
 
 // Largest co-resident grid of the persistent solve (cooperative launch bound), capped by tasks.
-int solve_grid_blocks(Ctx& c, int fp32) {
-  int& cached = c.solve_blocks[fp32 ? 1 : 0];
+int solve_grid_blocks(Ctx& c, int fp32, bool full) {
+  int& cached = c.solve_blocks[full ? 1 : 0][fp32 ? 1 : 0];
   if (cached > 0) return cached;
-  int per_sm = 0, per_sm_x = 0, nsm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, solve_kernel(c, fp32, false), kBlock, 0) !=
-          cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_x, solve_kernel(c, fp32, true), kBlock, 0) !=
-          cudaSuccess)
-    return -1;
-  if (per_sm_x < per_sm) per_sm = per_sm_x;    // one grid size for both variants
+  int per_sm = INT_MAX, nsm = 0;
+  const int smem = fp32 ? kPqSmem<float> : kPqSmem<double>;
+  for (bool x : {false, true}) {               // one grid size for both variants
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, solve_kernel(c, fp32, x, full), kBlock, smem) != cudaSuccess)
+      return -1;
+    per_sm = std::min(per_sm, n);
+  }
   if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c.device) != cudaSuccess) return -1;
   // every SM holds the same number of blocks; tasks are handed out one at a time, so the blocks
   // of busier SMs take fewer of them
   int64_t g = (int64_t)per_sm * nsm;
-  if (g > c.ntasks) g = c.ntasks;
+  g = std::min(g, full ? std::max(c.ntasks, c.ncg) : c.ncg);
   if (g < 1) return -1;
   cached = (int)g;
   return cached;
 }
 
-// Zero the control block, then launch the persistent solve cooperatively on the context stream.
-cudaError_t launch_solve(Ctx& c, unsigned long long wait_ns, int leaver) {
+// Zero the control block (its counters: full = false), then launch the persistent solve cooperatively
+// on the context stream.
+cudaError_t launch_solve(Ctx& c, bool full, unsigned long long wait_ns, int leaver) {
   const bool fp32 = c.opts.precision == HF_PREC_MIXED;
-  const int g = solve_grid_blocks(c, fp32 ? 1 : 0);
+  const int g = solve_grid_blocks(c, fp32 ? 1 : 0, full);
   if (g < 1) return cudaErrorInvalidConfiguration;
-  cudaError_t e = cudaMemsetAsync(c.d_sctl, 0, solve_ctl_bytes(c.ninst), c.stream);
+  const size_t skip = full ? 0 : offsetof(SolveCtl, arrived);
+  cudaError_t e = cudaMemsetAsync(reinterpret_cast<char*>(c.d_sctl) + skip, 0, solve_ctl_bytes(c.ninst) - skip,
+                                  c.stream);
   if (e != cudaSuccess) return e;
   const int64_t per = fp32 ? c.opts.inner_itmax : c.opts.itmax;
-  const int64_t limit = (int64_t)(c.opts.max_refine + 3) * (3 * per + 6) + 8;
+  const int64_t limit = (int64_t)(c.opts.max_refine + 3) * (2 * per + 6) + 8;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)g);
   cfg.blockDim = dim3(kBlock);
-  cfg.dynamicSmemBytes = 0;
+  cfg.dynamicSmemBytes = fp32 ? kPqSmem<float> : kPqSmem<double>;
   cfg.stream = c.stream;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeCooperative;
   at[0].val.cooperative = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, solve_kernel(c, fp32 ? 1 : 0, c.A.xout != nullptr), c.A, c.d_sctl, limit,
+  return cudaLaunchKernelEx(&cfg, solve_kernel(c, fp32 ? 1 : 0, c.A.xout != nullptr, full), c.A, c.d_sctl, limit,
                             wait_ns, leaver);
 }
 
@@ -1931,36 +1889,35 @@ cudaError_t launch_step_end(Ctx& c) {
 }
 
 // mode 0: initial residual (+ finalize); mode 1: solution update + residual (+ finalize)
+template <typename T>
+static void launch_res(Ctx& c, int mode, int log) {
+  const unsigned nb = (unsigned)c.ntasks;
+  if (mode == 0) {
+    k_residual<true, T><<<nb, kBlock, 0, c.stream>>>(c.A, log);
+    return;
+  }
+  k_xupdate<T><<<nb, kBlock, 0, c.stream>>>(c.A);
+  if (c.A.xout) k_residual<false, T, true><<<nb, kBlock, 0, c.stream>>>(c.A, log);
+  else k_residual<false, T><<<nb, kBlock, 0, c.stream>>>(c.A, log);
+}
 cudaError_t launch_residual(Ctx& c, int mode, CtrlState* ctrl, cudaGraphConditionalHandle hw,
                             int graph) {
-  const unsigned nb = (unsigned)c.ntasks;
-  const bool mixed = c.opts.precision == HF_PREC_MIXED;
-  if (mode == 0) {
-    if (mixed) k_residual<true, float><<<nb, kBlock, 0, c.stream>>>(c.A);
-    else k_residual<true, double><<<nb, kBlock, 0, c.stream>>>(c.A);
-    return launch_finalize(c, FIN_RES_INIT, ctrl, hw, graph);
-  }
-  if (mixed) {
-    k_xupdate<float><<<nb, kBlock, 0, c.stream>>>(c.A);
-    k_residual<false, float><<<nb, kBlock, 0, c.stream>>>(c.A);
-  } else {
-    k_xupdate<double><<<nb, kBlock, 0, c.stream>>>(c.A);
-    k_residual<false, double><<<nb, kBlock, 0, c.stream>>>(c.A);
-  }
-  return launch_finalize(c, FIN_RES, ctrl, hw, graph);
+  if (c.opts.precision == HF_PREC_MIXED) launch_res<float>(c, mode, graph == 2);
+  else launch_res<double>(c, mode, graph == 2);
+  return launch_finalize(c, mode == 0 ? FIN_RES_INIT : FIN_RES, ctrl, hw, graph);
+}
+
+template <typename T>
+static cudaError_t launch_cg_pq(Ctx& c) {
+  k_cg_pq<T><<<(unsigned)c.ncg, kBlock, kPqSmem<T>, c.stream>>>(c.A);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_inner_iteration(Ctx& c, int fp32, CtrlState* ctrl,
                                    cudaGraphConditionalHandle hw, int graph) {
-  const unsigned nb = (unsigned)c.ntasks;
-  if (fp32) {
-    k_cg_p<float><<<nb, kBlock, 0, c.stream>>>(c.A);
-    k_cg_spmv<float><<<nb, kBlock, 0, c.stream>>>(c.A);
-  } else {
-    k_cg_p<double><<<nb, kBlock, 0, c.stream>>>(c.A);
-    k_cg_spmv<double><<<nb, kBlock, 0, c.stream>>>(c.A);
-  }
-  cudaError_t e = launch_finalize(c, FIN_SPMV, ctrl, hw, graph);
+  const unsigned nb = (unsigned)c.ncg;
+  cudaError_t e = fp32 ? launch_cg_pq<float>(c) : launch_cg_pq<double>(c);
+  if (e == cudaSuccess) e = launch_finalize(c, FIN_SPMV, ctrl, hw, graph);
   if (e != cudaSuccess) return e;
   if (fp32) k_cg_upd<float><<<nb, kBlock, 0, c.stream>>>(c.A);
   else k_cg_upd<double><<<nb, kBlock, 0, c.stream>>>(c.A);
@@ -2009,36 +1966,24 @@ cudaError_t launch_single(Ctx& c, int which) {
   switch (which) {
     case HF_KERNEL_RHS: return launch_rhs(c);
     case HF_KERNEL_RESIDUAL:
-      if (fp32) k_residual<false, float><<<nb, kBlock, 0, c.stream>>>(c.A);
-      else k_residual<false, double><<<nb, kBlock, 0, c.stream>>>(c.A);
+      if (fp32) k_residual<false, float><<<nb, kBlock, 0, c.stream>>>(c.A, 0);
+      else k_residual<false, double><<<nb, kBlock, 0, c.stream>>>(c.A, 0);
       break;
     case HF_KERNEL_RESIDUAL_INIT:
-      if (fp32) k_residual<true, float><<<nb, kBlock, 0, c.stream>>>(c.A);
-      else k_residual<true, double><<<nb, kBlock, 0, c.stream>>>(c.A);
+      if (fp32) k_residual<true, float><<<nb, kBlock, 0, c.stream>>>(c.A, 0);
+      else k_residual<true, double><<<nb, kBlock, 0, c.stream>>>(c.A, 0);
       break;
     case HF_KERNEL_XUPDATE:
       if (fp32) k_xupdate<float><<<nb, kBlock, 0, c.stream>>>(c.A);
       else k_xupdate<double><<<nb, kBlock, 0, c.stream>>>(c.A);
       break;
+    // the direction update and the SpMV are one pass
     case HF_KERNEL_CG_P:
-      if (fp32) k_cg_p<float><<<nb, kBlock, 0, c.stream>>>(c.A);
-      else k_cg_p<double><<<nb, kBlock, 0, c.stream>>>(c.A);
-      break;
     case HF_KERNEL_CG_SPMV:
-      if (fp32) k_cg_spmv<float><<<nb, kBlock, 0, c.stream>>>(c.A);
-      else k_cg_spmv<double><<<nb, kBlock, 0, c.stream>>>(c.A);
-      break;
+    case HF_KERNEL_CG_PQ: return fp32 ? launch_cg_pq<float>(c) : launch_cg_pq<double>(c);
     case HF_KERNEL_CG_UPDATE:
-      if (fp32) k_cg_upd<float><<<nb, kBlock, 0, c.stream>>>(c.A);
-      else k_cg_upd<double><<<nb, kBlock, 0, c.stream>>>(c.A);
-      break;
-    case HF_KERNEL_CG_PQ:
-      if (fp32) {
-        k_cg_pq_f32<<<nb, kBlock, 0, c.stream>>>(c.A);
-      } else {
-        k_cg_p<double><<<nb, kBlock, 0, c.stream>>>(c.A);
-        k_cg_spmv<double><<<nb, kBlock, 0, c.stream>>>(c.A);
-      }
+      if (fp32) k_cg_upd<float><<<(unsigned)c.ncg, kBlock, 0, c.stream>>>(c.A);
+      else k_cg_upd<double><<<(unsigned)c.ncg, kBlock, 0, c.stream>>>(c.A);
       break;
     default: return cudaErrorInvalidValue;
   }

@@ -98,7 +98,7 @@ typedef struct hf_solver_opts {
   int32_t check_every;  /* iterations launched between host convergence polls */
   int32_t use_graph;    /* hf_run's step loop: 0 = kernels launched and polled by the host;
                            1 = the whole loop as one CUDA graph (a WHILE node around a step whose
-                           solve is one persistent cooperative kernel: no host round trip);
+                           inner solves are persistent cooperative kernels: no host round trip);
                            2 = a CUDA graph per step with conditional WHILE/SWITCH nodes;
                            3 = as 1, but one graph launch per step (kernels visible to profilers,
                            which do not see kernels inside conditional nodes) */
@@ -237,14 +237,14 @@ int hf_host_unregister(void* ptr);
 enum {
   HF_KERNEL_RHS = 0,         /* per-step right-hand side */
   HF_KERNEL_RESIDUAL = 1,    /* FP64 solution update + true residual sweep */
-  HF_KERNEL_CG_P = 2,        /* inner CG direction update p = r + beta p */
-  HF_KERNEL_CG_SPMV = 3,     /* inner CG SpMV q = A p and p.q */
-  HF_KERNEL_CG_UPDATE = 4,   /* inner CG solution/residual update + r.r */
+  HF_KERNEL_CG_P = 2,        /* the same pass as HF_KERNEL_CG_PQ */
+  HF_KERNEL_CG_SPMV = 3,     /* the same pass as HF_KERNEL_CG_PQ */
+  HF_KERNEL_CG_UPDATE = 4,   /* inner CG residual update r -= alpha q and r.r */
   HF_KERNEL_XUPDATE = 5,     /* FP64 solution update x += S^-1 y */
-  HF_KERNEL_SOLVE = 6,       /* the persistent solve kernel: one whole solve of the next step's
-                                system (the step's RHS runs before each timed launch) */
-  HF_KERNEL_CG_PQ = 7,       /* the fused direction update + SpMV pass of the persistent solve's
-                                FP32 inner CG, launched on its own (FP64: CG_P then CG_SPMV) */
+  HF_KERNEL_SOLVE = 6,       /* one whole solve of the next step's system, as a captured step runs
+                                it (the step's RHS runs before each timed solve) */
+  HF_KERNEL_CG_PQ = 7,       /* inner CG solution and direction update and SpMV in one pass:
+                                y += alpha p, p = r + beta p, q = A p and p.q */
   HF_KERNEL_RESIDUAL_INIT = 8 /* the step-start residual sweep r = S - H (x0 + TINY) */
 };
 /* Timeline of the latest step, from %globaltimer stamps its kernels write when they start
@@ -261,22 +261,22 @@ int hf_time_kernel(hf_ctx* ctx, int kernel, int reps, double* ms_per_launch);
  * every SM, CUDA-event timed).  On GB300 the FP64 rate bounds the FP64 kernels of a step. */
 int hf_measure_fp_rates(double* fp64_tflops, double* fp32_tflops);
 
-/* Phases of the persistent solve kernel, one per grid-wide round. */
+/* Phases of the solve, one per grid-wide round. */
 enum {
   HF_PHASE_IDLE = 0,      /* nothing left (step finished) */
   HF_PHASE_START = 1,     /* reserved */
   HF_PHASE_RES_INIT = 2,  /* first true residual r = S - H x0 */
-  HF_PHASE_CG_P = 3,      /* FP64 inner CG: p = r + beta p */
-  HF_PHASE_CG_Q = 4,      /* FP64 inner CG: q = Ah p, p.q */
-  HF_PHASE_CG_PQ = 5,     /* FP32 inner CG: p = r + beta p and q = Ah p in one pass */
-  HF_PHASE_CG_B = 6,      /* inner CG: y += alpha p, r -= alpha q, r.r */
+  HF_PHASE_CG_P = 3,      /* reserved (a direction update of its own) */
+  HF_PHASE_CG_Q = 4,      /* reserved (an SpMV of its own) */
+  HF_PHASE_CG_PQ = 5,     /* inner CG: y += alpha p, p = r + beta p, q = Ah p, p.q */
+  HF_PHASE_CG_B = 6,      /* inner CG: r -= alpha q, r.r */
   HF_PHASE_XUPD = 7,      /* x += sigma S^-1 y */
   HF_PHASE_RES = 8,       /* true residual of the updated x */
   HF_PHASE_RES_INIT_HX = 9, /* first true residual from the stored H T^n and H T^(n-1) (pointwise) */
   HF_PHASE_CG_BX = 10     /* inner CG update that also forms x += sigma S^-1 y: the iteration
                              predicted to end the inner solve (true-residual criterion) */
 };
-/* Round profile of the context's last persistent solve (use_graph = 1, or hf_time_kernel with
+/* Round profile of the context's last solve (use_graph 1 or 3, or hf_time_kernel with
  * HF_KERNEL_SOLVE).  No counterpart in the reference.  *rounds = grid-wide rounds run; for the
  * first min(rounds, cap, 512) rounds, phases[r] = the phase instance 0 ran and round_us[r] = the
  * round's length in microseconds (device %globaltimer; round 0 counts from the kernel's start). */
