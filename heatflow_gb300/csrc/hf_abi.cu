@@ -397,7 +397,7 @@ int capture_solve(Ctx& c, std::string& err) {
   const cudaGraphNode_t* deps = nullptr;
   size_t nd = 0;
   cudaGraphConditionalHandle hw;
-  if (!chk(cudaMemsetAsync(c.d_sctl, 0, solve_ctl_bytes(c.ninst), cs), "control block")) return HF_ECUDA;
+  if (!chk(cudaMemsetAsync(c.d_sctl, 0, solve_ctl_bytes(c.ninst, c.ncg), cs), "control block")) return HF_ECUDA;
   if (!chk(cudaStreamGetCaptureInfo(cs, &st, nullptr, &g, &deps, nullptr, &nd), "capture info")) return HF_ECUDA;
   if (!chk(cudaGraphConditionalHandleCreate(&hw, g, 0, cudaGraphCondAssignDefault), "handle(solve)")) return HF_ECUDA;
   if (!chk(launch_residual(c, 0, c.d_ctrl, hw, 2), "first residual")) return HF_ECUDA;
@@ -842,7 +842,18 @@ int cg_plan(Ctx& c) {
     c.A.cg_inst = p;
     c.ncg_cap = total;
   }
-  if (std::max(c.ntasks, total) > c.A.pcap) {   // two tables (the one-grid solve alternates)
+  const size_t ctl = solve_ctl_bytes(c.ninst, total);
+  if (ctl > c.sctl_cap) {
+    regrow(c.d_sctl);
+    c.d_sctl = c.A.sctl = nullptr;
+    c.sctl_cap = 0;
+    char* p = nullptr;
+    if (int r = dalloc(c, &p, ctl)) return r;
+    c.d_sctl = c.A.sctl = reinterpret_cast<SolveCtl*>(p);
+    c.sctl_cap = ctl;
+  }
+  CU(cudaMemsetAsync(c.d_sctl, 0, ctl, c.stream));
+  if (std::max(c.ntasks, total) > c.A.pcap) {   // two tables
     regrow(c.A.partials);
     c.A.partials = nullptr;
     c.A.pcap = 0;
@@ -1034,11 +1045,6 @@ int create_impl(const hf_problem* probs, int64_t count, const hf_solver_opts* op
   A.task_heat = d_task_heat;
   A.tasks = d_tasks;
   A.ntasks = c.ntasks;
-  {
-    char* sctl;                 // the control block and, behind it, the instances' queue entries
-    ALLOC(sctl, solve_ctl_bytes(count));
-    c.d_sctl = A.sctl = reinterpret_cast<SolveCtl*>(sctl);
-  }
   ALLOC(A.counters, (size_t)count);
   ALLOC(c.d_bc, (size_t)count);
   A.inst = d_inst; A.scal = d_scal; A.tile_inst = d_tile_inst;
@@ -1068,7 +1074,6 @@ int create_impl(const hf_problem* probs, int64_t count, const hf_solver_opts* op
 #define CK(call) do { cudaError_t e_ = (call); if (e_ != cudaSuccess) return fail(set_err(HF_ECUDA, std::string(#call) + ": " + cudaGetErrorString(e_))); } while (0)
   CK(cudaMemsetAsync(A.counters, 0, sizeof(unsigned) * count, c.stream));
   CK(cudaMemsetAsync(d_scal, 0, sizeof(InstScal) * count, c.stream));
-  CK(cudaMemsetAsync(c.d_sctl, 0, solve_ctl_bytes(count), c.stream));
   CK(cudaMemsetAsync(A.stamps, 0, sizeof(unsigned long long) * kStamps, c.stream));
   CK(cudaMemsetAsync(A.check, 0, sizeof(unsigned long long) * 4, c.stream));
   for (void* p : {(void*)A.diag, (void*)A.cx, (void*)A.cy, (void*)A.cz, (void*)c.asm_.kappa,
@@ -1883,7 +1888,7 @@ int hf_check_barrier_timeout(hf_ctx* h, int32_t wait_ms, int32_t* status, double
   CU(cudaEventCreate(&e0));
   CU(cudaEventCreate(&e1));
   CU(cudaEventRecord(e0, c.stream));
-  CU(cudaMemsetAsync(c.d_sctl, 0, solve_ctl_bytes(c.ninst), c.stream));
+  CU(cudaMemsetAsync(c.d_sctl, 0, solve_ctl_bytes(c.ninst, c.ncg), c.stream));
   if (c.split) CU(launch_residual(c, 0));
   CU(launch_solve(c, !c.split, (unsigned long long)wait_ms * 1000000ull, 0));
   CU(cudaEventRecord(e1, c.stream));

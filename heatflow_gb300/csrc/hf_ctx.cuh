@@ -30,6 +30,7 @@ struct Ctx {
   int64_t ncg = 0;               // tasks of the inner solve's passes, planned for a precision
   int cg_precision = -1;
   int64_t ncg_cap = 0;           // entries of cg_inst
+  size_t sctl_cap = 0;           // bytes at d_sctl
   std::vector<InstDesc> h_inst;
   std::vector<InstBC> h_bc;
   std::vector<int64_t> h_tile0;

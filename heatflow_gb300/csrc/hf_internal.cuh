@@ -153,20 +153,20 @@ struct SolveCtl {
   unsigned long long t_start;                 // %globaltimer at kernel start (ns)
   unsigned long long t_round[kRoundLog];      // %globaltimer when round r ended
   int32_t phase_log[kRoundLog];               // phase instance 0 ran in round r
-  // counters, one grid
+  // counters of one grid
   alignas(128) unsigned long long arrived;   // blocks arrived at all grid barriers so far
-  alignas(128) unsigned next_task[4];        // tasks handed out in a round (by round mod 4)
-  // counters, several grids
+  // counters of several grids
   alignas(128) unsigned long long ticket;    // tickets handed out
   alignas(128) unsigned long long tail;      // tickets published beyond the first phase's
   unsigned long long phases;                 // phases published
   unsigned finished;                         // instances without work left
 };
 
-// Several grids: behind the control block, each instance's published ticket range, then its count
-// of finished tasks.
-__host__ __device__ inline size_t solve_ctl_bytes(int64_t ninst) {
-  return sizeof(SolveCtl) + (size_t)ninst * (sizeof(unsigned long long) + sizeof(unsigned));
+// Behind the control block.  Several grids: each instance's published ticket range, then its count of
+// finished tasks.  One grid: its blocks' sums, three tables of two values per task.
+__host__ __device__ inline size_t solve_ctl_bytes(int64_t ninst, int64_t ncg) {
+  return sizeof(SolveCtl) + (ninst == 1 ? (size_t)ncg * 6 * sizeof(unsigned long long)
+                                        : (size_t)ninst * (sizeof(unsigned long long) + sizeof(unsigned)));
 }
 __device__ __forceinline__ unsigned long long* solve_slots(SolveCtl* ctl) {
   return reinterpret_cast<unsigned long long*>(ctl + 1);
@@ -190,8 +190,8 @@ struct DevArrays {
   InstScal* scal;
   const int32_t* tile_inst;
   double* partials;       // partial sums of the tasks: value k of task t at [k * pcap + t]; two such
-                          // tables of kNR values: the persistent solve of one grid uses them in
-                          // alternate rounds, that of several for the two kinds of tasks
+                          // tables of kNR values: the persistent solve of several grids uses the
+                          // second for the inner solve's passes, whose tasks are numbered apart
   unsigned int* counters; // per instance, last-block detection
   DevOpts opts;
   // static
@@ -423,7 +423,15 @@ __device__ __forceinline__ double tree8(const double (&t)[8]) {
 // dst[k * stride].  FP64 values go through shared memory and only warp 0 adds them (8 + 5 adds per
 // value per block): on GB300 every FP64 warp instruction costs the slow FP64 pipe, so a shuffle
 // tree in all eight warps would cost more than the kernel's own arithmetic.
-template <int NRV>
+// POSTED: for the blocks of the same launch that wait for the sums (post_sum).
+__device__ __forceinline__ void post_sum(double* dst, double v) {
+  // release: what the block wrote before (all of it behind a block barrier) is visible to whoever
+  // sees the sum.  A place that holds 0 has no sum yet, so +0 is posted as -0.
+  unsigned long long b = dbits(v);
+  if (b == 0ull) b = 0x8000000000000000ull;
+  asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(dst), "l"(b) : "memory");
+}
+template <int NRV, bool POSTED = false>
 __device__ __forceinline__ void tile_store(double* dst, int64_t stride, const double (&v)[NRV]) {
   static_assert(NRV <= kNR, "reduction slots");
   static_assert(kBlock == 256, "eight warps");
@@ -449,7 +457,10 @@ __device__ __forceinline__ void tile_store(double* dst, int64_t stride, const do
     }
     if (lane == 0) {
 #pragma unroll
-      for (int k = 0; k < NRV; ++k) dst[k * stride] = t[k];
+      for (int k = 0; k < NRV; ++k) {
+        if (POSTED) post_sum(dst + k * stride, t[k]);
+        else dst[k * stride] = t[k];
+      }
     }
   }
 }

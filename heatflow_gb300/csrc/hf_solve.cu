@@ -145,6 +145,7 @@ __device__ __forceinline__ T plane_above(const TCell& c, int j, V v, int z) {
 }
 
 // FP32 block sum of one value into *dst, a partial sum of a task (one conversion per block).
+template <bool POSTED = false>
 __device__ __forceinline__ void task_store_f(double* dst, float v) {
   __shared__ float red[kBlock / 32];
   __syncthreads();
@@ -157,7 +158,10 @@ __device__ __forceinline__ void task_store_f(double* dst, float v) {
     v = lane < kBlock / 32 ? red[lane] : 0.f;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
-    if (lane == 0) *dst = (double)v;
+    if (lane == 0) {
+      if (POSTED) post_sum(dst, (double)v);
+      else *dst = (double)v;
+    }
   }
 }
 
@@ -647,20 +651,19 @@ __device__ __forceinline__ void xupd_any(const DevArrays& A, double* part, int64
 // rounds.  Iteration 0 has p_0 = r and no y.
 //
 // Tasks (InstDesc::cgn of them): a block's thread owns one 16-byte vector (4 FP32 or 2 FP64 cells)
-// of a tile of 2^cqx vectors x kBlock / 2^cqx rows and marches the task's planes along z.  p is
-// formed once per cell, from r and p_(k-1), and shared through shared memory: three planes of the
-// tile, with the cells around it, whose p is formed from their r and p_(k-1) as well (the value that
-// their own tile stores) by threads that take one such vector or cell each.  The operands of the
-// plane after next are loaded into registers while a plane is computed, those beyond the tile into
-// shared memory (cp.async: few threads have any, but registers are the same for all).  The
-// neighbours' p comes from shared memory, so that few registers are live at the same time: spilled,
-// the pass took 1.8 times as long.
+// of a tile of 2^cqx vectors x kBlock / 2^cqx rows and marches the task's planes along z.  The operands
+// come through shared memory (cp.async), two planes ahead of the one that is computed: loads to
+// registers left the distance to the compiler, whose schedule of the same loop took 110 to 157 us at
+// 256^3 depending on the code around it.  p is formed once per cell, from r and p_(k-1), and shared:
+// three planes of the tile with the cells around it, whose p is formed from their r and p_(k-1) as well
+// (the value that their own tile stores) by threads that take one such vector or cell each.  One
+// block barrier per plane.
 // The rows of the inner solve's layout are padded to 4 cells: in a row's last vector the cells past
 // nx have zero coefficients, and q and r are kept zero there.  A face that does not exist has a
 // zero coefficient or a zero neighbour.
 // Bound by HBM in FP32 and by the FP64 pipe in FP64 (9 instructions per cell).  Measured on the
-// layered slab: 256^3 FP32, pq 115 us (5.2 TB/s) and upd 34 us (5.9 TB/s), where the direction
-// update, the SpMV and the update took 38 + 68 + 75 us; 190 x 192 x 192 FP64, 134 + 31 us against
+// layered slab: 256^3 FP32, pq 111 us (5.4 TB/s) and upd 31 us (6.5 TB/s), where the direction
+// update, the SpMV and the update took 38 + 68 + 75 us; 190 x 192 x 192 FP64, 134 + 30 us against
 // 34 + 111 + 68 us.
 template <typename T>
 struct alignas(16) Vec16 {
@@ -679,17 +682,22 @@ __device__ __forceinline__ void st16(T* p, const Vec16<T>& v) {
 
 // p of three planes: rows -1..rows of a tile, each of nq vectors with one more at either end (the
 // cell beside the row's first is the last of its vector, the cell beside its last the first of its
-// vector); the y faces of two planes, rows -1..rows-1; the x faces beside the rows' first cells.
+// vector).  A stage holds what one plane's step needs, by thread: r, p_(k-1) and y of the plane above
+// and the plane's own faces; and of the vectors and cells beyond the tile r and p_(k-1) of the plane
+// above and the plane's y or x faces.
+constexpr int kPqStages = 3;
 template <typename T>
 struct PqShared {
-  Vec16<T> p[3][340], ay[2][288];
-  Vec16<T> hr[80], hpo[80], hf[80];   // operands of the vectors and cells beyond the tile, by thread
-  T ax[2][32];
+  struct Stage {
+    Vec16<T> r[kBlock], po[kBlock], y[kBlock], ax[kBlock], ay[kBlock], az[kBlock];
+    Vec16<T> hr[80], hpo[80], hf[80];
+  } st[kPqStages];
+  Vec16<T> p[3][340];
 };
 template <typename T>
-constexpr int kPqSmem = (int)sizeof(PqShared<T>);   // (beside at most 11 KB of the kernels' own: below 48 KB)
-static_assert(kBlock == 256 && (8 + 2) * (32 + 2) <= 340 && (16 + 2) * (16 + 2) <= 340 && 8 * (32 + 1) <= 288 &&
-                  16 * (16 + 1) <= 288 && 32 * (8 + 1) <= 288, "tiles of 8, 16 or 32 vectors a row");
+constexpr int kPqSmem = (int)sizeof(PqShared<T>);   // 99 KB: two blocks per SM
+static_assert(kBlock == 256 && (8 + 2) * (32 + 2) <= 340 && (16 + 2) * (16 + 2) <= 340 && 2 * (8 + 32) <= 80,
+              "tiles of 8, 16 or 32 vectors a row");
 
 __device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 template <typename T>
@@ -701,8 +709,10 @@ __device__ __forceinline__ void cp1(T* dst, const T* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_addr(dst)), "l"(src), "n"((int)sizeof(T))
                : "memory");
 }
-// This thread's copies have arrived.
-__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// This thread's groups of copies have arrived, but for the newest N.
+template <int N>
+__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // Place of a thread in task `local` of the inner solve's passes.
 struct CgPos {
@@ -726,10 +736,10 @@ __device__ __forceinline__ CgPos cg_pos(const InstDesc& d, int local) {
 }
 
 // off: the instance's first cell (d.off4; a constant 0 where there is one instance keeps the base
-// pointers out of the registers).  pslot: the task's place in the table of partial sums; dyn:
-// kPqSmem<T> bytes of shared memory.
-template <typename T>
-__device__ __forceinline__ void pq_task(const DevArrays& A, const InstDesc& d, int64_t off, int local,
+// pointers out of the registers).  pslot: the place of the task's sum; dyn: kPqSmem<T> bytes of
+// shared memory.
+template <typename T, bool POSTED, bool FIRST>
+__device__ __forceinline__ void pq_form(const DevArrays& A, const InstDesc& d, int64_t off, int local,
                                         const InstScal& s, double* pslot, char* dyn) {
   constexpr int V = Vec16<T>::N;
   typedef Vec16<T> VT;
@@ -741,7 +751,6 @@ __device__ __forceinline__ void pq_task(const DevArrays& A, const InstDesc& d, i
   const bool act = c.act;
   const int last = min(V - 1, nx - 1 - c.x);   // the vector's last grid cell; cells past it are padding
   const int64_t k = s.iter;
-  const bool first = k == 0;
   const T beta = (T)s.beta, alpha = (T)s.alpha;      // alpha: of the previous iteration
   const T* R = Vec<T>::r(A) + off;
   const T* Po = Vec<T>::pb(A, k + 1) + off;
@@ -752,7 +761,7 @@ __device__ __forceinline__ void pq_task(const DevArrays& A, const InstDesc& d, i
   const T* __restrict__ ay = Vec<T>::ay(A) + off;
   const T* __restrict__ az = Vec<T>::az(A) + off;
   const int lxy = c.y * sx + c.x;
-  const int own = (c.ry + 1) * prow + c.vx + 1, ownay = (c.ry + 1) * nq + c.vx;
+  const int own = (c.ry + 1) * prow + c.vx + 1;
   // the vector or cell beyond the tile that this thread also forms: threads 0..nq-1 the row above
   // the tile's last one, nq..2nq-1 the row below its first (with that row's y faces), then the
   // cells beside the first column (with their x faces) and beside the last
@@ -791,124 +800,138 @@ __device__ __forceinline__ void pq_task(const DevArrays& A, const InstDesc& d, i
       }
     }
   }
+  // where the faces below this thread's row and beside its first cell come from
+  const bool hsouth = ny > 1 && (c.y > 0 || d.py), hwest = nx > 1 && (c.x > 0 || d.px);
   const VT zero{};
   auto form = [&](const VT& r, const VT& po) -> VT {
     VT p;
 #pragma unroll
-    for (int i = 0; i < V; ++i) p.v[i] = first ? r.v[i] : fma(beta, po.v[i], r.v[i]);
+    for (int i = 0; i < V; ++i) p.v[i] = FIRST ? r.v[i] : fma(beta, po.v[i], r.v[i]);
     return p;
   };
   auto above = [&](int z) { return z < nz || (d.pz && nz > 1); };   // plane z, or the wrap of z = nz
-  VT r = zero, po = zero, yv = zero;           // of the next plane to form
-  VT cx = zero, cy = zero, cz = zero;          // faces of the plane formed last
   const bool rdy = act && k > 1;
-  auto load_p = [&](int z) {                  // r, p_(k-1), y and the vector beyond of plane z
-    const int zp = (z < nz ? z : 0) * nxy;
-    if (act) {
-      const int l = HF_IXV(A, lxy + zp, n4, V);
-      r = ld16(R + l);
-      if (!first) po = ld16(Po + l);
-      if (rdy && z < z1) yv = ld16(Y + l);
-    }
-    if (hl >= 0 && z < z1) {
-      if (hvec) {
-        const int l = HF_IXV(A, hl + zp, n4, V);
-        cp16(&sm.hr[tid], R + l);
-        if (!first) cp16(&sm.hpo[tid], Po + l);
-      } else {
-        const int l = HF_IX(A, hl + zp, n4);
-        cp1(&sm.hr[tid].v[0], R + l);
-        if (!first) cp1(&sm.hpo[tid].v[0], Po + l);
-      }
-    }
-  };
-  auto load_c = [&](int z) {                  // the faces of plane z
-    if (act) {
-      const int l = HF_IXV(A, lxy + z * nxy, n4, V);
-      cx = ld16(ax + l);
-      cy = ld16(ay + l);
-      cz = ld16(az + l);
-    }
-    if (hl >= 0 && hc) {
-      if (hvec) cp16(&sm.hf[tid], ay + HF_IXV(A, hl + z * nxy, n4, V));
-      else cp1(&sm.hf[tid].v[0], ax + HF_IX(A, hl + z * nxy, n4));
-    }
-  };
-  // p of plane z into shared memory; the task's own planes are stored, and p_(k-1) goes into y
-  auto put_p = [&](int z, VT* pl) {
-    if (act) {
-      const VT p = above(z) ? form(r, po) : zero;
-      pl[own] = p;
-      if (z < z1) {
+  // the copies of plane z's step
+  auto issue = [&](int z, typename PqShared<T>::Stage& st) {
+    if (z < z1) {
+      const int za = z + 1 < nz ? z + 1 : 0;   // the plane above (or its wrap)
+      if (act) {
+        if (above(z + 1)) {
+          const int l = HF_IXV(A, lxy + za * nxy, n4, V);
+          cp16(&st.r[tid], R + l);
+          if (!FIRST) cp16(&st.po[tid], Po + l);
+          if (rdy && z + 1 < z1) cp16(&st.y[tid], Y + l);
+        }
         const int l = HF_IXV(A, lxy + z * nxy, n4, V);
-        st16(Pn + l, p);
-        if (!first) {
-          VT yn;
-#pragma unroll
-          for (int i = 0; i < V; ++i) yn.v[i] = fma(alpha, po.v[i], yv.v[i]);   // y is 0 before p_0
-          st16(Y + l, yn);
+        cp16(&st.ax[tid], ax + l);
+        cp16(&st.ay[tid], ay + l);
+        cp16(&st.az[tid], az + l);
+      }
+      if (hl >= 0) {
+        if (hvec) {
+          if (z + 1 < z1) {
+            const int l = HF_IXV(A, hl + za * nxy, n4, V);
+            cp16(&st.hr[tid], R + l);
+            if (!FIRST) cp16(&st.hpo[tid], Po + l);
+          }
+          if (hc) cp16(&st.hf[tid], ay + HF_IXV(A, hl + z * nxy, n4, V));
+        } else {
+          if (z + 1 < z1) {
+            const int l = HF_IX(A, hl + za * nxy, n4);
+            cp1(&st.hr[tid].v[0], R + l);
+            if (!FIRST) cp1(&st.hpo[tid].v[0], Po + l);
+          }
+          if (hc) cp1(&st.hf[tid].v[0], ax + HF_IX(A, hl + z * nxy, n4));
         }
       }
     }
-    if (hl >= 0 && z < z1) {
-      if (hvec) {
-        pl[hp] = form(sm.hr[tid], first ? zero : sm.hpo[tid]);
-      } else {
-        const T h = first ? sm.hr[tid].v[0] : fma(beta, sm.hpo[tid].v[0], sm.hr[tid].v[0]);
-        pl[hp].v[hc ? V - 1 : 0] = h;
-      }
-    }
+    cp_commit();
+  };
+  // p of a plane of the task: stored, and p_(k-1) goes into y
+  auto keep = [&](int z, const VT& p, const VT& po, const VT& yv) {
+    const int l = HF_IXV(A, lxy + z * nxy, n4, V);
+    st16(Pn + l, p);
+    if (FIRST) return;
+    VT yn;
+#pragma unroll
+    for (int i = 0; i < V; ++i) yn.v[i] = fma(alpha, po.v[i], yv.v[i]);   // y is 0 before p_0
+    st16(Y + l, yn);
   };
   __syncthreads();                            // the block's previous task is done with shared memory
-  load_p(z0);
-  load_c(z0);
-  VT azm = zero, pb = zero;
-  if (act && nz > 1) {                        // the plane below the task
+#pragma unroll
+  for (int i = 0; i < kPqStages - 1; ++i) issue(z0 + i, sm.st[i]);
+  // the first plane and the one below the task, on their way at the same time
+  VT r = zero, po = zero, yv = zero, rb = zero, pob = zero, azm = zero, hr = zero, hpo = zero;
+  if (act) {
+    const int l = HF_IXV(A, lxy + z0 * nxy, n4, V);
+    r = ld16(R + l);
+    if (!FIRST) po = ld16(Po + l);
+    if (rdy) yv = ld16(Y + l);
     int lb = -1;
-    if (z0 > 0) lb = lxy + (z0 - 1) * nxy;
-    else if (d.pz) lb = lxy + (nz - 1) * nxy;
+    if (nz > 1 && z0 > 0) lb = lxy + (z0 - 1) * nxy;
+    else if (nz > 1 && d.pz) lb = lxy + (nz - 1) * nxy;
     if (lb >= 0) {
       lb = HF_IXV(A, lb, n4, V);
-      pb = form(ld16(R + lb), first ? zero : ld16(Po + lb));
+      rb = ld16(R + lb);
+      if (!FIRST) pob = ld16(Po + lb);
       azm = ld16(az + lb);
     }
   }
-  for (int i = tid; i < 3 * 340; i += kBlock) sm.p[0][i] = zero;
-  for (int i = tid; i < 2 * 288; i += kBlock) sm.ay[0][i] = zero;
-  if (tid < 64) sm.ax[0][tid] = T(0);
-  __syncthreads();
-  sm.p[2][own] = pb;
-  cp_wait();
-  if (hl >= 0 && hc) {                        // the faces beyond the tile of plane z0
-    if (hvec) sm.ay[0][hp - 1] = sm.hf[tid];
-    else sm.ax[0][hp / prow - 1] = sm.hf[tid].v[0];
+  if (hl >= 0) {
+    if (hvec) {
+      const int l = HF_IXV(A, hl + z0 * nxy, n4, V);
+      hr = ld16(R + l);
+      if (!FIRST) hpo = ld16(Po + l);
+    } else {
+      const int l = HF_IX(A, hl + z0 * nxy, n4);
+      hr.v[0] = R[l];
+      if (!FIRST) hpo.v[0] = Po[l];
+    }
   }
-  put_p(z0, sm.p[0]);
-  if (above(z0 + 1)) load_p(z0 + 1);
+  for (int i = tid; i < 3 * 340; i += kBlock) sm.p[0][i] = zero;
+  __syncthreads();
+  auto put_beyond = [&](VT* pl, const VT& hr, const VT& hpo) {
+    if (hvec) pl[hp] = form(hr, hpo);
+    else pl[hp].v[hc ? V - 1 : 0] = FIRST ? hr.v[0] : fma(beta, hpo.v[0], hr.v[0]);
+  };
+  if (act) {
+    const VT p = form(r, po);
+    sm.p[0][own] = p;
+    sm.p[2][own] = form(rb, pob);
+    keep(z0, p, po, yv);
+  }
+  if (hl >= 0) put_beyond(sm.p[0], hr, hpo);
   // FP32 sums: per-thread sums of 8 planes, added up, so that no chain is longer than where four
   // groups of threads marched a quarter of a task's planes each
   T dot = T(0), dot8 = T(0);
   VT *pm = sm.p[2], *pc = sm.p[0], *pu = sm.p[1];
+  int si = 0;
   for (int z = z0; z < z1; ++z) {
-    const int b = (z - z0) & 1;
-    cp_wait();
-    if (hl >= 0 && hc && z > z0) {
-      if (hvec) sm.ay[b][hp - 1] = sm.hf[tid];
-      else sm.ax[b][hp / prow - 1] = sm.hf[tid].v[0];
-    }
-    put_p(z + 1, pu);
-    const VT axv = cx, azv = cz;
-    if (act) sm.ay[b][ownay] = cy;
-    if (z + 1 < z1) {
-      load_c(z + 1);
-      if (above(z + 2)) load_p(z + 2);
-    }
-    __syncthreads();                          // p of planes z and z + 1 and the y faces of z are there
-    T axw = __shfl_up_sync(kFull, axv.v[V - 1], 1);
-    if (c.vx == 0) axw = sm.ax[b][c.ry];
+    typename PqShared<T>::Stage& st = sm.st[si];
+    cp_wait<kPqStages - 2>();                 // plane z's step has arrived
     if (act) {
+      VT p = zero;
+      if (above(z + 1)) {
+        const VT po = FIRST ? zero : st.po[tid];
+        p = form(st.r[tid], po);
+        if (z + 1 < z1) keep(z + 1, p, po, rdy ? st.y[tid] : zero);
+      }
+      pu[own] = p;
+    }
+    if (hl >= 0 && z + 1 < z1) put_beyond(pu, st.hr[tid], FIRST ? zero : st.hpo[tid]);
+    __syncthreads();                          // p of planes z and z + 1 and all faces of z are there
+    {                                         // the stage of plane z - 1, which every thread has left
+      int sn = si + kPqStages - 1;
+      if (sn >= kPqStages) sn -= kPqStages;
+      issue(z + kPqStages - 1, sm.st[sn]);
+    }
+    if (act) {
+      const VT axv = st.ax[tid], azv = st.az[tid], ayv = st.ay[tid];
       const VT p = pc[own], pn = pc[own + prow], ps = pc[own - prow], pa = pu[own], pd = pm[own];
-      const VT ayv = sm.ay[b][ownay], ays = sm.ay[b][ownay - nq];
+      VT ays = zero;
+      if (hsouth) ays = c.ry > 0 ? st.ay[tid - nq] : st.hf[nq + c.vx];
+      T axw = T(0);
+      if (hwest) axw = c.vx > 0 ? st.ax[tid - 1].v[V - 1] : st.hf[2 * nq + c.ry].v[0];
       const T pw = pc[own - 1].v[V - 1], pe = pc[own + 1].v[0];
       VT qv;
 #pragma unroll
@@ -916,8 +939,7 @@ __device__ __forceinline__ void pq_task(const DevArrays& A, const InstDesc& d, i
         const T pi = p.v[i];
         T acc = pi;
         acc = fma(axv.v[i], i < last ? p.v[i < V - 1 ? i + 1 : i] : pe, acc);
-        if (i > 0) acc = fma(axv.v[i > 0 ? i - 1 : 0], p.v[i > 0 ? i - 1 : 0], acc);
-        else acc = fma(axw, pw, acc);
+        acc = fma(i > 0 ? axv.v[i > 0 ? i - 1 : 0] : axw, i > 0 ? p.v[i > 0 ? i - 1 : 0] : pw, acc);
         acc = fma(ayv.v[i], pn.v[i], acc);
         acc = fma(ays.v[i], ps.v[i], acc);
         acc = fma(azv.v[i], pa.v[i], acc);
@@ -927,24 +949,32 @@ __device__ __forceinline__ void pq_task(const DevArrays& A, const InstDesc& d, i
         qv.v[i] = acc;
       }
       st16(Q + HF_IXV(A, lxy + z * nxy, n4, V), qv);
+      azm = azv;
     }
     if (sizeof(T) == 4 && ((z - z0) & 7) == 7) {
       dot += dot8;
       dot8 = T(0);
     }
-    azm = azv;
     VT* t = pm;
     pm = pc;
     pc = pu;
     pu = t;
+    if (++si == kPqStages) si = 0;
   }
   dot += dot8;
   if constexpr (sizeof(T) == 4) {
-    task_store_f(pslot, dot);
+    task_store_f<POSTED>(pslot, dot);
   } else {
     const double v[1] = {dot};
-    tile_store<1>(pslot, A.pcap, v);
+    tile_store<1, POSTED>(pslot, 0, v);
   }
+}
+// Iteration 0 (p = r, no y) is a form of its own.
+template <typename T, bool POSTED>
+__device__ __forceinline__ void pq_task(const DevArrays& A, const InstDesc& d, int64_t off, int local,
+                                        const InstScal& s, double* pslot, char* dyn) {
+  if (s.iter == 0) pq_form<T, POSTED, true>(A, d, off, local, s, pslot, dyn);
+  else pq_form<T, POSTED, false>(A, d, off, local, s, pslot, dyn);
 }
 
 // r -= alpha q and r.r (and the unscaled ||r||^2 for the reference rule).  The planes are walked
@@ -953,124 +983,155 @@ __device__ __forceinline__ void pq_task(const DevArrays& A, const InstDesc& d, i
 // layouts index alike).
 // WEIGHTED is a form of its own: as a condition in the loop its FP64 instructions, predicated off,
 // took the FP64 pipe all the same (ncu: pipe 72 % busy for 2 FMAs per cell).
-template <typename T, bool WEIGHTED>
+// Operands arrive through shared memory (cp.async), two stages ahead of the one that is computed: the
+// pq pass's shared memory leaves little L1 for loads in flight (31 us at 256^3 against 39 with loads to
+// registers, the form with the x update 119 against 132).
+template <typename T>
+struct UpdStage { Vec16<T> q[4][kBlock], r[4][kBlock]; };     // four planes
+template <typename T>
+struct UpdXStage {                                            // one plane
+  Vec16<T> q[kBlock], r[kBlock], p[kBlock], y[kBlock], s[kBlock];
+  Vec16<double> x[Vec16<T>::N / 2][kBlock];
+};
+static_assert(3 * sizeof(UpdStage<float>) <= sizeof(PqShared<float>) && 3 * sizeof(UpdStage<double>) <= sizeof(PqShared<double>) &&
+                  3 * sizeof(UpdXStage<float>) <= sizeof(PqShared<float>) && 3 * sizeof(UpdXStage<double>) <= sizeof(PqShared<double>),
+              "the update's stages fit the pq pass's shared memory");
+template <typename T, bool WEIGHTED, bool POSTED>
 __device__ __forceinline__ void upd_form(const DevArrays& A, const InstDesc& d, int local, const InstScal& s,
-                                         double* pslot) {
+                                         double* pslot, int64_t stride, char* dyn) {
   constexpr int V = Vec16<T>::N;
   typedef Vec16<T> VT;
   const CgPos c = cg_pos<T>(d, local);
   const T alpha = (T)s.alpha;
+  const int tid = threadIdx.x;
   const int nxy = d.sx * d.ny, n4 = nxy * d.nz, lxy = c.y * d.sx + c.x;
   const int last = min(V - 1, d.nx - 1 - c.x);
   T* R = Vec<T>::r(A) + d.off4;
   const T* Q = Vec<T>::q(A) + d.off4;
   T rr = T(0), rr8 = T(0);
   double rw = 0.0;
-  if (!WEIGHTED && c.act && (s.xw & kXwThis)) {   // (never under the reference's rule)
+  if (!WEIGHTED && (s.xw & kXwThis)) {        // (never under the reference's rule)
+    UpdXStage<T>* st = reinterpret_cast<UpdXStage<T>*>(dyn);
     const bool first = s.iter == 0;
     const T* P = Vec<T>::pb(A, s.iter) + d.off4;
     const T* Y = Vec<T>::y(A) + d.off4;
     const double* XR = A.tbuf[s.role[2]] + d.off;
     double* XW = A.tbuf[s.role[3]] + d.off;
-    const double* __restrict__ sinv = A.sinv + d.off;
-    const float* __restrict__ sinv32 = A.sinv32 + d.off;
+    const double* sinv = A.sinv + d.off;
+    const float* sinv32 = A.sinv32 + d.off;
     const float sig = (float)s.sigma_prev;
+    auto issue = [&](int z, UpdXStage<T>& o) {
+      if (c.act && z >= c.z0) {
+        const int l = HF_IXV(A, lxy + z * nxy, n4, V);
+        cp16(&o.q[tid], Q + l);
+        cp16(&o.r[tid], R + l);
+        cp16(&o.p[tid], P + l);
+        if (!first) cp16(&o.y[tid], Y + l);
+        if constexpr (sizeof(T) == 8) cp16(&o.s[tid], sinv + l);
+        else cp16(&o.s[tid], sinv32 + l);
+#pragma unroll
+        for (int i = 0; i < V / 2; ++i) cp16(&o.x[i][tid], XR + l + 2 * i);
+      }
+      cp_commit();
+    };
+    issue(c.z1 - 1, st[0]);
+    issue(c.z1 - 2, st[1]);
+    int si = 0;
     for (int z = c.z1 - 1; z >= c.z0; --z) {
-      const int l = HF_IXV(A, lxy + z * nxy, n4, V);
-      const VT qv = ld16(Q + l), pv = ld16(P + l);
-      VT rv = ld16(R + l), yv{};
-      if (!first) yv = ld16(Y + l);
-      double xv[V], sv[V];
+      const UpdXStage<T>& o = st[si];
+      cp_wait<1>();
+      issue(z - 2, st[si == 0 ? 2 : si - 1]);
+      if (c.act) {
+        const int l = HF_IXV(A, lxy + z * nxy, n4, V);
+        const VT qv = o.q[tid], pv = o.p[tid], fv = o.s[tid];
+        VT rv = o.r[tid], yv{};
+        if (!first) yv = o.y[tid];
+        Vec16<double> xv[V / 2];
 #pragma unroll
-      for (int i = 0; i < V; i += 2) {
-        const double2 t = *reinterpret_cast<const double2*>(XR + l + i);
-        xv[i] = t.x;
-        xv[i + 1] = t.y;
-      }
-      if constexpr (sizeof(T) == 8) {
-        const double2 t = *reinterpret_cast<const double2*>(sinv + l);
-        sv[0] = t.x;
-        sv[1] = t.y;
-      }
-      VT fv{};
-      if constexpr (sizeof(T) == 4) fv = ld16(sinv32 + l);
+        for (int i = 0; i < V / 2; ++i) xv[i] = o.x[i][tid];
 #pragma unroll
-      for (int i = 0; i < V; ++i) {
-        const T yo = fma(alpha, pv.v[i], yv.v[i]);
-        rv.v[i] = fma(-alpha, qv.v[i], rv.v[i]);
-        rr8 = fma(rv.v[i], rv.v[i], rr8);
-        if constexpr (sizeof(T) == 8) xv[i] = fma(sv[i], yo, xv[i]);
-        else xv[i] = xv[i] + f32_to_f64(sig * fv.v[i] * yo);
-      }
-      st16(R + l, rv);
+        for (int i = 0; i < V; ++i) {
+          const T yo = fma(alpha, pv.v[i], yv.v[i]);
+          rv.v[i] = fma(-alpha, qv.v[i], rv.v[i]);
+          rr8 = fma(rv.v[i], rv.v[i], rr8);
+          double& x = xv[i / 2].v[i & 1];
+          if constexpr (sizeof(T) == 8) x = fma(fv.v[i], yo, x);
+          else x = x + f32_to_f64(sig * fv.v[i] * yo);
+        }
+        st16(R + l, rv);
 #pragma unroll
-      for (int i = 0; i < V; i += 2) *reinterpret_cast<double2*>(XW + l + i) = make_double2(xv[i], xv[i + 1]);
+        for (int i = 0; i < V / 2; ++i) st16(XW + l + 2 * i, xv[i]);
+      }
       if (sizeof(T) == 4 && ((c.z1 - 1 - z) & 7) == 7) {
         rr += rr8;
         rr8 = T(0);
       }
+      if (++si == 3) si = 0;
     }
-  } else if (c.act) {
-    // U planes of loads are in flight while the U before are computed
+  } else {
+    UpdStage<T>* st = reinterpret_cast<UpdStage<T>*>(dyn);
     constexpr int U = 4;
-    VT qn[U], rn[U];
-    auto load = [&](int zt) {
+    auto issue = [&](int zt, UpdStage<T>& o) {
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        if (zt - u < c.z0) continue;
+        if (!c.act || zt - u < c.z0) continue;
         const int l = HF_IXV(A, lxy + (zt - u) * nxy, n4, V);
-        qn[u] = ld16(Q + l);
-        rn[u] = ld16(R + l);
+        cp16(&o.q[u][tid], Q + l);
+        cp16(&o.r[u][tid], R + l);
       }
+      cp_commit();
     };
-    load(c.z1 - 1);
+    issue(c.z1 - 1, st[0]);
+    issue(c.z1 - 1 - U, st[1]);
+    int si = 0;
     for (int zt = c.z1 - 1; zt >= c.z0; zt -= U) {
-      VT qv[U], rv[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        qv[u] = qn[u];
-        rv[u] = rn[u];
-      }
-      load(zt - U);
+      const UpdStage<T>& o = st[si];
+      cp_wait<1>();
+      issue(zt - 2 * U, st[si == 0 ? 2 : si - 1]);
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const int z = zt - u;
-        if (z < c.z0) continue;
+        if (!c.act || z < c.z0) continue;
+        const VT qv = o.q[u][tid];
+        VT rv = o.r[u][tid];
 #pragma unroll
         for (int i = 0; i < V; ++i) {
-          T r = fma(-alpha, qv[u].v[i], rv[u].v[i]);
+          T r = fma(-alpha, qv.v[i], rv.v[i]);
           if (i > last) r = T(0);
-          rv[u].v[i] = r;
+          rv.v[i] = r;
           rr8 = fma(r, r, rr8);
           if (WEIGHTED && i <= last) {
             const double dg = A.diag[d.off + HF_IX(A, (z * d.ny + c.y) * d.nx + c.x + i, d.nx * d.ny * d.nz)];
             rw = fma(-dg * (double)r, (double)r, rw);
           }
         }
-        st16(R + HF_IXV(A, lxy + z * nxy, n4, V), rv[u]);
-        if (sizeof(T) == 4 && ((c.z1 - 1 - z) & 7) == 7) {
-          rr += rr8;
-          rr8 = T(0);
-        }
+        st16(R + HF_IXV(A, lxy + z * nxy, n4, V), rv);
       }
+      if (sizeof(T) == 4 && ((c.z1 - 1 - zt) & 4)) {
+        rr += rr8;
+        rr8 = T(0);
+      }
+      if (++si == 3) si = 0;
     }
   }
   rr += rr8;
   if constexpr (sizeof(T) == 4) {
-    task_store_f(pslot, rr);
+    task_store_f<POSTED>(pslot, rr);
   } else if constexpr (WEIGHTED) {
     const double v[2] = {rr, rw};
-    tile_store<2>(pslot, A.pcap, v);
+    tile_store<2, POSTED>(pslot, stride, v);
   } else {
     const double v[1] = {rr};
-    tile_store<1>(pslot, A.pcap, v);
+    tile_store<1, POSTED>(pslot, stride, v);
   }
 }
 template <typename T>
 __device__ __forceinline__ void upd_task(const DevArrays& A, const InstDesc& d, int local, const InstScal& s,
-                                         double* pslot) {
-  if (sizeof(T) == 8 && A.opts.criterion == HF_STOP_RECURSIVE) upd_form<T, sizeof(T) == 8>(A, d, local, s, pslot);
-  else upd_form<T, false>(A, d, local, s, pslot);
+                                         double* pslot, char* dyn) {
+  if (sizeof(T) == 8 && A.opts.criterion == HF_STOP_RECURSIVE)
+    upd_form<T, sizeof(T) == 8, false>(A, d, local, s, pslot, A.pcap, dyn);
+  else
+    upd_form<T, false, false>(A, d, local, s, pslot, A.pcap, dyn);
 }
 
 // ---- standalone kernels (host-polled loop, conditional-node graph, kernel timing) --------------
@@ -1112,16 +1173,17 @@ __global__ void __launch_bounds__(kBlock) k_cg_pq(DevArrays A) {
   const InstScal& s = A.scal[inst];
   if (!s.inner_active) return;
   const InstDesc& d = A.inst[inst];
-  pq_task<T>(A, d, d.off4, (int)(blockIdx.x - d.cg0), s, A.partials + blockIdx.x, dyn);
+  pq_task<T, false>(A, d, d.off4, (int)(blockIdx.x - d.cg0), s, A.partials + blockIdx.x, dyn);
 }
 
 template <typename T>
 __global__ void __launch_bounds__(kBlock) k_cg_upd(DevArrays A) {
+  extern __shared__ __align__(16) char dyn[];
   const int inst = A.cg_inst[blockIdx.x];
   const InstScal& s = A.scal[inst];
   if (!s.inner_active) return;
   const InstDesc& d = A.inst[inst];
-  upd_task<T>(A, d, (int)(blockIdx.x - d.cg0), s, A.partials + blockIdx.x);
+  upd_task<T>(A, d, (int)(blockIdx.x - d.cg0), s, A.partials + blockIdx.x, dyn);
 }
 
 // ---- summation of an instance's task partials ------------------------------------------------
@@ -1287,26 +1349,32 @@ __device__ void epi_spmv_s(InstScal& s, const double* tot) {
 }
 
 
+// What the epilogue of a CG update divides and roots: r.r over that of the iteration before, over
+// the inner solve's first, and the stopping criterion (the reference's on the unscaled recursive
+// residual r = -S rh sigma, mod_Sparse.f90:420).
+struct UpdRatios { double shrink, first, err; };
+__device__ __forceinline__ UpdRatios upd_ratios(const InstScal& s, const DevOpts& o, const double* tot) {
+  UpdRatios q;
+  q.shrink = tot[0] / s.rho;
+  q.first = tot[0] / s.gg0;
+  if (o.criterion == HF_STOP_RECURSIVE) q.err = s.bb > 0.0 ? sqrt(tot[1]) * s.sigma_prev / sqrt(s.bb) : 0.0;
+  else q.err = s.gg0 > 0.0 ? sqrt(q.first) : 0.0;
+  return q;
+}
+
 template <typename T>
-__device__ void epi_upd_s(InstScal& s, const DevOpts& o, const double* tot) {
+__device__ __forceinline__ void epi_upd_s(InstScal& s, const DevOpts& o, const double* tot, const UpdRatios& q) {
   const bool weighted = (o.criterion == HF_STOP_RECURSIVE);
-  const double rho_new = tot[0], rho_old = s.rho;
-  s.beta = rho_new / s.rho;
+  const double rho_new = tot[0];
+  s.beta = q.shrink;
   s.rho = rho_new;
   s.iter += 1;
   s.ypend = 1;
   s.step_iters += 1;
   if (sizeof(T) == 8) s.tot_iters += 1; else s.tot_inner += 1;
-  bool stop;
-  if (weighted) {
-    // err = ||r||/||b|| on the unscaled recursive residual r = -S rh sigma (mod_Sparse.f90:420)
-    s.rr_w = tot[1];
-    s.err = s.bb > 0.0 ? sqrt(tot[1]) * s.sigma_prev / sqrt(s.bb) : 0.0;
-    stop = (s.err <= o.tol);
-  } else {
-    s.err = s.gg0 > 0.0 ? sqrt(rho_new / s.gg0) : 0.0;
-    stop = (s.err <= s.eta);
-  }
+  if (weighted) s.rr_w = tot[1];
+  s.err = q.err;
+  bool stop = s.err <= (weighted ? o.tol : s.eta);
   const int64_t cap = (sizeof(T) == 8) ? o.itmax : (int64_t)o.inner_itmax;
   if (!stop && s.iter >= cap) {
     stop = true;
@@ -1320,7 +1388,7 @@ __device__ void epi_upd_s(InstScal& s, const DevOpts& o, const double* tot) {
   const int32_t wrote = (s.xw & kXwThis) ? kXwDone : 0;
   s.xw = (s.xw & kXwAllowed) | wrote;
   if (!stop && (s.xw & kXwAllowed)) {
-    const double next = (rho_new / s.gg0) * (rho_new / rho_old);
+    const double next = q.first * q.shrink;
     if (s.iter + 1 >= cap || next <= s.eta * s.eta) s.xw |= kXwThis;
   }
 }
@@ -1333,7 +1401,7 @@ __device__ void epi_residual(const DevArrays& A, int inst, const double* tot) {
 __device__ void epi_spmv(const DevArrays& A, int inst, const double* tot) { epi_spmv_s(A.scal[inst], tot); }
 template <typename T>
 __device__ void epi_upd(const DevArrays& A, int inst, const double* tot) {
-  epi_upd_s<T>(A.scal[inst], A.opts, tot);
+  epi_upd_s<T>(A.scal[inst], A.opts, tot, upd_ratios(A.scal[inst], A.opts, tot));
 }
 
 // Whether instance s took part in the producing kernel (the producers' own entry tests).
@@ -1471,6 +1539,9 @@ __device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long
   asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return v;
 }
+__device__ __forceinline__ void red_release_add_u64(unsigned long long* p, unsigned long long v) {
+  asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
 __device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long long* p) {
   unsigned long long v;
   asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
@@ -1479,10 +1550,6 @@ __device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long
 __device__ __forceinline__ void st_release_u64(unsigned long long* p, unsigned long long v) {
   asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
-__device__ __forceinline__ void red_release_add_u64(unsigned long long* p, unsigned long long v) {
-  asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-
 template <typename T>
 __device__ __forceinline__ int32_t phase_after(const InstScal& s) {
   if (!s.outer_active) return PH_IDLE;
@@ -1525,7 +1592,7 @@ __device__ __noinline__ void phase_epilogue(InstScal& sc, const InstDesc& d, con
       sc.phase = sc.inner_active ? PH_CG_B : phase_after<T>(sc);
       break;
     case PH_CG_B:
-      epi_upd_s<T>(sc, o, acc);
+      epi_upd_s<T>(sc, o, acc, upd_ratios(sc, o, acc));
       sc.phase = phase_after<T>(sc);
       break;
     case PH_XUPD: sc.phase = PH_RES; break;
@@ -1537,8 +1604,8 @@ __device__ __noinline__ void phase_epilogue(InstScal& sc, const InstDesc& d, con
 template <typename T, bool XOUT, bool FULL, bool WEIGHTED>
 __device__ __forceinline__ void round_task(const DevArrays& A, const InstDesc& d, double* part, int local,
                                            const InstScal& s, char* dyn) {
-  if (s.phase == PH_CG_PQ) pq_task<T>(A, d, d.off4, local, s, part + d.cg0 + local, dyn);
-  else if (s.phase == PH_CG_B) upd_form<T, WEIGHTED>(A, d, local, s, part + d.cg0 + local);
+  if (s.phase == PH_CG_PQ) pq_task<T, false>(A, d, d.off4, local, s, part + d.cg0 + local, dyn);
+  else if (s.phase == PH_CG_B) upd_form<T, WEIGHTED, false>(A, d, local, s, part + d.cg0 + local, A.pcap, dyn);
   if constexpr (FULL) {
     const int64_t task = d.task0 + local;
     switch (s.phase) {
@@ -1695,115 +1762,171 @@ __global__ void __launch_bounds__(kBlock, 2)
 }
 
 // ---- persistent solve of one grid ------------------------------------------------------------
-// With one grid every block can keep its scalars itself: after each grid barrier every block sums
-// all the tasks' partials (the same adds in the same order, so all blocks obtain the same bits) and
-// runs the scalar epilogue on its own copy in shared memory.  The barrier is then one arrival and
-// one wait.  Where the last block to arrive reads the scalars, sums, runs the epilogue, writes them
-// back and opens the barrier, and every block reads them again, each round holds six dependent
-// trips through L2, which was most of a small grid's round (a CG iteration of its three rounds took
-// 29 us on 625 cells and 34 us on 64^3, 15 and 17 with the epilogue in every block).
-// Partial sums alternate between two tables by round: a block may write round r + 1's while another
-// still sums round r's, and none writes round r + 2's before all have arrived at the barrier of
-// round r + 1.
-// Tasks: one each where the blocks suffice, else handed out one at a time from a per-round counter,
-// so blocks on busier SMs take fewer of them (counter r mod 4; block 0 clears the one of round
-// r + 2, which every block has left behind and none has reached).
-// Measured: the layered slab at 64^3, mixed, 20 steps 11.7 -> 6.1 ms; a 25 x 25 x 1 grid under the
-// reference's rule, 10 steps 17.3 -> 9.1 ms; 128^3 1.17 times as fast, 256^3 1.03 times.
+// The inner solve that is due, in grid-wide rounds (a pq or an update pass each).  Every block keeps
+// the scalars itself: after each round it adds the sums that all tasks posted (the same adds in the
+// same order, so all blocks obtain the same bits) and runs the scalar epilogue on its own copy in
+// shared memory.  Where the last block to arrive at a barrier does that for all, each round holds six
+// dependent trips through L2, which was most of a small grid's round.
+// Up to kDirectTasks tasks, a block waits for the sums themselves: posting one is the arrival, and a
+// round is one trip through L2 from the last task's end to the next round.  With more, that many
+// polls from every block get in each other's way (256 tasks: 8.2 against 5.3 us an update round), and
+// a counter is waited for first, by one thread.
+// Every block has at least one task, the tasks are dealt in turn, so no block passes round r before
+// all have posted round r: the sums of round r - 1 are then read by all, and each block clears its
+// places of that table, which round r + 2 uses (three tables).
+// Measured per CG iteration (two rounds; three at first): 25 x 25 x 1 under the reference's rule
+// 29 us with the epilogue in one block, 13.8 with a barrier and the epilogue in every block, 11.0 with
+// posted sums and the epilogue's divisions and roots side by side; the 64^3 slab, mixed, 34, 14.3 and
+// 11.8.
+constexpr int kDirectTasks = 32;
+// Wait until done() (one thread), in bounded time and polls; false: given up, and SolveCtl::err says so.
+template <class F>
+__device__ __forceinline__ int wait_for(SolveCtl* ctl, unsigned long long wait_ns, F done) {
+  unsigned long long t0 = 0;
+  for (unsigned polls = 0; !done(); ++polls) {
+    if (polls < 64u) continue;               // a round of a small grid is a few microseconds
+    if (*(volatile int*)&ctl->err) return 0;
+    if ((polls & 255u) == 64u) {
+      const unsigned long long now = gtimer();
+      if (t0 == 0) t0 = now;
+      if (now - t0 > wait_ns || polls > (1u << 27)) {
+        atomicExch(&ctl->err, 1);
+        return 0;
+      }
+    }
+    __nanosleep(32);
+  }
+  return 1;
+}
+
 // WEIGHTED: the reference's stopping rule (upd_form).
 template <typename T, bool WEIGHTED>
 __global__ void __launch_bounds__(kBlock, 2)
     k_solve_one(DevArrays A, SolveCtl* ctl, int64_t limit, unsigned long long wait_ns, int leaver) {
   __shared__ InstScal sh;
   __shared__ InstDesc sd;
-  __shared__ double red[kBlock * 2];
-  __shared__ unsigned s_next;
-  __shared__ int s_ok;
+  __shared__ double red[(WEIGHTED ? 2 : 1) * kBlock];
   extern __shared__ __align__(16) char dyn[];
   static_assert(sizeof(InstDesc) % 8 == 0 && sizeof(InstDesc) / 8 <= kBlock, "descriptor copy");
-  const unsigned G = gridDim.x;
-  if ((int)threadIdx.x < kScalWords)
-    reinterpret_cast<unsigned long long*>(&sh)[threadIdx.x] =
-        reinterpret_cast<const unsigned long long*>(A.scal)[threadIdx.x];
-  if (threadIdx.x < sizeof(InstDesc) / 8)
-    reinterpret_cast<unsigned long long*>(&sd)[threadIdx.x] =
-        reinterpret_cast<const unsigned long long*>(A.inst)[threadIdx.x];
+  const int tid = threadIdx.x, G = (int)gridDim.x;
+  if (tid < kScalWords)
+    reinterpret_cast<unsigned long long*>(&sh)[tid] = reinterpret_cast<const unsigned long long*>(A.scal)[tid];
+  if (tid < (int)(sizeof(InstDesc) / 8))
+    reinterpret_cast<unsigned long long*>(&sd)[tid] = reinterpret_cast<const unsigned long long*>(A.inst)[tid];
   __syncthreads();
   if (!sh.inner_active) return;              // no inner solve is due
   __syncthreads();
-  if (threadIdx.x == 0) sh.phase = PH_CG_PQ;
+  if (tid == 0) sh.phase = PH_CG_PQ;
+  const int nt = sd.cgn;
+  const bool direct = nt <= kDirectTasks;
+  double* const sums = reinterpret_cast<double*>(solve_slots(ctl));
+  const int64_t round0 = ctl->rounds;        // of the log
   __syncthreads();
   int64_t r = 0;
-  for (; cg_phase(sh.phase); ++r) {
+  for (int tab = 0; cg_phase(sh.phase); ++r, tab = tab == 2 ? 0 : tab + 1) {
     if (r >= limit) {
-      if (blockIdx.x == 0 && threadIdx.x == 0) ctl->guard_hit = 1;
+      if (blockIdx.x == 0 && tid == 0) ctl->guard_hit = 1;
       break;
     }
-    // odd rounds hand the tasks out backwards, so a round starts on the data the previous round wrote
-    // last, which is still in L2 (the partial sums have fixed slots: the order changes no bits)
-    double* part = A.partials + (r & 1) * (kNR * A.pcap);
     const int32_t ph = sh.phase;             // read before any thread can run the epilogue
-    const unsigned nt = (unsigned)sd.cgn;
-    const bool hand_out = nt > G;
-    unsigned k = blockIdx.x;
-    if (blockIdx.x == 0 && threadIdx.x == 32) ctl->next_task[(r + 2) & 3] = 0u;
-    if (hand_out) {
-      if (threadIdx.x == 0) s_next = atomicAdd(&ctl->next_task[r & 3], 1u);
-      __syncthreads();
-      k = s_next;
-    }
-    while (k < nt) {
-      if (hand_out) {
-        __syncthreads();                     // every thread has read s_next
-        if (threadIdx.x == 0) s_next = atomicAdd(&ctl->next_task[r & 3], 1u);
-      }
-      const int local = (int)(hand_out && (r & 1) ? nt - 1 - k : k);
-      if (ph == PH_CG_PQ) pq_task<T>(A, sd, 0, local, sh, part + local, dyn);
-      else upd_form<T, WEIGHTED>(A, sd, local, sh, part + local);
-      if (!hand_out) break;
-      __syncthreads();                       // s_next holds the block's next task
-      k = s_next;
-    }
-    // failure-path check only (leaver >= 0): that block leaves without arriving, so the others'
+    const int32_t logged = logged_phase(sh);
+    double* const mine = sums + tab * 2 * nt;
+    // failure-path check only (leaver >= 0): that block leaves without posting, so the others'
     // waits run out and record SolveCtl::err
     if ((int)blockIdx.x == leaver) return;
-    __syncthreads();                         // the block's work is done
-    if (threadIdx.x == 0) {
-      red_release_add_u64(&ctl->arrived, 1ull);   // releases what the block wrote before the barrier
-      const unsigned long long want = (unsigned long long)G * (unsigned long long)(r + 1);
-      int ok = 1;
-      unsigned long long t0 = 0;
-      for (unsigned polls = 0; ld_acquire_u64(&ctl->arrived) < want; ++polls) {
-        if (polls < 64u) continue;           // a round of a small grid is a few microseconds
-        if (*(volatile int*)&ctl->err) { ok = 0; break; }
-        if ((polls & 255u) == 64u) {
-          const unsigned long long t = gtimer();
-          if (t0 == 0) t0 = t;
-          if (t - t0 > wait_ns || polls > (1u << 27)) {
-            atomicExch(&ctl->err, 1);
-            ok = 0;
-            break;
-          }
-        }
-        __nanosleep(32);
-      }
-      s_ok = ok;
+    for (int k = blockIdx.x; k < nt; k += G) {
+      if (ph == PH_CG_PQ) pq_task<T, true>(A, sd, 0, k, sh, mine + k, dyn);
+      else upd_form<T, WEIGHTED, true>(A, sd, k, sh, mine + k, nt, dyn);
     }
-    __syncthreads();
-    if (!s_ok) return;
-    double acc[2] = {0.0, 0.0};
-    if (phase_partials(ph) > 0) instance_sum<2>(part, A.pcap, 0, nt, acc, red);
-    if (threadIdx.x == 0) {
-      if (blockIdx.x == 0) log_round(ctl, logged_phase(sh));
-      phase_epilogue<T>(sh, sd, A.opts, acc);
+    const bool two = WEIGHTED && ph == PH_CG_B;
+    int ok = 1;
+    if (!direct) {
+      __syncthreads();                       // the block's work is done
+      if (tid == 0) {
+        red_release_add_u64(&ctl->arrived, 1ull);
+        ok = wait_for(ctl, wait_ns, [&] {
+          return ld_acquire_u64(&ctl->arrived) >= (unsigned long long)G * (unsigned long long)(r + 1);
+        });
+      }
+      if (!__syncthreads_and(ok)) return;
+    }
+    double a0 = 0.0, a1 = 0.0;
+    for (int t = tid; t < nt && ok; t += kBlock) {
+      for (int v = 0; v < (two ? 2 : 1); ++v) {
+        const unsigned long long* p = reinterpret_cast<const unsigned long long*>(mine + v * nt + t);
+        unsigned long long b = ld_relaxed_u64(p);
+        if (direct && b == 0ull) ok = wait_for(ctl, wait_ns, [&] { return (b = ld_relaxed_u64(p)) != 0ull; });
+        if (v == 0) a0 += bitsd(b);
+        else a1 += bitsd(b);
+      }
+    }
+    if (direct && tid < nt) __threadfence();   // what the posting blocks wrote before is visible
+    red[tid] = a0;
+    if (WEIGHTED) red[(WEIGHTED ? 1 : 0) * kBlock + tid] = a1;
+    if (!__syncthreads_and(ok)) return;
+    if (tid >= 32) {
+      if (tid == 32 && blockIdx.x == 0) {    // the log, beside the epilogue
+        if (round0 + r < kRoundLog) {
+          ctl->phase_log[round0 + r] = logged;
+          ctl->t_round[round0 + r] = gtimer();
+        }
+      } else if (tid == 64 && r > 0) {       // this block's places of the round before
+        double* old = sums + (tab == 0 ? 2 : tab - 1) * 2 * nt;
+        for (int k = blockIdx.x; k < nt; k += G) {
+          old[k] = 0.0;
+          if (WEIGHTED) old[nt + k] = 0.0;
+        }
+      }
+    } else {
+      // the sums in every lane of the first warp: tree8 over the warps, then the lanes (those past
+      // the tasks hold zeros)
+      double tot[2] = {a0, a1};
+      if (nt > 32) {
+#pragma unroll
+        for (int v = 0; v < (WEIGHTED ? 2 : 1); ++v) {
+          double u[8];
+#pragma unroll
+          for (int w = 0; w < 8; ++w) u[w] = red[v * kBlock + tid + 32 * w];
+          tot[v] = tree8(u);
+        }
+      }
+      for (int o = 16; o > 0; o >>= 1) {
+        if (o >= nt) continue;
+        tot[0] += __shfl_xor_sync(kFull, tot[0], o);
+        if (two) tot[1] += __shfl_xor_sync(kFull, tot[1], o);
+      }
+      tot[0] = __shfl_sync(kFull, tot[0], 0);
+      if (two) tot[1] = __shfl_sync(kFull, tot[1], 0);
+      if (ph == PH_CG_PQ) {
+        if (tid == 0) {
+          epi_spmv_s(sh, tot);
+          sh.phase = sh.inner_active ? PH_CG_B : phase_after<T>(sh);
+        }
+      } else {
+        // upd_ratios with the two divisions and the two roots side by side in lanes 0 and 1
+        const double quot = tot[0] / (tid == 0 ? sh.rho : sh.gg0);
+        const double root = sqrt(WEIGHTED ? (tid == 0 ? tot[1] : sh.bb) : quot);
+        UpdRatios q;
+        q.shrink = quot;
+        q.first = __shfl_sync(kFull, quot, 1);
+        const double root1 = __shfl_sync(kFull, root, 1);
+        if (tid == 0) {
+          if (WEIGHTED) q.err = sh.bb > 0.0 ? root * sh.sigma_prev / root1 : 0.0;
+          else q.err = sh.gg0 > 0.0 ? root1 : 0.0;
+          epi_upd_s<T>(sh, A.opts, tot, q);
+          sh.phase = phase_after<T>(sh);
+        }
+      }
     }
     __syncthreads();
   }
   if (blockIdx.x != 0) return;
-  if ((int)threadIdx.x < kScalWords)
-    reinterpret_cast<unsigned long long*>(A.scal)[threadIdx.x] =
-        reinterpret_cast<const unsigned long long*>(&sh)[threadIdx.x];
-  if (threadIdx.x == 0) A.stamps[kStampSolveEnd] = gtimer();
+  if (tid < kScalWords)
+    reinterpret_cast<unsigned long long*>(A.scal)[tid] = reinterpret_cast<const unsigned long long*>(&sh)[tid];
+  if (tid == 0) {
+    ctl->rounds = round0 + r;
+    A.stamps[kStampSolveEnd] = gtimer();
+  }
 }
 
 typedef void (*SolveKernel)(DevArrays, SolveCtl*, int64_t, unsigned long long, int);
@@ -1819,6 +1942,11 @@ static SolveKernel solve_kernel(const Ctx& c, int fp32, bool xout, bool full) {
   return full ? solve_kernel_of<double, true, false>(c, xout) : solve_kernel_of<double, false, false>(c, xout);
 }
 
+template <typename K>
+static cudaError_t allow_smem(K kernel, int bytes) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+}
+
 // Largest co-resident grid of the persistent solve (cooperative launch bound), capped by tasks.
 int solve_grid_blocks(Ctx& c, int fp32, bool full) {
   int& cached = c.solve_blocks[full ? 1 : 0][fp32 ? 1 : 0];
@@ -1827,7 +1955,8 @@ int solve_grid_blocks(Ctx& c, int fp32, bool full) {
   const int smem = fp32 ? kPqSmem<float> : kPqSmem<double>;
   for (bool x : {false, true}) {               // one grid size for both variants
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, solve_kernel(c, fp32, x, full), kBlock, smem) != cudaSuccess)
+    if (allow_smem(solve_kernel(c, fp32, x, full), smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, solve_kernel(c, fp32, x, full), kBlock, smem) != cudaSuccess)
       return -1;
     per_sm = std::min(per_sm, n);
   }
@@ -1835,7 +1964,7 @@ int solve_grid_blocks(Ctx& c, int fp32, bool full) {
   // every SM holds the same number of blocks; tasks are handed out one at a time, so the blocks
   // of busier SMs take fewer of them
   int64_t g = (int64_t)per_sm * nsm;
-  g = std::min(g, full ? std::max(c.ntasks, c.ncg) : c.ncg);
+  g = std::min(g, full && c.ninst > 1 ? std::max(c.ntasks, c.ncg) : c.ncg);
   if (g < 1) return -1;
   cached = (int)g;
   return cached;
@@ -1848,8 +1977,8 @@ cudaError_t launch_solve(Ctx& c, bool full, unsigned long long wait_ns, int leav
   const int g = solve_grid_blocks(c, fp32 ? 1 : 0, full);
   if (g < 1) return cudaErrorInvalidConfiguration;
   const size_t skip = full ? 0 : offsetof(SolveCtl, arrived);
-  cudaError_t e = cudaMemsetAsync(reinterpret_cast<char*>(c.d_sctl) + skip, 0, solve_ctl_bytes(c.ninst) - skip,
-                                  c.stream);
+  cudaError_t e = cudaMemsetAsync(reinterpret_cast<char*>(c.d_sctl) + skip, 0,
+                                  solve_ctl_bytes(c.ninst, c.ncg) - skip, c.stream);
   if (e != cudaSuccess) return e;
   const int64_t per = fp32 ? c.opts.inner_itmax : c.opts.itmax;
   const int64_t limit = (int64_t)(c.opts.max_refine + 3) * (2 * per + 6) + 8;
@@ -1858,6 +1987,8 @@ cudaError_t launch_solve(Ctx& c, bool full, unsigned long long wait_ns, int leav
   cfg.blockDim = dim3(kBlock);
   cfg.dynamicSmemBytes = fp32 ? kPqSmem<float> : kPqSmem<double>;
   cfg.stream = c.stream;
+  e = allow_smem(solve_kernel(c, fp32 ? 1 : 0, c.A.xout != nullptr, full), (int)cfg.dynamicSmemBytes);
+  if (e != cudaSuccess) return e;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeCooperative;
   at[0].val.cooperative = 1;
@@ -1909,19 +2040,26 @@ cudaError_t launch_residual(Ctx& c, int mode, CtrlState* ctrl, cudaGraphConditio
 
 template <typename T>
 static cudaError_t launch_cg_pq(Ctx& c) {
+  const cudaError_t e = allow_smem(k_cg_pq<T>, kPqSmem<T>);
+  if (e != cudaSuccess) return e;
   k_cg_pq<T><<<(unsigned)c.ncg, kBlock, kPqSmem<T>, c.stream>>>(c.A);
+  return cudaGetLastError();
+}
+
+template <typename T>
+static cudaError_t launch_cg_upd(Ctx& c) {
+  const cudaError_t e = allow_smem(k_cg_upd<T>, kPqSmem<T>);
+  if (e != cudaSuccess) return e;
+  k_cg_upd<T><<<(unsigned)c.ncg, kBlock, kPqSmem<T>, c.stream>>>(c.A);
   return cudaGetLastError();
 }
 
 cudaError_t launch_inner_iteration(Ctx& c, int fp32, CtrlState* ctrl,
                                    cudaGraphConditionalHandle hw, int graph) {
-  const unsigned nb = (unsigned)c.ncg;
   cudaError_t e = fp32 ? launch_cg_pq<float>(c) : launch_cg_pq<double>(c);
   if (e == cudaSuccess) e = launch_finalize(c, FIN_SPMV, ctrl, hw, graph);
-  if (e != cudaSuccess) return e;
-  if (fp32) k_cg_upd<float><<<nb, kBlock, 0, c.stream>>>(c.A);
-  else k_cg_upd<double><<<nb, kBlock, 0, c.stream>>>(c.A);
-  return launch_finalize(c, FIN_UPD, ctrl, hw, graph);
+  if (e == cudaSuccess) e = fp32 ? launch_cg_upd<float>(c) : launch_cg_upd<double>(c);
+  return e == cudaSuccess ? launch_finalize(c, FIN_UPD, ctrl, hw, graph) : e;
 }
 
 cudaError_t launch_graph_step_begin(Ctx& c, CtrlState* ctrl, int launches_per_step) {
@@ -1981,10 +2119,7 @@ cudaError_t launch_single(Ctx& c, int which) {
     case HF_KERNEL_CG_P:
     case HF_KERNEL_CG_SPMV:
     case HF_KERNEL_CG_PQ: return fp32 ? launch_cg_pq<float>(c) : launch_cg_pq<double>(c);
-    case HF_KERNEL_CG_UPDATE:
-      if (fp32) k_cg_upd<float><<<(unsigned)c.ncg, kBlock, 0, c.stream>>>(c.A);
-      else k_cg_upd<double><<<(unsigned)c.ncg, kBlock, 0, c.stream>>>(c.A);
-      break;
+    case HF_KERNEL_CG_UPDATE: return fp32 ? launch_cg_upd<float>(c) : launch_cg_upd<double>(c);
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
