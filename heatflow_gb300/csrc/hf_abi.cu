@@ -245,27 +245,40 @@ int diagnose(Ctx& c) {
   return sync_scal(c);
 }
 
-// Drive one step's solve after the RHS / initial residual kernels are queued.
+int solve_grids(Ctx& c) {
+  const int fp32 = c.opts.precision == HF_PREC_MIXED ? 1 : 0;
+  if (solve_grid_blocks(c, fp32, true) < 1 || solve_grid_blocks(c, fp32, false) < 1)
+    return set_err(HF_ECUDA, "no co-resident grid for the persistent solve kernel");
+  if (!c.d_ctrl) {
+    int r = dalloc(c, &c.d_ctrl, 1);
+    if (r) return r;
+    CU(cudaMemset(c.d_ctrl, 0, sizeof(CtrlState)));
+  }
+  return HF_OK;
+}
+
+int solve_error(int32_t err, int32_t guard_hit) {
+  if (err) return set_err(HF_EDEVICE, "persistent solve: a grid barrier wait reached its time limit");
+  if (guard_hit) return set_err(HF_EDEVICE, "persistent solve reached its round bound");
+  return HF_OK;
+}
+
+// Drive one step's solve after the RHS / initial residual kernels are queued: the inner solves that
+// are due (one launch), the x update and the residual, polled once per refinement.
 int solve_loop(Ctx& c) {
-  const bool fp32 = c.opts.precision == HF_PREC_MIXED;
-  const int64_t per_solve = fp32 ? c.opts.inner_itmax : c.opts.itmax;
-  const int64_t guard = (int64_t)(c.opts.max_refine + 3) * (per_solve / c.opts.check_every + 3);
-  for (int64_t it = 0; it < guard; ++it) {
+  if (int r = solve_grids(c)) return r;
+  CU(cudaMemsetAsync(c.d_sctl, 0, solve_ctl_bytes(c.ninst, c.ncg), c.stream));
+  for (int64_t it = 0; it < (int64_t)c.opts.max_refine + 3; ++it) {
+    CU(launch_solve(c, false));
+    CU(launch_residual(c, 1));
+    c.launches += 4;
+    CU(cudaMemcpyAsync(c.h_flags, c.d_sctl, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, c.stream));
     int rc = sync_scal(c);
     if (rc) return rc;
-    bool any_outer = false, any_inner = false;
-    for (int64_t i = 0; i < c.ninst; ++i) {
-      any_outer |= c.h_scal[i].outer_active != 0;
-      any_inner |= c.h_scal[i].inner_active != 0;
-    }
+    if ((rc = solve_error(c.h_flags[0], c.h_flags[1]))) return rc;
+    bool any_outer = false;
+    for (int64_t i = 0; i < c.ninst; ++i) any_outer |= c.h_scal[i].outer_active != 0;
     if (!any_outer) return HF_OK;
-    if (any_inner) {
-      for (int k = 0; k < c.opts.check_every; ++k) CU(launch_inner_iteration(c, fp32 ? 1 : 0));
-      c.launches += 4 * c.opts.check_every;
-    } else {
-      CU(launch_residual(c, 1));
-      c.launches += 3;
-    }
   }
   return set_err(HF_EDEVICE, "solve loop did not terminate within its bound");
 }
@@ -287,110 +300,15 @@ int run_one_step(Ctx& c, int64_t itime) {
   return HF_OK;
 }
 
-// Capture one step as a CUDA graph: the solve loop is a WHILE node whose body selects, through a
-// SWITCH node, one inner CG iteration or one residual sweep; control kernels set the conditions
-// from the per-instance phase flags, so a step runs without any host round trip.
-int build_graph_cond(Ctx& c) {
-  if (!c.d_ctrl) {
-    int r = dalloc(c, &c.d_ctrl, 1);
-    if (r) return r;
-    CU(cudaMemset(c.d_ctrl, 0, sizeof(CtrlState)));
-  }
-  const bool fp32 = c.opts.precision == HF_PREC_MIXED;
-  cudaStream_t cs = nullptr, cs2 = nullptr;
-  CU(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
-  CU(cudaStreamCreateWithFlags(&cs2, cudaStreamNonBlocking));
-  cudaStream_t saved = c.stream;
-  cudaGraph_t g = nullptr;
-  std::string err;
-  auto chk = [&](cudaError_t e, const char* what) {
-    if (e != cudaSuccess && err.empty()) err = std::string(what) + ": " + cudaGetErrorString(e);
-    return e == cudaSuccess;
-  };
-  do {
-    if (!chk(cudaGraphCreate(&g, 0), "cudaGraphCreate")) break;
-    cudaGraphConditionalHandle hw;
-    if (!chk(cudaGraphConditionalHandleCreate(&hw, g, 0, cudaGraphCondAssignDefault), "handle(while)")) break;
-    if (!chk(cudaStreamBeginCaptureToGraph(cs, g, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed), "capture")) break;
-    c.stream = cs;
-    chk(launch_graph_step_begin(c, c.d_ctrl, c.tempdep ? 10 : 6), "step begin");
-    chk(launch_rhs(c), "rhs");
-    chk(launch_finalize(c, FIN_RHS, c.d_ctrl, hw, 1), "rhs finalize");
-    chk(launch_residual(c, 0, c.d_ctrl, hw, 1), "residual init");
-    cudaStreamCaptureStatus st;
-    cudaGraph_t cg = nullptr;
-    const cudaGraphNode_t* deps = nullptr;
-    size_t nd = 0;
-    chk(cudaStreamGetCaptureInfo(cs, &st, nullptr, &cg, &deps, nullptr, &nd), "capture info");
-    cudaGraphNodeParams wp = {};
-    wp.type = cudaGraphNodeTypeConditional;
-    wp.conditional.handle = hw;
-    wp.conditional.type = cudaGraphCondTypeWhile;
-    wp.conditional.size = 1;
-    cudaGraphNode_t wnode = nullptr;
-    if (!chk(cudaGraphAddNode(&wnode, cg, deps, nullptr, nd, &wp), "while node")) { cudaStreamEndCapture(cs, &g); break; }
-    cudaGraph_t body = wp.conditional.phGraph_out[0];
-    chk(cudaStreamUpdateCaptureDependencies(cs, &wnode, nullptr, 1, cudaStreamSetCaptureDependencies), "deps");
-    // loop body: select, switch, condition
-    cudaGraphConditionalHandle hs;
-    chk(cudaGraphConditionalHandleCreate(&hs, body, 2, cudaGraphCondAssignDefault), "handle(switch)");
-    chk(cudaStreamBeginCaptureToGraph(cs2, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed), "capture body");
-    c.stream = cs2;
-    chk(launch_ctrl_select(c, c.d_ctrl, hs, hw), "select");
-    cudaGraph_t cg2 = nullptr;
-    const cudaGraphNode_t* deps2 = nullptr;
-    size_t nd2 = 0;
-    chk(cudaStreamGetCaptureInfo(cs2, &st, nullptr, &cg2, &deps2, nullptr, &nd2), "capture info body");
-    cudaGraphNodeParams sp = {};
-    sp.type = cudaGraphNodeTypeConditional;
-    sp.conditional.handle = hs;
-    sp.conditional.type = cudaGraphCondTypeSwitch;
-    sp.conditional.size = 2;
-    cudaGraphNode_t snode = nullptr;
-    chk(cudaGraphAddNode(&snode, cg2, deps2, nullptr, nd2, &sp), "switch node");
-    chk(cudaStreamUpdateCaptureDependencies(cs2, &snode, nullptr, 1, cudaStreamSetCaptureDependencies), "deps body");
-    cudaGraph_t tmp = nullptr;
-    chk(cudaStreamEndCapture(cs2, &tmp), "end body");
-    if (err.empty()) {
-      chk(cudaStreamBeginCaptureToGraph(cs2, sp.conditional.phGraph_out[0], nullptr, nullptr, 0,
-                                        cudaStreamCaptureModeRelaxed), "capture cg");
-      chk(launch_inner_iteration(c, fp32 ? 1 : 0, c.d_ctrl, hw, 1), "cg iteration");
-      chk(cudaStreamEndCapture(cs2, &tmp), "end cg");
-      chk(cudaStreamBeginCaptureToGraph(cs2, sp.conditional.phGraph_out[1], nullptr, nullptr, 0,
-                                        cudaStreamCaptureModeRelaxed), "capture residual");
-      chk(launch_residual(c, 1, c.d_ctrl, hw, 1), "residual");
-      chk(cudaStreamEndCapture(cs2, &tmp), "end residual");
-    }
-    c.stream = cs;
-    chk(launch_graph_step_end(c, c.d_ctrl, nullptr), "step end");
-    if (c.tempdep) chk(launch_tempdep(c), "properties");
-    cudaGraph_t outg = nullptr;
-    chk(cudaStreamEndCapture(cs, &outg), "end capture");
-    if (err.empty()) chk(cudaGraphInstantiate(&c.graph_exec, g, 0), "instantiate");
-  } while (0);
-  c.stream = saved;
-  cudaStreamDestroy(cs);
-  cudaStreamDestroy(cs2);
-  if (!err.empty()) {
-    if (c.graph_exec) cudaGraphExecDestroy(c.graph_exec);
-    c.graph_exec = nullptr;
-    if (g) cudaGraphDestroy(g);
-    cudaGetLastError();
-    return set_err(HF_ECUDA, "graph capture: " + err);
-  }
-  c.graph = g;
-  return HF_OK;
-}
-
 // The solve of a captured step, on the capturing stream c.stream.  Whole: one cooperative kernel.
 // Split: the first residual, then a WHILE node around [the inner solves that are due as one
 // cooperative kernel, x update, residual], as kernels of their own (split_solve says where).
-int capture_solve(Ctx& c, std::string& err) {
+int capture_solve(Ctx& c, bool split, std::string& err) {
   auto chk = [&](cudaError_t e, const char* what) {
     if (e != cudaSuccess && err.empty()) err = std::string(what) + ": " + cudaGetErrorString(e);
     return e == cudaSuccess;
   };
-  if (!c.split) return chk(launch_solve(c), "persistent solve") ? HF_OK : HF_ECUDA;
+  if (!split) return chk(launch_solve(c), "persistent solve") ? HF_OK : HF_ECUDA;
   cudaStream_t cs = c.stream, cb = nullptr;
   cudaStreamCaptureStatus st;
   cudaGraph_t g = nullptr, tmp = nullptr;
@@ -424,18 +342,6 @@ int capture_solve(Ctx& c, std::string& err) {
   return err.empty() ? HF_OK : HF_ECUDA;
 }
 
-int solve_grids(Ctx& c) {
-  const int fp32 = c.opts.precision == HF_PREC_MIXED ? 1 : 0;
-  if (solve_grid_blocks(c, fp32, true) < 1 || solve_grid_blocks(c, fp32, false) < 1)
-    return set_err(HF_ECUDA, "no co-resident grid for the persistent solve kernel");
-  if (!c.d_ctrl) {
-    int r = dalloc(c, &c.d_ctrl, 1);
-    if (r) return r;
-    CU(cudaMemset(c.d_ctrl, 0, sizeof(CtrlState)));
-  }
-  return HF_OK;
-}
-
 // One solve on the context stream, outside a captured step.
 int run_solve(Ctx& c) {
   if (int r = solve_grids(c)) return r;
@@ -451,7 +357,7 @@ int run_solve(Ctx& c) {
     cudaError_t e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeRelaxed);
     if (e == cudaSuccess) {
       c.stream = cs;
-      capture_solve(c, err);
+      capture_solve(c, true, err);
       c.stream = saved;
       e = cudaStreamEndCapture(cs, &g);
     }
@@ -472,6 +378,7 @@ int run_solve(Ctx& c) {
 // solve kernel (zeroing its control block first), step end.  Five kernels per step.
 int build_graph_persistent(Ctx& c) {
   if (int r = solve_grids(c)) return r;
+  const bool split = c.split || c.opts.use_graph == 2;
   cudaStream_t cs = nullptr;
   CU(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
   cudaStream_t saved = c.stream;
@@ -483,10 +390,10 @@ int build_graph_persistent(Ctx& c) {
   };
   if (chk(cudaStreamBeginCapture(cs, cudaStreamCaptureModeRelaxed), "capture")) {
     c.stream = cs;
-    chk(launch_graph_step_begin(c, c.d_ctrl, (c.split ? 6 : 5) + (c.tempdep ? 4 : 0)), "step begin");
+    chk(launch_graph_step_begin(c, c.d_ctrl, (split ? 6 : 5) + (c.tempdep ? 4 : 0)), "step begin");
     chk(launch_rhs(c), "rhs");
     chk(launch_finalize(c, FIN_RHS, nullptr, 0, 0), "rhs finalize");
-    capture_solve(c, err);
+    capture_solve(c, split, err);
     chk(launch_graph_step_end(c, c.d_ctrl, c.d_sctl), "step end");
     if (c.tempdep) chk(launch_tempdep(c), "properties");
     chk(cudaStreamEndCapture(cs, &g), "end capture");
@@ -542,7 +449,7 @@ int build_loop_graph(Ctx& c) {
     chk(launch_graph_step_begin(c, c.d_ctrl, (c.split ? 6 : 5) + (c.tempdep ? 4 : 0)), "step begin");
     chk(launch_rhs(c), "rhs");
     chk(launch_finalize(c, FIN_RHS, nullptr, 0, 0), "rhs finalize");
-    capture_solve(c, err);
+    capture_solve(c, c.split, err);
     chk(launch_graph_step_end(c, c.d_ctrl, c.d_sctl, hl, 1), "step end");
     if (c.tempdep) chk(launch_tempdep(c), "properties");
     cudaGraph_t tmp = nullptr;
@@ -568,7 +475,7 @@ int build_graph(Ctx& c) {
       c.graph_criterion == c.opts.criterion && c.graph_mode == c.opts.use_graph)
     return HF_OK;
   drop_graph(c);
-  const int rc = c.opts.use_graph == 2 ? build_graph_cond(c) : build_graph_persistent(c);
+  const int rc = build_graph_persistent(c);
   if (rc) return rc;
   c.graph_precision = c.opts.precision;
   c.graph_criterion = c.opts.criterion;
@@ -604,7 +511,7 @@ int build_post_graph(Ctx& c) {
       c.stream = cs;
       c.A.xout = c.d_stage_x[j];
       chk(launch_finalize(c, FIN_RHS, nullptr, 0, 0), "rhs finalize");
-      capture_solve(c, err);
+      capture_solve(c, c.split, err);
       chk(launch_stage_fallback(c), "result fallback");
       chk(launch_graph_step_end(c, c.d_ctrl, c.d_sctl), "step end");
       if (c.tempdep) chk(launch_tempdep(c), "properties");
@@ -1067,9 +974,10 @@ int create_impl(const hf_problem* probs, int64_t count, const hf_solver_opts* op
   ALLOC(d_rho, N); ALLOC(d_hc, N); ALLOC(d_tau, N);
   if (c.any_em) ALLOC(d_em, N);
 #undef ALLOC
-  if (cudaMallocHost((void**)&c.h_scal, sizeof(InstScal) * count) != cudaSuccess) {
+  if (cudaMallocHost((void**)&c.h_scal, sizeof(InstScal) * count + 2 * sizeof(int32_t)) != cudaSuccess) {
     free_all(c); delete h; return set_err(HF_ENOMEM, "cudaMallocHost failed");
   }
+  c.h_flags = reinterpret_cast<int32_t*>(c.h_scal + count);
   auto fail = [&](int r) { free_all(c); delete h; return r; };
 #define CK(call) do { cudaError_t e_ = (call); if (e_ != cudaSuccess) return fail(set_err(HF_ECUDA, std::string(#call) + ": " + cudaGetErrorString(e_))); } while (0)
   CK(cudaMemsetAsync(A.counters, 0, sizeof(unsigned) * count, c.stream));
@@ -1420,10 +1328,9 @@ int hf_step_host_async(hf_ctx* h, int64_t itime, const double* tp, const double*
     CU(cudaEventRecord(ps.free, c.stream));
     c.async_host_kernels += 1;
   }
-  const int64_t per = c.opts.precision == HF_PREC_MIXED ? c.opts.inner_itmax : c.opts.itmax;
   if (early) {
     // begin the step from the device's copy of the inputs; the whole RHS as one launch
-    CU(launch_ctrl_init(c, itime, 2 * (int64_t)(c.opts.max_refine + 3) * (per + 3)));
+    CU(launch_ctrl_init(c, itime));
     CU(launch_graph_step_begin(c, c.d_ctrl, 1 + (c.split ? 6 : 5) + (c.tempdep ? 4 : 0)));
     CU(launch_rhs(c));
     c.async_host_kernels += 1;                    // control reset
@@ -1432,7 +1339,7 @@ int hf_step_host_async(hf_ctx* h, int64_t itime, const double* tp, const double*
     // its tasks (the later chunks are still on the link)
     CU(cudaStreamWaitEvent(c.stream, st.in_pp, 0));
     CU(launch_host_in(c, st.pp, 1, c.stream));
-    CU(launch_ctrl_init(c, itime, 2 * (int64_t)(c.opts.max_refine + 3) * (per + 3)));
+    CU(launch_ctrl_init(c, itime));
     // kernels of the step outside the host copies: begin, RHS per chunk, finalize, solve, result
     // fallback, end
     CU(launch_graph_step_begin(c, c.d_ctrl, nch + (c.split ? 6 : 5) + (c.tempdep ? 4 : 0)));
@@ -1498,10 +1405,8 @@ int hf_host_sync(hf_ctx* h, hf_stats* stats) {
   const int64_t steps = c.async_steps;
   c.async_steps = 0;
   c.launches += cs.launches + c.async_host_kernels;
-  if (cs.guard_hit & 2)
-    return set_err(HF_EDEVICE, "persistent solve: a grid barrier wait reached its time limit");
-  if (cs.guard_hit) return set_err(HF_EDEVICE, "captured solve loop reached its iteration bound");
   int rc;
+  if ((rc = solve_error(cs.guard_hit & 2, cs.guard_hit))) return rc;
   if (first_bad != INT64_MAX) {
     // An early-started call's uploaded inputs differed from the device copy it started from (a
     // queued array was changed): from that call on, every step runs again from its own uploaded
@@ -1551,12 +1456,9 @@ int run_steps(Ctx& c, int64_t itime0, int64_t nsteps, hf_stats* stats) {
   if (c.opts.use_graph && nsteps > 0) {
     if ((rc = build_graph(c))) return rc;
     const bool loop = c.opts.use_graph == 1 && build_loop_graph(c) == HF_OK;   // 3: per-step graphs
-    const bool fp32 = c.opts.precision == HF_PREC_MIXED;
-    const int64_t per = fp32 ? c.opts.inner_itmax : c.opts.itmax;
     CtrlState cs{};
     cs.itime = itime0;
     cs.itime_end = itime0 + nsteps;
-    cs.limit = 2 * (int64_t)(c.opts.max_refine + 3) * (per + 3);
     CU(cudaMemcpyAsync(c.d_ctrl, &cs, sizeof(cs), cudaMemcpyHostToDevice, c.stream));
     if (loop) {
       CU(cudaGraphLaunch(c.loop_exec, c.stream));                    // the whole time loop
@@ -1565,9 +1467,7 @@ int run_steps(Ctx& c, int64_t itime0, int64_t nsteps, hf_stats* stats) {
     }
     CU(cudaMemcpyAsync(&cs, c.d_ctrl, sizeof(cs), cudaMemcpyDeviceToHost, c.stream));
     CU(cudaStreamSynchronize(c.stream));
-    if (cs.guard_hit & 2)
-      return set_err(HF_EDEVICE, "persistent solve: a grid barrier wait reached its time limit");
-    if (cs.guard_hit) return set_err(HF_EDEVICE, "captured solve loop reached its iteration bound");
+    if ((rc = solve_error(cs.guard_hit & 2, cs.guard_hit))) return rc;
     c.launches += cs.launches;
     done = nsteps;
     nsteps = 0;
@@ -1861,8 +1761,7 @@ int time_solve(Ctx& c, int reps, double* ms) {
   CU(cudaMemcpy(&sc, c.d_sctl, sizeof(sc), cudaMemcpyDeviceToHost));
   std::memcpy(c.h_scal, saved.data(), sizeof(InstScal) * c.ninst);
   if ((rc = push_scal(c, true))) return rc;
-  if (sc.err) return set_err(HF_EDEVICE, "persistent solve: a grid barrier wait reached its time limit");
-  if (sc.guard_hit) return set_err(HF_EDEVICE, "persistent solve reached its round bound");
+  if ((rc = solve_error(sc.err, sc.guard_hit))) return rc;
   *ms = total / reps;
   return HF_OK;
 }
@@ -2082,21 +1981,18 @@ int hf_get_rhs(hf_ctx* h, int64_t itime, double* B, double* Q, double* Qd, doubl
 }  // extern "C"
 
 namespace {
-// The solve of hf_solve / hf_solve_device after the scalars were set up: one persistent launch
-// (use_graph = 1) or the host-polled kernels.
+// The solve of hf_solve / hf_solve_device after the scalars were set up: as a captured step runs it, or
+// polled by the host.
 int device_solve(Ctx& c) {
-  if (c.opts.use_graph == 1 || c.opts.use_graph == 3) {
-    if (int r = run_solve(c)) return r;
-    SolveCtl sc;
-    CU(cudaMemcpyAsync(&sc, c.d_sctl, sizeof(sc), cudaMemcpyDeviceToHost, c.stream));
-    CU(cudaStreamSynchronize(c.stream));
-    c.launches += 1;
-    if (sc.err) return set_err(HF_EDEVICE, "persistent solve: a grid barrier wait reached its time limit");
-    if (sc.guard_hit) return set_err(HF_EDEVICE, "persistent solve reached its round bound");
-    return HF_OK;
+  if (c.opts.use_graph == 0) {
+    CU(launch_residual(c, 0));
+    return solve_loop(c);
   }
-  CU(launch_residual(c, 0));
-  return solve_loop(c);
+  if (int r = run_solve(c)) return r;
+  CU(cudaMemcpyAsync(c.h_flags, c.d_sctl, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, c.stream));
+  CU(cudaStreamSynchronize(c.stream));
+  c.launches += 1;
+  return solve_error(c.h_flags[0], c.h_flags[1]);
 }
 }  // namespace
 

@@ -40,6 +40,7 @@ struct Ctx {
   InstBC* d_bc = nullptr;
   std::vector<void*> allocs;
   InstScal* h_scal = nullptr;    // pinned mirror for polling
+  int32_t* h_flags = nullptr;    // behind it: SolveCtl's err and guard_hit
   bool state_set = false;
   bool any_heater = false, any_power = false, any_em = false, any_case5 = false;
   // graph of one step (hf_run replays it once per step, no host synchronisation in between)

@@ -124,9 +124,7 @@ constexpr int32_t kXwThis = 1, kXwDone = 2, kXwAllowed = 4;
 // Device-side control of a captured step (CUDA graph with conditional nodes).
 struct CtrlState {
   int64_t itime;      // step index of the next step
-  int64_t loop_iter;  // body iterations of the current step's solve loop
-  int64_t limit;      // bound on body iterations per step (termination guarantee)
-  int32_t guard_hit;  // the bound was reached (reported as HF_EDEVICE)
+  int32_t guard_hit;  // a solve gave up: 2 a wait's time limit, 1 the round bound (HF_EDEVICE)
   uint32_t fin_count; // finalize blocks arrived (last one sets the loop condition)
   int64_t launches;   // kernels the captured steps launched
   int64_t itime_end;  // one past the last step of a whole-loop graph launch
@@ -531,7 +529,7 @@ cudaError_t launch_stage_fallback(Ctx& c);
 cudaError_t launch_host_check(Ctx& c, const double* sp, const double* spp, int64_t call,
                               int64_t* first, cudaStream_t stream);
 // Control block of a one-step graph launch queued without the host (async host-buffer steps).
-cudaError_t launch_ctrl_init(Ctx& c, int64_t itime, int64_t limit);
+cudaError_t launch_ctrl_init(Ctx& c, int64_t itime);
 cudaError_t launch_rhs_parts(Ctx& c, double* B, double* Q, double* Qd, double* Sc);
 cudaError_t launch_rhs_diagnose(Ctx& c);
 cudaError_t launch_adj_rhs(Ctx& c, const double* g, const double* l1, const double* l2, double* out);
@@ -540,8 +538,6 @@ cudaError_t launch_adj_grad(Ctx& c, const double* lam, const double* x, int64_t 
 cudaError_t launch_sumsq(Ctx& c, const double* b, int64_t n);
 cudaError_t launch_residual(Ctx& c, int mode, CtrlState* ctrl = nullptr,
                             cudaGraphConditionalHandle hw = 0, int graph = 0);
-cudaError_t launch_inner_iteration(Ctx& c, int fp32, CtrlState* ctrl = nullptr,
-                                   cudaGraphConditionalHandle hw = 0, int graph = 0);
 cudaError_t launch_step_end(Ctx& c);
 // Persistent solve: one cooperative launch runs the whole refinement loop of a step, or (full =
 // false) the inner solves that are due.
@@ -553,12 +549,10 @@ cudaError_t launch_single(Ctx& c, int which);
 cudaError_t launch_graph_step_begin(Ctx& c, CtrlState* ctrl, int launches_per_step);
 cudaError_t launch_graph_step_end(Ctx& c, CtrlState* ctrl, const SolveCtl* sctl,
                                   cudaGraphConditionalHandle hloop = 0, int loop = 0);
-cudaError_t launch_ctrl_select(Ctx& c, CtrlState* ctrl, cudaGraphConditionalHandle hs,
-                               cudaGraphConditionalHandle hw);
 // Finalize kernels: sum the tile partials of each instance and run the scalar epilogue of the
-// kernel that produced them.  With graph != 0 the last block also sets the loop condition hw; graph
-// = 2: the split solve's loop, whose rounds are logged.
-enum { FIN_RHS = 0, FIN_RHS_DIAG, FIN_RES_INIT, FIN_RES, FIN_SPMV, FIN_UPD };
+// kernel that produced them.  With graph != 0 (a captured split solve) the last block also sets the
+// loop condition hw, and the rounds are logged.
+enum { FIN_RHS = 0, FIN_RHS_DIAG, FIN_RES_INIT, FIN_RES };
 cudaError_t launch_finalize(Ctx& c, int kind, CtrlState* ctrl, cudaGraphConditionalHandle hw,
                             int graph);
 #ifdef HF_CHECKED

@@ -621,11 +621,9 @@ __global__ void k_stage_fallback(DevArrays A) {
 
 // itime of the next one-step launch; the kernel count and the failure flag accumulate over the
 // queued steps (reset = first step of a queue).
-__global__ void k_ctrl_init(CtrlState* ctrl, int64_t itime, int64_t limit, int reset) {
+__global__ void k_ctrl_init(CtrlState* ctrl, int64_t itime, int reset) {
   ctrl->itime = itime;
   ctrl->itime_end = itime + 1;
-  ctrl->loop_iter = 0;
-  ctrl->limit = limit;
   ctrl->fin_count = 0u;
   if (reset) {
     ctrl->guard_hit = 0;
@@ -660,8 +658,8 @@ cudaError_t launch_stage_fallback(Ctx& c) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_ctrl_init(Ctx& c, int64_t itime, int64_t limit) {
-  k_ctrl_init<<<1, 1, 0, c.stream>>>(c.d_ctrl, itime, limit, c.async_steps == 0 ? 1 : 0);
+cudaError_t launch_ctrl_init(Ctx& c, int64_t itime) {
+  k_ctrl_init<<<1, 1, 0, c.stream>>>(c.d_ctrl, itime, c.async_steps == 0 ? 1 : 0);
   return cudaGetLastError();
 }
 

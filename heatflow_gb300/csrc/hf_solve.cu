@@ -166,9 +166,8 @@ __device__ __forceinline__ void task_store_f(double* dst, float v) {
 }
 
 // ---- task bodies ---------------------------------------------------------------------------------
-// Each body does one kernel's work for one task; the standalone kernels (host-polled loop, the
-// conditional-node graph, kernel timing) and the persistent solve kernel call the same bodies, so
-// every path computes the same bits.  Vectors that some phase of the persistent kernel writes
+// Each body does one kernel's work for one task; the kernels of the split solve and the persistent
+// solve kernels call the same bodies, so every path computes the same bits.  Vectors that some phase of the persistent kernel writes
 // (temperature buffers, CG vectors) are read through plain pointers: within one launch they change
 // between rounds, so they must not be taken for read-only data.  The operator, S and the scalings
 // do not change during a solve and are read through const __restrict__ pointers.
@@ -746,7 +745,8 @@ __device__ __forceinline__ void pq_form(const DevArrays& A, const InstDesc& d, i
   PqShared<T>& sm = *reinterpret_cast<PqShared<T>*>(dyn);
   const CgPos c = cg_pos<T>(d, local);
   const int tid = threadIdx.x, nq = 1 << d.cqx, rows = kBlock >> d.cqx, prow = nq + 2;
-  const int nx = d.nx, ny = d.ny, nz = d.nz, sx = d.sx, nxy = sx * ny, n4 = nxy * nz;
+  const int nx = d.nx, ny = d.ny, nz = d.nz, sx = d.sx, nxy = sx * ny;
+  [[maybe_unused]] const int n4 = nxy * nz;
   const int z0 = c.z0, z1 = c.z1;
   const bool act = c.act;
   const int last = min(V - 1, nx - 1 - c.x);   // the vector's last grid cell; cells past it are padding
@@ -851,11 +851,12 @@ __device__ __forceinline__ void pq_form(const DevArrays& A, const InstDesc& d, i
   auto keep = [&](int z, const VT& p, const VT& po, const VT& yv) {
     const int l = HF_IXV(A, lxy + z * nxy, n4, V);
     st16(Pn + l, p);
-    if (FIRST) return;
-    VT yn;
+    if constexpr (!FIRST) {
+      VT yn;
 #pragma unroll
-    for (int i = 0; i < V; ++i) yn.v[i] = fma(alpha, po.v[i], yv.v[i]);   // y is 0 before p_0
-    st16(Y + l, yn);
+      for (int i = 0; i < V; ++i) yn.v[i] = fma(alpha, po.v[i], yv.v[i]);   // y is 0 before p_0
+      st16(Y + l, yn);
+    }
   };
   __syncthreads();                            // the block's previous task is done with shared memory
 #pragma unroll
@@ -1004,7 +1005,8 @@ __device__ __forceinline__ void upd_form(const DevArrays& A, const InstDesc& d, 
   const CgPos c = cg_pos<T>(d, local);
   const T alpha = (T)s.alpha;
   const int tid = threadIdx.x;
-  const int nxy = d.sx * d.ny, n4 = nxy * d.nz, lxy = c.y * d.sx + c.x;
+  const int nxy = d.sx * d.ny, lxy = c.y * d.sx + c.x;
+  [[maybe_unused]] const int n4 = nxy * d.nz;
   const int last = min(V - 1, d.nx - 1 - c.x);
   T* R = Vec<T>::r(A) + d.off4;
   const T* Q = Vec<T>::q(A) + d.off4;
@@ -1134,7 +1136,7 @@ __device__ __forceinline__ void upd_task(const DevArrays& A, const InstDesc& d, 
     upd_form<T, false, false>(A, d, local, s, pslot, A.pcap, dyn);
 }
 
-// ---- standalone kernels (host-polled loop, conditional-node graph, kernel timing) --------------
+// ---- kernels of the split solve; the inner passes on their own only for timing -------------------
 // A round of the split solve in its log (one thread).
 __device__ __forceinline__ void log_round(SolveCtl* ctl, int32_t phase) {
   const int64_t r = ctl->rounds;
@@ -1398,12 +1400,6 @@ template <bool INIT>
 __device__ void epi_residual(const DevArrays& A, int inst, const double* tot) {
   epi_residual_s<INIT>(A.scal[inst], A.inst[inst], A.opts, tot);
 }
-__device__ void epi_spmv(const DevArrays& A, int inst, const double* tot) { epi_spmv_s(A.scal[inst], tot); }
-template <typename T>
-__device__ void epi_upd(const DevArrays& A, int inst, const double* tot) {
-  epi_upd_s<T>(A.scal[inst], A.opts, tot, upd_ratios(A.scal[inst], A.opts, tot));
-}
-
 // Whether instance s took part in the producing kernel (the producers' own entry tests).
 template <int KIND>
 __device__ __forceinline__ bool took_part(const InstScal& s) {
@@ -1411,19 +1407,18 @@ __device__ __forceinline__ bool took_part(const InstScal& s) {
     case FIN_RHS: return s.outer_active != 0;
     case FIN_RHS_DIAG: return (s.status & kStatusRhsNan) != 0;
     case FIN_RES_INIT: return s.outer_active && !s.inner_active && s.refine == 0;
-    case FIN_RES: return s.outer_active && !s.inner_active && s.refine != 0;
-    default: return s.inner_active != 0;      // FIN_SPMV, FIN_UPD
+    default: return s.outer_active && !s.inner_active && s.refine != 0;      // FIN_RES
   }
 }
 
-template <int KIND, bool FP32>
+template <int KIND>
 __global__ void __launch_bounds__(kBlock) k_finalize(DevArrays A, CtrlState* ctrl,
                                                   cudaGraphConditionalHandle hw, int graph) {
-  constexpr int NR = (KIND == FIN_RHS_DIAG) ? 5 : (KIND == FIN_SPMV ? 1 : 2);
+  constexpr int NR = KIND == FIN_RHS_DIAG ? 5 : 2;
   const int inst = blockIdx.x;
   if (KIND == FIN_RHS && inst == 0 && threadIdx.x == 0) A.stamps[kStampFin] = gtimer();
   const InstDesc& d = A.inst[inst];
-  if (graph == 2 && inst == 0 && threadIdx.x == 0 && took_part<KIND>(A.scal[0])) {
+  if (graph && inst == 0 && threadIdx.x == 0 && took_part<KIND>(A.scal[0])) {
     log_round(A.sctl, KIND == FIN_RES ? (int32_t)HF_PHASE_RES
                                       : A.scal[0].hx_ok >= 2 ? (int32_t)HF_PHASE_RES_INIT_HX : (int32_t)HF_PHASE_RES_INIT);
     A.stamps[kStampSolveEnd] = gtimer();
@@ -1431,23 +1426,18 @@ __global__ void __launch_bounds__(kBlock) k_finalize(DevArrays A, CtrlState* ctr
   if (took_part<KIND>(A.scal[inst])) {
     double acc[NR];
     __shared__ double red[kBlock * NR];
-    constexpr bool cg = KIND == FIN_SPMV || KIND == FIN_UPD;
-    instance_sum<NR>(A.partials, A.pcap, cg ? d.cg0 : d.task0, cg ? d.cgn : d.ntask, acc, red);
+    instance_sum<NR>(A.partials, A.pcap, d.task0, d.ntask, acc, red);
     if (threadIdx.x == 0) {
       switch (KIND) {
         case FIN_RHS: epi_rhs(A, inst, acc); break;
         case FIN_RHS_DIAG: epi_rhs_diag(A, inst, acc); break;
         case FIN_RES_INIT: epi_residual<true>(A, inst, acc); break;
-        case FIN_RES: epi_residual<false>(A, inst, acc); break;
-        case FIN_SPMV: epi_spmv(A, inst, acc); break;
-        default:
-          if (FP32) epi_upd<float>(A, inst, acc); else epi_upd<double>(A, inst, acc);
-          break;
+        default: epi_residual<false>(A, inst, acc); break;
       }
     }
   }
   // loop condition of the captured solve loop: set by the last instance block to finish
-  if (graph && (KIND == FIN_RES_INIT || KIND == FIN_RES || KIND == FIN_UPD)) {
+  if (graph && (KIND == FIN_RES_INIT || KIND == FIN_RES)) {
     __shared__ bool last;
     if (threadIdx.x == 0) {
       __threadfence();
@@ -1460,11 +1450,9 @@ __global__ void __launch_bounds__(kBlock) k_finalize(DevArrays A, CtrlState* ctr
       int any_outer = 0;
       for (int64_t i = 0; i < A.ninst; ++i) any_outer |= __ldcg(&A.scal[i].outer_active);
       ctrl->fin_count = 0u;
-      if (graph == 2) {
-        // a split solve's kernel that gave up leaves its instance as it was: the loop ends there
-        if (A.sctl->err || A.sctl->guard_hit) any_outer = 0;
-        ctrl->launches += KIND == FIN_RES ? 4 : 0;
-      }
+      // a kernel of the inner solves that gave up leaves its instance as it was: the loop ends there
+      if (A.sctl->err || A.sctl->guard_hit) any_outer = 0;
+      ctrl->launches += KIND == FIN_RES ? 4 : 0;
       cudaGraphSetConditional(hw, any_outer ? 1u : 0u);
     }
   }
@@ -1475,7 +1463,6 @@ __global__ void k_graph_step_begin(DevArrays A, CtrlState* ctrl, int launches_pe
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < kStamps) A.stamps[i] = i == kStampBegin ? gtimer() : 0ull;
   if (i == 0) {
-    ctrl->loop_iter = 0;
     ctrl->launches += launches_per_step;   // the step's kernels outside the solve loop
   }
   if (i < A.ninst) begin_step(A.scal[i], ctrl->itime);
@@ -1495,29 +1482,6 @@ __global__ void k_graph_step_end(DevArrays A, CtrlState* ctrl, const SolveCtl* s
     if (sctl && (sctl->err || sctl->guard_hit)) ctrl->guard_hit |= sctl->err ? 2 : 1;
     if (loop) cudaGraphSetConditional(hloop, (ctrl->itime < ctrl->itime_end && !ctrl->guard_hit) ? 1u : 0u);
   }
-}
-
-// Branch of the solve loop body: 0 = one inner CG iteration, 1 = update + residual, 2 = nothing.
-// It also bounds the loop: past ctrl->limit body iterations (or with nothing to do) it clears the
-// loop condition, so the WHILE node always terminates.
-__global__ void k_ctrl_select(DevArrays A, CtrlState* ctrl, cudaGraphConditionalHandle hs,
-                              cudaGraphConditionalHandle hw) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  int any_inner = 0, any_outer = 0;
-  for (int64_t i = 0; i < A.ninst; ++i) {
-    any_inner |= A.scal[i].inner_active;
-    any_outer |= A.scal[i].outer_active;
-  }
-  unsigned branch = any_inner ? 0u : (any_outer ? 1u : 2u);
-  const int64_t it = ctrl->loop_iter + 1;
-  ctrl->loop_iter = it;
-  if (it > ctrl->limit) {
-    ctrl->guard_hit = 1;
-    branch = 2u;
-  }
-  ctrl->launches += 1 + (branch == 0u ? 4 : (branch == 1u ? 3 : 0));
-  if (branch == 2u) cudaGraphSetConditional(hw, 0u);
-  cudaGraphSetConditional(hs, branch);
 }
 
 // ---- persistent solve ------------------------------------------------------------------------
@@ -2033,8 +1997,8 @@ static void launch_res(Ctx& c, int mode, int log) {
 }
 cudaError_t launch_residual(Ctx& c, int mode, CtrlState* ctrl, cudaGraphConditionalHandle hw,
                             int graph) {
-  if (c.opts.precision == HF_PREC_MIXED) launch_res<float>(c, mode, graph == 2);
-  else launch_res<double>(c, mode, graph == 2);
+  if (c.opts.precision == HF_PREC_MIXED) launch_res<float>(c, mode, graph);
+  else launch_res<double>(c, mode, graph);
   return launch_finalize(c, mode == 0 ? FIN_RES_INIT : FIN_RES, ctrl, hw, graph);
 }
 
@@ -2054,14 +2018,6 @@ static cudaError_t launch_cg_upd(Ctx& c) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_inner_iteration(Ctx& c, int fp32, CtrlState* ctrl,
-                                   cudaGraphConditionalHandle hw, int graph) {
-  cudaError_t e = fp32 ? launch_cg_pq<float>(c) : launch_cg_pq<double>(c);
-  if (e == cudaSuccess) e = launch_finalize(c, FIN_SPMV, ctrl, hw, graph);
-  if (e == cudaSuccess) e = fp32 ? launch_cg_upd<float>(c) : launch_cg_upd<double>(c);
-  return e == cudaSuccess ? launch_finalize(c, FIN_UPD, ctrl, hw, graph) : e;
-}
-
 cudaError_t launch_graph_step_begin(Ctx& c, CtrlState* ctrl, int launches_per_step) {
   k_graph_step_begin<<<(unsigned)((c.ninst + 127) / 128), 128, 0, c.stream>>>(c.A, ctrl,
                                                                                launches_per_step);
@@ -2072,26 +2028,14 @@ cudaError_t launch_graph_step_end(Ctx& c, CtrlState* ctrl, const SolveCtl* sctl,
   k_graph_step_end<<<1, 256, 0, c.stream>>>(c.A, ctrl, sctl, hloop, loop);
   return cudaGetLastError();
 }
-cudaError_t launch_ctrl_select(Ctx& c, CtrlState* ctrl, cudaGraphConditionalHandle hs,
-                               cudaGraphConditionalHandle hw) {
-  k_ctrl_select<<<1, 32, 0, c.stream>>>(c.A, ctrl, hs, hw);
-  return cudaGetLastError();
-}
-
 cudaError_t launch_finalize(Ctx& c, int kind, CtrlState* ctrl, cudaGraphConditionalHandle hw,
                             int graph) {
   const unsigned nb = (unsigned)c.ninst;
-  const bool fp32 = c.opts.precision == HF_PREC_MIXED;
   switch (kind) {
-    case FIN_RHS: k_finalize<FIN_RHS, false><<<nb, 256, 0, c.stream>>>(c.A, ctrl, hw, graph); break;
-    case FIN_RHS_DIAG: k_finalize<FIN_RHS_DIAG, false><<<nb, 256, 0, c.stream>>>(c.A, ctrl, hw, graph); break;
-    case FIN_RES_INIT: k_finalize<FIN_RES_INIT, false><<<nb, 256, 0, c.stream>>>(c.A, ctrl, hw, graph); break;
-    case FIN_RES: k_finalize<FIN_RES, false><<<nb, 256, 0, c.stream>>>(c.A, ctrl, hw, graph); break;
-    case FIN_SPMV: k_finalize<FIN_SPMV, false><<<nb, 256, 0, c.stream>>>(c.A, ctrl, hw, graph); break;
-    case FIN_UPD:
-      if (fp32) k_finalize<FIN_UPD, true><<<nb, 256, 0, c.stream>>>(c.A, ctrl, hw, graph);
-      else k_finalize<FIN_UPD, false><<<nb, 256, 0, c.stream>>>(c.A, ctrl, hw, graph);
-      break;
+    case FIN_RHS: k_finalize<FIN_RHS><<<nb, 256, 0, c.stream>>>(c.A, ctrl, hw, graph); break;
+    case FIN_RHS_DIAG: k_finalize<FIN_RHS_DIAG><<<nb, 256, 0, c.stream>>>(c.A, ctrl, hw, graph); break;
+    case FIN_RES_INIT: k_finalize<FIN_RES_INIT><<<nb, 256, 0, c.stream>>>(c.A, ctrl, hw, graph); break;
+    case FIN_RES: k_finalize<FIN_RES><<<nb, 256, 0, c.stream>>>(c.A, ctrl, hw, graph); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();

@@ -95,13 +95,14 @@ typedef struct hf_solver_opts {
   double inner_tol;     /* mixed: relative reduction asked of each FP32 inner solve */
   int32_t inner_itmax;  /* mixed: max FP32 CG iterations per inner solve */
   int32_t max_refine;   /* mixed: max FP64 refinement sweeps per step */
-  int32_t check_every;  /* iterations launched between host convergence polls */
-  int32_t use_graph;    /* hf_run's step loop: 0 = kernels launched and polled by the host;
+  int32_t check_every;  /* >= 1; without effect (inner solves run on the device to their end) */
+  int32_t use_graph;    /* hf_run's step loop: 0 = kernels launched by the host, which polls once
+                           per refinement;
                            1 = the whole loop as one CUDA graph (a WHILE node around a step whose
                            inner solves are persistent cooperative kernels: no host round trip);
-                           2 = a CUDA graph per step with conditional WHILE/SWITCH nodes;
-                           3 = as 1, but one graph launch per step (kernels visible to profilers,
-                           which do not see kernels inside conditional nodes) */
+                           2 = as 3, the solve always as a WHILE node around its kernels;
+                           3 = as 1, but one graph launch per step (profilers, which do not see
+                           kernels inside conditional nodes, then see those outside the solve) */
   int32_t task_depth;   /* z-planes per task of the step kernels (0: 32, or 16/8/4 when the
                            grids would give fewer than 912 tasks; otherwise 4..1024) */
 } hf_solver_opts;
