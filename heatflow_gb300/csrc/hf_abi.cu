@@ -816,6 +816,7 @@ int build_tasks(Ctx& c, int depth) {
   CU(cudaStreamSynchronize(c.stream));
   c.depth = depth;
   for (auto& b : c.solve_blocks) b[0] = b[1] = 0;
+  c.res_depth = -1;
   c.split = split_solve(c);
   drop_graph(c);
   return HF_OK;
@@ -1115,6 +1116,7 @@ int hf_set_opts(hf_ctx* h, const hf_solver_opts* opts) {
   h->c.opts = *opts;
   h->c.A.opts = dev_opts(*opts);
   drop_graph(h->c);   // captured kernels hold the options by value
+  h->c.res_depth = -1;
   if (effective_depth(h->c, *opts) != h->c.depth || opts->precision != h->c.cg_precision)
     return build_tasks(h->c, effective_depth(h->c, *opts));
   return HF_OK;

@@ -49,6 +49,9 @@ struct Ctx {
   CtrlState* d_ctrl = nullptr;
   SolveCtl* d_sctl = nullptr;    // control block of the persistent solve kernel
   int solve_blocks[2][2] = {{0, 0}, {0, 0}};  // its co-resident grid: [full][FP64, FP32]
+  // choose_solve of one grid: planes per task of k_solve_res (0: not taken, -1: not asked yet), blocks of
+  // k_solve_cluster (0: not taken)
+  int res_depth = -1, cluster_blocks = 0;
   bool split = false;            // the solve as several kernels (split_solve)
   cudaGraphExec_t solve_exec = nullptr;   // the split solve on its own (hf_solve, timing)
   cudaGraph_t solve_graph = nullptr;

@@ -161,9 +161,9 @@ struct SolveCtl {
 };
 
 // Behind the control block.  Several grids: each instance's published ticket range, then its count of
-// finished tasks.  One grid: its blocks' sums, three tables of two values per task.
+// finished tasks.  One grid: its tasks' sums, two tables of two values per task.
 __host__ __device__ inline size_t solve_ctl_bytes(int64_t ninst, int64_t ncg) {
-  return sizeof(SolveCtl) + (ninst == 1 ? (size_t)ncg * 6 * sizeof(unsigned long long)
+  return sizeof(SolveCtl) + (ninst == 1 ? (size_t)ncg * 4 * sizeof(unsigned long long)
                                         : (size_t)ninst * (sizeof(unsigned long long) + sizeof(unsigned)));
 }
 __device__ __forceinline__ unsigned long long* solve_slots(SolveCtl* ctl) {
@@ -421,15 +421,7 @@ __device__ __forceinline__ double tree8(const double (&t)[8]) {
 // dst[k * stride].  FP64 values go through shared memory and only warp 0 adds them (8 + 5 adds per
 // value per block): on GB300 every FP64 warp instruction costs the slow FP64 pipe, so a shuffle
 // tree in all eight warps would cost more than the kernel's own arithmetic.
-// POSTED: for the blocks of the same launch that wait for the sums (post_sum).
-__device__ __forceinline__ void post_sum(double* dst, double v) {
-  // release: what the block wrote before (all of it behind a block barrier) is visible to whoever
-  // sees the sum.  A place that holds 0 has no sum yet, so +0 is posted as -0.
-  unsigned long long b = dbits(v);
-  if (b == 0ull) b = 0x8000000000000000ull;
-  asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(dst), "l"(b) : "memory");
-}
-template <int NRV, bool POSTED = false>
+template <int NRV>
 __device__ __forceinline__ void tile_store(double* dst, int64_t stride, const double (&v)[NRV]) {
   static_assert(NRV <= kNR, "reduction slots");
   static_assert(kBlock == 256, "eight warps");
@@ -455,10 +447,7 @@ __device__ __forceinline__ void tile_store(double* dst, int64_t stride, const do
     }
     if (lane == 0) {
 #pragma unroll
-      for (int k = 0; k < NRV; ++k) {
-        if (POSTED) post_sum(dst + k * stride, t[k]);
-        else dst[k * stride] = t[k];
-      }
+      for (int k = 0; k < NRV; ++k) dst[k * stride] = t[k];
     }
   }
 }

@@ -145,7 +145,6 @@ __device__ __forceinline__ T plane_above(const TCell& c, int j, V v, int z) {
 }
 
 // FP32 block sum of one value into *dst, a partial sum of a task (one conversion per block).
-template <bool POSTED = false>
 __device__ __forceinline__ void task_store_f(double* dst, float v) {
   __shared__ float red[kBlock / 32];
   __syncthreads();
@@ -158,10 +157,7 @@ __device__ __forceinline__ void task_store_f(double* dst, float v) {
     v = lane < kBlock / 32 ? red[lane] : 0.f;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
-    if (lane == 0) {
-      if (POSTED) post_sum(dst, (double)v);
-      else *dst = (double)v;
-    }
+    if (lane == 0) *dst = (double)v;
   }
 }
 
@@ -675,6 +671,11 @@ __device__ __forceinline__ Vec16<T> ld16(const T* p) {
   return *reinterpret_cast<const Vec16<T>*>(&u);
 }
 template <typename T>
+__device__ __forceinline__ Vec16<T> ld16cg(const T* p) {   // from L2
+  const uint4 u = __ldcg(reinterpret_cast<const uint4*>(p));
+  return *reinterpret_cast<const Vec16<T>*>(&u);
+}
+template <typename T>
 __device__ __forceinline__ void st16(T* p, const Vec16<T>& v) {
   *reinterpret_cast<uint4*>(p) = *reinterpret_cast<const uint4*>(&v);
 }
@@ -734,10 +735,57 @@ __device__ __forceinline__ CgPos cg_pos(const InstDesc& d, int local) {
   return c;
 }
 
+// The vector or cell beyond a tile that a thread also forms: threads 0..nq-1 the row above the tile's
+// last one, nq..2nq-1 the row below its first (with that row's y faces), then the cells beside the first
+// column (with their x faces) and beside the last.  hl: its cell in a plane, or -1; hp: its place in the
+// tile's plane of p; hvec: a vector; hc: with a face (ay, or ax for a cell).
+struct Beyond { int hl, hp; bool hvec, hc; };
+template <typename T>
+__device__ __forceinline__ Beyond beyond_of(const InstDesc& d, const CgPos& c) {
+  constexpr int V = Vec16<T>::N;
+  const int tid = threadIdx.x, nq = 1 << d.cqx, rows = kBlock >> d.cqx, prow = nq + 2;
+  const int nx = d.nx, ny = d.ny, sx = d.sx;
+  const int nv = min(nq, (nx - c.x0 + V - 1) / V), nr = min(rows, ny - c.y0);   // vectors, rows in use
+  Beyond b{-1, 0, true, false};
+  if (tid < 2 * nq) {
+    const int v = tid & (nq - 1), xv = c.x0 + v * V;
+    if (v < nv && ny > 1) {
+      if (tid < nq) {
+        if (c.y0 + nr < ny) b.hl = (c.y0 + nr) * sx + xv;
+        else if (d.py) b.hl = xv;
+        b.hp = (nr + 1) * prow + v + 1;
+      } else {
+        if (c.y0 > 0) b.hl = (c.y0 - 1) * sx + xv;
+        else if (d.py) b.hl = (ny - 1) * sx + xv;
+        b.hp = v + 1;
+        b.hc = true;
+      }
+    }
+  } else if (tid < 2 * nq + 2 * rows) {
+    const bool west = tid < 2 * nq + rows;
+    const int row = tid - 2 * nq - (west ? 0 : rows);
+    b.hvec = false;
+    if (row < nr) {
+      const int lr = (c.y0 + row) * sx, xe = c.x0 + nv * V;
+      if (west) {
+        if (c.x0 > 0) b.hl = lr + c.x0 - 1;
+        else if (d.px && nx > 1) b.hl = lr + nx - 1;
+        b.hp = (row + 1) * prow;
+        b.hc = true;
+      } else {
+        if (xe < nx) b.hl = lr + xe;
+        else if (d.px && nx > 1) b.hl = lr;
+        b.hp = (row + 1) * prow + nv + 1;
+      }
+    }
+  }
+  return b;
+}
+
 // off: the instance's first cell (d.off4; a constant 0 where there is one instance keeps the base
 // pointers out of the registers).  pslot: the place of the task's sum; dyn: kPqSmem<T> bytes of
 // shared memory.
-template <typename T, bool POSTED, bool FIRST>
+template <typename T, bool FIRST>
 __device__ __forceinline__ void pq_form(const DevArrays& A, const InstDesc& d, int64_t off, int local,
                                         const InstScal& s, double* pslot, char* dyn) {
   constexpr int V = Vec16<T>::N;
@@ -762,44 +810,9 @@ __device__ __forceinline__ void pq_form(const DevArrays& A, const InstDesc& d, i
   const T* __restrict__ az = Vec<T>::az(A) + off;
   const int lxy = c.y * sx + c.x;
   const int own = (c.ry + 1) * prow + c.vx + 1;
-  // the vector or cell beyond the tile that this thread also forms: threads 0..nq-1 the row above
-  // the tile's last one, nq..2nq-1 the row below its first (with that row's y faces), then the
-  // cells beside the first column (with their x faces) and beside the last
-  const int nv = min(nq, (nx - c.x0 + V - 1) / V), nr = min(rows, ny - c.y0);   // vectors, rows in use
-  int hl = -1, hp = 0;                         // its cell in a plane, its place in sm.p
-  bool hvec = true, hc = false;                // a vector; with a face (ay, or ax for a cell)
-  if (tid < 2 * nq) {
-    const int v = tid & (nq - 1), xv = c.x0 + v * V;
-    if (v < nv && ny > 1) {
-      if (tid < nq) {
-        if (c.y0 + nr < ny) hl = (c.y0 + nr) * sx + xv;
-        else if (d.py) hl = xv;
-        hp = (nr + 1) * prow + v + 1;
-      } else {
-        if (c.y0 > 0) hl = (c.y0 - 1) * sx + xv;
-        else if (d.py) hl = (ny - 1) * sx + xv;
-        hp = v + 1;
-        hc = true;
-      }
-    }
-  } else if (tid < 2 * nq + 2 * rows) {
-    const bool west = tid < 2 * nq + rows;
-    const int row = tid - 2 * nq - (west ? 0 : rows);
-    hvec = false;
-    if (row < nr) {
-      const int lr = (c.y0 + row) * sx, xe = c.x0 + nv * V;
-      if (west) {
-        if (c.x0 > 0) hl = lr + c.x0 - 1;
-        else if (d.px && nx > 1) hl = lr + nx - 1;
-        hp = (row + 1) * prow;
-        hc = true;
-      } else {
-        if (xe < nx) hl = lr + xe;
-        else if (d.px && nx > 1) hl = lr;
-        hp = (row + 1) * prow + nv + 1;
-      }
-    }
-  }
+  const Beyond by = beyond_of<T>(d, c);
+  const int hl = by.hl, hp = by.hp;
+  const bool hvec = by.hvec, hc = by.hc;
   // where the faces below this thread's row and beside its first cell come from
   const bool hsouth = ny > 1 && (c.y > 0 || d.py), hwest = nx > 1 && (c.x > 0 || d.px);
   const VT zero{};
@@ -964,18 +977,18 @@ __device__ __forceinline__ void pq_form(const DevArrays& A, const InstDesc& d, i
   }
   dot += dot8;
   if constexpr (sizeof(T) == 4) {
-    task_store_f<POSTED>(pslot, dot);
+    task_store_f(pslot, dot);
   } else {
     const double v[1] = {dot};
-    tile_store<1, POSTED>(pslot, 0, v);
+    tile_store<1>(pslot, 0, v);
   }
 }
 // Iteration 0 (p = r, no y) is a form of its own.
-template <typename T, bool POSTED>
+template <typename T>
 __device__ __forceinline__ void pq_task(const DevArrays& A, const InstDesc& d, int64_t off, int local,
                                         const InstScal& s, double* pslot, char* dyn) {
-  if (s.iter == 0) pq_form<T, POSTED, true>(A, d, off, local, s, pslot, dyn);
-  else pq_form<T, POSTED, false>(A, d, off, local, s, pslot, dyn);
+  if (s.iter == 0) pq_form<T, true>(A, d, off, local, s, pslot, dyn);
+  else pq_form<T, false>(A, d, off, local, s, pslot, dyn);
 }
 
 // r -= alpha q and r.r (and the unscaled ||r||^2 for the reference rule).  The planes are walked
@@ -997,7 +1010,7 @@ struct UpdXStage {                                            // one plane
 static_assert(3 * sizeof(UpdStage<float>) <= sizeof(PqShared<float>) && 3 * sizeof(UpdStage<double>) <= sizeof(PqShared<double>) &&
                   3 * sizeof(UpdXStage<float>) <= sizeof(PqShared<float>) && 3 * sizeof(UpdXStage<double>) <= sizeof(PqShared<double>),
               "the update's stages fit the pq pass's shared memory");
-template <typename T, bool WEIGHTED, bool POSTED>
+template <typename T, bool WEIGHTED>
 __device__ __forceinline__ void upd_form(const DevArrays& A, const InstDesc& d, int local, const InstScal& s,
                                          double* pslot, int64_t stride, char* dyn) {
   constexpr int V = Vec16<T>::N;
@@ -1118,22 +1131,22 @@ __device__ __forceinline__ void upd_form(const DevArrays& A, const InstDesc& d, 
   }
   rr += rr8;
   if constexpr (sizeof(T) == 4) {
-    task_store_f<POSTED>(pslot, rr);
+    task_store_f(pslot, rr);
   } else if constexpr (WEIGHTED) {
     const double v[2] = {rr, rw};
-    tile_store<2, POSTED>(pslot, stride, v);
+    tile_store<2>(pslot, stride, v);
   } else {
     const double v[1] = {rr};
-    tile_store<1, POSTED>(pslot, stride, v);
+    tile_store<1>(pslot, stride, v);
   }
 }
 template <typename T>
 __device__ __forceinline__ void upd_task(const DevArrays& A, const InstDesc& d, int local, const InstScal& s,
                                          double* pslot, char* dyn) {
   if (sizeof(T) == 8 && A.opts.criterion == HF_STOP_RECURSIVE)
-    upd_form<T, sizeof(T) == 8, false>(A, d, local, s, pslot, A.pcap, dyn);
+    upd_form<T, sizeof(T) == 8>(A, d, local, s, pslot, A.pcap, dyn);
   else
-    upd_form<T, false, false>(A, d, local, s, pslot, A.pcap, dyn);
+    upd_form<T, false>(A, d, local, s, pslot, A.pcap, dyn);
 }
 
 // ---- kernels of the split solve; the inner passes on their own only for timing -------------------
@@ -1175,7 +1188,7 @@ __global__ void __launch_bounds__(kBlock) k_cg_pq(DevArrays A) {
   const InstScal& s = A.scal[inst];
   if (!s.inner_active) return;
   const InstDesc& d = A.inst[inst];
-  pq_task<T, false>(A, d, d.off4, (int)(blockIdx.x - d.cg0), s, A.partials + blockIdx.x, dyn);
+  pq_task<T>(A, d, d.off4, (int)(blockIdx.x - d.cg0), s, A.partials + blockIdx.x, dyn);
 }
 
 template <typename T>
@@ -1568,8 +1581,8 @@ __device__ __noinline__ void phase_epilogue(InstScal& sc, const InstDesc& d, con
 template <typename T, bool XOUT, bool FULL, bool WEIGHTED>
 __device__ __forceinline__ void round_task(const DevArrays& A, const InstDesc& d, double* part, int local,
                                            const InstScal& s, char* dyn) {
-  if (s.phase == PH_CG_PQ) pq_task<T, false>(A, d, d.off4, local, s, part + d.cg0 + local, dyn);
-  else if (s.phase == PH_CG_B) upd_form<T, WEIGHTED, false>(A, d, local, s, part + d.cg0 + local, A.pcap, dyn);
+  if (s.phase == PH_CG_PQ) pq_task<T>(A, d, d.off4, local, s, part + d.cg0 + local, dyn);
+  else if (s.phase == PH_CG_B) upd_form<T, WEIGHTED>(A, d, local, s, part + d.cg0 + local, A.pcap, dyn);
   if constexpr (FULL) {
     const int64_t task = d.task0 + local;
     switch (s.phase) {
@@ -1727,22 +1740,13 @@ __global__ void __launch_bounds__(kBlock, 2)
 
 // ---- persistent solve of one grid ------------------------------------------------------------
 // The inner solve that is due, in grid-wide rounds (a pq or an update pass each).  Every block keeps
-// the scalars itself: after each round it adds the sums that all tasks posted (the same adds in the
-// same order, so all blocks obtain the same bits) and runs the scalar epilogue on its own copy in
-// shared memory.  Where the last block to arrive at a barrier does that for all, each round holds six
-// dependent trips through L2, which was most of a small grid's round.
-// Up to kDirectTasks tasks, a block waits for the sums themselves: posting one is the arrival, and a
-// round is one trip through L2 from the last task's end to the next round.  With more, that many
-// polls from every block get in each other's way (256 tasks: 8.2 against 5.3 us an update round), and
-// a counter is waited for first, by one thread.
-// Every block has at least one task, the tasks are dealt in turn, so no block passes round r before
-// all have posted round r: the sums of round r - 1 are then read by all, and each block clears its
-// places of that table, which round r + 2 uses (three tables).
-// Measured per CG iteration (two rounds; three at first): 25 x 25 x 1 under the reference's rule
-// 29 us with the epilogue in one block, 13.8 with a barrier and the epilogue in every block, 11.0 with
-// posted sums and the epilogue's divisions and roots side by side; the 64^3 slab, mixed, 34, 14.3 and
-// 11.8.
-constexpr int kDirectTasks = 32;
+// the scalars itself: after each round it adds the sums of all tasks (the same adds in the same order,
+// so all blocks obtain the same bits) and runs the scalar epilogue on its own copy in shared memory.
+// Where the last block to arrive at a barrier does that for all, each round holds six dependent trips
+// through L2, which was most of a small grid's round (64^3 slab, mixed, per iteration: 34 us in that
+// form and three rounds, 14.3 in two with the epilogue in every block, 11.8 with the epilogue's
+// divisions and roots side by side).  No block passes round r before all have arrived at its end, and
+// the sums of round r - 1 have then been read by all: two tables, taken in turn.
 // Wait until done() (one thread), in bounded time and polls; false: given up, and SolveCtl::err says so.
 template <class F>
 __device__ __forceinline__ int wait_for(SolveCtl* ctl, unsigned long long wait_ns, F done) {
@@ -1761,6 +1765,90 @@ __device__ __forceinline__ int wait_for(SolveCtl* ctl, unsigned long long wait_n
     __nanosleep(32);
   }
   return 1;
+}
+
+// The scalar epilogue of a round, by the first warp: tot[] valid in lane 0.  The divisions and the roots
+// of upd_ratios side by side in lanes 0 and 1.
+template <typename T, bool WEIGHTED>
+__device__ __forceinline__ void round_epilogue(InstScal& sh, const DevOpts& o, int32_t ph, double (&tot)[2]) {
+  const int lane = threadIdx.x & 31;
+  tot[0] = __shfl_sync(kFull, tot[0], 0);
+  if (WEIGHTED) tot[1] = __shfl_sync(kFull, tot[1], 0);
+  if (ph == PH_CG_PQ) {
+    if (lane == 0) {
+      epi_spmv_s(sh, tot);
+      sh.phase = sh.inner_active ? PH_CG_B : phase_after<T>(sh);
+    }
+    return;
+  }
+  const double quot = tot[0] / (lane == 0 ? sh.rho : sh.gg0);
+  const double root = sqrt(WEIGHTED ? (lane == 0 ? tot[1] : sh.bb) : quot);
+  UpdRatios q;
+  q.shrink = quot;
+  q.first = __shfl_sync(kFull, quot, 1);
+  const double root1 = __shfl_sync(kFull, root, 1);
+  if (lane == 0) {
+    if (WEIGHTED) q.err = sh.bb > 0.0 ? root * sh.sigma_prev / root1 : 0.0;
+    else q.err = sh.gg0 > 0.0 ? root1 : 0.0;
+    epi_upd_s<T>(sh, o, tot, q);
+    sh.phase = phase_after<T>(sh);
+  }
+}
+
+// A block's arrival at the end of a round, after its last task's sums (which thread 0 wrote, behind a
+// block barrier after all else that the task wrote).
+__device__ __forceinline__ void round_arrive(SolveCtl* ctl) {
+  if (threadIdx.x == 0) red_release_add_u64(&ctl->arrived, 1ull);
+}
+// The end of round r, whose sums lie at `sums` (nt first values, then nt second ones): wait for all
+// blocks, add the sums, run the round's epilogue on sh.  false: the wait gave up.
+template <typename T, bool WEIGHTED>
+__device__ __forceinline__ bool round_finish(const DevArrays& A, SolveCtl* ctl, unsigned long long wait_ns, InstScal& sh,
+                                             double* red, const double* sums, int nt, int64_t r, int64_t round0,
+                                             int32_t ph, int32_t logged) {
+  const int tid = threadIdx.x, G = (int)gridDim.x;
+  const bool two = WEIGHTED && ph == PH_CG_B;
+  int ok = 1;
+  if (tid == 0)
+    ok = wait_for(ctl, wait_ns, [&] {
+      return ld_acquire_u64(&ctl->arrived) >= (unsigned long long)G * (unsigned long long)(r + 1);
+    });
+  if (!__syncthreads_and(ok)) return false;
+  double a0 = 0.0, a1 = 0.0;
+  for (int t = tid; t < nt; t += kBlock) {
+    a0 += bitsd(ld_relaxed_u64(reinterpret_cast<const unsigned long long*>(sums + t)));
+    if (two) a1 += bitsd(ld_relaxed_u64(reinterpret_cast<const unsigned long long*>(sums + nt + t)));
+  }
+  red[tid] = a0;
+  if (WEIGHTED) red[(WEIGHTED ? 1 : 0) * kBlock + tid] = a1;
+  __syncthreads();
+  if (tid >= 32) {
+    if (tid == 32 && blockIdx.x == 0 && round0 + r < kRoundLog) {   // the log, beside the epilogue
+      ctl->phase_log[round0 + r] = logged;
+      ctl->t_round[round0 + r] = gtimer();
+    }
+  } else {
+    // the sums in every lane of the first warp: tree8 over the warps, then the lanes (those past
+    // the tasks hold zeros)
+    double tot[2] = {a0, a1};
+    if (nt > 32) {
+#pragma unroll
+      for (int v = 0; v < (WEIGHTED ? 2 : 1); ++v) {
+        double u[8];
+#pragma unroll
+        for (int w = 0; w < 8; ++w) u[w] = red[v * kBlock + tid + 32 * w];
+        tot[v] = tree8(u);
+      }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      if (o >= nt) continue;
+      tot[0] += __shfl_xor_sync(kFull, tot[0], o);
+      if (two) tot[1] += __shfl_xor_sync(kFull, tot[1], o);
+    }
+    round_epilogue<T, WEIGHTED>(sh, A.opts, ph, tot);
+  }
+  __syncthreads();
+  return true;
 }
 
 // WEIGHTED: the reference's stopping rule (upd_form).
@@ -1782,109 +1870,637 @@ __global__ void __launch_bounds__(kBlock, 2)
   __syncthreads();
   if (tid == 0) sh.phase = PH_CG_PQ;
   const int nt = sd.cgn;
-  const bool direct = nt <= kDirectTasks;
-  double* const sums = reinterpret_cast<double*>(solve_slots(ctl));
+  double* const sums = reinterpret_cast<double*>(solve_slots(ctl));   // two tables
   const int64_t round0 = ctl->rounds;        // of the log
   __syncthreads();
   int64_t r = 0;
-  for (int tab = 0; cg_phase(sh.phase); ++r, tab = tab == 2 ? 0 : tab + 1) {
+  for (; cg_phase(sh.phase); ++r) {
     if (r >= limit) {
       if (blockIdx.x == 0 && tid == 0) ctl->guard_hit = 1;
       break;
     }
     const int32_t ph = sh.phase;             // read before any thread can run the epilogue
     const int32_t logged = logged_phase(sh);
-    double* const mine = sums + tab * 2 * nt;
+    double* const mine = sums + (r & 1) * 2 * nt;
     // failure-path check only (leaver >= 0): that block leaves without posting, so the others'
     // waits run out and record SolveCtl::err
     if ((int)blockIdx.x == leaver) return;
     for (int k = blockIdx.x; k < nt; k += G) {
-      if (ph == PH_CG_PQ) pq_task<T, true>(A, sd, 0, k, sh, mine + k, dyn);
-      else upd_form<T, WEIGHTED, true>(A, sd, k, sh, mine + k, nt, dyn);
+      if (ph == PH_CG_PQ) pq_task<T>(A, sd, 0, k, sh, mine + k, dyn);
+      else upd_form<T, WEIGHTED>(A, sd, k, sh, mine + k, nt, dyn);
     }
-    const bool two = WEIGHTED && ph == PH_CG_B;
-    int ok = 1;
-    if (!direct) {
-      __syncthreads();                       // the block's work is done
-      if (tid == 0) {
-        red_release_add_u64(&ctl->arrived, 1ull);
-        ok = wait_for(ctl, wait_ns, [&] {
-          return ld_acquire_u64(&ctl->arrived) >= (unsigned long long)G * (unsigned long long)(r + 1);
-        });
+    round_arrive(ctl);
+    if (!round_finish<T, WEIGHTED>(A, ctl, wait_ns, sh, red, mine, nt, r, round0, ph, logged)) return;
+  }
+  if (blockIdx.x != 0) return;
+  if (tid < kScalWords)
+    reinterpret_cast<unsigned long long*>(A.scal)[tid] = reinterpret_cast<const unsigned long long*>(&sh)[tid];
+  if (tid == 0) {
+    ctl->rounds = round0 + r;
+    A.stamps[kStampSolveEnd] = gtimer();
+  }
+}
+
+// ---- persistent solve of one grid that fits on the chip ------------------------------------------
+// As k_solve_one, one task per block, with the task's vectors and faces in shared memory for the whole
+// inner solve, where the tasks are no more than the blocks that run at once and their planes fit.  Of
+// the cells around the task a block also keeps p and r, and updates them as their owner does, so only
+// q crosses memory: a round's passes touch no memory before their sum is posted but to store q, and what
+// else there is (y, the neighbours' q, the fused x update) is done while the sums travel.  q lies in
+// the p buffers by the iteration's parity: a block may still read iteration k's while another stores
+// that of k + 1.  A direction enters y in the update that follows it, so y is complete at the end
+// (InstScal::ypend = 0).  The arithmetic and its order are those of pq_form and upd_form.
+// Bound by the latency of a round (post, poll, the sums' adds and the epilogue's division).  Measured per
+// CG iteration, against k_solve_one: the 64^3 slab, mixed, 8.8 us (11.8); 48^3 mixed 7.3 (9.6); 40 FP64
+// tiles under the reference's rule 10.4 (13.3).
+template <typename T>
+struct ResLayout {                             // offsets in 16-byte vectors, for tasks of D planes
+  static constexpr int kPlane = 340, kHalo = 80;
+  int r, q, ax, ay, az, hr, hf, ur, azm, dg, n;
+  bool has_dg;
+  __host__ __device__ ResLayout(int D, bool weighted) {
+    r = (D + 2) * kPlane;                      // p first: the task's planes and the two beside them
+    q = r + D * kBlock;
+    ax = q + D * kBlock;
+    ay = ax + D * kBlock;
+    az = ay + D * kBlock;
+    hr = az + D * kBlock;                      // r and the faces of the cells beyond the tile (Beyond)
+    hf = hr + D * kHalo;
+    ur = hf + D * kHalo;                       // r of the planes above and below
+    azm = ur + 2 * kBlock;                     // faces to the plane below
+    dg = azm + kBlock;                         // diag (the reference's rule), if two blocks still fit
+    has_dg = weighted && D <= 2;
+    n = dg + (has_dg ? D * kBlock : 0);
+  }
+};
+
+template <typename T, bool WEIGHTED>
+__global__ void __launch_bounds__(kBlock, 2)
+    k_solve_res(DevArrays A, SolveCtl* ctl, int64_t limit, unsigned long long wait_ns, int leaver, int depth) {
+  constexpr int V = Vec16<T>::N, kPlane = ResLayout<T>::kPlane, kHalo = ResLayout<T>::kHalo;
+  typedef Vec16<T> VT;
+  __shared__ InstScal sh;
+  __shared__ InstDesc sd;
+  __shared__ double red[(WEIGHTED ? 2 : 1) * kBlock];
+  extern __shared__ __align__(16) char dyn[];
+  const int tid = threadIdx.x;
+  if (tid < kScalWords)
+    reinterpret_cast<unsigned long long*>(&sh)[tid] = reinterpret_cast<const unsigned long long*>(A.scal)[tid];
+  if (tid < (int)(sizeof(InstDesc) / 8))
+    reinterpret_cast<unsigned long long*>(&sd)[tid] = reinterpret_cast<const unsigned long long*>(A.inst)[tid];
+  __syncthreads();
+  if (!sh.inner_active) return;                // no inner solve is due
+  __syncthreads();
+  if (tid == 0) sh.phase = PH_CG_PQ;
+  const int nt = sd.cgn;
+  double* const sums = reinterpret_cast<double*>(solve_slots(ctl));
+  const int64_t round0 = ctl->rounds;          // of the log
+
+  const ResLayout<T> lay(depth, WEIGHTED);
+  VT* const P = reinterpret_cast<VT*>(dyn);
+  const CgPos c = cg_pos<T>(sd, (int)blockIdx.x);
+  const Beyond by = beyond_of<T>(sd, c);
+  const int nq = 1 << sd.cqx, prow = nq + 2, nx = sd.nx, ny = sd.ny, nz = sd.nz, sx = sd.sx, nxy = sx * ny;
+  [[maybe_unused]] const int n4 = nxy * nz;
+  const int z0 = c.z0, D = c.z1 - c.z0, lxy = c.y * sx + c.x, own = (c.ry + 1) * prow + c.vx + 1;
+  const bool act = c.act;
+  const int last = min(V - 1, nx - 1 - c.x);
+  const bool hsouth = ny > 1 && (c.y > 0 || sd.py), hwest = nx > 1 && (c.x > 0 || sd.px);
+  // the planes above and below the task (or their wraps), or -1
+  const int zu = nz < 2 ? -1 : c.z1 < nz ? c.z1 : sd.pz ? 0 : -1, zd = nz < 2 ? -1 : z0 > 0 ? z0 - 1 : sd.pz ? nz - 1 : -1;
+  const VT zero{};
+  // this thread's vectors
+  VT* const R = P + lay.r + tid;
+  VT* const Qs = P + lay.q + tid;
+  VT* const AX = P + lay.ax + tid;
+  VT* const AY = P + lay.ay + tid;
+  VT* const AZ = P + lay.az + tid;
+  VT* const HR = P + lay.hr + tid;             // (threads below kHalo)
+  VT* const UR = P + lay.ur + tid;
+  auto at = [&](int l, int z) { return HF_IXV(A, l + z * nxy, n4, V); };
+  auto diag_of = [&](int k) -> VT {
+    VT g = zero;
+#pragma unroll
+    for (int i = 0; i < V; ++i)
+      if (i <= last) g.v[i] = (T)A.diag[HF_IX(A, ((z0 + k) * ny + c.y) * nx + c.x + i, nx * ny * nz)];
+    return g;
+  };
+  for (int i = tid; i < (D + 2) * kPlane; i += kBlock) P[i] = zero;
+  for (int k = 0; k < D; ++k) {
+    const int l = act ? at(lxy, z0 + k) : 0;
+    R[k * kBlock] = act ? ld16(Vec<T>::r(A) + l) : zero;
+    AX[k * kBlock] = act ? ld16(Vec<T>::ax(A) + l) : zero;
+    AY[k * kBlock] = act ? ld16(Vec<T>::ay(A) + l) : zero;
+    AZ[k * kBlock] = act ? ld16(Vec<T>::az(A) + l) : zero;
+    Qs[k * kBlock] = zero;
+    if (WEIGHTED && lay.has_dg) P[lay.dg + k * kBlock + tid] = act ? diag_of(k) : zero;
+    if (by.hl >= 0) {
+      VT h = zero, f = zero;
+      if (by.hvec) {
+        const int lh = at(by.hl, z0 + k);
+        h = ld16(Vec<T>::r(A) + lh);
+        if (by.hc) f = ld16(Vec<T>::ay(A) + lh);
+      } else {
+        const int lh = HF_IX(A, by.hl + (z0 + k) * nxy, n4);
+        h.v[0] = Vec<T>::r(A)[lh];
+        if (by.hc) f.v[0] = Vec<T>::ax(A)[lh];
       }
-      if (!__syncthreads_and(ok)) return;
+      HR[k * kHalo] = h;
+      P[lay.hf + k * kHalo + tid] = f;
     }
-    double a0 = 0.0, a1 = 0.0;
-    for (int t = tid; t < nt && ok; t += kBlock) {
-      for (int v = 0; v < (two ? 2 : 1); ++v) {
-        const unsigned long long* p = reinterpret_cast<const unsigned long long*>(mine + v * nt + t);
-        unsigned long long b = ld_relaxed_u64(p);
-        if (direct && b == 0ull) ok = wait_for(ctl, wait_ns, [&] { return (b = ld_relaxed_u64(p)) != 0ull; });
-        if (v == 0) a0 += bitsd(b);
-        else a1 += bitsd(b);
-      }
+  }
+  UR[0] = act && zu >= 0 ? ld16(Vec<T>::r(A) + at(lxy, zu)) : zero;
+  UR[kBlock] = act && zd >= 0 ? ld16(Vec<T>::r(A) + at(lxy, zd)) : zero;
+  P[lay.azm + tid] = act && zd >= 0 ? ld16(Vec<T>::az(A) + at(lxy, zd)) : zero;
+  __syncthreads();
+
+  int64_t r = 0;
+  for (; cg_phase(sh.phase); ++r) {
+    if (r >= limit) {
+      if (blockIdx.x == 0 && tid == 0) ctl->guard_hit = 1;
+      break;
     }
-    if (direct && tid < nt) __threadfence();   // what the posting blocks wrote before is visible
-    red[tid] = a0;
-    if (WEIGHTED) red[(WEIGHTED ? 1 : 0) * kBlock + tid] = a1;
-    if (!__syncthreads_and(ok)) return;
-    if (tid >= 32) {
-      if (tid == 32 && blockIdx.x == 0) {    // the log, beside the epilogue
-        if (round0 + r < kRoundLog) {
-          ctl->phase_log[round0 + r] = logged;
-          ctl->t_round[round0 + r] = gtimer();
+    const int32_t ph = sh.phase;               // read before any thread can run the epilogue
+    const int32_t logged = logged_phase(sh);
+    double* const mine = sums + (r & 1) * 2 * nt;
+    if ((int)blockIdx.x == leaver) return;     // failure-path check only (k_solve_one)
+    const bool first = sh.iter == 0;
+    const T alpha = (T)sh.alpha;
+    T* const Q = Vec<T>::pb(A, sh.iter);
+    if (ph == PH_CG_PQ) {
+      const T beta = (T)sh.beta;
+      auto form = [&](VT* p, const VT& rv) {   // p = r + beta p
+        VT t = rv;
+        if (!first) {
+          const VT po = *p;
+#pragma unroll
+          for (int i = 0; i < V; ++i) t.v[i] = fma(beta, po.v[i], t.v[i]);
         }
-      } else if (tid == 64 && r > 0) {       // this block's places of the round before
-        double* old = sums + (tab == 0 ? 2 : tab - 1) * 2 * nt;
-        for (int k = blockIdx.x; k < nt; k += G) {
-          old[k] = 0.0;
-          if (WEIGHTED) old[nt + k] = 0.0;
+        *p = t;
+      };
+      if (act) {
+        for (int k = 0; k < D; ++k) form(P + (k + 1) * kPlane + own, R[k * kBlock]);
+        if (zd >= 0) form(P + own, UR[kBlock]);
+        if (zu >= 0) form(P + (D + 1) * kPlane + own, UR[0]);
+      }
+      if (by.hl >= 0) {
+        for (int k = 0; k < D; ++k) {
+          VT* const p = P + (k + 1) * kPlane + by.hp;
+          if (by.hvec) {
+            form(p, HR[k * kHalo]);
+          } else {
+            T& e = p->v[by.hc ? V - 1 : 0];
+            const T h = HR[k * kHalo].v[0];
+            e = first ? h : fma(beta, e, h);
+          }
         }
       }
+      __syncthreads();
+      T dot = T(0);
+      if (act) {
+        VT azm = P[lay.azm + tid];
+        for (int k = 0; k < D; ++k) {
+          const VT *pc = P + (k + 1) * kPlane, *hf = P + lay.hf + k * kHalo;
+          const VT axv = AX[k * kBlock], ayv = AY[k * kBlock], azv = AZ[k * kBlock];
+          const VT p = pc[own], pn = pc[own + prow], ps = pc[own - prow], pa = pc[own + kPlane], pd = pc[own - kPlane];
+          VT ays = zero;
+          if (hsouth) ays = c.ry > 0 ? AY[k * kBlock - nq] : hf[nq + c.vx];
+          T axw = T(0);
+          if (hwest) axw = c.vx > 0 ? AX[k * kBlock - 1].v[V - 1] : hf[2 * nq + c.ry].v[0];
+          const T pw = pc[own - 1].v[V - 1], pe = pc[own + 1].v[0];
+          VT qv;
+#pragma unroll
+          for (int i = 0; i < V; ++i) {
+            const T pi = p.v[i];
+            T acc = pi;
+            acc = fma(axv.v[i], i < last ? p.v[i < V - 1 ? i + 1 : i] : pe, acc);
+            acc = fma(i > 0 ? axv.v[i > 0 ? i - 1 : 0] : axw, i > 0 ? p.v[i > 0 ? i - 1 : 0] : pw, acc);
+            acc = fma(ayv.v[i], pn.v[i], acc);
+            acc = fma(ays.v[i], ps.v[i], acc);
+            acc = fma(azv.v[i], pa.v[i], acc);
+            acc = fma(azm.v[i], pd.v[i], acc);
+            if (i > last) acc = T(0);          // padding: q stays 0
+            dot = fma(pi, acc, dot);
+            qv.v[i] = acc;
+          }
+          Qs[k * kBlock] = qv;
+          st16(Q + at(lxy, z0 + k), qv);
+          azm = azv;
+        }
+      }
+      if constexpr (sizeof(T) == 4) {
+        task_store_f(mine + blockIdx.x, dot);
+      } else {
+        const double v[1] = {dot};
+        tile_store<1>(mine + blockIdx.x, 0, v);
+      }
+      round_arrive(ctl);
     } else {
-      // the sums in every lane of the first warp: tree8 over the warps, then the lanes (those past
-      // the tasks hold zeros)
-      double tot[2] = {a0, a1};
-      if (nt > 32) {
+      T rr = T(0);
+      double rw = 0.0;
+      for (int k = D - 1; k >= 0 && act; --k) {   // (the order of upd_form)
+        const VT qv = Qs[k * kBlock];
+        VT rv = R[k * kBlock], dg = zero;
+        if (WEIGHTED) dg = lay.has_dg ? P[lay.dg + k * kBlock + tid] : diag_of(k);
 #pragma unroll
-        for (int v = 0; v < (WEIGHTED ? 2 : 1); ++v) {
-          double u[8];
-#pragma unroll
-          for (int w = 0; w < 8; ++w) u[w] = red[v * kBlock + tid + 32 * w];
-          tot[v] = tree8(u);
+        for (int i = 0; i < V; ++i) {
+          T x = fma(-alpha, qv.v[i], rv.v[i]);
+          if (i > last) x = T(0);
+          rv.v[i] = x;
+          rr = fma(x, x, rr);
+          if (WEIGHTED && i <= last) rw = fma(-(double)dg.v[i] * (double)x, (double)x, rw);
         }
+        R[k * kBlock] = rv;
+      }
+      if constexpr (sizeof(T) == 4) {
+        task_store_f(mine + blockIdx.x, rr);
+      } else if constexpr (WEIGHTED) {
+        const double v[2] = {rr, rw};
+        tile_store<2>(mine + blockIdx.x, nt, v);
+      } else {
+        const double v[1] = {rr};
+        tile_store<1>(mine + blockIdx.x, 0, v);
+      }
+      round_arrive(ctl);
+      // while the sums travel
+      auto upd = [&](VT* x, int l) {           // r of the cells beside the task
+        const VT q = ld16cg(Q + l);
+        VT t = *x;
+#pragma unroll
+        for (int i = 0; i < V; ++i) t.v[i] = fma(-alpha, q.v[i], t.v[i]);
+        *x = t;
+      };
+      if (act) {
+        if (zu >= 0) upd(UR, at(lxy, zu));
+        if (zd >= 0) upd(UR + kBlock, at(lxy, zd));
+      }
+      if (by.hl >= 0) {
+        for (int k = 0; k < D; ++k) {
+          if (by.hvec) {
+            upd(HR + k * kHalo, at(by.hl, z0 + k));
+          } else {
+            T& e = HR[k * kHalo].v[0];
+            e = fma(-alpha, __ldcg(Q + HF_IX(A, by.hl + (z0 + k) * nxy, n4)), e);
+          }
+        }
+      }
+      const bool form_x = !WEIGHTED && (sh.xw & kXwThis);   // (never under the reference's rule)
+      for (int k = 0; k < D && act; ++k) {
+        const int l = at(lxy, z0 + k);
+        const VT p = P[(k + 1) * kPlane + own];
+        VT y = zero;
+        if (!first) y = ld16(Vec<T>::y(A) + l);
+#pragma unroll
+        for (int i = 0; i < V; ++i) y.v[i] = fma(alpha, p.v[i], y.v[i]);
+        st16(Vec<T>::y(A) + l, y);
+        if (form_x) {                          // rows of 4k cells: both layouts index alike
+          const double* XR = A.tbuf[sh.role[2]];
+          double* XW = A.tbuf[sh.role[3]];
+          const float sig = (float)sh.sigma_prev;
+#pragma unroll
+          for (int i = 0; i < V; ++i) {
+            if constexpr (sizeof(T) == 8) XW[l + i] = fma(A.sinv[l + i], y.v[i], XR[l + i]);
+            else XW[l + i] = XR[l + i] + f32_to_f64(sig * A.sinv32[l + i] * y.v[i]);
+          }
+        }
+      }
+    }
+    if (!round_finish<T, WEIGHTED>(A, ctl, wait_ns, sh, red, mine, nt, r, round0, ph, logged)) return;
+  }
+  if (blockIdx.x != 0) return;
+  if (tid == 0) sh.ypend = 0;
+  __syncthreads();
+  if (tid < kScalWords)
+    reinterpret_cast<unsigned long long*>(A.scal)[tid] = reinterpret_cast<const unsigned long long*>(&sh)[tid];
+  if (tid == 0) {
+    ctl->rounds = round0 + r;
+    A.stamps[kStampSolveEnd] = gtimer();
+  }
+}
+
+// ---- persistent solve of one small grid --------------------------------------------------------
+// The inner solve of a grid of up to kClusterTasks tasks of one plane each: one thread-block cluster, whose
+// blocks keep the vectors and the faces of their tasks (a run of consecutive ones) in shared memory for
+// the whole solve.  A neighbour's p and faces are read from the shared memory of the block that owns
+// them, each task's sums are written into every block's table, and the cluster barrier (three per
+// iteration: p, p.q, r.r) takes the place of the trips through L2, which are most of a small grid's
+// rounds in k_solve_one.  The same thread does the same cell's arithmetic as in pq_form and upd_form,
+// and the sums are added in the same order: the same bits.  A direction enters y in the update that
+// follows it, so y is complete at the end (InstScal::ypend = 0).
+// Bound by the FP64 pipe of the SMs it has (1.2 us for 512 cells' products) and by latency.  25 x 25 x 1
+// under the reference's rule: 6.9 us per iteration, 8.8 in k_solve_res and 11.7 in k_solve_one.
+constexpr int kClusterMax = 16, kClusterSlots = 2, kClusterTasks = kClusterMax * kClusterSlots;
+template <typename T, bool WEIGHTED>
+struct ClusterSlot {
+  Vec16<T> p[kBlock], r[kBlock], q[kBlock], y[kBlock], ax[kBlock], ay[kBlock], az[kBlock];
+  Vec16<T> dg[WEIGHTED ? kBlock : 1];
+  T red[sizeof(T) == 4 ? kBlock / 32 : (WEIGHTED ? 2 : 1) * kBlock];   // values of the sums (cluster_put)
+};
+
+__device__ __forceinline__ void cluster_sync() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The address of this block's shared object `p` in block `rank` of the cluster.
+__device__ __forceinline__ unsigned in_block(const void* p, int rank) {
+  unsigned a;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ Vec16<float> ld_cluster(unsigned a, float) {
+  Vec16<float> v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];"
+               : "=f"(v.v[0]), "=f"(v.v[1]), "=f"(v.v[2]), "=f"(v.v[3]) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ Vec16<double> ld_cluster(unsigned a, double) {
+  Vec16<double> v;
+  asm volatile("ld.shared::cluster.v2.f64 {%0,%1}, [%2];" : "=d"(v.v[0]), "=d"(v.v[1]) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ void st_cluster(unsigned a, double v) {
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+
+// A thread's values of the sums of a slot (FP32: its warp's sum).
+template <typename T, int NRV, class S>
+__device__ __forceinline__ void cluster_put(S& slot, const T (&v)[NRV]) {
+  if constexpr (sizeof(T) == 4) {
+    float s = v[0];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
+    if ((threadIdx.x & 31) == 0) slot.red[threadIdx.x >> 5] = s;
+  } else {
+#pragma unroll
+    for (int k = 0; k < NRV; ++k) slot.red[k * kBlock + threadIdx.x] = v[k];
+  }
+}
+// The slots' sums, in the order of task_store_f (FP32) and tile_store (FP64), into every block's table:
+// value k of task t at table[k * kClusterTasks + t].
+template <typename T, int NRV, class S>
+__device__ __forceinline__ void cluster_post(const S* slot, int slots, int task0, int C, double* table) {
+  const int lane = threadIdx.x & 31, j = threadIdx.x >> 5;
+  __syncthreads();
+  if (j >= slots) return;
+  double t[NRV];
+  if constexpr (sizeof(T) == 4) {
+    float v = lane < kBlock / 32 ? slot[j].red[lane] : 0.f;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
+    t[0] = (double)v;
+  } else {
+#pragma unroll
+    for (int k = 0; k < NRV; ++k) {
+      double u[8];
+#pragma unroll
+      for (int w = 0; w < 8; ++w) u[w] = slot[j].red[k * kBlock + lane + 32 * w];
+      t[k] = tree8(u);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+      for (int k = 0; k < NRV; ++k) t[k] += __shfl_xor_sync(kFull, t[k], o);
+    }
+  }
+  if (lane < C) {
+#pragma unroll
+    for (int k = 0; k < NRV; ++k) st_cluster(in_block(table + k * kClusterTasks + task0 + j, lane), t[k]);
+  }
+}
+
+template <typename T, bool WEIGHTED>
+__global__ void __launch_bounds__(kBlock, 1) k_solve_cluster(DevArrays A, SolveCtl* ctl, int64_t limit) {
+  constexpr int V = Vec16<T>::N, NRV = WEIGHTED ? 2 : 1;
+  typedef Vec16<T> VT;
+  typedef ClusterSlot<T, WEIGHTED> Slot;
+  __shared__ InstScal sh;
+  __shared__ InstDesc sd;
+  __shared__ double table[3 * kClusterTasks];          // p.q; r.r and the weighted r.r
+  __shared__ unsigned beside[kClusterSlots][6];          // per slot: the slots e, w, n, s, up, down of it
+  __shared__ int4 origin[kClusterSlots];                 // per slot: x, y, z and first cell of its tile
+  extern __shared__ __align__(16) char dyn[];
+  const int tid = threadIdx.x, C = (int)gridDim.x, rank = (int)blockIdx.x;
+  if (tid < kScalWords)
+    reinterpret_cast<unsigned long long*>(&sh)[tid] = reinterpret_cast<const unsigned long long*>(A.scal)[tid];
+  if (tid < (int)(sizeof(InstDesc) / 8))
+    reinterpret_cast<unsigned long long*>(&sd)[tid] = reinterpret_cast<const unsigned long long*>(A.inst)[tid];
+  __syncthreads();
+  if (!sh.inner_active) return;                         // no inner solve is due (in any block)
+  Slot* slot = reinterpret_cast<Slot*>(dyn);
+  const int nt = sd.cgn, nxy_t = sd.cgnx * sd.cgny, task0 = rank * nt / C, slots = (rank + 1) * nt / C - task0;
+  const int nx = sd.nx, ny = sd.ny, nz = sd.nz, sx = sd.sx, nxy = sx * ny, nq = 1 << sd.cqx, rows = kBlock >> sd.cqx;
+  [[maybe_unused]] const int n4 = nxy * nz;
+  const int vx = tid & (nq - 1), ry = tid >> sd.cqx, lt = ry * sx + vx * V;
+  const VT zero{};
+  if (tid < slots) {
+    const int t = task0 + tid, x = t % sd.cgnx * nq * V, y = t / sd.cgnx % sd.cgny * rows, z = t / nxy_t;
+    origin[tid] = make_int4(x, y, z, z * nxy + y * sx + x);
+  }
+  if (tid >= 32 && tid - 32 < slots * 6) {
+    const int j = (tid - 32) / 6, dir = (tid - 32) % 6, t = task0 + j;
+    const int bx = t % sd.cgnx, by = t / sd.cgnx % sd.cgny, bz = t / nxy_t;
+    int o;                                              // the task beside it (across a wrap, too)
+    if (dir == 0) o = bx + 1 < sd.cgnx ? t + 1 : t - bx;
+    else if (dir == 1) o = bx > 0 ? t - 1 : t + sd.cgnx - 1;
+    else if (dir == 2) o = by + 1 < sd.cgny ? t + sd.cgnx : t - by * sd.cgnx;
+    else if (dir == 3) o = by > 0 ? t - sd.cgnx : t + (sd.cgny - 1) * sd.cgnx;
+    else if (dir == 4) o = bz + 1 < nz ? t + nxy_t : t - bz * nxy_t;
+    else o = bz > 0 ? t - nxy_t : t + (nz - 1) * nxy_t;
+    const int owner = ((o + 1) * C - 1) / nt;           // the block whose run of tasks holds it
+    beside[j][dir] = in_block(slot + (o - owner * nt / C), owner);
+  }
+  for (int i = tid; i < 3 * kClusterTasks; i += kBlock) table[i] = 0.0;
+  __syncthreads();
+  auto active = [&](const int4& o) { return o.x + vx * V < nx && o.y + ry < ny; };
+  for (int j = 0; j < slots; ++j) {
+    const int4 o = origin[j];
+    Slot& s = slot[j];
+    const bool act = active(o);
+    const int l = act ? HF_IXV(A, o.w + lt, n4, V) : 0;
+    s.r[tid] = act ? ld16(Vec<T>::r(A) + l) : zero;
+    s.ax[tid] = act ? ld16(Vec<T>::ax(A) + l) : zero;
+    s.ay[tid] = act ? ld16(Vec<T>::ay(A) + l) : zero;
+    s.az[tid] = act ? ld16(Vec<T>::az(A) + l) : zero;
+    s.p[tid] = s.q[tid] = s.y[tid] = zero;
+    if constexpr (WEIGHTED) {
+      VT dg{};
+      for (int i = 0; i < V; ++i)
+        if (act && o.x + vx * V + i < nx)
+          dg.v[i] = A.diag[HF_IX(A, (o.z * ny + o.y + ry) * nx + o.x + vx * V + i, nx * ny * nz)];
+      s.dg[tid] = dg;
+    }
+  }
+  if (tid == 0) sh.phase = PH_CG_PQ;
+  const int64_t round0 = ctl->rounds;
+  cluster_sync();                                       // every block's state is in place
+  int64_t r = 0;
+  for (; cg_phase(sh.phase); ++r) {
+    if (r >= limit) {                                   // (the same in every block)
+      if (rank == 0 && tid == 0) ctl->guard_hit = 1;
+      break;
+    }
+    const int32_t ph = sh.phase, logged = logged_phase(sh);
+    const T alpha = (T)sh.alpha;
+    const bool first = sh.iter == 0;
+    if (ph == PH_CG_PQ) {
+      const T beta = (T)sh.beta;
+      for (int j = 0; j < slots; ++j) {
+        VT p = slot[j].r[tid];
+        if (!first) {
+          const VT po = slot[j].p[tid];
+#pragma unroll
+          for (int i = 0; i < V; ++i) p.v[i] = fma(beta, po.v[i], p.v[i]);
+        }
+        slot[j].p[tid] = p;
+      }
+      cluster_sync();                                   // p of every block is there
+      for (int j = 0; j < slots; ++j) {
+        Slot& s = slot[j];
+        const int4 o = origin[j];
+        T dot = T(0);
+        if (active(o)) {
+          constexpr unsigned kAx = offsetof(Slot, ax), kAy = offsetof(Slot, ay), kAz = offsetof(Slot, az);
+          const int x = o.x + vx * V, y = o.y + ry, z = o.z;
+          const int last = min(V - 1, nx - 1 - x);
+          VT pn = zero, ps = zero, ays = zero, pa = zero, pd = zero, azm = zero;
+          T pe = T(0), pw = T(0), axw = T(0);
+          if (nz > 1) {
+            if (z + 1 < nz || sd.pz) pa = ld_cluster(beside[j][4] + tid * 16, T(0));
+            if (z > 0 || sd.pz) {
+              pd = ld_cluster(beside[j][5] + tid * 16, T(0));
+              azm = ld_cluster(beside[j][5] + kAz + tid * 16, T(0));
+            }
+          }
+          if (ny > 1) {
+            if (y + 1 < ny && ry < rows - 1) pn = s.p[tid + nq];
+            else if (y + 1 < ny || sd.py) pn = ld_cluster(beside[j][2] + vx * 16, T(0));
+            if (ry > 0) {
+              ps = s.p[tid - nq];
+              ays = s.ay[tid - nq];
+            } else if (y > 0 || sd.py) {
+              const int row = y > 0 ? rows - 1 : (ny - 1) & (rows - 1);
+              const unsigned a = beside[j][3] + (row * nq + vx) * 16;
+              ps = ld_cluster(a, T(0));
+              ays = ld_cluster(a + kAy, T(0));
+            }
+          }
+          if (x + V < nx && vx < nq - 1) pe = s.p[tid + 1].v[0];
+          else if (x + V < nx || (sd.px && nx > 1)) pe = ld_cluster(beside[j][0] + (tid - vx) * 16, T(0)).v[0];
+          if (vx > 0) {
+            pw = s.p[tid - 1].v[V - 1];
+            axw = s.ax[tid - 1].v[V - 1];
+          } else if (x > 0 || (sd.px && nx > 1)) {      // the last cell of the tile, or of the row
+            const int e = x > 0 ? nq * V - 1 : (nx - 1) & (nq * V - 1);
+            const unsigned a = beside[j][1] + (tid + e / V) * 16;
+            const VT w = ld_cluster(a, T(0)), f = ld_cluster(a + kAx, T(0));
+#pragma unroll
+            for (int i = 0; i < V; ++i) {
+              if (i == e % V) {
+                pw = w.v[i];
+                axw = f.v[i];
+              }
+            }
+          }
+          const VT p = s.p[tid], axv = s.ax[tid], ayv = s.ay[tid], azv = s.az[tid];
+          VT qv;
+#pragma unroll
+          for (int i = 0; i < V; ++i) {
+            const T pi = p.v[i];
+            T acc = pi;
+            acc = fma(axv.v[i], i < last ? p.v[i < V - 1 ? i + 1 : i] : pe, acc);
+            acc = fma(i > 0 ? axv.v[i > 0 ? i - 1 : 0] : axw, i > 0 ? p.v[i > 0 ? i - 1 : 0] : pw, acc);
+            acc = fma(ayv.v[i], pn.v[i], acc);
+            acc = fma(ays.v[i], ps.v[i], acc);
+            acc = fma(azv.v[i], pa.v[i], acc);
+            acc = fma(azm.v[i], pd.v[i], acc);
+            if (i > last) acc = T(0);
+            dot = fma(pi, acc, dot);
+            qv.v[i] = acc;
+          }
+          s.q[tid] = qv;
+        }
+        const T v[1] = {dot};
+        cluster_put<T, 1>(s, v);
+      }
+      cluster_post<T, 1>(slot, slots, task0, C, table);
+    } else {
+      const bool form_x = !WEIGHTED && (sh.xw & kXwThis);
+      for (int j = 0; j < slots; ++j) {
+        Slot& s = slot[j];
+        const int4 o = origin[j];
+        T rr = T(0), rw = T(0);
+        if (active(o)) {
+          const int last = min(V - 1, nx - 1 - (o.x + vx * V)), l = HF_IXV(A, o.w + lt, n4, V);
+          VT y = s.y[tid], rv = s.r[tid];
+          const VT q = s.q[tid], p = s.p[tid];
+          VT dg{};
+          if constexpr (WEIGHTED) dg = s.dg[tid];
+#pragma unroll
+          for (int i = 0; i < V; ++i) {
+            T x = fma(-alpha, q.v[i], rv.v[i]);
+            if (i > last) x = T(0);
+            rv.v[i] = x;
+            rr = fma(x, x, rr);
+            if (WEIGHTED && i <= last) rw = fma(-dg.v[i] * x, x, rw);
+            y.v[i] = fma(alpha, p.v[i], y.v[i]);
+          }
+          s.r[tid] = rv;
+          s.y[tid] = y;
+          if (form_x) {                                 // rows of 4k cells: both layouts index alike
+            const double* XR = A.tbuf[sh.role[2]];
+            double* XW = A.tbuf[sh.role[3]];
+            const float sig = (float)sh.sigma_prev;
+#pragma unroll
+            for (int i = 0; i < V; ++i) {
+              if constexpr (sizeof(T) == 8) XW[l + i] = fma(A.sinv[l + i], y.v[i], XR[l + i]);
+              else XW[l + i] = XR[l + i] + f32_to_f64(sig * A.sinv32[l + i] * y.v[i]);
+            }
+          }
+        }
+        if constexpr (WEIGHTED) {
+          const T v[2] = {rr, rw};
+          cluster_put<T, 2>(s, v);
+        } else {
+          const T v[1] = {rr};
+          cluster_put<T, 1>(s, v);
+        }
+      }
+      cluster_post<T, NRV>(slot, slots, task0, C, table + kClusterTasks);
+    }
+    cluster_sync();                                     // the sums of every block are there
+    if (tid < 32) {
+      // one task a lane: the order of instance_sum
+      double tot[2] = {0.0, 0.0};
+      const double* p = table + (ph == PH_CG_PQ ? 0 : kClusterTasks);
+      if (tid < nt) {
+        tot[0] = 0.0 + p[tid];
+        if (WEIGHTED && ph == PH_CG_B) tot[1] = 0.0 + p[kClusterTasks + tid];
       }
       for (int o = 16; o > 0; o >>= 1) {
-        if (o >= nt) continue;
+        if (o >= nt) continue;                          // (lanes past the tasks hold zeros)
         tot[0] += __shfl_xor_sync(kFull, tot[0], o);
-        if (two) tot[1] += __shfl_xor_sync(kFull, tot[1], o);
+        if (WEIGHTED) tot[1] += __shfl_xor_sync(kFull, tot[1], o);
       }
-      tot[0] = __shfl_sync(kFull, tot[0], 0);
-      if (two) tot[1] = __shfl_sync(kFull, tot[1], 0);
-      if (ph == PH_CG_PQ) {
-        if (tid == 0) {
-          epi_spmv_s(sh, tot);
-          sh.phase = sh.inner_active ? PH_CG_B : phase_after<T>(sh);
-        }
-      } else {
-        // upd_ratios with the two divisions and the two roots side by side in lanes 0 and 1
-        const double quot = tot[0] / (tid == 0 ? sh.rho : sh.gg0);
-        const double root = sqrt(WEIGHTED ? (tid == 0 ? tot[1] : sh.bb) : quot);
-        UpdRatios q;
-        q.shrink = quot;
-        q.first = __shfl_sync(kFull, quot, 1);
-        const double root1 = __shfl_sync(kFull, root, 1);
-        if (tid == 0) {
-          if (WEIGHTED) q.err = sh.bb > 0.0 ? root * sh.sigma_prev / root1 : 0.0;
-          else q.err = sh.gg0 > 0.0 ? root1 : 0.0;
-          epi_upd_s<T>(sh, A.opts, tot, q);
-          sh.phase = phase_after<T>(sh);
-        }
-      }
+      round_epilogue<T, WEIGHTED>(sh, A.opts, ph, tot);
+    } else if (tid == 32 && rank == 0 && round0 + r < kRoundLog) {
+      ctl->phase_log[round0 + r] = logged;
+      ctl->t_round[round0 + r] = gtimer();
     }
     __syncthreads();
   }
-  if (blockIdx.x != 0) return;
+  if (sh.iter > 0) {
+    for (int j = 0; j < slots; ++j) {
+      const int4 o = origin[j];
+      if (active(o)) {
+        const int l = HF_IXV(A, o.w + lt, n4, V);
+        st16(Vec<T>::y(A) + l, slot[j].y[tid]);
+      }
+    }
+  }
+  cluster_sync();                                       // no block leaves while its memory may be read
+  if (rank != 0) return;
+  if (tid == 0) sh.ypend = 0;
+  __syncthreads();
   if (tid < kScalWords)
     reinterpret_cast<unsigned long long*>(A.scal)[tid] = reinterpret_cast<const unsigned long long*>(&sh)[tid];
   if (tid == 0) {
@@ -1934,6 +2550,74 @@ int solve_grid_blocks(Ctx& c, int fp32, bool full) {
   return cached;
 }
 
+// k_solve_cluster's launch: C blocks, one cluster.
+template <typename T, bool WEIGHTED>
+static cudaError_t cluster_config(Ctx& c, int C, cudaLaunchConfig_t& cfg, cudaLaunchAttribute& at) {
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = (unsigned)C;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg = {};
+  cfg.gridDim = dim3((unsigned)C);
+  cfg.blockDim = dim3(kBlock);
+  cfg.dynamicSmemBytes = kClusterSlots * sizeof(ClusterSlot<T, WEIGHTED>);
+  cfg.stream = c.stream;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  auto kernel = k_solve_cluster<T, WEIGHTED>;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  return e == cudaSuccess ? allow_smem(kernel, (int)cfg.dynamicSmemBytes) : e;
+}
+// Blocks of the cluster that runs a grid's inner solves, or 0.
+template <typename T, bool WEIGHTED>
+static int cluster_blocks_of(Ctx& c) {
+  const InstDesc& d = c.h_inst[0];
+  if (d.cgnz != d.nz || d.cgn > (sizeof(T) == 8 ? kClusterMax : kClusterTasks)) return 0;
+  const int C = std::min(kClusterMax, d.cgn);
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute at;
+  int n = 0;
+  if (cluster_config<T, WEIGHTED>(c, C, cfg, at) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, k_solve_cluster<T, WEIGHTED>, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return n >= 1 ? C : 0;
+}
+template <typename T, bool WEIGHTED>
+static cudaError_t launch_cluster(Ctx& c, int64_t limit) {
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute at;
+  const cudaError_t e = cluster_config<T, WEIGHTED>(c, c.cluster_blocks, cfg, at);
+  return e == cudaSuccess ? cudaLaunchKernelEx(&cfg, k_solve_cluster<T, WEIGHTED>, c.A, c.d_sctl, limit) : e;
+}
+
+// Planes of the deepest task where k_solve_res serves the inner solves of a grid, or 0: all of its
+// blocks run at once with the task's state in shared memory.
+template <typename T, bool WEIGHTED>
+static int res_depth_of(Ctx& c) {
+  const InstDesc& d = c.h_inst[0];
+  const int D = (d.nz + d.cgnz - 1) / d.cgnz, smem = ResLayout<T>(D, WEIGHTED).n * 16;
+  auto kernel = k_solve_res<T, WEIGHTED>;
+  int n = 0, nsm = 0, most = 0;
+  if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c.device) != cudaSuccess ||
+      cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, c.device) != cudaSuccess)
+    return 0;
+  if (smem > most - 8192 || allow_smem(kernel, smem) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kBlock, smem) != cudaSuccess)
+    return 0;
+  return (int64_t)n * nsm >= d.cgn ? D : 0;
+}
+// Which kernel runs the inner solves of one grid: k_solve_cluster, k_solve_res or k_solve_one, each where
+// the one before does not take the grid.  The cluster has 16 SMs, and its latency advantage is spent when
+// each has more than one FP64 task (its pipe's work) or two FP32 ones; us per iteration, cluster against
+// k_solve_res: FP64 under the reference's rule, 8 tasks 7.3 and 9.5, 16 tasks 7.7 and 9.5, 32 tasks 9.8
+// and 9.4; FP32, 16 tasks 4.6 and 6.3, 32 tasks 5.5 and 6.3, 48 (three a block) 7.8 and 6.7.
+template <typename T, bool WEIGHTED>
+static void choose_solve(Ctx& c) {
+  c.cluster_blocks = cluster_blocks_of<T, WEIGHTED>(c);
+  c.res_depth = res_depth_of<T, WEIGHTED>(c);
+}
+
 // Zero the control block (its counters: full = false), then launch the persistent solve cooperatively
 // on the context stream.
 cudaError_t launch_solve(Ctx& c, bool full, unsigned long long wait_ns, int leaver) {
@@ -1951,13 +2635,32 @@ cudaError_t launch_solve(Ctx& c, bool full, unsigned long long wait_ns, int leav
   cfg.blockDim = dim3(kBlock);
   cfg.dynamicSmemBytes = fp32 ? kPqSmem<float> : kPqSmem<double>;
   cfg.stream = c.stream;
-  e = allow_smem(solve_kernel(c, fp32 ? 1 : 0, c.A.xout != nullptr, full), (int)cfg.dynamicSmemBytes);
-  if (e != cudaSuccess) return e;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeCooperative;
   at[0].val.cooperative = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
+  const bool weighted = !fp32 && c.opts.criterion == HF_STOP_RECURSIVE;
+  if (c.ninst == 1) {
+    if (c.res_depth < 0) {
+      if (fp32) choose_solve<float, false>(c);
+      else if (weighted) choose_solve<double, true>(c);
+      else choose_solve<double, false>(c);
+    }
+    if (c.cluster_blocks > 0 && leaver < 0)    // (the failure-path check is of the waits of the others)
+      return fp32 ? launch_cluster<float, false>(c, limit)
+                  : weighted ? launch_cluster<double, true>(c, limit) : launch_cluster<double, false>(c, limit);
+    if (const int D = c.res_depth) {
+      auto kernel = fp32 ? k_solve_res<float, false> : weighted ? k_solve_res<double, true> : k_solve_res<double, false>;
+      cfg.gridDim = dim3((unsigned)c.h_inst[0].cgn);
+      cfg.dynamicSmemBytes = (size_t)16 * (fp32 ? ResLayout<float>(D, false).n : ResLayout<double>(D, weighted).n);
+      e = allow_smem(kernel, (int)cfg.dynamicSmemBytes);
+      if (e != cudaSuccess) return e;
+      return cudaLaunchKernelEx(&cfg, kernel, c.A, c.d_sctl, limit, wait_ns, leaver, D);
+    }
+  }
+  e = allow_smem(solve_kernel(c, fp32 ? 1 : 0, c.A.xout != nullptr, full), (int)cfg.dynamicSmemBytes);
+  if (e != cudaSuccess) return e;
   return cudaLaunchKernelEx(&cfg, solve_kernel(c, fp32 ? 1 : 0, c.A.xout != nullptr, full), c.A, c.d_sctl, limit,
                             wait_ns, leaver);
 }
