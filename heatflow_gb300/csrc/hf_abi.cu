@@ -539,10 +539,9 @@ int build_post_graph(Ctx& c) {
   return HF_OK;
 }
 
-// Chunks of the host arrays for hf_step_host_async: whole z-slabs of tasks (instance i, task
-// planes [bz*zc, (bz+1)*zc)), which are contiguous in the compact host layout, in the device
-// layout and in the task table, merged in order into at most kHostChunks chunks of about equal
-// cells.
+// Chunks of the host arrays for hf_step_host_async: the cells of groups of tasks (Chunk in
+// hf_internal.cuh), which are contiguous in the compact host layout, in the device layout and in the
+// task table, in at most kHostChunks chunks of about equal cells.
 void build_host_chunks(Ctx& c) {
   if (c.host_chunks_depth == c.depth && !c.host_chunks.empty()) return;
   int64_t total = 0;
@@ -552,13 +551,10 @@ void build_host_chunks(Ctx& c) {
   Ctx::HostChunk cur{0, 0, 0, 0, 0, 0};
   bool open = false;
   for (const auto& d : c.h_inst) {
-    const int64_t nbx = (d.nx + kTX - 1) / kTX, nby = (d.ny + kTY - 1) / kTY;
-    const int64_t nxy = (int64_t)d.nx * d.ny;
-    for (int64_t z0 = 0, bz = 0; z0 < d.nz; z0 += d.zc, ++bz) {
-      const int64_t z1 = std::min<int64_t>(z0 + d.zc, d.nz);
-      const Ctx::HostChunk g{d.hoff + z0 * nxy, d.hoff + z1 * nxy, d.off + z0 * nxy,
-                             d.off + z1 * nxy, d.task0 + bz * nbx * nby,
-                             d.task0 + (bz + 1) * nbx * nby};
+    for (int64_t t = 0; t < d.ntask; t += d.fg) {
+      const int64_t t1 = std::min<int64_t>(t + d.fg, d.ntask);
+      const int64_t l0 = std::min<int64_t>(t * d.fc, d.n), l1 = std::min<int64_t>(t1 * d.fc, d.n);
+      const Ctx::HostChunk g{d.hoff + l0, d.hoff + l1, d.off + l0, d.off + l1, d.task0 + t, d.task0 + t1};
       if (!open) {
         cur = g;
         open = true;
@@ -799,6 +795,8 @@ int build_tasks(Ctx& c, int depth) {
     d.task0 = (int64_t)tasks.size();
     d.ntask = nbx * nby * nbz;
     d.zc = depth;
+    d.fc = ((d.n + d.ntask - 1) / d.ntask + kPiece - 1) / kPiece * kPiece;
+    d.fg = (d.ntask + 7) / 8;
     for (int bz = 0; bz < nbz; ++bz)
       for (int by = 0; by < nby; ++by)
         for (int bx = 0; bx < nbx; ++bx)

@@ -60,6 +60,7 @@ struct InstDesc {
   int64_t task0;      // first task of the step kernels
   int32_t ntask;      // tasks of this instance
   int32_t zc;         // planes per task (the task depth)
+  int32_t fc, fg;     // element-wise passes (Chunk): cells per task, tasks per group
   int64_t hoff;       // first cell in the compact host layout (instances back to back, no padding)
   // The vectors of the inner solve (a32x/y/z, y32, r32, p32, p232, q32 and their FP64 twins) use
   // their own layout: rows of sx = nx rounded up to 4 cells (the padding cells hold zeros), so every
@@ -213,7 +214,7 @@ struct DevArrays {
   // solver
   double *b, *y, *r, *p, *q, *p2;
   float *y32, *r32, *p32, *q32, *p232;   // p / p2: search directions, ping-pong by iteration
-  const int8_t* task_heat;  // per task: some cell holds a heater
+  const int8_t* task_heat;  // per task: some cell of its run (Chunk) holds a heater
   const int4* tasks;        // (instance, x0, y0, z0) per task
   const int32_t* cg_inst;   // instance per task of the inner solve's passes
   int64_t ncells, ntiles, ninst, ntasks, ncg;   // ncg: tasks of the inner solve's passes
@@ -230,12 +231,12 @@ struct DevArrays {
 
 // ---- index checks of the checked build ----------------------------------------------------------
 // Compiled with -DHF_CHECKED (build_library(checked=True): a separate library for tests), every
-// global load and store of the step kernels takes its index through HF_IX (one cell), HF_IX4 (a
-// 4-cell vector, which must also start on a multiple of 4 cells: a 16-byte boundary for FP32, two
-// for FP64) or HF_IXV (a vector of v = 2 or 4 cells).  An index outside [0, n) -- n the extent of that array in the instance's layout -- is
+// global load and store of the step kernels takes its index through HF_IX (one cell), HF_IXV (a
+// vector of v = 2 or 4 cells, which must also start on a multiple of v) or HF_IXP (a pair, or one cell at
+// the end).  An index outside [0, n) -- n the extent of that array in the instance's layout -- is
 // recorded in DevArrays::check and replaced by 0, so the access stays inside the array and the
 // kernel goes on: no trap, no fault.  The host reports a record as HF_EDEVICE (the site is
-// 100000 * file + line).  In the normal build both macros are the index itself.
+// 100000 * file + line).  In the normal build the macros are the index itself.
 #ifdef HF_CHECKED
 __device__ __noinline__ inline long long hf_check_ix(unsigned long long* rec, int site, long long i,
                                                      long long n, int vec) {
@@ -253,24 +254,16 @@ __device__ __noinline__ inline long long hf_check_ix(unsigned long long* rec, in
 }
 #define HF_SITE (HF_FILE_ID * 100000 + __LINE__)
 #define HF_IX(A, i, n) ((int)hf_check_ix((A).check, HF_SITE, (long long)(i), (long long)(n), 1))
-#define HF_IX4(A, i, n) ((int)hf_check_ix((A).check, HF_SITE, (long long)(i), (long long)(n), 4))
 #define HF_IXV(A, i, n, v) ((int)hf_check_ix((A).check, HF_SITE, (long long)(i), (long long)(n), (v)))
 #else
 #define HF_IX(A, i, n) (i)
-#define HF_IX4(A, i, n) (i)
 #define HF_IXV(A, i, n, v) (i)
 #endif
+#define HF_IXP(A, i, n, two) ((two) ? HF_IXV(A, i, n, 2) : HF_IX(A, i, n))
 
 // Slots of DevArrays::stamps: step begin, RHS start, RHS finalize start, solve start, end of the
 // solve's last round, step end.
 enum { kStampBegin = 0, kStampRhs, kStampFin, kStampSolve, kStampSolveEnd, kStampEnd, kStamps = 8 };
-
-// Ask L2 for the line holding p (no register, no result): planes a pass streams in its next z
-// steps, so their DRAM latency overlaps the current step's work at the persistent solve's 3 blocks
-// per SM.  Only ever given addresses inside the arrays (planes the task itself reads next).
-__device__ __forceinline__ void prefetch_l2(const void* p) {
-  asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
-}
 
 __device__ __forceinline__ unsigned long long gtimer() {
   unsigned long long t;
@@ -454,6 +447,55 @@ __device__ __forceinline__ void tile_store(double* dst, int64_t stride, const do
 template <int NRV>
 __device__ __forceinline__ void tile_store(const DevArrays& A, int64_t task, const double (&v)[NRV]) {
   tile_store<NRV>(A.partials + task, A.pcap, v);
+}
+
+// The element-wise passes (right-hand side, first residual from the stored products, x update) take the
+// same tasks as the stencil passes, but of each an equal share of the cells: no lane lies past a row's
+// end (grids of 16 to 96 cells an edge fill 72 % of the 32 x 8 column tiles).  Groups of fg tasks (an
+// eighth of the instance) own runs of consecutive cells and deal them in turn in pieces of 2 kBlock, a pair of
+// cells per thread: the blocks that run at the same time read neighbouring pieces, and cells that cost
+// more (a heated layer) are spread over the group.  Pieces start at even cells, so pairs are 16-byte
+// aligned.
+// The x update as a kernel splits each share into kFine parts, a block each: 256^3 has 2048 tasks, 3.4
+// times what is resident at once, and the fourth wave was nearly empty.
+constexpr int kFine = 4, kPiece = 2 * kBlock;
+struct Chunk {
+  const InstDesc* d;
+  // first cell of its first piece, end of its group's cells, from piece to piece (unsigned: l + step may
+  // pass 2^31)
+  unsigned l0, end, step;
+  bool rows4;                 // the inner solve's layout indexes like the cells
+  __device__ __forceinline__ unsigned first() const { return l0 + 2 * threadIdx.x; }
+  // index of cell l in the inner solve's layout
+  __device__ __forceinline__ int inner(int l) const { return rows4 ? l : l + l / d->nx * (d->sx - d->nx); }
+};
+__device__ __forceinline__ int task_inst(const DevArrays& A, int64_t task) {
+  return A.ninst == 1 ? 0 : A.tasks[task].x;    // (one load latency less at the start of a block)
+}
+// The cells of a task, or of part `part` of its `parts`.
+template <int parts = 1>
+__device__ __forceinline__ Chunk task_chunk(const DevArrays& A, int64_t task, int part = 0) {
+  Chunk c;
+  c.d = A.inst + task_inst(A, task);
+  const int t = (int)(task - c.d->task0), g0 = t / c.d->fg * c.d->fg, ng = min(c.d->fg, c.d->ntask - g0);
+  const int64_t n = c.d->n, base = min((int64_t)g0 * c.d->fc, n);
+  c.end = (unsigned)min(base + (int64_t)ng * c.d->fc, n);
+  c.l0 = (unsigned)min(base + (t - g0 + (int64_t)part * ng) * kPiece, n);
+  c.step = (unsigned)(ng * kPiece * parts);
+  c.rows4 = c.d->sx == c.d->nx;
+  return c;
+}
+// Values l and l + 1 of a vector by cell (two: l + 1 lies in the grid).
+__device__ __forceinline__ double2 ld_pair(const double* p, int l, bool two) {
+  return two ? *reinterpret_cast<const double2*>(p + l) : make_double2(p[l], 0.0);
+}
+__device__ __forceinline__ float2 ld_pair(const float* p, int l, bool two) {
+  return two ? *reinterpret_cast<const float2*>(p + l) : make_float2(p[l], 0.f);
+}
+template <typename T, typename P>
+__device__ __forceinline__ void st_pair(T* p, int l, bool two, const P& v) {
+  if (two) *reinterpret_cast<P*>(p + l) = v;
+  else p[l] = v.x;
 }
 
 // The columns of a task that this thread owns.

@@ -68,192 +68,78 @@ __device__ __forceinline__ bool x0_below_tiny(double tp, double d, double x0) {
   return dbl_lt_pos(x0 - tp, kTiny);
 }
 
-// The per-cell work of the step RHS (shared by the scalar and the vector forms): heater, S_cat,
-// S and the initial guess of cell l; returns S and sets x0 and the x0 - T < TINY flag.
-struct RhsCtx {
-  bool heater, has_power, has_em, case5, cat, steady;
-  bool fast;      // HF_STOP_TRUE, not steady: S from scoef (passed as rhoc), x0 in one FMA
-  int qmode;
-  double inv_dt, vol, hvol, power_in, tb4, dt2;
-  int64_t itime;
-};
-// Heat density of cell l (the heater branch, out of line so the common heater-free tasks keep
-// a small register footprint).
-__device__ __noinline__ double rhs_qdens(const DevArrays& A, const InstDesc& d, const RhsCtx& r,
-                                         int64_t off, int l, double tp) {
-  double q = 0.0, qd = 0.0;
-  {
-    l = HF_IX(A, l, d.n);
-    const int cs = A.icase[off + l];
-    if (cs > 0 && cs < 7) {
-      const double P = r.has_power ? A.power[off + l] : r.power_in;
-      const double tau = r.case5 ? A.tau_s[off + l] * r.dt2 : 0.0;
-      q = heat_case(cs, P, tau, r.itime, d);
-    }
-    if (r.has_em) q = q - A.emc[off + l] * (pow(tp, 4.0) - r.tb4);
-    if (!dbl_is_zero(q)) {
-      if (r.qmode == HF_QDENS_CELL_VOLUME) qd = q / r.vol;
-      else if (r.hvol > 0.0) qd = q / r.hvol;
-    }
-  }
-  return qd;
-}
-
-template <bool HEAT>
-__device__ __forceinline__ double rhs_cell(const DevArrays& A, const InstDesc& d, const RhsCtx& r,
-                                           int64_t off, int l, double tp, double tpp, double rhoc,
-                                           double ccat, double B, double& x0, int& flag) {
-  const double qd = HEAT ? rhs_qdens(A, d, r, off, l, tp) : 0.0;
-  double S;
-  if (r.fast) {                                     // rhoc holds scoef here
-    S = r.cat ? fma(tp, rhoc, ccat * tpp) : tp * rhoc;
-    if (!dbl_is_zero(qd)) S = S - qd;
-    if (!dbl_is_zero(B)) S = S - B;
-    x0 = fma(2.0, tp, -tpp);
-    return S;
-  }
-  if (!r.steady) {
-    S = -r.inv_dt * tp * rhoc;
-    if (!dbl_is_zero(qd)) S = S - qd;
-    if (!dbl_is_zero(B)) S = S - B;
-    if (r.cat) S = S + fma(-2.0, tp, tpp) * ccat;   // (tpp - 2 tp) * ccat: 2 tp is exact
-  } else {
-    S = -qd;
-    if (!dbl_is_zero(B)) S = S - B;
-  }
-  const double dt = tp - tpp;
-  x0 = tp + dt;
-  flag |= x0_below_tiny(tp, dt, x0) ? 1 : 0;
-  return S;
-}
-
-// The common task of a step under the true-residual criterion, on rows of 4k cells: no heated
-// cell, S = T^n scoef + ccat T^(n-1) - B and x0 = 2 T^n - T^(n-1) (3 FP64 instructions per cell),
-// the arithmetic and summation order of rhs4_task's fast form.  Kept apart from the general forms
-// (out of line) so that its operands stay in registers: with them in one body the kernel's 64
-// registers spilled, and the pass ran on local-memory traffic as large as its HBM traffic (ncu).
-// B is read only on the outer faces: boundary() (k_assemble, k_tempdep) gives it to no other
-// cell, where it is +0.0.
-__device__ __forceinline__ void rhs4_fast_task(const DevArrays& A, int64_t task, const InstDesc& d,
-                                               const InstScal& s) {
-  const int4 tk = A.tasks[task];
-  const int tid = threadIdx.x, grp = tid >> 6, w = tid & 63;
-  const int x = tk.y + 4 * (w & 7), y = tk.z + (w >> 3);
-  const int z1 = min(tk.w + d.zc, d.nz);
-  const int per = (z1 - tk.w + 3) >> 2;
-  const int za = min(tk.w + grp * per, z1), zb = min(za + per, z1);
-  const bool act = x < d.nx && y < d.ny;
-  const bool face_col = x == 0 || x + 4 >= d.nx || y == 0 || y == d.ny - 1;
-  const bool cat = d.icattaneo == 1;
+// The common task of a step under the true-residual criterion: no heated cell,
+// S = T^n scoef + ccat T^(n-1) - B and x0 = 2 T^n - T^(n-1) (3 FP64 instructions per cell).  Kept apart
+// from the general form so that its operands stay in registers.  B is read only on the outer faces:
+// boundary() (k_assemble, k_tempdep) gives it to no other cell, where it is +0.0.  Bound by HBM (48 B per
+// cell) and the FP64 pipe alike, which instructions that are predicated off take too: with the form without
+// ccat and the subtraction of B so in the loop, ncu saw 5.3 FP64 instructions per cell and the pipe 61 %
+// busy.  256^3 slab 200 -> 175 us, 190 x 192 x 192 130 -> 79, 64 grids of 16 to 96 cells an edge 276 -> 129.
+template <bool CAT>
+__device__ __forceinline__ void rhs_fast_task(const DevArrays& A, int64_t task, const Chunk& c, const InstScal& s) {
+  const InstDesc& d = *c.d;
   const int64_t off = d.off;
-  const int nxy = d.nx * d.ny, lxy = y * d.nx + x;
-  const double* Tp = A.tbuf[s.role[0]] + off;
-  const double* Tpp = A.tbuf[s.role[1]] + off;
-  double* X = A.tbuf[s.role[2]] + off;
+  const int nx = d.nx, ny = d.ny, nz = d.nz;
+  [[maybe_unused]] const int n = d.n;
+  const double* __restrict__ Tp = A.tbuf[s.role[0]] + off;
+  const double* __restrict__ Tpp = A.tbuf[s.role[1]] + off;
+  double* __restrict__ X = A.tbuf[s.role[2]] + off;
   const double* __restrict__ sc = A.scoef + off;
   const double* __restrict__ ccat = A.ccat + off;
   const double* __restrict__ bvec = A.bvec + off;
-  double* bout = A.b + off;
+  double* __restrict__ bout = A.b + off;
   SqSum sq;
-  if (act) {
-    for (int z = za; z < zb; ++z) {
-      const int l = HF_IX4(A, lxy + z * nxy, d.n);
-      const double2* tp2 = reinterpret_cast<const double2*>(Tp + l);
-      const double2* tq2 = reinterpret_cast<const double2*>(Tpp + l);
-      const double2* sc2 = reinterpret_cast<const double2*>(sc + l);
-      const double2* cc2 = reinterpret_cast<const double2*>(ccat + l);
-      const double2* bv2 = reinterpret_cast<const double2*>(bvec + l);
-      const double2 t0 = tp2[0], t1 = tp2[1], u0 = tq2[0], u1 = tq2[1], h0 = sc2[0], h1 = sc2[1];
-      double2 c0 = make_double2(0.0, 0.0), c1 = c0, b0 = c0, b1 = c0;
-      if (cat) { c0 = cc2[0]; c1 = cc2[1]; }
-      if (face_col || z == 0 || z == d.nz - 1) { b0 = bv2[0]; b1 = bv2[1]; }
-      const double tp[4] = {t0.x, t0.y, t1.x, t1.y}, tpp[4] = {u0.x, u0.y, u1.x, u1.y};
-      const double rh[4] = {h0.x, h0.y, h1.x, h1.y}, cc[4] = {c0.x, c0.y, c1.x, c1.y};
-      const double bv[4] = {b0.x, b0.y, b1.x, b1.y};
-      double S[4], x0[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        S[i] = cat ? fma(tp[i], rh[i], cc[i] * tpp[i]) : tp[i] * rh[i];
-        if (!dbl_is_zero(bv[i])) S[i] = S[i] - bv[i];
-        x0[i] = fma(2.0, tp[i], -tpp[i]);
-        sq.add(S[i]);
-      }
-      reinterpret_cast<double2*>(bout + l)[0] = make_double2(S[0], S[1]);
-      reinterpret_cast<double2*>(bout + l)[1] = make_double2(S[2], S[3]);
-      reinterpret_cast<double2*>(X + l)[0] = make_double2(x0[0], x0[1]);
-      reinterpret_cast<double2*>(X + l)[1] = make_double2(x0[2], x0[3]);
+  // where the pair that is loaded next lies; the thread's pairs are a fixed step apart
+  const int step_x = (int)(c.step % nx), step_q = (int)(c.step / nx), step_y = step_q % ny, step_z = step_q / ny;
+  int x = (int)(c.first() % nx), y = (int)(c.first() / nx % ny), z = (int)(c.first() / nx / ny);
+  // the operands of a pair; those of the thread's next pair are on their way while one is computed
+  struct Pair {
+    double2 tp, tpp, rh, cc, B;
+    bool face;
+  };
+  auto load = [&](unsigned m, Pair& o) {
+    o.face = false;
+    if (m >= c.end) return;
+    const int l = (int)m;
+    const bool two = m + 1 < c.end;
+    const int lc = HF_IXP(A, l, n, two);
+    o.tp = ld_pair(Tp, lc, two);
+    o.tpp = ld_pair(Tpp, lc, two);
+    o.rh = ld_pair(sc, lc, two);
+    if (CAT) o.cc = ld_pair(ccat, lc, two);
+    o.face = x == 0 || x + 2 >= nx || y == 0 || y == ny - 1 || z == 0 || z == nz - 1;
+    if (o.face) o.B = ld_pair(bvec, lc, two);
+    x += step_x;
+    const int cx = x >= nx ? 1 : 0;
+    x -= cx ? nx : 0;
+    y += step_y + cx;
+    const int cy = y >= ny ? 1 : 0;
+    y -= cy ? ny : 0;
+    z += step_z + cy;
+  };
+  Pair cur, nxt;
+  load(c.first(), cur);
+  for (unsigned l = c.first(); l < c.end; l += c.step) {
+    load(l + c.step, nxt);
+    const bool two = l + 1 < c.end;
+    double2 S, x0;
+    S.x = CAT ? fma(cur.tp.x, cur.rh.x, cur.cc.x * cur.tpp.x) : cur.tp.x * cur.rh.x;
+    S.y = CAT ? fma(cur.tp.y, cur.rh.y, cur.cc.y * cur.tpp.y) : cur.tp.y * cur.rh.y;
+    // a branch of the warp: predicated off, the subtractions would take the FP64 pipe all the same
+    if (__any_sync(__activemask(), cur.face)) {
+      if (cur.face && !dbl_is_zero(cur.B.x)) S.x = S.x - cur.B.x;
+      if (cur.face && !dbl_is_zero(cur.B.y)) S.y = S.y - cur.B.y;
     }
+    x0.x = fma(2.0, cur.tp.x, -cur.tpp.x);
+    x0.y = fma(2.0, cur.tp.y, -cur.tpp.y);
+    sq.add(S.x);
+    if (two) sq.add(S.y);
+    st_pair(bout, HF_IXP(A, l, n, two), two, S);
+    st_pair(X, HF_IXP(A, l, n, two), two, x0);
+    cur = nxt;
   }
   const double bb = sq.value();
   if (threadIdx.x == 0) A.partials[A.pcap + task] = 0.0;   // no x0 - T < TINY test here
-  const double v[1] = {bb};
-  tile_store<1>(A, task, v);
-}
-
-// Vector form for rows of 4k cells: each thread owns 4 consecutive x cells of a quarter of the
-// task's planes (the layout of the solver's vector passes), so every thread has 4 independent
-// cells of FP64 work in flight: the pass is bound by the FP64 pipe, and one cell per thread left
-// it partly idle.  ||S||^2 is summed per thread plane by plane, cells in x order.
-__device__ __noinline__ void rhs4_task(const DevArrays& A, int64_t task, const InstDesc& d,
-                                       const InstScal& s, const RhsCtx& r) {
-  const int4 tk = A.tasks[task];
-  const int tid = threadIdx.x, grp = tid >> 6, w = tid & 63;
-  const int x = tk.y + 4 * (w & 7), y = tk.z + (w >> 3);
-  const int z1 = min(tk.w + d.zc, d.nz);
-  const int per = (z1 - tk.w + 3) >> 2;
-  const int za = min(tk.w + grp * per, z1), zb = min(za + per, z1);
-  const bool act = x < d.nx && y < d.ny;
-  // boundary() gives B only to cells on the outer faces (k_assemble, k_tempdep): elsewhere it is
-  // +0.0, so a quad off the x/y faces reads B only in the first and last plane
-  const bool face_col = x == 0 || x + 4 >= d.nx || y == 0 || y == d.ny - 1;
-  const int64_t off = d.off;
-  const int nxy = d.nx * d.ny, lxy = y * d.nx + x;
-  const double* Tp = A.tbuf[s.role[0]] + off;
-  const double* Tpp = A.tbuf[s.role[1]] + off;
-  double* X = A.tbuf[s.role[2]] + off;
-  const double* __restrict__ rhoc = (r.fast ? A.scoef : A.rhoc) + off;
-  const double* __restrict__ ccat = A.ccat + off;
-  const double* __restrict__ bvec = A.bvec + off;
-  double* bout = A.b + off;
-  double bb = 0.0;
-  SqSum sq;
-  int flag = 0;
-  if (act) {
-    for (int z = za; z < zb; ++z) {
-      const int l = HF_IX4(A, lxy + z * nxy, d.n);
-      const double2* tp2 = reinterpret_cast<const double2*>(Tp + l);
-      const double2* tq2 = reinterpret_cast<const double2*>(Tpp + l);
-      const double2* rc2 = reinterpret_cast<const double2*>(rhoc + l);
-      const double2* cc2 = reinterpret_cast<const double2*>(ccat + l);
-      const double2* bv2 = reinterpret_cast<const double2*>(bvec + l);
-      const double2 t0 = tp2[0], t1 = tp2[1], u0 = tq2[0], u1 = tq2[1];
-      const double2 h0 = rc2[0], h1 = rc2[1], c0 = cc2[0], c1 = cc2[1];
-      double2 b0 = make_double2(0.0, 0.0), b1 = b0;
-      if (face_col || z == 0 || z == d.nz - 1) { b0 = bv2[0]; b1 = bv2[1]; }
-      const double tp[4] = {t0.x, t0.y, t1.x, t1.y}, tpp[4] = {u0.x, u0.y, u1.x, u1.y};
-      const double rh[4] = {h0.x, h0.y, h1.x, h1.y}, cc[4] = {c0.x, c0.y, c1.x, c1.y};
-      const double bv[4] = {b0.x, b0.y, b1.x, b1.y};
-      double S[4], x0[4];
-      if (r.heater) {               // unrolled too: a dynamic index would put the arrays in
-#pragma unroll                      // local memory for both branches
-        for (int i = 0; i < 4; ++i)
-          S[i] = rhs_cell<true>(A, d, r, off, l + i, tp[i], tpp[i], rh[i], cc[i], bv[i], x0[i], flag);
-      } else {
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          S[i] = rhs_cell<false>(A, d, r, off, l + i, tp[i], tpp[i], rh[i], cc[i], bv[i], x0[i], flag);
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i) sq.add(S[i]);
-      reinterpret_cast<double2*>(bout + l)[0] = make_double2(S[0], S[1]);
-      reinterpret_cast<double2*>(bout + l)[1] = make_double2(S[2], S[3]);
-      reinterpret_cast<double2*>(X + l)[0] = make_double2(x0[0], x0[1]);
-      reinterpret_cast<double2*>(X + l)[1] = make_double2(x0[2], x0[3]);
-    }
-  }
-  bb = sq.value();
-  const int any_flag = __syncthreads_or(flag);
-  if (threadIdx.x == 0) A.partials[A.pcap + task] = any_flag ? 1.0 : 0.0;
   const double v[1] = {bb};
   tile_store<1>(A, task, v);
 }
@@ -265,38 +151,19 @@ __global__ void __launch_bounds__(kBlock, 4) k_rhs(DevArrays A, double* oB, doub
                                                 double* oSc, int64_t task_base) {
   const int64_t task = task_base + blockIdx.x;
   if (!PARTS && !DIAG && task == 0 && threadIdx.x == 0) A.stamps[kStampRhs] = gtimer();
-  if (!PARTS && !DIAG) {          // the step's pass: vector form where the rows allow it
-    const int inst = A.tasks[task].x;
-    const InstDesc& d = A.inst[inst];
-    const InstScal& s = A.scal[inst];
-    if ((d.nx & 3) == 0) {
-      if (!s.outer_active) return;
-      const bool heater = d.heater && (d.has_em || A.task_heat[task]);
-      if (!heater && A.opts.criterion == HF_STOP_TRUE && d.isteady == 0) {
-        rhs4_fast_task(A, task, d, s);
-        return;
-      }
-      RhsCtx r;
-      r.heater = heater;
-      r.has_power = d.has_power; r.has_em = d.has_em; r.case5 = d.has_case5;
-      r.cat = d.icattaneo == 1; r.steady = d.isteady != 0;
-      r.qmode = d.qdens_mode;
-      r.inv_dt = d.inv_dt; r.vol = d.volume; r.hvol = d.heated_volume; r.power_in = d.power_in;
-      r.tb4 = d.has_em ? pow(d.t_bath, 4.0) : 0.0;
-      r.dt2 = d.has_case5 ? pow(d.time_step, 2.0) : 0.0;
-      r.itime = s.itime;
-      r.fast = A.opts.criterion == HF_STOP_TRUE && !r.steady;
-      rhs4_task(A, task, d, s, r);
-      return;
-    }
-  }
-  const TCell c = task_cell(A, task);
-  const InstDesc& d = A.inst[c.inst];
-  InstScal& s = A.scal[c.inst];
+  const Chunk c = task_chunk(A, task);
+  const InstDesc& d = *c.d;
+  InstScal& s = A.scal[task_inst(A, task)];
   if (!DIAG && !s.outer_active) return;
   if (DIAG && !(s.status & kStatusRhsNan)) return;
+  if (!PARTS && !DIAG && A.opts.criterion == HF_STOP_TRUE && d.isteady == 0 &&
+      !(d.heater && (d.has_em || A.task_heat[task]))) {
+    if (d.icattaneo == 1) rhs_fast_task<true>(A, task, c, s);
+    else rhs_fast_task<false>(A, task, c, s);
+    return;
+  }
   const int64_t itime = DIAG ? s.failed_step : s.itime;
-  const int64_t off = c.off;
+  const int64_t off = d.off;
   // heater() runs for every cell when any exists (mod_evolve.f90:79); with emissivity every cell
   // has a radiative term, otherwise only tasks holding a heated cell have nonzero Q
   const bool heater = d.heater && (d.has_em || A.task_heat[task]);
@@ -319,21 +186,38 @@ __global__ void __launch_bounds__(kBlock, 4) k_rhs(DevArrays A, double* oB, doub
   SqSum sq;
   int flag = 0;
   int nan_q = 0, nan_qd = 0, nan_sc = 0, nan_s = 0;
-  for (int z = c.z0; z < c.z1; ++z) {
+  constexpr int U = kPiece / kBlock;           // the loads of a piece are issued together
+  for (unsigned m = c.l0 + threadIdx.x; m < c.end; m += c.step) {
+    double tp[U], tpp[U], rh[U], cc[U], B[U], pw[U];
+    int cs[U];
 #pragma unroll
-    for (int j = 0; j < kXC; ++j) {
-      if (!c.act(j)) continue;
-      const int l = HF_IX(A, c.base(j) + z * c.nxy, c.n());
-      const double tp = Tp[l], tpp = Tpp[l];
+    for (int u = 0; u < U; ++u) {
+      tp[u] = tpp[u] = rh[u] = cc[u] = B[u] = pw[u] = 0.0;
+      cs[u] = 0;
+      if (m + kBlock * u >= c.end) continue;
+      const int l = HF_IX(A, (int)m + kBlock * u, d.n);
+      tp[u] = Tp[l];
+      tpp[u] = Tpp[l];
+      rh[u] = rhoc[l];
+      if (cat) cc[u] = ccat[l];
+      B[u] = bvec[l];
+      if (heater) {
+        cs[u] = A.icase[off + l];
+        if (has_power) pw[u] = A.power[off + l];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (m + kBlock * u >= c.end) continue;
+      const int l = HF_IX(A, (int)m + kBlock * u, d.n);
       double q = 0.0, qd = 0.0;
       if (heater) {
-        const int cs = A.icase[off + l];
-        if (cs > 0 && cs < 7) {
-          const double P = has_power ? A.power[off + l] : power_in;
+        if (cs[u] > 0 && cs[u] < 7) {
+          const double P = has_power ? pw[u] : power_in;
           const double tau = case5 ? A.tau_s[off + l] * dt2 : 0.0;
-          q = heat_case(cs, P, tau, itime, d);
+          q = heat_case(cs[u], P, tau, itime, d);
         }
-        if (has_em) q = q - A.emc[off + l] * (pow(tp, 4.0) - tb4);
+        if (has_em) q = q - A.emc[off + l] * (pow(tp[u], 4.0) - tb4);
         if (!dbl_is_zero(q)) {
           if (qmode == HF_QDENS_CELL_VOLUME) qd = q / vol;
           else if (hvol > 0.0) qd = q / hvol;
@@ -342,36 +226,35 @@ __global__ void __launch_bounds__(kBlock, 4) k_rhs(DevArrays A, double* oB, doub
       }
       double sc = 0.0;
       if (cat && !fast) {
-        sc = fma(-2.0, tp, tpp) * ccat[l];   // = (tpp - 2 tp) * ccat: 2 tp is exact
+        sc = fma(-2.0, tp[u], tpp[u]) * cc[u];   // = (tpp - 2 tp) * ccat: 2 tp is exact
         if (DIAG) nan_sc += dbl_is_nan(sc);
       }
-      const double B = bvec[l];
       double S, x0;
       if (fast) {
-        S = cat ? fma(tp, rhoc[l], ccat[l] * tpp) : tp * rhoc[l];
+        S = cat ? fma(tp[u], rh[u], cc[u] * tpp[u]) : tp[u] * rh[u];
         if (!dbl_is_zero(qd)) S = S - qd;
-        if (!dbl_is_zero(B)) S = S - B;
-        x0 = fma(2.0, tp, -tpp);
+        if (!dbl_is_zero(B[u])) S = S - B[u];
+        x0 = fma(2.0, tp[u], -tpp[u]);
       } else {
         if (!steady) {
-          S = -inv_dt * tp * rhoc[l];
+          S = -inv_dt * tp[u] * rh[u];
           if (!dbl_is_zero(qd)) S = S - qd;
-          if (!dbl_is_zero(B)) S = S - B;
+          if (!dbl_is_zero(B[u])) S = S - B[u];
           if (cat) S = S + sc;
         } else {
           S = -qd;
-          if (!dbl_is_zero(B)) S = S - B;
+          if (!dbl_is_zero(B[u])) S = S - B[u];
         }
-        const double dt = tp - tpp;
-        x0 = tp + dt;
-        flag |= x0_below_tiny(tp, dt, x0) ? 1 : 0;
+        const double dt = tp[u] - tpp[u];
+        x0 = tp[u] + dt;
+        flag |= x0_below_tiny(tp[u], dt, x0) ? 1 : 0;
       }
       if (DIAG) nan_s += dbl_is_nan(S);
       bout[l] = S;
       X[l] = x0;
       sq.add(S);
       if (PARTS) {
-        oB[off + l] = B;
+        oB[off + l] = B[u];
         oQ[off + l] = q;
         oQd[off + l] = qd;
         oSc[off + l] = sc;
@@ -519,11 +402,11 @@ __global__ void k_adj_grad(DevArrays A, const InstBC* bcs, const double* kappa, 
 // the other tasks.
 __global__ void k_task_heat(DevArrays A, int8_t* flag) {
   const int64_t task = blockIdx.x;
-  const TCell c = task_cell(A, task);
+  const Chunk c = task_chunk(A, task);
   int any = 0;
-  if (A.icase && c.act(0)) {
-    for (int z = c.z0; z < c.z1; ++z) any |= A.icase[c.off + c.base(0) + (int64_t)z * c.nxy] != 0;
-  }
+  if (A.icase)
+    for (unsigned m = c.l0; m < c.end; m += c.step)
+      for (unsigned l = m + threadIdx.x; l < min(m + kPiece, c.end); l += kBlock) any |= A.icase[c.d->off + l] != 0;
   any = __syncthreads_or(any);
   if (threadIdx.x == 0) flag[task] = (int8_t)(any ? 1 : 0);
 }

@@ -24,6 +24,7 @@
 #include <algorithm>
 #include <climits>
 #include <cstddef>
+#include <type_traits>
 
 #include "hf_ctx.cuh"
 
@@ -111,8 +112,17 @@ __global__ void k_step_end(DevArrays A) {
 // x, whatever the start, and this CG treats a zero residual itself, so the TINY is skipped: one
 // FP64 instruction per cell less in the first residual and in the x update (GB300's FP64 pipe
 // bounds both).
+// (The mixed solve has the true-residual criterion only.)
+template <typename T>
 __device__ __forceinline__ bool tiny_applies(const DevArrays& A, const InstScal& s) {
-  return s.x0flag != 0 && A.opts.criterion == HF_STOP_RECURSIVE;
+  return sizeof(T) == 8 && s.x0flag != 0 && A.opts.criterion == HF_STOP_RECURSIVE;
+}
+// f(true_type or false_type): a loop instantiated for either value of a uniform condition, because FP64
+// instructions that are predicated off take the FP64 pipe all the same.
+template <class F>
+__device__ __forceinline__ void for_flag(bool flag, F f) {
+  if (flag) f(std::true_type{});
+  else f(std::false_type{});
 }
 
 // ---- neighbour access for the columns of a task ------------------------------------------------
@@ -204,56 +214,88 @@ __device__ __forceinline__ int y_south(const TCell& c) {
   return c.py ? (c.ny - 1) * c.nx : kNoNbr;
 }
 
+__device__ __forceinline__ float2 pair_of(float a, float b) { return make_float2(a, b); }
+__device__ __forceinline__ double2 pair_of(double a, double b) { return make_double2(a, b); }
+
 // First residual of a step from the products the last two steps stored: x0 = T^n + (T^n - T^(n-1))
 // (mod_evolve.f90:141), so S - H x0 = S - 2 H T^n + H T^(n-1) up to the rounding of x0 (~1e-16 of
 // the terms).  Pointwise: 40 B and 4 FP64 instructions per cell (mixed) instead of the stencil
-// sweep's 64 B and 9.  The step's acceptance test stays the FP64 residual of the final x.
+// sweep's 64 B and 9.  The step's acceptance test stays the FP64 residual of the final x.  Bound by
+// HBM and the FP64 pipe alike; the loads of U pairs are issued together (256^3 slab 144 -> 120 us, 64
+// uneven grids 242 -> 121, against passes over column tiles).
 template <typename TR>
 __device__ __forceinline__ void res_hx_task(const DevArrays& A, double* part, int64_t task,
                                             const InstScal& s) {
-  const TCell c = task_cell(A, task);
-  const int64_t off = c.off;
-  const double* __restrict__ b = A.b + off;
-  const double* __restrict__ yc = A.hx[s.hx_role] + off;
-  const double* __restrict__ yp = A.hx[1 - s.hx_role] + off;
-  const double* __restrict__ rsum = A.rsum + off;
-  const float* __restrict__ sinv32 = A.sinv32 + off;
-  const double* __restrict__ sinv = A.sinv + off;
-  TR* R = Vec<TR>::r(A) + c.off4;             // the inner solve's layout
+  constexpr bool F32 = sizeof(TR) == 4;
+  constexpr int U = F32 ? 4 : 2;
+  const Chunk c = task_chunk(A, task);
+  const InstDesc& d = *c.d;
+  const double* __restrict__ b = A.b + d.off;
+  const double* __restrict__ yc = A.hx[s.hx_role] + d.off;
+  const double* __restrict__ yp = A.hx[1 - s.hx_role] + d.off;
+  const double* __restrict__ rsum = A.rsum + d.off;
+  const TR* __restrict__ sinv;
+  if constexpr (F32) sinv = A.sinv32 + d.off;
+  else sinv = A.sinv + d.off;
+  TR* R = Vec<TR>::r(A) + d.off4;             // the inner solve's layout
+  [[maybe_unused]] const int n = d.n, n4 = d.sx * d.ny * d.nz;
   const float isig = (float)(1.0 / s.sigma);
-  const bool tiny = tiny_applies(A, s);       // the residual of x0 + TINY: r(x0) - TINY * H1
+  const bool tiny = tiny_applies<TR>(A, s);       // the residual of x0 + TINY: r(x0) - TINY * H1
   double rr = 0.0, gg64 = 0.0;
   float gg = 0.f;
   SqSum rq;                                    // mixed: ||r||^2 off the FP64 pipe
-  if (c.act(0)) {
-    const int nxy = c.nxy, base = c.base(0);
-    const int rxy = c.nxy4, rbase = c.base4(0);
-#pragma unroll 4
-    for (int z = c.z0; z < c.z1; ++z) {
-      const int l = base + z * nxy, lr = rbase + z * rxy;
-      if (z + 4 < c.z1) {                       // four planes ahead
-        prefetch_l2(b + l + 4 * nxy);
-        prefetch_l2(yc + l + 4 * nxy);
-        prefetch_l2(yp + l + 4 * nxy);
+  auto cell = [&](auto with_tiny, double bv, double cv, double pv, TR si, int l) -> TR {
+    double a = fma(-2.0, cv, bv);
+    a = a + pv;
+    if constexpr (decltype(with_tiny)::value) a = fma(-kTiny, rsum[l], a);
+    if constexpr (F32) {
+      rq.add(a);
+      const float g = -si * f64_to_f32_trunc(a) * isig;
+      gg = fmaf(g, g, gg);
+      return g;
+    } else {
+      rr = fma(a, a, rr);
+      const double g = -si * a;
+      gg64 = fma(g, g, gg64);
+      return g;
+    }
+  };
+  auto cells = [&](auto with_tiny) {
+    for (unsigned l0 = c.first(); l0 < c.end; l0 += c.step * U) {
+      double2 bv[U], cv[U], pv[U];
+      decltype(ld_pair(sinv, 0, true)) sv[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const unsigned l = l0 + c.step * u;
+        if (l >= c.end) continue;
+        const bool two = l + 1 < c.end;
+        const int lc = HF_IXP(A, l, n, two);
+        bv[u] = ld_pair(b, lc, two);
+        cv[u] = ld_pair(yc, lc, two);
+        pv[u] = ld_pair(yp, lc, two);
+        sv[u] = ld_pair(sinv, lc, two);
       }
-      const int lc = HF_IX(A, l, c.n());
-      double a = fma(-2.0, yc[lc], b[lc]);
-      a = a + yp[lc];
-      if (tiny) a = fma(-kTiny, rsum[lc], a);
-      if (sizeof(TR) == 4) rq.add(a); else rr = fma(a, a, rr);
-      if (sizeof(TR) == 4) {
-        const float g = -sinv32[lc] * f64_to_f32_trunc(a) * isig;
-        R[HF_IX(A, lr, c.n4())] = (TR)g;
-        gg = fmaf(g, g, gg);
-      } else {
-        const double g = -sinv[lc] * a;
-        R[HF_IX(A, lr, c.n4())] = (TR)g;
-        gg64 = fma(g, g, gg64);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const unsigned l = l0 + c.step * u;
+        if (l >= c.end) continue;
+        const bool two = l + 1 < c.end;
+        const TR g0 = cell(with_tiny, bv[u].x, cv[u].x, pv[u].x, sv[u].x, l);
+        TR g1 = TR(0);
+        if (two) g1 = cell(with_tiny, bv[u].y, cv[u].y, pv[u].y, sv[u].y, l + 1);
+        if (c.rows4) {
+          st_pair(R, HF_IXP(A, l, n4, two), two, pair_of(g0, g1));
+        } else {
+          R[HF_IX(A, c.inner(l), n4)] = g0;
+          if (two) R[HF_IX(A, c.inner(l + 1), n4)] = g1;
+        }
       }
     }
-  }
-  if (sizeof(TR) == 4) rr = rq.value();
-  if (sizeof(TR) == 4) {
+  };
+  if constexpr (F32) cells(std::false_type{});
+  else for_flag(tiny, cells);
+  if constexpr (F32) {
+    rr = rq.value();
     task_store_f(part + A.pcap + task, gg);
     const double v[1] = {rr};
     tile_store<1>(part + task, A.pcap, v);
@@ -262,11 +304,6 @@ __device__ __forceinline__ void res_hx_task(const DevArrays& A, double* part, in
     tile_store<2>(part + task, A.pcap, v);
   }
 }
-
-__device__ __forceinline__ bool vec4_ok(const InstDesc& d);
-template <typename TR>
-__device__ __forceinline__ void res_hx4_task(const DevArrays& A, double* part, int64_t task,
-                                             const InstScal& s);
 
 // FP64 true residual of one task: r = S - H x with x in the x-read buffer (INIT: x0 from the RHS
 // kernel) or, after an update, in the x-write buffer (the epilogue then swaps the roles).  Writes
@@ -277,8 +314,7 @@ template <bool INIT, typename TR, bool XOUT = false>
 __device__ __forceinline__ void res_task(const DevArrays& A, double* part, int64_t task,
                                           const InstScal& s) {
   if (INIT && s.hx_ok >= 2) {
-    if (vec4_ok(A.inst[A.tasks[task].x])) res_hx4_task<TR>(A, part, task, s);
-    else res_hx_task<TR>(A, part, task, s);
+    res_hx_task<TR>(A, part, task, s);
     return;
   }
   const TCell c = task_cell(A, task);
@@ -302,7 +338,7 @@ __device__ __forceinline__ void res_task(const DevArrays& A, double* part, int64
   // this FP64-bound sweep)
   SqSum rq;
   // INIT: the residual of x0 + TINY (mod_evolve.f90:141) is r(x0) - TINY * H1
-  const bool tiny = INIT && tiny_applies(A, s);
+  const bool tiny = INIT && tiny_applies<TR>(A, s);
   const bool act = c.act(0);
   const int nz = c.nz, nxy = c.nxy, base = c.base(0);
   const XEdge xe = x_edges(c);
@@ -403,237 +439,66 @@ struct YEnd {
   }
 };
 
-// Solution update of one task: x_new = x + sigma S^-1 y (+ TINY once).
+// Solution update of some cells: x_new = x + sigma S^-1 y (+ TINY once).  Bound by HBM (256^3 slab 94 ->
+// 78 us, 5.9 TB/s).
 template <typename TY>
-__device__ __forceinline__ void xupd_task(const DevArrays& A, double* part, int64_t task,
-                                          const InstScal& s) {
-  const TCell c = task_cell(A, task);
-  if (!c.act(0)) return;
-  const int64_t off = c.off;
-  const double* XR = A.tbuf[s.role[2]] + off;
-  double* XW = A.tbuf[s.role[3]] + off;
-  const TY* Y = Vec<TY>::y(A) + c.off4;       // the inner solve's layout
-  const TY* P = Vec<TY>::pb(A, s.iter - 1) + c.off4;
+__device__ __forceinline__ void xupd_cells(const DevArrays& A, const Chunk& c, const InstScal& s) {
+  constexpr bool F32 = sizeof(TY) == 4;
+  constexpr int U = 1;
+  const InstDesc& d = *c.d;
+  const double* XR = A.tbuf[s.role[2]] + d.off;
+  double* XW = A.tbuf[s.role[3]] + d.off;
+  const TY* Y = Vec<TY>::y(A) + d.off4;       // the inner solve's layout
+  const TY* P = Vec<TY>::pb(A, s.iter - 1) + d.off4;
   const YEnd<TY> ye(s);
-  const double* __restrict__ sinv = A.sinv + off;
-  const float* __restrict__ sinv32 = A.sinv32 + off;
+  const TY* __restrict__ sinv;
+  if constexpr (F32) sinv = A.sinv32 + d.off;
+  else sinv = A.sinv + d.off;
+  [[maybe_unused]] const int n = d.n, n4 = d.sx * d.ny * d.nz;
   const bool use_y = s.iter > 0;
-  const bool tiny = s.tiny_pending != 0;
+  const bool tiny = !F32 && s.tiny_pending != 0;
   const float sig = (float)s.sigma_prev;
-  const int nxy = c.nxy, base = c.base(0);
-  const int yxy = c.nxy4, ybase = c.base4(0);
-  for (int z0 = c.z0; z0 < c.z1; z0 += 4) {
-    double xv[4], sv[4];
-    float sv32[4];
-    TY yv[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int l = base + (z0 + u) * nxy;
-      xv[u] = 0.0; yv[u] = TY(0); sv[u] = 0.0; sv32[u] = 0.f;
-      if (z0 + u < c.z1) {
-        const int lc = HF_IX(A, l, c.n());
-        xv[u] = XR[lc];
-        if (use_y) {
-          const int ly = HF_IX(A, ybase + (z0 + u) * yxy, c.n4());
-          yv[u] = ye(ye.old ? Y[ly] : TY(0), ye.last ? P[ly] : TY(0));
-          if (sizeof(TY) == 8) sv[u] = sinv[lc];
-          else sv32[u] = sinv32[lc];
-        }
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      if (z0 + u >= c.z1) continue;
-      const int l = base + (z0 + u) * nxy;
-      double x = xv[u];
-      if (tiny) x = x + kTiny;
-      if (use_y) {
-        if (sizeof(TY) == 8) x = fma(sv[u], (double)yv[u], x);   // sigma = 1 on the FP64 path
-        else x = x + f32_to_f64(sig * sv32[u] * (float)yv[u]);
-      }
-      XW[HF_IX(A, l, c.n())] = x;
-    }
-  }
-}
-
-__device__ __forceinline__ bool vec4_ok(const InstDesc& d) { return (d.nx & 3) == 0; }
-
-// ---- passes over the cell tasks on 4-cell vectors (rows of 4k cells) --------------------------
-// Four z-groups of 64 threads, 4 consecutive x cells per thread; FP32 vectors are one 16-byte
-// access, FP64 vectors two.  Two planes of loads are issued before they are used.  Reductions are
-// summed per thread plane by plane, cells in x order.
-template <typename T> struct V4 { T v[4]; };
-__device__ __forceinline__ V4<float> ldv4(const float* p) {
-  const float4 t = *reinterpret_cast<const float4*>(p);
-  return V4<float>{{t.x, t.y, t.z, t.w}};
-}
-__device__ __forceinline__ V4<double> ldv4(const double* p) {
-  const double2 a = reinterpret_cast<const double2*>(p)[0], b = reinterpret_cast<const double2*>(p)[1];
-  return V4<double>{{a.x, a.y, b.x, b.y}};
-}
-__device__ __forceinline__ void stv4(float* p, const V4<float>& v) {
-  *reinterpret_cast<float4*>(p) = make_float4(v.v[0], v.v[1], v.v[2], v.v[3]);
-}
-__device__ __forceinline__ void stv4(double* p, const V4<double>& v) {
-  reinterpret_cast<double2*>(p)[0] = make_double2(v.v[0], v.v[1]);
-  reinterpret_cast<double2*>(p)[1] = make_double2(v.v[2], v.v[3]);
-}
-
-// A thread's quad: 4 consecutive x cells of a quarter of the task's planes.
-struct Quad {
-  int64_t off;
-  int nxy, lxy, za, zb, n;
-  bool act;
-};
-__device__ __forceinline__ Quad quad_cell(const DevArrays& A, int64_t task) {
-  const int4 tk = A.tasks[task];
-  const InstDesc& d = A.inst[tk.x];
-  const int tid = threadIdx.x, grp = tid >> 6, w = tid & 63;
-  const int x = tk.y + 4 * (w & 7), y = tk.z + (w >> 3);
-  const int z1 = min(tk.w + d.zc, d.nz);
-  const int per = (z1 - tk.w + 3) >> 2;
-  Quad c;
-  c.off = d.off;
-  c.nxy = d.nx * d.ny;
-  c.lxy = y * d.nx + x;
-  c.za = min(tk.w + grp * per, z1);
-  c.zb = min(c.za + per, z1);
-  c.act = x < d.nx && y < d.ny;
-  c.n = c.nxy * d.nz;
-  return c;
-}
-
-template <typename TY>
-__device__ __forceinline__ void xupd4_task(const DevArrays& A, double* part, int64_t task,
-                                           const InstScal& s) {
-  const Quad c = quad_cell(A, task);   // rows of 4k cells: the two layouts agree in shape
-  if (!c.act) return;
-  const double* XR = A.tbuf[s.role[2]] + c.off;
-  double* XW = A.tbuf[s.role[3]] + c.off;
-  const int64_t off4 = A.inst[A.tasks[task].x].off4;
-  const TY* Y = Vec<TY>::y(A) + off4;
-  const TY* P = Vec<TY>::pb(A, s.iter - 1) + off4;
-  const YEnd<TY> ye(s);
-  auto ldy = [&](int l) -> V4<TY> {
-    V4<TY> y{}, p{};
-    if (ye.old) y = ldv4(Y + l);
-    if (ye.last) p = ldv4(P + l);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) y.v[i] = ye(y.v[i], p.v[i]);
-    return y;
+  auto inner = [&](const TY* v, int l, bool two) {
+    if (c.rows4) return ld_pair(v, HF_IXP(A, l, n4, two), two);
+    return pair_of(v[HF_IX(A, c.inner(l), n4)], two ? v[HF_IX(A, c.inner(l + 1), n4)] : TY(0));
   };
-  const double* __restrict__ sinv = A.sinv + c.off;
-  const float* __restrict__ sinv32 = A.sinv32 + c.off;
-  const bool use_y = s.iter > 0;
-  const bool tiny = s.tiny_pending != 0;
-  const float sig = (float)s.sigma_prev;
-  for (int z = c.za; z < c.zb; z += 2) {
-    const bool two = z + 1 < c.zb;
-    const int l0 = HF_IX4(A, c.lxy + z * c.nxy, c.n);
-    const int l1 = two ? HF_IX4(A, l0 + c.nxy, c.n) : 0;
-    V4<double> x0 = ldv4(XR + l0), x1{}, s0{}, s1{};
-    V4<TY> y0{}, y1{};
-    V4<float> f0{}, f1{};
+  auto cell = [&](auto with_tiny, double x, TY y, TY si) -> double {
+    if constexpr (decltype(with_tiny)::value) x = x + kTiny;
     if (use_y) {
-      y0 = ldy(l0);
-      if (sizeof(TY) == 8) s0 = ldv4(sinv + l0); else f0 = ldv4(sinv32 + l0);
+      if constexpr (F32) x = x + f32_to_f64(sig * si * y);
+      else x = fma(si, y, x);                 // sigma = 1 on the FP64 path
     }
-    if (two) {
-      x1 = ldv4(XR + l1);
-      if (use_y) {
-        y1 = ldy(l1);
-        if (sizeof(TY) == 8) s1 = ldv4(sinv + l1); else f1 = ldv4(sinv32 + l1);
-      }
-    }
+    return x;
+  };
+  auto cells = [&](auto with_tiny) {
+    for (unsigned l0 = c.first(); l0 < c.end; l0 += c.step * U) {
+      double2 xv[U];
+      decltype(ld_pair(sinv, 0, true)) yv[U], pv[U], sv[U];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      if (h == 1 && !two) break;
-      V4<double> xv = h ? x1 : x0;
-      const V4<TY>& yv = h ? y1 : y0;
-      const V4<double>& sv = h ? s1 : s0;
-      const V4<float>& fv = h ? f1 : f0;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        double x = xv.v[i];
-        if (tiny) x = x + kTiny;
+      for (int u = 0; u < U; ++u) {
+        const unsigned l = l0 + c.step * u;
+        yv[u] = pv[u] = sv[u] = pair_of(TY(0), TY(0));
+        if (l >= c.end) continue;
+        const bool two = l + 1 < c.end;
+        xv[u] = ld_pair(XR, HF_IXP(A, l, n, two), two);
         if (use_y) {
-          if (sizeof(TY) == 8) x = fma(sv.v[i], (double)yv.v[i], x);   // sigma = 1 on the FP64 path
-          else x = x + f32_to_f64(sig * fv.v[i] * (float)yv.v[i]);
+          if (ye.old) yv[u] = inner(Y, l, two);
+          if (ye.last) pv[u] = inner(P, l, two);
+          sv[u] = ld_pair(sinv, HF_IXP(A, l, n, two), two);
         }
-        xv.v[i] = x;
       }
-      stv4(XW + (h ? l1 : l0), xv);
-    }
-  }
-}
-
-// The step's first residual from the stored products (res_hx_task) on 4-cell vectors, for rows of
-// 4k cells: the same per-cell arithmetic; ||r||^2 and ||g||^2 summed per thread plane by plane,
-// cells in x order.  A quarter of the scalar form's load instructions keeps more bytes in flight
-// on this FP64-bound round.
-template <typename TR>
-__device__ __forceinline__ void res_hx4_task(const DevArrays& A, double* part, int64_t task,
-                                             const InstScal& s) {
-  const Quad c = quad_cell(A, task);   // rows of 4k cells: the two layouts agree in shape
-  const int64_t off = c.off;
-  const double* __restrict__ b = A.b + off;
-  const double* __restrict__ yc = A.hx[s.hx_role] + off;
-  const double* __restrict__ yp = A.hx[1 - s.hx_role] + off;
-  const double* __restrict__ rsum = A.rsum + off;
-  const float* __restrict__ sinv32 = A.sinv32 + off;
-  const double* __restrict__ sinv = A.sinv + off;
-  const bool f32 = sizeof(TR) == 4;
-  TR* R = Vec<TR>::r(A) + A.inst[A.tasks[task].x].off4;
-  const float isig = (float)(1.0 / s.sigma);
-  const bool tiny = tiny_applies(A, s);       // the residual of x0 + TINY: r(x0) - TINY * H1
-  double rr = 0.0, gg64 = 0.0;
-  float gg = 0.f;
-  SqSum rq;                                    // mixed: ||r||^2 off the FP64 pipe
-  if (c.act) {
-    for (int z = c.za; z < c.zb; ++z) {
-      const int l = HF_IX4(A, c.lxy + z * c.nxy, c.n);
-      const V4<double> bv = ldv4(b + l), cv = ldv4(yc + l), pv = ldv4(yp + l);
-      V4<double> rs{}, s64{};
-      V4<float> s32{};
-      if (tiny) rs = ldv4(rsum + l);
-      if (f32) s32 = ldv4(sinv32 + l);
-      else s64 = ldv4(sinv + l);
-      V4<TR> g4;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        double a = fma(-2.0, cv.v[i], bv.v[i]);
-        a = a + pv.v[i];
-        if (tiny) a = fma(-kTiny, rs.v[i], a);
-        if (f32) rq.add(a); else rr = fma(a, a, rr);
-        if (f32) {
-          const float g = -s32.v[i] * f64_to_f32_trunc(a) * isig;
-          g4.v[i] = (TR)g;
-          gg = fmaf(g, g, gg);
-        } else {
-          const double g = -s64.v[i] * a;
-          g4.v[i] = (TR)g;
-          gg64 = fma(g, g, gg64);
-        }
+      for (int u = 0; u < U; ++u) {
+        const unsigned l = l0 + c.step * u;
+        if (l >= c.end) continue;
+        const double2 x = make_double2(cell(with_tiny, xv[u].x, ye(yv[u].x, pv[u].x), sv[u].x),
+                                       cell(with_tiny, xv[u].y, ye(yv[u].y, pv[u].y), sv[u].y));
+        st_pair(XW, HF_IXP(A, l, n, l + 1 < c.end), l + 1 < c.end, x);
       }
-      stv4(R + l, g4);
     }
-  }
-  if (f32) rr = rq.value();
-  if (sizeof(TR) == 4) {
-    task_store_f(part + A.pcap + task, gg);
-    const double v[1] = {rr};
-    tile_store<1>(part + task, A.pcap, v);
-  } else {
-    const double v[2] = {rr, gg64};
-    tile_store<2>(part + task, A.pcap, v);
-  }
-}
-
-// Dispatch between the vector and the scalar form of the x update (same choice on every path).
-template <typename TY>
-__device__ __forceinline__ void xupd_any(const DevArrays& A, double* part, int64_t task, const InstScal& s) {
-  if (vec4_ok(A.inst[A.tasks[task].x])) xupd4_task<TY>(A, part, task, s);
-  else xupd_task<TY>(A, part, task, s);
+  };
+  if constexpr (F32) cells(std::false_type{});
+  else for_flag(tiny, cells);
 }
 
 // ---- the inner solve's passes ------------------------------------------------------------------
@@ -1176,9 +1041,10 @@ __global__ void __launch_bounds__(kBlock) k_residual(DevArrays A, int log) {
 
 template <typename TY>
 __global__ void __launch_bounds__(kBlock) k_xupdate(DevArrays A) {
-  const InstScal& s = A.scal[A.tasks[blockIdx.x].x];
+  const int64_t task = blockIdx.x / kFine;
+  const InstScal& s = A.scal[task_inst(A, task)];
   if (!s.outer_active || s.inner_active || s.refine == 0 || (s.xw & kXwDone)) return;
-  xupd_any<TY>(A, A.partials, blockIdx.x, s);
+  xupd_cells<TY>(A, task_chunk<kFine>(A, task, (int)(blockIdx.x % kFine)), s);
 }
 
 template <typename T>
@@ -1588,7 +1454,7 @@ __device__ __forceinline__ void round_task(const DevArrays& A, const InstDesc& d
     switch (s.phase) {
       case PH_RES_INIT: res_task<true, T>(A, part, task, s); break;
       case PH_RES: res_task<false, T, XOUT>(A, part, task, s); break;
-      case PH_XUPD: xupd_any<T>(A, part, task, s); break;
+      case PH_XUPD: xupd_cells<T>(A, task_chunk(A, task), s); break;
       default: break;
     }
   }
@@ -2694,7 +2560,7 @@ static void launch_res(Ctx& c, int mode, int log) {
     k_residual<true, T><<<nb, kBlock, 0, c.stream>>>(c.A, log);
     return;
   }
-  k_xupdate<T><<<nb, kBlock, 0, c.stream>>>(c.A);
+  k_xupdate<T><<<nb * kFine, kBlock, 0, c.stream>>>(c.A);
   if (c.A.xout) k_residual<false, T, true><<<nb, kBlock, 0, c.stream>>>(c.A, log);
   else k_residual<false, T><<<nb, kBlock, 0, c.stream>>>(c.A, log);
 }
@@ -2759,8 +2625,8 @@ cudaError_t launch_single(Ctx& c, int which) {
       else k_residual<true, double><<<nb, kBlock, 0, c.stream>>>(c.A, 0);
       break;
     case HF_KERNEL_XUPDATE:
-      if (fp32) k_xupdate<float><<<nb, kBlock, 0, c.stream>>>(c.A);
-      else k_xupdate<double><<<nb, kBlock, 0, c.stream>>>(c.A);
+      if (fp32) k_xupdate<float><<<nb * kFine, kBlock, 0, c.stream>>>(c.A);
+      else k_xupdate<double><<<nb * kFine, kBlock, 0, c.stream>>>(c.A);
       break;
     // the direction update and the SpMV are one pass
     case HF_KERNEL_CG_P:
