@@ -676,11 +676,12 @@ int64_t inner_cells(const Ctx& c) {
   return d.off4 + (n4 + kTile - 1) / kTile * kTile;
 }
 
-// The tasks of the inner solve's passes.  A tile is 2^cqx 16-byte vectors (4 FP32 or 2 FP64 cells)
-// wide and kBlock / 2^cqx rows high, of the shapes the one that covers the grid's plane with the
-// fewest tiles (of equals the one of 16 vectors: its halo rows and the sectors that its row ends
-// read beside it are fewest).  Along z a tile is cut into parts, whose ends read a plane of their
-// neighbours.  One grid: as many parts as make its longest chain of planes per block, over waves of
+// The tasks of the inner solve's passes.  A tile is cgw 16-byte vectors (4 FP32 or 2 FP64 cells) wide
+// and cgr rows high, 8 to 32 vectors and at most kBlock in all, of these shapes the one that covers the
+// grid's plane with the fewest tiles, evenly (of equals the one that reads least beside itself).  With
+// widths of 8, 16 and 32 vectors only, the tiles of 64 grids of 16 to 96 cells an edge held 1.47 threads
+// per vector, with these 1.22 (20 steps 71 -> 60 ms, with the 128-byte alignment of their
+// shared memory).  Along z a tile is cut into parts, whose ends read a plane of their neighbours.  One grid: as many parts as make its longest chain of planes per block, over waves of
 // kSolveBlocks blocks, shortest, the halo counted as one plane per part; a count above one wave
 // pays only where a wave could not be filled.  Several grids: parts of one length for all, such
 // that there are about kBatchWaves tasks per block -- they are handed out one at a time, and each
@@ -692,13 +693,21 @@ int cg_plan(Ctx& c) {
   const int vec = c.opts.precision == HF_PREC_MIXED ? 4 : 2;
   int64_t planes = 0;                 // tile planes of all grids
   for (InstDesc& d : c.h_inst) {
-    int64_t best = 0;
-    for (int q : {4, 5, 3}) {
-      const int w = vec << q, h = kBlock >> q;
-      const int64_t nbx = (d.nx + w - 1) / w, nby = (d.ny + h - 1) / h;
-      if (best != 0 && nbx * nby >= best) continue;
+    const int nv = (d.nx + vec - 1) / vec;
+    int64_t best = INT64_MAX, edge = 0;
+    for (int w0 = 32; w0 >= 8; --w0) {
+      const int64_t nbx = (nv + w0 - 1) / w0;
+      const int w = std::max<int>(8, (int)((nv + nbx - 1) / nbx));    // as even as they come
+      const int64_t nby = (d.ny + kBlock / w - 1) / (kBlock / w);
+      const int h = (int)((d.ny + nby - 1) / nby);
+      if ((w + 2) * (h + 2) > kTilePlane || 2 * (w + h) > kTileHalo) continue;
+      // fewest tiles; then the fewest bytes beyond a tile (a cell beside a row costs 32)
+      const int64_t e = 16 * w + 32 * h;
+      if (nbx * nby > best || (nbx * nby == best && e > edge)) continue;
       best = nbx * nby;
-      d.cqx = q;
+      edge = e;
+      d.cgw = w;
+      d.cgr = h;
       d.cgnx = (int32_t)nbx;
       d.cgny = (int32_t)nby;
     }

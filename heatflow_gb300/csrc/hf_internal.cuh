@@ -27,6 +27,9 @@ constexpr double kPi = 3.141592653589793;    // mod_constants.f90:12
 constexpr double kStefBoltz = 5.670373e-8;   // mod_constants.f90:16
 
 constexpr int kBlock = 256;                  // threads per block of the cell kernels
+// Tiles of the inner solve's passes: the vectors of a plane with those around it, and the vectors and
+// cells around it (PqShared), at most.
+constexpr int kTilePlane = 340, kTileHalo = 80;
 constexpr int kCellsPerThread = 4;
 constexpr int kTile = kBlock * kCellsPerThread;   // cells per tile (one block per tile)
 constexpr int kNR = 8;
@@ -68,9 +71,9 @@ struct InstDesc {
   // layout of the other FP64 arrays.
   int64_t off4;
   int32_t sx;
-  // Tasks of the inner solve's passes (cg_plan): tiles of 2^cqx 16-byte vectors x kBlock / 2^cqx rows,
+  // Tasks of the inner solve's passes (cg_plan): tiles of cgw 16-byte vectors x cgr rows,
   // cgnx x cgny of them, each cut into cgnz parts along z; cgn in all, the first at cg0.
-  int32_t cqx, cgnx, cgny, cgnz, cgn;
+  int32_t cgw, cgr, cgnx, cgny, cgnz, cgn;
   int64_t cg0;
 };
 

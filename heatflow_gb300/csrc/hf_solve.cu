@@ -511,18 +511,20 @@ __device__ __forceinline__ void xupd_cells(const DevArrays& A, const Chunk& c, c
 // rounds.  Iteration 0 has p_0 = r and no y.
 //
 // Tasks (InstDesc::cgn of them): a block's thread owns one 16-byte vector (4 FP32 or 2 FP64 cells)
-// of a tile of 2^cqx vectors x kBlock / 2^cqx rows and marches the task's planes along z.  The operands
+// of a tile of cgw vectors x cgr rows and marches the task's planes along z.  The operands
 // come through shared memory (cp.async), two planes ahead of the one that is computed: loads to
 // registers left the distance to the compiler, whose schedule of the same loop took 110 to 157 us at
 // 256^3 depending on the code around it.  p is formed once per cell, from r and p_(k-1), and shared:
 // three planes of the tile with the cells around it, whose p is formed from their r and p_(k-1) as well
 // (the value that their own tile stores) by threads that take one such vector or cell each.  One
 // block barrier per plane.
+// The shared memory starts on 128 bytes: 48 bytes off, the passes at 256^3 took 124 and 36 us instead of
+// 108 and 30 (32 bytes off: 111 and 30).
 // The rows of the inner solve's layout are padded to 4 cells: in a row's last vector the cells past
 // nx have zero coefficients, and q and r are kept zero there.  A face that does not exist has a
 // zero coefficient or a zero neighbour.
 // Bound by HBM in FP32 and by the FP64 pipe in FP64 (9 instructions per cell).  Measured on the
-// layered slab: 256^3 FP32, pq 111 us (5.4 TB/s) and upd 31 us (6.5 TB/s), where the direction
+// layered slab: 256^3 FP32, pq 108 us (5.6 TB/s) and upd 30 us (6.7 TB/s), where the direction
 // update, the SpMV and the update took 38 + 68 + 75 us; 190 x 192 x 192 FP64, 134 + 30 us against
 // 34 + 111 + 68 us.
 template <typename T>
@@ -555,15 +557,12 @@ template <typename T>
 struct PqShared {
   struct Stage {
     Vec16<T> r[kBlock], po[kBlock], y[kBlock], ax[kBlock], ay[kBlock], az[kBlock];
-    Vec16<T> hr[80], hpo[80], hf[80];
+    Vec16<T> hr[kTileHalo], hpo[kTileHalo], hf[kTileHalo];
   } st[kPqStages];
-  Vec16<T> p[3][340];
+  Vec16<T> p[3][kTilePlane];
 };
 template <typename T>
 constexpr int kPqSmem = (int)sizeof(PqShared<T>);   // 99 KB: two blocks per SM
-static_assert(kBlock == 256 && (8 + 2) * (32 + 2) <= 340 && (16 + 2) * (16 + 2) <= 340 && 2 * (8 + 32) <= 80,
-              "tiles of 8, 16 or 32 vectors a row");
-
 __device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 template <typename T>
 __device__ __forceinline__ void cp16(Vec16<T>* dst, const T* src) {
@@ -588,15 +587,15 @@ template <typename T>
 __device__ __forceinline__ CgPos cg_pos(const InstDesc& d, int local) {
   const int bx = local % d.cgnx, rest = local / d.cgnx, by = rest % d.cgny, bz = rest / d.cgny;
   CgPos c;
-  c.vx = (int)threadIdx.x & ((1 << d.cqx) - 1);
-  c.ry = (int)threadIdx.x >> d.cqx;
-  c.x0 = (bx << d.cqx) * Vec16<T>::N;
-  c.y0 = by * (kBlock >> d.cqx);
+  c.ry = (int)(threadIdx.x / (unsigned)d.cgw);
+  c.vx = (int)threadIdx.x - c.ry * d.cgw;
+  c.x0 = bx * d.cgw * Vec16<T>::N;
+  c.y0 = by * d.cgr;
   c.x = c.x0 + c.vx * Vec16<T>::N;
   c.y = c.y0 + c.ry;
   c.z0 = (int)((int64_t)bz * d.nz / d.cgnz);
   c.z1 = (int)((int64_t)(bz + 1) * d.nz / d.cgnz);
-  c.act = c.x < d.nx && c.y < d.ny;
+  c.act = c.x < d.nx && c.y < d.ny && c.ry < d.cgr;
   return c;
 }
 
@@ -608,12 +607,12 @@ struct Beyond { int hl, hp; bool hvec, hc; };
 template <typename T>
 __device__ __forceinline__ Beyond beyond_of(const InstDesc& d, const CgPos& c) {
   constexpr int V = Vec16<T>::N;
-  const int tid = threadIdx.x, nq = 1 << d.cqx, rows = kBlock >> d.cqx, prow = nq + 2;
+  const int tid = threadIdx.x, nq = d.cgw, rows = d.cgr, prow = nq + 2;
   const int nx = d.nx, ny = d.ny, sx = d.sx;
   const int nv = min(nq, (nx - c.x0 + V - 1) / V), nr = min(rows, ny - c.y0);   // vectors, rows in use
   Beyond b{-1, 0, true, false};
   if (tid < 2 * nq) {
-    const int v = tid & (nq - 1), xv = c.x0 + v * V;
+    const int v = tid < nq ? tid : tid - nq, xv = c.x0 + v * V;
     if (v < nv && ny > 1) {
       if (tid < nq) {
         if (c.y0 + nr < ny) b.hl = (c.y0 + nr) * sx + xv;
@@ -657,7 +656,7 @@ __device__ __forceinline__ void pq_form(const DevArrays& A, const InstDesc& d, i
   typedef Vec16<T> VT;
   PqShared<T>& sm = *reinterpret_cast<PqShared<T>*>(dyn);
   const CgPos c = cg_pos<T>(d, local);
-  const int tid = threadIdx.x, nq = 1 << d.cqx, rows = kBlock >> d.cqx, prow = nq + 2;
+  const int tid = threadIdx.x, nq = d.cgw, rows = d.cgr, prow = nq + 2;
   const int nx = d.nx, ny = d.ny, nz = d.nz, sx = d.sx, nxy = sx * ny;
   [[maybe_unused]] const int n4 = nxy * nz;
   const int z0 = c.z0, z1 = c.z1;
@@ -767,7 +766,7 @@ __device__ __forceinline__ void pq_form(const DevArrays& A, const InstDesc& d, i
       if (!FIRST) hpo.v[0] = Po[l];
     }
   }
-  for (int i = tid; i < 3 * 340; i += kBlock) sm.p[0][i] = zero;
+  for (int i = tid; i < 3 * kTilePlane; i += kBlock) sm.p[0][i] = zero;
   __syncthreads();
   auto put_beyond = [&](VT* pl, const VT& hr, const VT& hpo) {
     if (hvec) pl[hp] = form(hr, hpo);
@@ -1049,7 +1048,7 @@ __global__ void __launch_bounds__(kBlock) k_xupdate(DevArrays A) {
 
 template <typename T>
 __global__ void __launch_bounds__(kBlock) k_cg_pq(DevArrays A) {
-  extern __shared__ __align__(16) char dyn[];
+  extern __shared__ __align__(128) char dyn[];
   const int inst = A.cg_inst[blockIdx.x];
   const InstScal& s = A.scal[inst];
   if (!s.inner_active) return;
@@ -1059,7 +1058,7 @@ __global__ void __launch_bounds__(kBlock) k_cg_pq(DevArrays A) {
 
 template <typename T>
 __global__ void __launch_bounds__(kBlock) k_cg_upd(DevArrays A) {
-  extern __shared__ __align__(16) char dyn[];
+  extern __shared__ __align__(128) char dyn[];
   const int inst = A.cg_inst[blockIdx.x];
   const InstScal& s = A.scal[inst];
   if (!s.inner_active) return;
@@ -1493,7 +1492,7 @@ __global__ void __launch_bounds__(kBlock, 2)
   __shared__ double red[kBlock * 2];
   __shared__ unsigned long long s_ticket, s_slot;
   __shared__ int s_inst, s_last, s_stop;
-  extern __shared__ __align__(16) char dyn[];
+  extern __shared__ __align__(128) char dyn[];
   const int ninst = (int)A.ninst;
   // the first phase's tickets: all instances' cell tasks, or those of the inner solve's passes
   const unsigned long long first = (unsigned long long)(FULL ? A.ntasks : A.ncg);
@@ -1724,7 +1723,7 @@ __global__ void __launch_bounds__(kBlock, 2)
   __shared__ InstScal sh;
   __shared__ InstDesc sd;
   __shared__ double red[(WEIGHTED ? 2 : 1) * kBlock];
-  extern __shared__ __align__(16) char dyn[];
+  extern __shared__ __align__(128) char dyn[];
   static_assert(sizeof(InstDesc) % 8 == 0 && sizeof(InstDesc) / 8 <= kBlock, "descriptor copy");
   const int tid = threadIdx.x, G = (int)gridDim.x;
   if (tid < kScalWords)
@@ -1781,7 +1780,7 @@ __global__ void __launch_bounds__(kBlock, 2)
 // tiles under the reference's rule 10.4 (13.3).
 template <typename T>
 struct ResLayout {                             // offsets in 16-byte vectors, for tasks of D planes
-  static constexpr int kPlane = 340, kHalo = 80;
+  static constexpr int kPlane = kTilePlane, kHalo = kTileHalo;
   int r, q, ax, ay, az, hr, hf, ur, azm, dg, n;
   bool has_dg;
   __host__ __device__ ResLayout(int D, bool weighted) {
@@ -1808,7 +1807,7 @@ __global__ void __launch_bounds__(kBlock, 2)
   __shared__ InstScal sh;
   __shared__ InstDesc sd;
   __shared__ double red[(WEIGHTED ? 2 : 1) * kBlock];
-  extern __shared__ __align__(16) char dyn[];
+  extern __shared__ __align__(128) char dyn[];
   const int tid = threadIdx.x;
   if (tid < kScalWords)
     reinterpret_cast<unsigned long long*>(&sh)[tid] = reinterpret_cast<const unsigned long long*>(A.scal)[tid];
@@ -1826,7 +1825,7 @@ __global__ void __launch_bounds__(kBlock, 2)
   VT* const P = reinterpret_cast<VT*>(dyn);
   const CgPos c = cg_pos<T>(sd, (int)blockIdx.x);
   const Beyond by = beyond_of<T>(sd, c);
-  const int nq = 1 << sd.cqx, prow = nq + 2, nx = sd.nx, ny = sd.ny, nz = sd.nz, sx = sd.sx, nxy = sx * ny;
+  const int nq = sd.cgw, prow = nq + 2, nx = sd.nx, ny = sd.ny, nz = sd.nz, sx = sd.sx, nxy = sx * ny;
   [[maybe_unused]] const int n4 = nxy * nz;
   const int z0 = c.z0, D = c.z1 - c.z0, lxy = c.y * sx + c.x, own = (c.ry + 1) * prow + c.vx + 1;
   const bool act = c.act;
@@ -2144,7 +2143,7 @@ __global__ void __launch_bounds__(kBlock, 1) k_solve_cluster(DevArrays A, SolveC
   __shared__ double table[3 * kClusterTasks];          // p.q; r.r and the weighted r.r
   __shared__ unsigned beside[kClusterSlots][6];          // per slot: the slots e, w, n, s, up, down of it
   __shared__ int4 origin[kClusterSlots];                 // per slot: x, y, z and first cell of its tile
-  extern __shared__ __align__(16) char dyn[];
+  extern __shared__ __align__(128) char dyn[];
   const int tid = threadIdx.x, C = (int)gridDim.x, rank = (int)blockIdx.x;
   if (tid < kScalWords)
     reinterpret_cast<unsigned long long*>(&sh)[tid] = reinterpret_cast<const unsigned long long*>(A.scal)[tid];
@@ -2154,9 +2153,9 @@ __global__ void __launch_bounds__(kBlock, 1) k_solve_cluster(DevArrays A, SolveC
   if (!sh.inner_active) return;                         // no inner solve is due (in any block)
   Slot* slot = reinterpret_cast<Slot*>(dyn);
   const int nt = sd.cgn, nxy_t = sd.cgnx * sd.cgny, task0 = rank * nt / C, slots = (rank + 1) * nt / C - task0;
-  const int nx = sd.nx, ny = sd.ny, nz = sd.nz, sx = sd.sx, nxy = sx * ny, nq = 1 << sd.cqx, rows = kBlock >> sd.cqx;
+  const int nx = sd.nx, ny = sd.ny, nz = sd.nz, sx = sd.sx, nxy = sx * ny, nq = sd.cgw, rows = sd.cgr;
   [[maybe_unused]] const int n4 = nxy * nz;
-  const int vx = tid & (nq - 1), ry = tid >> sd.cqx, lt = ry * sx + vx * V;
+  const int ry = tid / nq, vx = tid - ry * nq, lt = ry * sx + vx * V;
   const VT zero{};
   if (tid < slots) {
     const int t = task0 + tid, x = t % sd.cgnx * nq * V, y = t / sd.cgnx % sd.cgny * rows, z = t / nxy_t;
@@ -2177,7 +2176,7 @@ __global__ void __launch_bounds__(kBlock, 1) k_solve_cluster(DevArrays A, SolveC
   }
   for (int i = tid; i < 3 * kClusterTasks; i += kBlock) table[i] = 0.0;
   __syncthreads();
-  auto active = [&](const int4& o) { return o.x + vx * V < nx && o.y + ry < ny; };
+  auto active = [&](const int4& o) { return o.x + vx * V < nx && o.y + ry < ny && ry < rows; };
   for (int j = 0; j < slots; ++j) {
     const int4 o = origin[j];
     Slot& s = slot[j];
@@ -2244,7 +2243,7 @@ __global__ void __launch_bounds__(kBlock, 1) k_solve_cluster(DevArrays A, SolveC
               ps = s.p[tid - nq];
               ays = s.ay[tid - nq];
             } else if (y > 0 || sd.py) {
-              const int row = y > 0 ? rows - 1 : (ny - 1) & (rows - 1);
+              const int row = y > 0 ? rows - 1 : (ny - 1) % rows;
               const unsigned a = beside[j][3] + (row * nq + vx) * 16;
               ps = ld_cluster(a, T(0));
               ays = ld_cluster(a + kAy, T(0));
@@ -2256,7 +2255,7 @@ __global__ void __launch_bounds__(kBlock, 1) k_solve_cluster(DevArrays A, SolveC
             pw = s.p[tid - 1].v[V - 1];
             axw = s.ax[tid - 1].v[V - 1];
           } else if (x > 0 || (sd.px && nx > 1)) {      // the last cell of the tile, or of the row
-            const int e = x > 0 ? nq * V - 1 : (nx - 1) & (nq * V - 1);
+            const int e = x > 0 ? nq * V - 1 : (nx - 1) % (nq * V);
             const unsigned a = beside[j][1] + (tid + e / V) * 16;
             const VT w = ld_cluster(a, T(0)), f = ld_cluster(a + kAx, T(0));
 #pragma unroll
