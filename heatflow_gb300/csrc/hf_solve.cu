@@ -1232,18 +1232,16 @@ __device__ void epi_spmv_s(InstScal& s, const double* tot) {
 // What the epilogue of a CG update divides and roots: r.r over that of the iteration before, over
 // the inner solve's first, and the stopping criterion (the reference's on the unscaled recursive
 // residual r = -S rh sigma, mod_Sparse.f90:420).
-struct UpdRatios { double shrink, first, err; };
-__device__ __forceinline__ UpdRatios upd_ratios(const InstScal& s, const DevOpts& o, const double* tot) {
-  UpdRatios q;
-  q.shrink = tot[0] / s.rho;
-  q.first = tot[0] / s.gg0;
-  if (o.criterion == HF_STOP_RECURSIVE) q.err = s.bb > 0.0 ? sqrt(tot[1]) * s.sigma_prev / sqrt(s.bb) : 0.0;
-  else q.err = s.gg0 > 0.0 ? sqrt(q.first) : 0.0;
-  return q;
+struct UpdRatios { double shrink, first; };
+__device__ __forceinline__ double upd_err(const InstScal& s, bool weighted, double rr_w, double first) {
+  if (weighted) return s.bb > 0.0 ? sqrt(rr_w) * s.sigma_prev / sqrt(s.bb) : 0.0;
+  return s.gg0 > 0.0 ? sqrt(first) : 0.0;
 }
 
+// stop: the criterion is met.  The caller sets s.err.
 template <typename T>
-__device__ __forceinline__ void epi_upd_s(InstScal& s, const DevOpts& o, const double* tot, const UpdRatios& q) {
+__device__ __forceinline__ void epi_upd_s(InstScal& s, const DevOpts& o, const double* tot, const UpdRatios& q,
+                                          bool stop) {
   const bool weighted = (o.criterion == HF_STOP_RECURSIVE);
   const double rho_new = tot[0];
   s.beta = q.shrink;
@@ -1253,8 +1251,6 @@ __device__ __forceinline__ void epi_upd_s(InstScal& s, const DevOpts& o, const d
   s.step_iters += 1;
   if (sizeof(T) == 8) s.tot_iters += 1; else s.tot_inner += 1;
   if (weighted) s.rr_w = tot[1];
-  s.err = q.err;
-  bool stop = s.err <= (weighted ? o.tol : s.eta);
   const int64_t cap = (sizeof(T) == 8) ? o.itmax : (int64_t)o.inner_itmax;
   if (!stop && s.iter >= cap) {
     stop = true;
@@ -1273,6 +1269,14 @@ __device__ __forceinline__ void epi_upd_s(InstScal& s, const DevOpts& o, const d
   }
 }
 
+
+template <typename T>
+__device__ __forceinline__ void epi_upd(InstScal& s, const DevOpts& o, const double* tot) {
+  const bool weighted = o.criterion == HF_STOP_RECURSIVE;
+  const UpdRatios q{tot[0] / s.rho, tot[0] / s.gg0};
+  s.err = upd_err(s, weighted, tot[1], q.first);
+  epi_upd_s<T>(s, o, tot, q, s.err <= (weighted ? o.tol : s.eta));
+}
 
 template <bool INIT>
 __device__ void epi_residual(const DevArrays& A, int inst, const double* tot) {
@@ -1434,7 +1438,7 @@ __device__ __noinline__ void phase_epilogue(InstScal& sc, const InstDesc& d, con
       sc.phase = sc.inner_active ? PH_CG_B : phase_after<T>(sc);
       break;
     case PH_CG_B:
-      epi_upd_s<T>(sc, o, acc, upd_ratios(sc, o, acc));
+      epi_upd<T>(sc, o, acc);
       sc.phase = phase_after<T>(sc);
       break;
     case PH_XUPD: sc.phase = PH_RES; break;
@@ -1632,30 +1636,47 @@ __device__ __forceinline__ int wait_for(SolveCtl* ctl, unsigned long long wait_n
   return 1;
 }
 
-// The scalar epilogue of a round, by the first warp: tot[] valid in lane 0.  The divisions and the roots
-// of upd_ratios side by side in lanes 0 and 1.
+// The value up to which the criterion is met (of ||r||_w^2 under the reference's rule, of r.r over the
+// solve's first r.r otherwise), or NaN where it was not found; by the first warp.  The criterion, of which
+// every rounded operation is monotone, is a root, a product and a division deep, a fifth of a small grid's
+// round; an iteration then only compares, with the same outcome.  The lanes try the 32 values around the
+// one that exact arithmetic gives.
+template <bool WEIGHTED>
+__device__ __forceinline__ double stop_limit(const InstScal& s, const DevOpts& o) {
+  const double bound = WEIGHTED ? o.tol : s.eta;
+  const double root = WEIGHTED ? bound * sqrt(s.bb) / s.sigma_prev : bound;
+  const double mid = root * root;
+  const bool found = mid > 1e-290 && mid < 1e290 && (WEIGHTED ? s.bb > 0.0 : s.gg0 > 0.0);   // (bb, gg0 > 0)
+  const double v = bitsd(dbits(mid) + (unsigned long long)(threadIdx.x & 31) - 16ull);
+  const unsigned met = __ballot_sync(kFull, found && upd_err(s, WEIGHTED, v, v) <= bound);
+  const int n = __popc(met);                   // the first n lanes, not none of them and not all
+  const double lim = __shfl_sync(kFull, v, n > 0 ? n - 1 : 0);
+  return n > 0 && n < 32 && met == (1u << n) - 1u ? lim : (double)NAN;
+}
+
+// The scalar epilogue of a round, by the first warp: tot[] valid in lane 0.  The two divisions side by
+// side in lanes 0 and 1.  lim: stop_limit.
 template <typename T, bool WEIGHTED>
-__device__ __forceinline__ void round_epilogue(InstScal& sh, const DevOpts& o, int32_t ph, double (&tot)[2]) {
+__device__ __forceinline__ void round_epilogue(InstScal& sh, const DevOpts& o, int32_t ph, double (&tot)[2], double lim) {
   const int lane = threadIdx.x & 31;
-  tot[0] = __shfl_sync(kFull, tot[0], 0);
-  if (WEIGHTED) tot[1] = __shfl_sync(kFull, tot[1], 0);
   if (ph == PH_CG_PQ) {
     if (lane == 0) {
       epi_spmv_s(sh, tot);
+      if (!sh.inner_active && sh.iter > 0) sh.err = upd_err(sh, WEIGHTED, sh.rr_w, sh.rho / sh.gg0);   // the last update's
       sh.phase = sh.inner_active ? PH_CG_B : phase_after<T>(sh);
     }
     return;
   }
-  const double quot = tot[0] / (lane == 0 ? sh.rho : sh.gg0);
-  const double root = sqrt(WEIGHTED ? (lane == 0 ? tot[1] : sh.bb) : quot);
+  tot[0] = __shfl_sync(kFull, tot[0], 0);
   UpdRatios q;
-  q.shrink = quot;
-  q.first = __shfl_sync(kFull, quot, 1);
-  const double root1 = __shfl_sync(kFull, root, 1);
+  q.shrink = tot[0] / (lane == 0 ? sh.rho : sh.gg0);
+  q.first = __shfl_sync(kFull, q.shrink, 1);
   if (lane == 0) {
-    if (WEIGHTED) q.err = sh.bb > 0.0 ? root * sh.sigma_prev / root1 : 0.0;
-    else q.err = sh.gg0 > 0.0 ? root1 : 0.0;
-    epi_upd_s<T>(sh, o, tot, q);
+    const double v = WEIGHTED ? tot[1] : q.first;
+    const bool known = !isnan(lim);
+    if (!known) sh.err = upd_err(sh, WEIGHTED, tot[1], q.first);
+    epi_upd_s<T>(sh, o, tot, q, known ? v >= 0.0 && v <= lim : sh.err <= (WEIGHTED ? o.tol : sh.eta));
+    if (known && !sh.inner_active) sh.err = upd_err(sh, WEIGHTED, tot[1], q.first);
     sh.phase = phase_after<T>(sh);
   }
 }
@@ -1670,7 +1691,7 @@ __device__ __forceinline__ void round_arrive(SolveCtl* ctl) {
 template <typename T, bool WEIGHTED>
 __device__ __forceinline__ bool round_finish(const DevArrays& A, SolveCtl* ctl, unsigned long long wait_ns, InstScal& sh,
                                              double* red, const double* sums, int nt, int64_t r, int64_t round0,
-                                             int32_t ph, int32_t logged) {
+                                             int32_t ph, int32_t logged, double lim) {
   const int tid = threadIdx.x, G = (int)gridDim.x;
   const bool two = WEIGHTED && ph == PH_CG_B;
   int ok = 1;
@@ -1710,7 +1731,7 @@ __device__ __forceinline__ bool round_finish(const DevArrays& A, SolveCtl* ctl, 
       tot[0] += __shfl_xor_sync(kFull, tot[0], o);
       if (two) tot[1] += __shfl_xor_sync(kFull, tot[1], o);
     }
-    round_epilogue<T, WEIGHTED>(sh, A.opts, ph, tot);
+    round_epilogue<T, WEIGHTED>(sh, A.opts, ph, tot, lim);
   }
   __syncthreads();
   return true;
@@ -1732,6 +1753,7 @@ __global__ void __launch_bounds__(kBlock, 2)
     reinterpret_cast<unsigned long long*>(&sd)[tid] = reinterpret_cast<const unsigned long long*>(A.inst)[tid];
   __syncthreads();
   if (!sh.inner_active) return;              // no inner solve is due
+  const double lim = tid < 32 ? stop_limit<WEIGHTED>(sh, A.opts) : 0.0;
   __syncthreads();
   if (tid == 0) sh.phase = PH_CG_PQ;
   const int nt = sd.cgn;
@@ -1755,7 +1777,7 @@ __global__ void __launch_bounds__(kBlock, 2)
       else upd_form<T, WEIGHTED>(A, sd, k, sh, mine + k, nt, dyn);
     }
     round_arrive(ctl);
-    if (!round_finish<T, WEIGHTED>(A, ctl, wait_ns, sh, red, mine, nt, r, round0, ph, logged)) return;
+    if (!round_finish<T, WEIGHTED>(A, ctl, wait_ns, sh, red, mine, nt, r, round0, ph, logged, lim)) return;
   }
   if (blockIdx.x != 0) return;
   if (tid < kScalWords)
@@ -1815,6 +1837,7 @@ __global__ void __launch_bounds__(kBlock, 2)
     reinterpret_cast<unsigned long long*>(&sd)[tid] = reinterpret_cast<const unsigned long long*>(A.inst)[tid];
   __syncthreads();
   if (!sh.inner_active) return;                // no inner solve is due
+  const double lim = tid < 32 ? stop_limit<WEIGHTED>(sh, A.opts) : 0.0;
   __syncthreads();
   if (tid == 0) sh.phase = PH_CG_PQ;
   const int nt = sd.cgn;
@@ -2030,7 +2053,7 @@ __global__ void __launch_bounds__(kBlock, 2)
         }
       }
     }
-    if (!round_finish<T, WEIGHTED>(A, ctl, wait_ns, sh, red, mine, nt, r, round0, ph, logged)) return;
+    if (!round_finish<T, WEIGHTED>(A, ctl, wait_ns, sh, red, mine, nt, r, round0, ph, logged, lim)) return;
   }
   if (blockIdx.x != 0) return;
   if (tid == 0) sh.ypend = 0;
@@ -2151,6 +2174,7 @@ __global__ void __launch_bounds__(kBlock, 1) k_solve_cluster(DevArrays A, SolveC
     reinterpret_cast<unsigned long long*>(&sd)[tid] = reinterpret_cast<const unsigned long long*>(A.inst)[tid];
   __syncthreads();
   if (!sh.inner_active) return;                         // no inner solve is due (in any block)
+  const double lim = tid < 32 ? stop_limit<WEIGHTED>(sh, A.opts) : 0.0;
   Slot* slot = reinterpret_cast<Slot*>(dyn);
   const int nt = sd.cgn, nxy_t = sd.cgnx * sd.cgny, task0 = rank * nt / C, slots = (rank + 1) * nt / C - task0;
   const int nx = sd.nx, ny = sd.ny, nz = sd.nz, sx = sd.sx, nxy = sx * ny, nq = sd.cgw, rows = sd.cgr;
@@ -2346,7 +2370,7 @@ __global__ void __launch_bounds__(kBlock, 1) k_solve_cluster(DevArrays A, SolveC
         tot[0] += __shfl_xor_sync(kFull, tot[0], o);
         if (WEIGHTED) tot[1] += __shfl_xor_sync(kFull, tot[1], o);
       }
-      round_epilogue<T, WEIGHTED>(sh, A.opts, ph, tot);
+      round_epilogue<T, WEIGHTED>(sh, A.opts, ph, tot, lim);
     } else if (tid == 32 && rank == 0 && round0 + r < kRoundLog) {
       ctl->phase_log[round0 + r] = logged;
       ctl->t_round[round0 + r] = gtimer();
