@@ -17,7 +17,13 @@
 //
 // GB300 issues FP64 at ~1 TFLOP/s, so the FP64 kernels (residual, x update, FP64 CG) are bound by
 // FP64 instructions: they spend them only on the arithmetic itself (no FP64 compares, no FP64
-// accumulation of FP32 quantities).  The FP32 kernels accumulate in FP32 within a block.
+// accumulation of FP32 quantities), and where a condition is the same for a whole launch it selects a
+// loop: an FP64 instruction that is predicated off takes the pipe all the same.  The FP32 kernels
+// accumulate in FP32 within a block.
+//
+// The inner solve of one grid is one persistent kernel, of three (choose_solve): k_solve_cluster,
+// k_solve_res, k_solve_one.  Batches: k_solve_batch.  Residuals and x update are kernels of their own
+// but in small batches (split_solve).
 //
 // All solver state is per instance in device memory; tiles of instances that are not in the
 // phase a kernel serves return at once (per-instance convergence masks).
