@@ -918,6 +918,7 @@ int create_impl(const hf_problem* probs, int64_t count, const hf_solver_opts* op
       bc.pd[f] = 0.0;
     }
     bc.br = p.br;
+    for (int a = 0; a < 3; ++a) bc.rl2[a] = 1.0 / (d.len[a] * d.len[a]);
     // Neumann power densities, mod_boundary.f90:43-66 (T_BathCG / (volume * n_a * n_b))
     const double nxd = (double)p.nx, nyd = (double)p.ny, nzd = (double)p.nz;
     if (bc.cg[4]) bc.pd[4] = p.t_bath_cg / (d.volume * nxd * nyd);

@@ -221,40 +221,81 @@ __global__ void k_assemble(DevArrays A, const InstBC* bcs, const double* kappa) 
 // The coefficients of k_assemble + k_sinv, bit for bit, with each conductivity evaluated once.
 // Interior face P|Q (Q the + neighbour): calculate_conductivity(P->Q) (kin = kappa_P) is both the
 // stored slot of P (hmatrixfunc(Q,P)) and the - face term of Q's diagonal; (Q->P) is P's + face
-// term.  The products (L+L)*kin*kout round differently in the two orders, so both are evaluated.
-// Pass 1 writes P->Q per axis into the a64 arrays, by cell (k_scale rewrites them afterwards, in the
-// inner solve's layout); on the last
-// cell of a periodic axis it writes last->first, the - face term of the first cell.  Pass 2 forms
-// the + face terms, the diagonal in hmatrixfunc's summation order, the wrap slots (the + face term
-// of the last cell), the boundary vector and 1/sqrt|H_II|.  k_assemble instead evaluates
-// hmatrixfunc whole per stored slot (six conductivities each) and checks slot consistency, which
-// the one-time set-up affords and a rebuild on every step does not.
-__global__ void k_faces_step(DevArrays A, const InstBC* bcs, const double* kappa) {
-  int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= A.ncells) return;
-  const int inst = A.tile_inst[g / kTile];
-  const InstDesc& d = A.inst[inst];
-  HM h{d, bcs[inst], kappa + d.off, A.rhoc + d.off, A.tau_s + d.off};
-  const int64_t l = g - d.off;
-  if (l >= d.n) return;
-  const int64_t nx = d.nx, ny = d.ny, nz = d.nz;
-  const int64_t x = l % nx + 1, y = (l / nx) % ny + 1, z = l / (nx * ny) + 1;
-  A.a64x[g] = x < nx ? h.cond(x, y, z, x + 1, y, z) : (d.px ? h.cond(x, y, z, 1, y, z) : 0.0);
-  A.a64y[g] = y < ny ? h.cond(x, y, z, x, y + 1, z) : (d.py ? h.cond(x, y, z, x, 1, z) : 0.0);
-  A.a64z[g] = z < nz ? h.cond(x, y, z, x, y, z + 1) : (d.pz ? h.cond(x, y, z, x, y, 1) : 0.0);
+// term.  The products (L+L)*kin*kout round differently in the two orders, so both are evaluated; the
+// denominator is the same.  Pass 1 writes P->Q per axis into the a64 arrays, by cell (k_scale rewrites
+// them afterwards, in the inner solve's layout), and Q->P into the arrays of the stored products H T and
+// of S, which a rebuild makes void; the faces of the last cell of a periodic axis are those between it and
+// the first.  Pass 2 forms the diagonal in hmatrixfunc's summation order, the wrap slots (the + face term
+// of the last cell), the outer faces with the boundary vector, and 1/sqrt|H_II|.  k_assemble instead
+// evaluates hmatrixfunc whole per stored slot (six conductivities each) and checks slot consistency,
+// which the one-time set-up affords and a rebuild on every step does not.
+// Bound by the FP64 pipe, of which a division takes about ten instructions: a face's two quotients share
+// the reciprocal of their denominator, those by L*L the host's.  96 x 100 x 90 (ncu): the
+// faces 168 us where one orientation took 118, the diagonal 84 where it took 224 with the other.
+
+// The correctly rounded a / b from y, the correctly rounded 1 / b: two corrections of a * y, the first
+// of which brings it within one unit of a / b, whence the second is exact (P. Markstein, Computation of
+// elementary functions on the IBM RISC System/6000, 1990), where no step over- or underflows and b's
+// significand is not all ones; the division itself elsewhere.
+__device__ __forceinline__ bool mid_range(double v) {   // 2^-400 < |v| < 2^400
+  return (unsigned)((dbits(v) >> 52) & 0x7ffull) - 623u < 800u;
+}
+__device__ __forceinline__ bool recip_ok(double b) {
+  return mid_range(b) && (~dbits(b) & 0xfffffffffffffull) != 0ull;
+}
+__device__ __forceinline__ double quotient(double a, double b, double y, bool ok) {
+  if (!ok || !mid_range(a)) return a / b;
+  double q = a * y;
+  q = fma(fma(-b, q, a), y, q);
+  return fma(fma(-b, q, a), y, q);
 }
 
-__global__ void k_diag_step(DevArrays A, const InstBC* bcs, const double* kappa) {
-  int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(256) k_faces_step(DevArrays A, const InstBC* bcs, const double* kappa) {
+  const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= A.ncells) return;
   const int inst = A.tile_inst[g / kTile];
   const InstDesc& d = A.inst[inst];
   const InstBC& bc = bcs[inst];
-  HM h{d, bc, kappa + d.off, A.rhoc + d.off, A.tau_s + d.off};
-  const int64_t l = g - d.off;
+  const int l = (int)(g - d.off);
+  if (l >= d.n) return;
+  const int nx = d.nx, ny = d.ny, nz = d.nz, nxy = nx * ny;
+  const int row = l / nx, x = l - row * nx, z = row / ny, y = row - z * ny;
+  const double* K = kappa + d.off;
+  const double kp = K[l];
+  // calculate_conductivity of the face to cell m along axis a, from here (pq) and from there (qp)
+  auto face = [&](int a, int m, double* pq, double* qp) {
+    double f = 0.0, r = 0.0;
+    if (m >= 0 && m != l) {                    // (a cell beside itself has no length)
+      const double kq = K[m], L = d.len[a], L2 = L * L, twoL = L + L;
+      const double den = L * kq + L * kp;
+      const bool ok = recip_ok(den), ok2 = recip_ok(L2);
+      const double y = ok ? __drcp_rn(den) : 0.0, y2 = bc.rl2[a];
+      f = quotient(quotient(twoL * kp * kq, den, y, ok), L2, y2, ok2);
+      r = quotient(quotient(twoL * kq * kp, den, y, ok), L2, y2, ok2);
+      if (kp != kq) {
+        f = f * bc.br;
+        r = r * bc.br;
+      }
+    }
+    pq[g] = f;
+    qp[g] = r;
+  };
+  face(0, x + 1 < nx ? l + 1 : (d.px ? l - (nx - 1) : -1), A.a64x, A.hx[0]);
+  face(1, y + 1 < ny ? l + nx : (d.py ? l - (ny - 1) * nx : -1), A.a64y, A.hx[1]);
+  face(2, z + 1 < nz ? l + nxy : (d.pz ? l - (nz - 1) * nxy : -1), A.a64z, A.b);
+}
+
+__global__ void __launch_bounds__(256) k_diag_step(DevArrays A, const InstBC* bcs, const double* kappa) {
+  const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (g >= A.ncells) return;
+  const int inst = A.tile_inst[g / kTile];
+  const InstDesc& d = A.inst[inst];
+  const InstBC& bc = bcs[inst];
+  const int l = (int)(g - d.off);
   if (l >= d.n) { A.sinv[g] = 0.0; return; }
-  const int64_t nx = d.nx, ny = d.ny, nz = d.nz, nxy = nx * ny;
-  const int64_t x = l % nx + 1, y = (l / nx) % ny + 1, z = l / nxy + 1;
+  const int nx = d.nx, ny = d.ny, nz = d.nz, nxy = nx * ny;
+  const int row = l / nx, x = l - row * nx, z = row / ny, y = row - z * ny;
+  const double kap = kappa[g];
   // hmatrixfunc(I,I): alpha, then the six face terms (mod_hmatrix.f90:62-248)
   double alpha = 0.0;
   if (d.isteady == 0) {
@@ -262,67 +303,48 @@ __global__ void k_diag_step(DevArrays A, const InstBC* bcs, const double* kappa)
     if (d.icattaneo == 0) tau = 0.0;
     alpha = (tau * A.rhoc[g]) + (d.inv_dt * A.rhoc[g]);
   }
-  int64_t xp = x + 1, xm = x - 1, yp = y + 1, ym = y - 1, zp = z + 1, zm = z - 1;
-  if (d.px) { if (xp > nx) xp = 1; if (xm < 1) xm = nx; }
-  if (d.py) { if (yp > ny) yp = 1; if (ym < 1) ym = ny; }
-  if (d.pz) { if (zp > nz) zp = 1; if (zm < 1) zm = nz; }
-  const double Af = x > 1 ? A.a64x[g - 1] : (d.px ? A.a64x[g + nx - 1] : h.cond(xm, y, z, x, y, z));
-  const double Bf = h.cond(xp, y, z, x, y, z);
-  const double Df = y > 1 ? A.a64y[g - nx] : (d.py ? A.a64y[g + (ny - 1) * nx] : h.cond(x, ym, z, x, y, z));
-  const double Ef = h.cond(x, yp, z, x, y, z);
-  const double Ff = z > 1 ? A.a64z[g - nxy] : (d.pz ? A.a64z[g + (nz - 1) * nxy] : h.cond(x, y, zm, x, y, z));
-  const double Gf = h.cond(x, y, zp, x, y, z);
+  // the half cell to the bath of outer face f: the diagonal's term (boundry_diag_term) and the
+  // boundary vector's (mod_boundary.f90:72-150), whose numerators 2 kb k round alike
+  double Bv = 0.0;
+  auto outer = [&](int f) -> double {
+    const double kb = bc.kb[f], L = d.len[f / 2], L2 = L * L, den = kb + kap;
+    const bool ok = recip_ok(den);
+    double kh = quotient(quotient((2.0 * kb) * kap, den, ok ? __drcp_rn(den) : 0.0, ok), L2, bc.rl2[f / 2], recip_ok(L2));
+    if (kap != kb) kh = kh * bc.br;
+    if (bc.cg[f]) Bv = bc.pd[f];
+    else Bv = Bv + kh * bc.tb[f];
+    return kh;
+  };
+  double Af, Bf, Df, Ef, Ff, Gf;               // the boundary vector takes the faces in this order
+  if (x > 0 || d.px) Af = A.a64x[x > 0 ? g - 1 : g + (nx - 1)]; else Af = outer(0);
+  if (x + 1 < nx || d.px) Bf = A.hx[0][g]; else Bf = outer(1);
+  if (y > 0 || d.py) Df = A.a64y[y > 0 ? g - nx : g + (ny - 1) * nx]; else Df = outer(2);
+  if (y + 1 < ny || d.py) Ef = A.hx[1][g]; else Ef = outer(3);
+  if (z > 0 || d.pz) Ff = A.a64z[z > 0 ? g - nxy : g + (int64_t)(nz - 1) * nxy]; else Ff = outer(4);
+  if (z + 1 < nz || d.pz) Gf = A.b[g]; else Gf = outer(5);
   const double dg = -(Af + Bf + Df + Ef + Ff + Gf) - alpha;
   A.diag[g] = dg;
   auto keep = [](double v) { return fabs(v) < kTiny ? 0.0 : v; };   // sparse_Hmatrix's drop rule
   double cxv = 0.0, cyv = 0.0, czv = 0.0;
-  if (x < nx) cxv = keep(A.a64x[g]);
+  if (x + 1 < nx) cxv = keep(A.a64x[g]);
   else if (d.px && nx > 1) cxv = keep(Bf);
   if (ny > 1) {
-    if (y < ny) cyv = keep(A.a64y[g]);
+    if (y + 1 < ny) cyv = keep(A.a64y[g]);
     else if (d.py) cyv = keep(Ef);
   }
   if (nz > 1) {
-    if (z < nz) czv = keep(A.a64z[g]);
+    if (z + 1 < nz) czv = keep(A.a64z[g]);
     else if (d.pz) czv = keep(Gf);
   }
   A.cx[g] = cxv;
   A.cy[g] = cyv;
   A.cz[g] = czv;
-  // boundary(B), mod_boundary.f90:72-150
-  double Bv = 0.0;
-  const double kap = kappa[g];
-  const int64_t c[3] = {x, y, z}, n[3] = {nx, ny, nz};
-  const int per[3] = {d.px, d.py, d.pz};
-  for (int a = 0; a < 3; ++a) {
-    if (per[a]) continue;
-    double L = d.len[a];
-    if (c[a] == 1) {
-      int f = 2 * a;
-      if (bc.cg[f]) {
-        Bv = bc.pd[f];
-      } else {
-        double kh = (2.0 * kap * bc.kb[f] / (kap + bc.kb[f])) / (L * L);
-        if (kap != bc.kb[f]) kh = kh * bc.br;
-        Bv = Bv + (kh) * bc.tb[f];
-      }
-    }
-    if (c[a] == n[a]) {
-      int f = 2 * a + 1;
-      if (bc.cg[f]) {
-        Bv = bc.pd[f];
-      } else {
-        double kh = (2.0 * kap * bc.kb[f] / (kap + bc.kb[f])) / (L * L);
-        if (kap != bc.kb[f]) kh = kh * bc.br;
-        Bv = Bv + (kh) * bc.tb[f];
-      }
-    }
-  }
   A.bvec[g] = Bv;
   if (isnan(Bv)) atomicOr(&A.scal[inst].status, 1 << (HF_ENAN_B - HF_ENAN_B));
   if (dg >= 0.0) atomicOr(&A.scal[inst].devcheck, 2);
-  A.sinv[g] = 1.0 / sqrt(fabs(dg));
-  A.sinv32[g] = (float)A.sinv[g];
+  const double si = 1.0 / sqrt(fabs(dg));
+  A.sinv[g] = si;
+  A.sinv32[g] = (float)si;
 }
 
 // ---- Jacobi scaling: sinv = 1/sqrt|H_II|, a = -c * sinv_I * sinv_E ----------------------------
@@ -338,21 +360,21 @@ __global__ void k_sinv(DevArrays A) {
 }
 
 __global__ void k_scale(DevArrays A) {
-  int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= A.ncells) return;
   const InstDesc& d = A.inst[A.tile_inst[g / kTile]];
-  const int64_t l = g - d.off;
+  const int l = (int)(g - d.off);
   if (l >= d.n) return;
-  const int64_t nx = d.nx, ny = d.ny, nz = d.nz, nxy = nx * ny;
-  const int64_t x = l % nx, y = (l / nx) % ny, z = l / nxy;
+  const int nx = d.nx, ny = d.ny, nz = d.nz, nxy = nx * ny;
+  const int row = l / nx, x = l - row * nx, z = row / ny, y = row - z * ny;
   const double si = A.sinv[g];
   int64_t ex = x + 1 < nx ? g + 1 : g - (nx - 1);
   int64_t ey = y + 1 < ny ? g + nx : g - (ny - 1) * nx;
-  int64_t ez = z + 1 < nz ? g + nxy : g - (nz - 1) * nxy;
+  int64_t ez = z + 1 < nz ? g + nxy : g - (int64_t)(nz - 1) * nxy;
   double ax = -A.cx[g] * si * A.sinv[ex];
   double ay = -A.cy[g] * si * A.sinv[ey];
   double az = -A.cz[g] * si * A.sinv[ez];
-  const int64_t g4 = d.off4 + (z * ny + y) * d.sx + x;   // the inner solve's layout (rows of sx cells)
+  const int64_t g4 = d.off4 + (int64_t)row * d.sx + x;   // the inner solve's layout (rows of sx cells)
   A.a64x[g4] = ax; A.a64y[g4] = ay; A.a64z[g4] = az;
   A.a32x[g4] = (float)ax; A.a32y[g4] = (float)ay; A.a32z[g4] = (float)az;
   if (x == nx - 1)                       // padding cells: a rebuild used them as scratch

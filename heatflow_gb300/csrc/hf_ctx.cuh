@@ -16,6 +16,7 @@ struct AsmArrays {
 
 struct InstBC {
   double kb[6], tb[6], pd[6], br;
+  double rl2[3];      // 1 / len^2, rounded to nearest (the rebuild's exact quotients)
   int32_t cg[6];
 };
 
