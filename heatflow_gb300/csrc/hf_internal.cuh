@@ -34,8 +34,8 @@ constexpr int kCellsPerThread = 4;
 constexpr int kTile = kBlock * kCellsPerThread;   // cells per tile (one block per tile)
 constexpr int kNR = 8;
 // Step kernels work on tasks: a block of 32 x kTY threads owns kXC*32 x kTY columns of one
-// instance (one warp per row; lane L holds columns x0 + L + 32 j, j < kXC) and marches the task
-// depth (InstDesc::zc planes, an option; kZC by default) along z.  (kXC > 1 trades occupancy for
+// instance (one warp per row, or 256 consecutive columns of the plane: InstDesc::flat) and marches the
+// task depth (InstDesc::zc planes, an option; kZC by default) along z.  (kXC > 1 trades occupancy for
 // per-thread parallelism; on GB300 kXC = 1 is faster.)
 constexpr int kXC = 1, kTX = 32 * kXC, kTY = 8, kZC = 32;
 constexpr int kMinTaskDepth = 4;   // task buffers are sized for the shallowest task depth
@@ -71,6 +71,7 @@ struct InstDesc {
   // layout of the other FP64 arrays.
   int64_t off4;
   int32_t sx;
+  int32_t flat;       // cell tasks are runs of kBlock columns instead of kTX x kTY tiles (build_tasks)
   // Tasks of the inner solve's passes (cg_plan): tiles of cgw 16-byte vectors x cgr rows,
   // cgnx x cgny of them, each cut into cgnz parts along z; cgn in all, the first at cg0.
   int32_t cgw, cgr, cgnx, cgny, cgnz, cgn;
@@ -507,10 +508,10 @@ struct TCell {
   int64_t off;
   int nx, ny, nz, nxy;
   bool px, py, pz;
-  int x0, y, z0, z1, lane;
+  int xc, y, z0, z1, lane;
   int64_t off4;       // the FP32 vectors' layout (rows of sx cells)
   int sx, nxy4;
-  __device__ int x(int j) const { return x0 + 32 * j + lane; }
+  __device__ int x(int) const { return xc; }
   __device__ bool act(int j) const { return x(j) < nx && y < ny; }   // column inside the grid
   __device__ int base(int j) const { return y * nx + x(j); }          // local index of (x, y, 0)
   __device__ int base4(int j) const { return y * sx + x(j); }         // the same in the FP32 layout
@@ -526,8 +527,14 @@ __device__ __forceinline__ TCell task_cell(const DevArrays& A, int64_t task) {
   c.nx = d.nx; c.ny = d.ny; c.nz = d.nz; c.nxy = d.nx * d.ny;
   c.px = d.px; c.py = d.py; c.pz = d.pz;
   c.lane = threadIdx.x & 31;
-  c.x0 = t.y;
-  c.y = t.z + (int)(threadIdx.x >> 5);
+  if (d.flat) {
+    const int col = t.y + (int)threadIdx.x;
+    c.y = col / d.nx;
+    c.xc = col - c.y * d.nx;
+  } else {
+    c.xc = t.y + c.lane;
+    c.y = t.z + (int)(threadIdx.x >> 5);
+  }
   c.z0 = t.w;
   c.z1 = min(t.w + d.zc, d.nz);
   c.off4 = d.off4;

@@ -189,17 +189,18 @@ __device__ __forceinline__ void task_store_f(double* dst, float v) {
 // prove distinct.
 
 // x-neighbour loads of a column (offsets from the cell, or kNoNbr): lane 0 loads its west
-// neighbour, lane 31 its east neighbour, and a last column of a periodic axis its wrap; all other
-// x neighbours come from the adjacent lanes by shuffles.
+// neighbour, lane 31 its east neighbour, and the first and last columns of a periodic axis their wraps;
+// all other x neighbours come from the adjacent lanes by shuffles.
 constexpr int kNoNbr = -2147483647 - 1;
 struct XEdge { int w, e; };
 __device__ __forceinline__ XEdge x_edges(const TCell& c) {
   XEdge r{kNoNbr, kNoNbr};
   if (!c.act(0)) return r;
   const int x = c.x(0), nx = c.nx;
-  if (c.lane == 0) {
-    if (x > 0) r.w = -1;
-    else if (c.px && nx > 1) r.w = nx - 1;
+  if (x == 0) {
+    if (c.px && nx > 1) r.w = nx - 1;
+  } else if (c.lane == 0) {
+    r.w = -1;
   }
   if (x + 1 < nx) {
     if (c.lane == 31) r.e = 1;
@@ -388,7 +389,8 @@ __device__ __forceinline__ void res_task(const DevArrays& A, double* part, int64
     const double up = __shfl_up_sync(kFull, xc, 1), cup = __shfl_up_sync(kFull, cur.cx, 1);
     const double dn = __shfl_down_sync(kFull, xc, 1);
     if (act) {
-      const double xw = c.lane > 0 ? up : cur.xw, cxw = c.lane > 0 ? cup : cur.cxw;
+      const bool west = c.lane > 0 && c.x(0) > 0;
+      const double xw = west ? up : cur.xw, cxw = west ? cup : cur.cxw;
       const double xeast = (c.x(0) + 1 < c.nx && c.lane < 31) ? dn : cur.xe;
       double a = fma(-cur.diag, xc, cur.b);
       if (tiny) a = fma(-kTiny, cur.rs, a);
@@ -1320,6 +1322,7 @@ __global__ void __launch_bounds__(kBlock) k_finalize(DevArrays A, CtrlState* ctr
   __shared__ InstDesc sd;
   __shared__ double red[kBlock * NR];
   const unsigned long long start = gtimer();
+  if (RES && A.ninst == 1 && tid == 0) A.sctl->arrived = 0ull;   // of the inner solve that may follow
   if (KIND == FIN_RHS && inst == 0 && tid == 0) A.stamps[kStampFin] = start;
   const bool loop = graph && RES, one = A.ninst == 1;
   int32_t gave_up = 0;
@@ -2550,9 +2553,11 @@ cudaError_t launch_solve(Ctx& c, bool full, unsigned long long wait_ns, int leav
   const int g = solve_grid_blocks(c, fp32 ? 1 : 0, full);
   if (g < 1) return cudaErrorInvalidConfiguration;
   const size_t skip = full ? 0 : offsetof(SolveCtl, arrived);
-  cudaError_t e = cudaMemsetAsync(reinterpret_cast<char*>(c.d_sctl) + skip, 0,
-                                  solve_ctl_bytes(c.ninst, c.ncg) - skip, c.stream);
-  if (e != cudaSuccess) return e;
+  cudaError_t e = cudaSuccess;
+  if (full || c.ninst > 1 || leaver >= 0) {    // (one grid's counter: k_finalize)
+    e = cudaMemsetAsync(reinterpret_cast<char*>(c.d_sctl) + skip, 0, solve_ctl_bytes(c.ninst, c.ncg) - skip, c.stream);
+    if (e != cudaSuccess) return e;
+  }
   const int64_t per = fp32 ? c.opts.inner_itmax : c.opts.itmax;
   const int64_t limit = (int64_t)(c.opts.max_refine + 3) * (2 * per + 6) + 8;
   cudaLaunchConfig_t cfg = {};
