@@ -680,14 +680,15 @@ int64_t inner_cells(const Ctx& c) {
 // and cgr rows high, 8 to 32 vectors and at most kBlock in all, of these shapes the one that covers the
 // grid's plane with the fewest tiles, evenly (of equals the one that reads least beside itself).  With
 // widths of 8, 16 and 32 vectors only, the tiles of 64 grids of 16 to 96 cells an edge held 1.47 threads
-// per vector, with these 1.22 (20 steps 71 -> 60 ms, with the 128-byte alignment of their
-// shared memory).  Along z a tile is cut into parts, whose ends read a plane of their neighbours.  One grid: as many parts as make its longest chain of planes per block, over waves of
-// kSolveBlocks blocks, shortest, the halo counted as one plane per part; a count above one wave
-// pays only where a wave could not be filled.  Several grids: parts of one length for all, such
-// that there are about kBatchWaves tasks per block -- they are handed out one at a time, and each
-// costs a few trips through L2.  Small grids get one plane per part either way, so a grid's bits
-// do not depend on the batch it is in there.
-constexpr int64_t kBatchWaves = 4;
+// per vector, with these 1.22 (20 steps 71 -> 60 ms, with the 128-byte alignment of their shared
+// memory).  Along z a tile is cut into parts, whose ends read a plane of their neighbours.  One grid: as
+// many parts as make its longest chain of planes per block, over waves of kSolveBlocks blocks, shortest,
+// the halo counted as one plane per part; a count above one wave pays only where a wave could not be
+// filled.  Several grids: parts of one length for all, such that there are about kBatchWaves tasks per
+// block -- they are handed out one at a time, and each costs a few trips through L2 (64 uneven grids, 20
+// steps, with 2, 3, 4 and 5 per block: 56.2, 56.0, 58.0 and 64.6 ms).  Small grids get one plane per part
+// either way, so a grid's bits do not depend on the batch it is in there.
+constexpr int64_t kBatchWaves = 3;
 int cg_plan(Ctx& c) {
   const int64_t kSolveBlocks = 2 * 152;
   const int vec = c.opts.precision == HF_PREC_MIXED ? 4 : 2;

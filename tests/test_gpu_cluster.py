@@ -39,6 +39,6 @@ def test_small_grid_equals_batch(cuda_lib, dims, periodic, precision, criterion,
 @pytest.mark.parametrize("precision,criterion,tol", OPTS)
 @pytest.mark.parametrize("ny,nz,periodic", [(16, 304, (0, 0, 1)), (15, 456, WRAP), (16, 608, OPEN)])
 def test_deep_tasks_equal_batch(cuda_lib, ny, nz, periodic, precision, criterion, tol):
-    """Two tiles side by side, tasks of 2, 3 and 4 planes (the last do not fit), in a batch of four of
+    """Two tiles side by side, tasks of 2, 3 and 4 planes (the last do not fit), in a batch of three of
     which the tasks are cut the same."""
-    _check(_problem((128 if precision == "mixed" else 64, ny, nz), periodic), 4, precision, criterion, tol)
+    _check(_problem((128 if precision == "mixed" else 64, ny, nz), periodic), 3, precision, criterion, tol)
