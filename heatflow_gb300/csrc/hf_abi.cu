@@ -1593,10 +1593,14 @@ int hf_set_property_tables(hf_ctx* h, int32_t ntables, const int32_t* offsets, c
   c.d_toff = nullptr;
   c.d_trows = nullptr;
   int r = dalloc(c, &c.d_toff, (size_t)ntables + 1);
-  if (!r) r = dalloc(c, &c.d_trows, 4 * (size_t)offsets[ntables]);
+  if (!r) r = dalloc(c, &c.d_trows, 5 * (size_t)offsets[ntables]);   // behind the rows: 1 / (T of the next row - T)
   if (r) return r;
   CU(cudaMemcpy(c.d_toff, offsets, sizeof(int32_t) * ((size_t)ntables + 1), cudaMemcpyHostToDevice));
   CU(cudaMemcpy(c.d_trows, rows, sizeof(double) * 4 * (size_t)offsets[ntables], cudaMemcpyHostToDevice));
+  c.table_rows = offsets[ntables];
+  std::vector<double> recip((size_t)offsets[ntables], 0.0);
+  for (int32_t k = 0; k + 1 < offsets[ntables]; ++k) recip[(size_t)k] = 1.0 / (rows[4 * (k + 1)] - rows[4 * k]);
+  CU(cudaMemcpy(c.d_trows + 4 * (size_t)offsets[ntables], recip.data(), sizeof(double) * recip.size(), cudaMemcpyHostToDevice));
   CU(cudaMemcpy(c.d_cell_table, ct.data(), sizeof(int32_t) * ct.size(), cudaMemcpyHostToDevice));
   c.tempdep = true;
   drop_graph(c);                              // the captured steps gain the rebuild kernels

@@ -483,12 +483,22 @@ struct TableAt {
   bool inside;
 };
 
-__device__ __forceinline__ TableAt table_at(const double* rows, int m, double T) {
-  if (T <= rows[0]) return {rows, rows, 0.0, false};
-  if (T >= rows[4 * (m - 1)]) return {rows + 4 * (m - 1), rows + 4 * (m - 1), 0.0, false};
+// Order of doubles as integers (NaN aside): a compare on the FP64 pipe costs as much as an FMA.
+__device__ __forceinline__ unsigned long long order_key(double v) {
+  unsigned long long b = dbits(v);
+  if (dbl_is_zero(v)) b = 0ull;                       // -0 as 0
+  return b >> 63 ? ~b : b | 0x8000000000000000ull;
+}
+// recip: 1 / (T of the next row - T), by row, correctly rounded.
+__device__ __forceinline__ TableAt table_at(const double* rows, const double* recip, int m, double T) {
+  const unsigned long long key = order_key(T);
+  const bool nan = dbl_is_nan(T);                     // (a NaN takes the last interval, and stays one)
+  if (!nan && key <= order_key(rows[0])) return {rows, rows, 0.0, false};
+  if (!nan && key >= order_key(rows[4 * (m - 1)])) return {rows + 4 * (m - 1), rows + 4 * (m - 1), 0.0, false};
   int k = 0;
-  while (k + 1 < m - 1 && !(T < rows[4 * (k + 1)])) ++k;
-  const double f = (T - rows[4 * k]) / (rows[4 * (k + 1)] - rows[4 * k]);
+  while (k + 1 < m - 1 && (nan || key >= order_key(rows[4 * (k + 1)]))) ++k;
+  const double den = rows[4 * (k + 1)] - rows[4 * k];
+  const double f = quotient(T - rows[4 * k], den, recip[k], recip_ok(den));
   return {rows + 4 * k, rows + 4 * (k + 1), f, true};
 }
 
@@ -497,7 +507,7 @@ __device__ __forceinline__ double table_col(const TableAt& t, int col) {
   return t.r0[col] + t.f * (t.r1[col] - t.r0[col]);
 }
 
-__global__ void k_tempdep(DevArrays A, const int32_t* toff, const double* trows,
+__global__ void k_tempdep(DevArrays A, const int32_t* toff, const double* trows, int32_t nrows,
                           const int32_t* cell_table, double* kappa) {
   int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= A.ncells) return;
@@ -510,7 +520,7 @@ __global__ void k_tempdep(DevArrays A, const int32_t* toff, const double* trows,
   const double* rows = trows + 4 * (int64_t)toff[t];
   const int m = toff[t + 1] - toff[t];
   const double T = A.tbuf[A.scal[inst].role[0]][g];
-  const TableAt at = table_at(rows, m, T);
+  const TableAt at = table_at(rows, trows + 4 * (int64_t)nrows + toff[t], m, T);
   kappa[g] = table_col(at, 1);
   const double rc = table_col(at, 2) * table_col(at, 3);
   A.rhoc[g] = rc;
@@ -519,7 +529,7 @@ __global__ void k_tempdep(DevArrays A, const int32_t* toff, const double* trows,
 }
 
 cudaError_t launch_tempdep(Ctx& c) {
-  k_tempdep<<<nblk(c.ncells, 256), 256, 0, c.stream>>>(c.A, c.d_toff, c.d_trows, c.d_cell_table,
+  k_tempdep<<<nblk(c.ncells, 256), 256, 0, c.stream>>>(c.A, c.d_toff, c.d_trows, c.table_rows, c.d_cell_table,
                                                        c.asm_.kappa);
   k_faces_step<<<nblk(c.ncells, 256), 256, 0, c.stream>>>(c.A, c.d_bc, c.asm_.kappa);
   k_diag_step<<<nblk(c.ncells, 256), 256, 0, c.stream>>>(c.A, c.d_bc, c.asm_.kappa);

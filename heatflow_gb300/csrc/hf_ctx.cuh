@@ -137,6 +137,7 @@ struct Ctx {
   // tabulated properties re-evaluated after every step (hf_set_property_tables)
   bool tempdep = false;
   int32_t* d_toff = nullptr;
+  int32_t table_rows = 0;        // rows of all tables
   double* d_trows = nullptr;
   int32_t* d_cell_table = nullptr;
 };
