@@ -2519,6 +2519,22 @@ static cudaError_t launch_cluster(Ctx& c, int64_t limit) {
   return e == cudaSuccess ? cudaLaunchKernelEx(&cfg, k_solve_cluster<T, WEIGHTED>, c.A, c.d_sctl, limit) : e;
 }
 
+// The dynamic shared memory a block of `kernel` may have beside its static one, which becomes its limit;
+// or 0.  The limit belongs to the process: with one value for every context, no thread lowers it between
+// another's occupancy query or launch and its own.
+template <typename K>
+static int most_smem(const Ctx& c, K kernel) {
+  int most = 0;
+  cudaFuncAttributes fa;
+  if (cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, c.device) == cudaSuccess &&
+      cudaFuncGetAttributes(&fa, kernel) == cudaSuccess) {
+    most -= (int)fa.sharedSizeBytes;
+    if (allow_smem(kernel, most) == cudaSuccess) return most;
+  }
+  cudaGetLastError();                          // a refusal is an answer: no later launch reports it
+  return 0;
+}
+
 // Planes of the deepest task where k_solve_res serves the inner solves of a grid, or 0: all of its
 // blocks run at once with the task's state in shared memory.
 template <typename T, bool WEIGHTED>
@@ -2526,13 +2542,13 @@ static int res_depth_of(Ctx& c) {
   const InstDesc& d = c.h_inst[0];
   const int D = (d.nz + d.cgnz - 1) / d.cgnz, smem = ResLayout<T>(D, WEIGHTED).n * 16;
   auto kernel = k_solve_res<T, WEIGHTED>;
-  int n = 0, nsm = 0, most = 0;
+  int n = 0, nsm = 0;
+  if (smem > most_smem(c, kernel)) return 0;
   if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c.device) != cudaSuccess ||
-      cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, c.device) != cudaSuccess)
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kBlock, smem) != cudaSuccess) {
+    cudaGetLastError();
     return 0;
-  if (smem > most - 8192 || allow_smem(kernel, smem) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kBlock, smem) != cudaSuccess)
-    return 0;
+  }
   return (int64_t)n * nsm >= d.cgn ? D : 0;
 }
 // Which kernel runs the inner solves of one grid: k_solve_cluster, k_solve_res or k_solve_one, each where
@@ -2584,8 +2600,6 @@ cudaError_t launch_solve(Ctx& c, bool full, unsigned long long wait_ns, int leav
       auto kernel = fp32 ? k_solve_res<float, false> : weighted ? k_solve_res<double, true> : k_solve_res<double, false>;
       cfg.gridDim = dim3((unsigned)c.h_inst[0].cgn);
       cfg.dynamicSmemBytes = (size_t)16 * (fp32 ? ResLayout<float>(D, false).n : ResLayout<double>(D, weighted).n);
-      e = allow_smem(kernel, (int)cfg.dynamicSmemBytes);
-      if (e != cudaSuccess) return e;
       return cudaLaunchKernelEx(&cfg, kernel, c.A, c.d_sctl, limit, wait_ns, leaver, D);
     }
   }
