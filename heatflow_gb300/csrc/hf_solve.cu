@@ -1335,6 +1335,7 @@ __global__ void __launch_bounds__(kBlock) k_finalize(DevArrays A, CtrlState* ctr
   double acc[NR];
   instance_sum<NR>(A.partials, A.pcap, one ? 0 : sd.task0, one ? A.ntasks : (int64_t)sd.ntask, acc, red);
   const bool part = took_part<KIND>(sh);       // (instance_sum holds a block barrier)
+  __syncthreads();                             // every thread has looked before the epilogue changes sh
   if (part && tid < 32) {
     double rel = 0.0, rms = 0.0;
     if (RES) {
