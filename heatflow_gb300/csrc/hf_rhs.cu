@@ -119,23 +119,27 @@ __device__ __forceinline__ void rhs_fast_task(const DevArrays& A, int64_t task, 
   };
   Pair cur, nxt;
   load(c.first(), cur);
-  for (unsigned l = c.first(); l < c.end; l += c.step) {
+  // as many rounds for every lane of a warp as for its first: they vote below
+  const unsigned rounds_end = c.end + 2 * (threadIdx.x & 31);
+  for (unsigned l = c.first(); l < rounds_end; l += c.step) {
     load(l + c.step, nxt);
-    const bool two = l + 1 < c.end;
+    const bool in = l < c.end, two = l + 1 < c.end;
     double2 S, x0;
     S.x = CAT ? fma(cur.tp.x, cur.rh.x, cur.cc.x * cur.tpp.x) : cur.tp.x * cur.rh.x;
     S.y = CAT ? fma(cur.tp.y, cur.rh.y, cur.cc.y * cur.tpp.y) : cur.tp.y * cur.rh.y;
     // a branch of the warp: predicated off, the subtractions would take the FP64 pipe all the same
-    if (__any_sync(__activemask(), cur.face)) {
+    if (__any_sync(0xffffffffu, cur.face)) {
       if (cur.face && !dbl_is_zero(cur.B.x)) S.x = S.x - cur.B.x;
       if (cur.face && !dbl_is_zero(cur.B.y)) S.y = S.y - cur.B.y;
     }
     x0.x = fma(2.0, cur.tp.x, -cur.tpp.x);
     x0.y = fma(2.0, cur.tp.y, -cur.tpp.y);
-    sq.add(S.x);
-    if (two) sq.add(S.y);
-    st_pair(bout, HF_IXP(A, l, n, two), two, S);
-    st_pair(X, HF_IXP(A, l, n, two), two, x0);
+    if (in) {
+      sq.add(S.x);
+      if (two) sq.add(S.y);
+      st_pair(bout, HF_IXP(A, l, n, two), two, S);
+      st_pair(X, HF_IXP(A, l, n, two), two, x0);
+    }
     cur = nxt;
   }
   const double bb = sq.value();

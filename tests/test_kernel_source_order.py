@@ -25,3 +25,11 @@ def test_finalize_reads_flags_before_the_epilogue_writes_them():
     read, write = body.index("took_part<KIND>(sh)"), body.index("epi_rhs(sh")
     assert read < write
     assert "__syncthreads()" in body[read:write]
+
+
+def test_warp_votes_name_lanes_that_arrive():
+    """A vote over __activemask() names whichever lanes happen to run together and then waits for them:
+    the kernels vote with all lanes, which take the same number of rounds."""
+    for unit in os.listdir(os.path.join(ROOT, "heatflow_gb300", "csrc")):
+        text = open(os.path.join(ROOT, "heatflow_gb300", "csrc", unit)).read()
+        assert "__activemask" not in text, unit
