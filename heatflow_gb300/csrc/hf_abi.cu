@@ -686,12 +686,15 @@ int64_t inner_cells(const Ctx& c) {
 // the halo counted as one plane per part; a count above one wave pays only where a wave could not be
 // filled.  Several grids: parts of one length for all, such that there are about kBatchWaves tasks per
 // block -- they are handed out one at a time, and each costs a few trips through L2 (64 uneven grids, 20
-// steps, with 2, 3, 4 and 5 per block: 56.2, 56.0, 58.0 and 64.6 ms).  Small grids get one plane per part
-// either way, so a grid's bits do not depend on the batch it is in there.
+// steps, with 2, 3, 4 and 5 per block: 56.2, 56.0, 58.0 and 64.6 ms).  The order of a grid's sums, and
+// with it its bits, then depends on the grids beside it.  Where the caller gives a task depth it does not:
+// every grid of a batch is cut as it would be alone, into tasks of no fewer cells than a cell task of
+// that depth has (the 64 grids at depths 8, 16, 32 and 64: 5.1, 3.7, 2.9 and 2.6 ms a step, 2.6 without).
 constexpr int64_t kBatchWaves = 3;
 int cg_plan(Ctx& c) {
   const int64_t kSolveBlocks = 2 * 152;
   const int vec = c.opts.precision == HF_PREC_MIXED ? 4 : 2;
+  const int64_t depth = c.opts.task_depth;
   int64_t planes = 0;                 // tile planes of all grids
   for (InstDesc& d : c.h_inst) {
     const int nv = (d.nx + vec - 1) / vec;
@@ -718,9 +721,10 @@ int cg_plan(Ctx& c) {
   for (InstDesc& d : c.h_inst) {
     const int64_t tiles = (int64_t)d.cgnx * d.cgny;
     int64_t parts = 1;
-    if (c.ninst == 1) {
+    if (c.ninst == 1 || depth != 0) {
       int64_t best = INT64_MAX;
-      for (int64_t n = 1; n <= d.nz && (n == 1 || n * tiles <= 16 * kSolveBlocks); ++n) {
+      const int64_t least = std::max<int64_t>(1, depth / vec);   // planes: a tile has kBlock * vec cells in each
+      for (int64_t n = 1; n <= d.nz && (n == 1 || (n * tiles <= 16 * kSolveBlocks && (d.nz + n - 1) / n >= least)); ++n) {
         const int64_t waves = (n * tiles + kSolveBlocks - 1) / kSolveBlocks;
         const int64_t cost = waves * ((d.nz + n - 1) / n + 1);
         if (cost < best) {
@@ -739,6 +743,7 @@ int cg_plan(Ctx& c) {
   }
   c.ncg = c.A.ncg = total;
   c.cg_precision = c.opts.precision;
+  c.cg_depth = c.opts.task_depth;
   std::vector<int32_t> inst((size_t)total);
   for (int64_t i = 0; i < c.ninst; ++i)
     std::fill_n(inst.begin() + c.h_inst[i].cg0, c.h_inst[i].cgn, (int32_t)i);
@@ -1132,7 +1137,8 @@ int hf_set_opts(hf_ctx* h, const hf_solver_opts* opts) {
   h->c.A.opts = dev_opts(*opts);
   drop_graph(h->c);   // captured kernels hold the options by value
   h->c.res_depth = -1;
-  if (effective_depth(h->c, *opts) != h->c.depth || opts->precision != h->c.cg_precision)
+  if (effective_depth(h->c, *opts) != h->c.depth || opts->precision != h->c.cg_precision ||
+      opts->task_depth != h->c.cg_depth)
     return build_tasks(h->c, effective_depth(h->c, *opts));
   return HF_OK;
 }

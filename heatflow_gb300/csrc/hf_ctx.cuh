@@ -29,7 +29,7 @@ struct Ctx {
   int64_t ntasks_cap = 0;        // task buffers' capacity (shallowest task depth)
   int depth = 0;                 // task depth of the current table
   int64_t ncg = 0;               // tasks of the inner solve's passes, planned for a precision
-  int cg_precision = -1;
+  int cg_precision = -1, cg_depth = -1;   // and a task_depth option
   int64_t ncg_cap = 0;           // entries of cg_inst
   size_t sctl_cap = 0;           // bytes at d_sctl
   std::vector<InstDesc> h_inst;

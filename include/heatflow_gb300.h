@@ -104,7 +104,9 @@ typedef struct hf_solver_opts {
                            3 = as 1, but one graph launch per step (profilers, which do not see
                            kernels inside conditional nodes, then see those outside the solve) */
   int32_t task_depth;   /* z-planes per task of the step kernels (0: 32, or 16/8/4 when the
-                           grids would give fewer than 912 tasks; otherwise 4..1024) */
+                           grids would give fewer than 912 tasks; otherwise 4..1024).  With 0 a
+                           batch's tasks are cut by all of its grids, so the last bits of a grid's
+                           field depend on the grids beside it; with a depth they do not */
 } hf_solver_opts;
 
 typedef struct hf_stats {
