@@ -654,6 +654,47 @@ __device__ __forceinline__ Beyond beyond_of(const InstDesc& d, const CgPos& c) {
   return b;
 }
 
+// The sum of a pass over a task.  FP32 sums cover at most 8192 cells, 8 planes of the 4 cells of each
+// thread: a task of no more planes is added up in FP32, of a deeper one every 8 planes a warp's, and
+// these in FP64 (64 uneven grids 2.57 -> 2.60 ms a step, 256^3 1.400 -> 1.402).
+template <typename T>
+struct TaskSum {
+  static constexpr int kPlanes = 8;
+  T part = T(0);                              // of the present group of planes
+  double whole = 0.0;                         // of those before it: the warp's
+  // a group of kPlanes ends, and not the task with it (all threads)
+  __device__ __forceinline__ void group() {
+    if constexpr (sizeof(T) == 4) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(kFull, part, o);
+      whole += f32_to_f64(part);
+      part = T(0);
+    }
+  }
+  __device__ __forceinline__ void store(double* slot, int planes) {
+    if constexpr (sizeof(T) == 4) {
+      if (planes <= kPlanes) {
+        task_store_f(slot, part);
+        return;
+      }
+      __shared__ double red[kBlock / 32];
+      group();
+      __syncthreads();
+      if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = whole;
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        double u[8];
+#pragma unroll
+        for (int w = 0; w < 8; ++w) u[w] = red[w];
+        *slot = tree8(u);
+      }
+    } else {
+      const double v[1] = {part};
+      tile_store<1>(slot, 0, v);
+    }
+  }
+};
+
 // off: the instance's first cell (d.off4; a constant 0 where there is one instance keeps the base
 // pointers out of the registers).  pslot: the place of the task's sum; dyn: kPqSmem<T> bytes of
 // shared memory.
@@ -787,9 +828,7 @@ __device__ __forceinline__ void pq_form(const DevArrays& A, const InstDesc& d, i
     keep(z0, p, po, yv);
   }
   if (hl >= 0) put_beyond(sm.p[0], hr, hpo);
-  // FP32 sums: per-thread sums of 8 planes, added up, so that no chain is longer than where four
-  // groups of threads marched a quarter of a task's planes each
-  T dot = T(0), dot8 = T(0);
+  TaskSum<T> dot;
   VT *pm = sm.p[2], *pc = sm.p[0], *pu = sm.p[1];
   int si = 0;
   for (int z = z0; z < z1; ++z) {
@@ -831,29 +870,20 @@ __device__ __forceinline__ void pq_form(const DevArrays& A, const InstDesc& d, i
         acc = fma(azv.v[i], pa.v[i], acc);
         acc = fma(azm.v[i], pd.v[i], acc);
         if (i > last) acc = T(0);             // padding: q stays 0
-        dot8 = fma(pi, acc, dot8);
+        dot.part = fma(pi, acc, dot.part);
         qv.v[i] = acc;
       }
       st16(Q + HF_IXV(A, lxy + z * nxy, n4, V), qv);
       azm = azv;
     }
-    if (sizeof(T) == 4 && ((z - z0) & 7) == 7) {
-      dot += dot8;
-      dot8 = T(0);
-    }
+    if (((z - z0) & 7) == 7 && z + 1 < z1) dot.group();
     VT* t = pm;
     pm = pc;
     pc = pu;
     pu = t;
     if (++si == kPqStages) si = 0;
   }
-  dot += dot8;
-  if constexpr (sizeof(T) == 4) {
-    task_store_f(pslot, dot);
-  } else {
-    const double v[1] = {dot};
-    tile_store<1>(pslot, 0, v);
-  }
+  dot.store(pslot, z1 - z0);
 }
 // Iteration 0 (p = r, no y) is a form of its own.
 template <typename T>
@@ -895,7 +925,7 @@ __device__ __forceinline__ void upd_form(const DevArrays& A, const InstDesc& d, 
   const int last = min(V - 1, d.nx - 1 - c.x);
   T* R = Vec<T>::r(A) + d.off4;
   const T* Q = Vec<T>::q(A) + d.off4;
-  T rr = T(0), rr8 = T(0);
+  TaskSum<T> rr;
   double rw = 0.0;
   if (!WEIGHTED && (s.xw & kXwThis)) {        // (never under the reference's rule)
     UpdXStage<T>* st = reinterpret_cast<UpdXStage<T>*>(dyn);
@@ -940,7 +970,7 @@ __device__ __forceinline__ void upd_form(const DevArrays& A, const InstDesc& d, 
         for (int i = 0; i < V; ++i) {
           const T yo = fma(alpha, pv.v[i], yv.v[i]);
           rv.v[i] = fma(-alpha, qv.v[i], rv.v[i]);
-          rr8 = fma(rv.v[i], rv.v[i], rr8);
+          rr.part = fma(rv.v[i], rv.v[i], rr.part);
           double& x = xv[i / 2].v[i & 1];
           if constexpr (sizeof(T) == 8) x = fma(fv.v[i], yo, x);
           else x = x + f32_to_f64(sig * fv.v[i] * yo);
@@ -949,10 +979,7 @@ __device__ __forceinline__ void upd_form(const DevArrays& A, const InstDesc& d, 
 #pragma unroll
         for (int i = 0; i < V / 2; ++i) st16(XW + l + 2 * i, xv[i]);
       }
-      if (sizeof(T) == 4 && ((c.z1 - 1 - z) & 7) == 7) {
-        rr += rr8;
-        rr8 = T(0);
-      }
+      if (((c.z1 - 1 - z) & 7) == 7 && z > c.z0) rr.group();
       if (++si == 3) si = 0;
     }
   } else {
@@ -986,7 +1013,7 @@ __device__ __forceinline__ void upd_form(const DevArrays& A, const InstDesc& d, 
           T r = fma(-alpha, qv.v[i], rv.v[i]);
           if (i > last) r = T(0);
           rv.v[i] = r;
-          rr8 = fma(r, r, rr8);
+          rr.part = fma(r, r, rr.part);
           if (WEIGHTED && i <= last) {
             const double dg = A.diag[d.off + HF_IX(A, (z * d.ny + c.y) * d.nx + c.x + i, d.nx * d.ny * d.nz)];
             rw = fma(-dg * (double)r, (double)r, rw);
@@ -994,22 +1021,15 @@ __device__ __forceinline__ void upd_form(const DevArrays& A, const InstDesc& d, 
         }
         st16(R + HF_IXV(A, lxy + z * nxy, n4, V), rv);
       }
-      if (sizeof(T) == 4 && ((c.z1 - 1 - zt) & 4)) {
-        rr += rr8;
-        rr8 = T(0);
-      }
+      if (((c.z1 - 1 - zt) & 4) && zt - U >= c.z0) rr.group();
       if (++si == 3) si = 0;
     }
   }
-  rr += rr8;
-  if constexpr (sizeof(T) == 4) {
-    task_store_f(pslot, rr);
-  } else if constexpr (WEIGHTED) {
-    const double v[2] = {rr, rw};
+  if constexpr (WEIGHTED) {
+    const double v[2] = {rr.part, rw};
     tile_store<2>(pslot, stride, v);
   } else {
-    const double v[1] = {rr};
-    tile_store<1>(pslot, stride, v);
+    rr.store(pslot, c.z1 - c.z0);
   }
 }
 template <typename T>
