@@ -1137,6 +1137,7 @@ int hf_set_opts(hf_ctx* h, const hf_solver_opts* opts) {
   h->c.A.opts = dev_opts(*opts);
   drop_graph(h->c);   // captured kernels hold the options by value
   h->c.res_depth = -1;
+  for (auto& b : h->c.solve_blocks) b[0] = b[1] = 0;   // (the criterion picks the kernel, too)
   if (effective_depth(h->c, *opts) != h->c.depth || opts->precision != h->c.cg_precision ||
       opts->task_depth != h->c.cg_depth)
     return build_tasks(h->c, effective_depth(h->c, *opts));
