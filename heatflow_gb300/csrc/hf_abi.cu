@@ -8,6 +8,7 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "hf_ctx.cuh"
@@ -91,6 +92,9 @@ template <typename T>
 int dalloc(Ctx& c, T** p, size_t count) {
   void* q = nullptr;
   size_t bytes = std::max<size_t>(count, 1) * sizeof(T);
+#ifdef HF_CHECKED
+  if (c.fail_alloc > 0 && --c.fail_alloc == 0) return set_err(HF_ENOMEM, "allocation refused for a test");
+#endif
   cudaError_t e = cudaMalloc(&q, bytes);
   if (e != cudaSuccess) {
     cudaGetLastError();
@@ -742,43 +746,41 @@ int cg_plan(Ctx& c) {
     total += tiles * parts;
   }
   c.ncg = c.A.ncg = total;
-  c.cg_precision = c.opts.precision;
-  c.cg_depth = c.opts.task_depth;
   std::vector<int32_t> inst((size_t)total);
   for (int64_t i = 0; i < c.ninst; ++i)
     std::fill_n(inst.begin() + c.h_inst[i].cg0, c.h_inst[i].cgn, (int32_t)i);
-  auto regrow = [&](void* old) {
-    if (!old) return;
-    cudaFree(old);
-    c.allocs.erase(std::remove(c.allocs.begin(), c.allocs.end(), old), c.allocs.end());
+  // a larger buffer in the place of p; p stays where there is no memory for one
+  auto regrow = [&](auto*& p, size_t n) -> int {
+    std::remove_reference_t<decltype(p)> fresh = nullptr;
+    if (int r = dalloc(c, &fresh, n)) return r;
+    if (p) {
+      cudaFree((void*)p);
+      c.allocs.erase(std::remove(c.allocs.begin(), c.allocs.end(), (void*)p), c.allocs.end());
+    }
+    p = fresh;
+    return HF_OK;
   };
   if (total > c.ncg_cap) {
-    regrow(const_cast<int32_t*>(c.A.cg_inst));
-    c.A.cg_inst = nullptr;
-    int32_t* p = nullptr;
-    if (int r = dalloc(c, &p, (size_t)total)) return r;
+    int32_t* p = const_cast<int32_t*>(c.A.cg_inst);
+    if (int r = regrow(p, (size_t)total)) return r;
     c.A.cg_inst = p;
     c.ncg_cap = total;
   }
   const size_t ctl = solve_ctl_bytes(c.ninst, total);
   if (ctl > c.sctl_cap) {
-    regrow(c.d_sctl);
-    c.d_sctl = c.A.sctl = nullptr;
-    c.sctl_cap = 0;
-    char* p = nullptr;
-    if (int r = dalloc(c, &p, ctl)) return r;
+    char* p = reinterpret_cast<char*>(c.d_sctl);
+    if (int r = regrow(p, ctl)) return r;
     c.d_sctl = c.A.sctl = reinterpret_cast<SolveCtl*>(p);
     c.sctl_cap = ctl;
   }
   CU(cudaMemsetAsync(c.d_sctl, 0, ctl, c.stream));
   if (std::max(c.ntasks, total) > c.A.pcap) {   // two tables
-    regrow(c.A.partials);
-    c.A.partials = nullptr;
-    c.A.pcap = 0;
     const int64_t cap = std::max(c.ntasks_cap, total);
-    if (int r = dalloc(c, &c.A.partials, (size_t)cap * kNR * 2)) return r;
+    if (int r = regrow(c.A.partials, (size_t)cap * kNR * 2)) return r;
     c.A.pcap = cap;
   }
+  c.cg_precision = c.opts.precision;
+  c.cg_depth = c.opts.task_depth;
   CU(cudaMemcpyAsync(const_cast<int32_t*>(c.A.cg_inst), inst.data(), sizeof(int32_t) * inst.size(),
                      cudaMemcpyHostToDevice, c.stream));
   CU(cudaStreamSynchronize(c.stream));
@@ -802,6 +804,7 @@ bool split_solve(const Ctx& c) {
 // planes, ordered (z, y, x); uploads the table and the instance descriptors, recomputes the
 // per-task heater flags and forgets what depended on the old table (captured graph, grid size).
 int build_tasks(Ctx& c, int depth) {
+  c.cg_precision = -1;                // until the plan and its buffers are there
   std::vector<int4> tasks;
   for (int64_t i = 0; i < c.ninst; ++i) {
     InstDesc& d = c.h_inst[i];
@@ -839,6 +842,17 @@ int build_tasks(Ctx& c, int depth) {
   c.split = split_solve(c);
   drop_graph(c);
   return HF_OK;
+}
+
+// Take over options, and plan anew what follows from them.
+int apply_opts(Ctx& c, const hf_solver_opts& o) {
+  c.opts = o;
+  c.A.opts = dev_opts(o);
+  drop_graph(c);                 // captured kernels hold the options by value
+  c.res_depth = -1;
+  for (auto& b : c.solve_blocks) b[0] = b[1] = 0;   // (the criterion picks the kernel, too)
+  const int depth = effective_depth(c, o);
+  return depth != c.depth || o.precision != c.cg_precision || o.task_depth != c.cg_depth ? build_tasks(c, depth) : HF_OK;
 }
 
 int create_impl(const hf_problem* probs, int64_t count, const hf_solver_opts* opts, hf_ctx** out) {
@@ -1133,14 +1147,13 @@ int hf_set_opts(hf_ctx* h, const hf_solver_opts* opts) {
     return set_err(HF_ESTATE, "host-buffer steps are queued: call hf_host_sync first");
   int rc = validate_opts(*opts);
   if (rc) return rc;
-  h->c.opts = *opts;
-  h->c.A.opts = dev_opts(*opts);
-  drop_graph(h->c);   // captured kernels hold the options by value
-  h->c.res_depth = -1;
-  for (auto& b : h->c.solve_blocks) b[0] = b[1] = 0;   // (the criterion picks the kernel, too)
-  if (effective_depth(h->c, *opts) != h->c.depth || opts->precision != h->c.cg_precision ||
-      opts->task_depth != h->c.cg_depth)
-    return build_tasks(h->c, effective_depth(h->c, *opts));
+  const hf_solver_opts old = h->c.opts;
+  rc = apply_opts(h->c, *opts);
+  if (rc) {                      // back to the options before, whose buffers are still there
+    const std::string why = g_err;
+    apply_opts(h->c, old);
+    return set_err(rc, why);
+  }
   return HF_OK;
 }
 
@@ -1873,7 +1886,8 @@ int hf_index_checks(hf_ctx* h, int32_t probe, int32_t* enabled, int64_t* record)
   if (int r = refuse_queued(c)) return r;
 #ifdef HF_CHECKED
   *enabled = 1;
-  if (probe) {
+  c.fail_alloc = std::max(probe - 1, 0);
+  if (probe == 1) {
     CU(launch_check_probe(c));
     CU(cudaStreamSynchronize(c.stream));
   }

@@ -40,6 +40,7 @@ struct Ctx {
   AsmArrays asm_{};
   InstBC* d_bc = nullptr;
   std::vector<void*> allocs;
+  int fail_alloc = 0;            // checked build: the allocation from now on that is refused (hf_index_checks)
   InstScal* h_scal = nullptr;    // pinned mirror for polling
   int32_t* h_flags = nullptr;    // behind it: SolveCtl's err and guard_hit
   bool state_set = false;

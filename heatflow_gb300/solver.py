@@ -79,9 +79,10 @@ class HeatFlow:
     def _check(self, code: int, where: str):
         abi.check(code, where, self.lib)
 
-    def index_checks(self, probe: bool = False):
+    def index_checks(self, probe: int = 0):
         """(enabled, record) of the index checks: enabled is True in the checked build; record =
-        [failed checks, site of the first, its index, the extent]; the record is cleared."""
+        [failed checks, site of the first, its index, the extent]; the record is cleared.  probe: as
+        hf_index_checks (1: a failed check; 1 + k: the k-th allocation from now on is refused)."""
         en = C.c_int32()
         rec = (C.c_int64 * 4)()
         self._check(self.lib.hf_index_checks(self.h, int(probe), C.byref(en), rec), "hf_index_checks")

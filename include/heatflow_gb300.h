@@ -295,8 +295,9 @@ int hf_solve_profile(hf_ctx* ctx, int64_t cap, int64_t* rounds, int32_t* phases,
  * finishes steps returns HF_EDEVICE naming the first failed check's site in hf_last_error.
  * hf_index_checks sets *enabled = 1 in the checked build (0 otherwise), copies the record
  * {failed checks, site of the first (100000 * file + line), its index, the extent} to record
- * (4 values, or NULL) and clears it.  probe != 0 (checked build only) first runs one check on an
- * index outside its range without any memory access, so a test can see a failure recorded. */
+ * (4 values, or NULL) and clears it.  probe = 1 (checked build only) first runs one check on an
+ * index outside its range without any memory access, so a test can see a failure recorded;
+ * probe = 1 + k has the context's k-th device allocation from now on refused (0 or 1: none). */
 int hf_index_checks(hf_ctx* ctx, int32_t probe, int32_t* enabled, int64_t* record);
 
 /* ---- temperature-dependent properties -------------------------------------------------------
