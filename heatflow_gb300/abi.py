@@ -139,8 +139,10 @@ _SIGNATURES = {
     "hf_adjoint_rhs": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
     "hf_adjoint_accumulate": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p,
                                         C.c_void_p]),
+    "hf_inner_solver": (C.c_int, [C.c_void_p, C.c_int32, C.POINTER(C.c_int32)]),
     "hf_index_checks": (C.c_int, [C.c_void_p, C.c_int32, C.POINTER(C.c_int32), C.POINTER(C.c_int64)]),
 }
+INNER_NAMES = ("auto", "cluster", "resident", "general", "launches")     # HF_INNER_*
 HF_KERNEL_RHS, HF_KERNEL_RESIDUAL, HF_KERNEL_CG_P, HF_KERNEL_CG_SPMV, HF_KERNEL_CG_UPDATE = 0, 1, 2, 3, 4
 HF_KERNEL_XUPDATE, HF_KERNEL_SOLVE, HF_KERNEL_CG_PQ, HF_KERNEL_RESIDUAL_INIT = 5, 6, 7, 8
 (HF_PHASE_IDLE, HF_PHASE_START, HF_PHASE_RES_INIT, HF_PHASE_CG_P, HF_PHASE_CG_Q, HF_PHASE_CG_PQ,

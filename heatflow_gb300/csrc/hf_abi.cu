@@ -267,9 +267,37 @@ int solve_error(int32_t err, int32_t guard_hit) {
   return HF_OK;
 }
 
+// As solve_loop, no kernel of which waits for another block: every pass of the inner solves is a launch,
+// and the host looks every check_every iterations.
+int solve_loop_launches(Ctx& c) {
+  const int64_t per = c.opts.precision == HF_PREC_MIXED ? c.opts.inner_itmax : c.opts.itmax;
+  const int64_t bound = ((int64_t)c.opts.max_refine + 3) * (per / c.opts.check_every + 3);
+  for (int64_t it = 0; it < bound; ++it) {
+    if (int r = sync_scal(c)) return r;
+    bool any_outer = false, any_inner = false;
+    for (int64_t i = 0; i < c.ninst; ++i) {
+      any_outer |= c.h_scal[i].outer_active != 0;
+      any_inner |= c.h_scal[i].inner_active != 0;
+    }
+    if (!any_outer) return HF_OK;
+    if (any_inner) {
+      for (int k = 0; k < c.opts.check_every; ++k) CU(launch_inner_iteration(c));
+      c.launches += 4 * c.opts.check_every;
+    } else {
+      CU(launch_residual(c, 1));
+      c.launches += 3;
+    }
+  }
+  return set_err(HF_EDEVICE, "solve loop did not terminate within its bound");
+}
+
 // Drive one step's solve after the RHS / initial residual kernels are queued: the inner solves that
 // are due (one launch), the x update and the residual, polled once per refinement.
 int solve_loop(Ctx& c) {
+  if (c.inner_from == HF_INNER_LAUNCHES || solve_grid_blocks(c, c.opts.precision == HF_PREC_MIXED ? 1 : 0, false) < 1) {
+    cudaGetLastError();                        // (no co-resident grid is no error here)
+    return solve_loop_launches(c);
+  }
   if (int r = solve_grids(c)) return r;
   CU(cudaMemsetAsync(c.d_sctl, 0, solve_ctl_bytes(c.ninst, c.ncg), c.stream));
   for (int64_t it = 0; it < (int64_t)c.opts.max_refine + 3; ++it) {
@@ -1154,6 +1182,19 @@ int hf_set_opts(hf_ctx* h, const hf_solver_opts* opts) {
     apply_opts(h->c, old);
     return set_err(rc, why);
   }
+  return HF_OK;
+}
+
+int hf_inner_solver(hf_ctx* h, int32_t from, int32_t* kernel) {
+  if (!h || from > HF_INNER_LAUNCHES) return set_err(HF_EARG, "null context or unknown kernel");
+  Ctx& c = h->c;
+  if (int r_ = refuse_queued(c)) return r_;
+  if (from >= 0 && from != c.inner_from) {
+    c.inner_from = from;
+    c.res_depth = -1;
+    drop_graph(c);                             // the captured steps hold the kernel
+  }
+  if (kernel) *kernel = inner_kernel(c);
   return HF_OK;
 }
 

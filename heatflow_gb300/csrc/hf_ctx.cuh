@@ -54,6 +54,7 @@ struct Ctx {
   // choose_solve of one grid: planes per task of k_solve_res (0: not taken, -1: not asked yet), blocks of
   // k_solve_cluster (0: not taken)
   int res_depth = -1, cluster_blocks = 0;
+  int inner_from = HF_INNER_AUTO;   // the first kernel that may run the inner solves (hf_inner_solver)
   bool split = false;            // the solve as several kernels (split_solve)
   cudaGraphExec_t solve_exec = nullptr;   // the split solve on its own (hf_solve, timing)
   cudaGraph_t solve_graph = nullptr;

@@ -585,6 +585,11 @@ cudaError_t launch_step_end(Ctx& c);
 cudaError_t launch_solve(Ctx& c, bool full = true, unsigned long long wait_ns = 4000000000ull,
                          int leaver = -1);
 int solve_grid_blocks(Ctx& c, int fp32, bool full = true);
+// The kernel that runs the inner solves (HF_INNER_*).
+int inner_kernel(Ctx& c);
+// One iteration of the inner solves that are due, as launches that wait for nothing (two passes, each
+// with its finalize).
+cudaError_t launch_inner_iteration(Ctx& c);
 cudaError_t launch_apply(Ctx& c, const double* x, double* y);
 cudaError_t launch_single(Ctx& c, int which);
 cudaError_t launch_graph_step_begin(Ctx& c, CtrlState* ctrl, int launches_per_step);
@@ -593,7 +598,7 @@ cudaError_t launch_graph_step_end(Ctx& c, CtrlState* ctrl, const SolveCtl* sctl,
 // Finalize kernels: sum the tile partials of each instance and run the scalar epilogue of the
 // kernel that produced them.  With graph != 0 (a captured split solve) the last block also sets the
 // loop condition hw, and the rounds are logged.
-enum { FIN_RHS = 0, FIN_RHS_DIAG, FIN_RES_INIT, FIN_RES };
+enum { FIN_RHS = 0, FIN_RHS_DIAG, FIN_RES_INIT, FIN_RES, FIN_PQ, FIN_UPD };
 cudaError_t launch_finalize(Ctx& c, int kind, CtrlState* ctrl, cudaGraphConditionalHandle hw,
                             int graph);
 #ifdef HF_CHECKED

@@ -1041,7 +1041,7 @@ __device__ __forceinline__ void upd_task(const DevArrays& A, const InstDesc& d, 
     upd_form<T, false>(A, d, local, s, pslot, A.pcap, dyn);
 }
 
-// ---- kernels of the split solve; the inner passes on their own only for timing -------------------
+// ---- kernels of the split solve; the inner passes on their own -----------------------------------
 // A round of the split solve in its log (one thread).
 __device__ __forceinline__ void log_round(SolveCtl* ctl, int32_t phase, unsigned long long now) {
   const int64_t r = ctl->rounds;
@@ -1324,6 +1324,8 @@ __device__ __forceinline__ bool took_part(const InstScal& s) {
     case FIN_RHS: return s.outer_active != 0;
     case FIN_RHS_DIAG: return (s.status & kStatusRhsNan) != 0;
     case FIN_RES_INIT: return s.outer_active && !s.inner_active && s.refine == 0;
+    case FIN_PQ:
+    case FIN_UPD: return s.inner_active != 0;
     default: return s.outer_active && !s.inner_active && s.refine != 0;      // FIN_RES
   }
 }
@@ -1353,7 +1355,10 @@ __global__ void __launch_bounds__(kBlock) k_finalize(DevArrays A, CtrlState* ctr
     reinterpret_cast<unsigned long long*>(&sd)[tid] = reinterpret_cast<const unsigned long long*>(A.inst + inst)[tid];
   if (!one) __syncthreads();
   double acc[NR];
-  instance_sum<NR>(A.partials, A.pcap, one ? 0 : sd.task0, one ? A.ntasks : (int64_t)sd.ntask, acc, red);
+  if (KIND == FIN_PQ || KIND == FIN_UPD)
+    instance_sum<NR>(A.partials, A.pcap, one ? 0 : sd.cg0, one ? A.ncg : (int64_t)sd.cgn, acc, red);
+  else
+    instance_sum<NR>(A.partials, A.pcap, one ? 0 : sd.task0, one ? A.ntasks : (int64_t)sd.ntask, acc, red);
   const bool part = took_part<KIND>(sh);       // (instance_sum holds a block barrier)
   __syncthreads();                             // every thread has looked before the epilogue changes sh
   if (part && tid < 32) {
@@ -1374,6 +1379,11 @@ __global__ void __launch_bounds__(kBlock) k_finalize(DevArrays A, CtrlState* ctr
         case FIN_RHS: epi_rhs(sh, sd, A.opts, acc); break;
         case FIN_RHS_DIAG: epi_rhs_diag(sh, acc); break;
         case FIN_RES_INIT: epi_residual_s<true>(sh, sd, A.opts, acc, rel, rms); break;
+        case FIN_PQ: epi_spmv_s(sh, acc); break;
+        case FIN_UPD:
+          if (A.opts.precision == HF_PREC_MIXED) epi_upd<float>(sh, A.opts, acc);
+          else epi_upd<double>(sh, A.opts, acc);
+          break;
         default: epi_residual_s<false>(sh, sd, A.opts, acc, rel, rms); break;
       }
     }
@@ -2578,9 +2588,21 @@ static int res_depth_of(Ctx& c) {
 // k_solve_res: FP64 under the reference's rule, 8 tasks 7.3 and 9.5, 16 tasks 7.7 and 9.5, 32 tasks 9.8
 // and 9.4; FP32, 16 tasks 4.6 and 6.3, 32 tasks 5.5 and 6.3, 48 (three a block) 7.8 and 6.7.
 template <typename T, bool WEIGHTED>
+static void choose_of(Ctx& c) {
+  c.cluster_blocks = c.inner_from <= HF_INNER_CLUSTER ? cluster_blocks_of<T, WEIGHTED>(c) : 0;
+  c.res_depth = c.inner_from <= HF_INNER_RESIDENT ? res_depth_of<T, WEIGHTED>(c) : 0;
+}
 static void choose_solve(Ctx& c) {
-  c.cluster_blocks = cluster_blocks_of<T, WEIGHTED>(c);
-  c.res_depth = res_depth_of<T, WEIGHTED>(c);
+  if (c.res_depth >= 0) return;
+  if (c.opts.precision == HF_PREC_MIXED) choose_of<float, false>(c);
+  else if (c.opts.criterion == HF_STOP_RECURSIVE) choose_of<double, true>(c);
+  else choose_of<double, false>(c);
+}
+int inner_kernel(Ctx& c) {
+  if (c.opts.use_graph == 0 && c.inner_from == HF_INNER_LAUNCHES) return HF_INNER_LAUNCHES;
+  if (c.ninst > 1) return HF_INNER_GENERAL;
+  choose_solve(c);
+  return c.cluster_blocks > 0 ? HF_INNER_CLUSTER : c.res_depth > 0 ? HF_INNER_RESIDENT : HF_INNER_GENERAL;
 }
 
 // Zero the control block (its counters: full = false), then launch the persistent solve cooperatively
@@ -2609,11 +2631,7 @@ cudaError_t launch_solve(Ctx& c, bool full, unsigned long long wait_ns, int leav
   cfg.numAttrs = 1;
   const bool weighted = !fp32 && c.opts.criterion == HF_STOP_RECURSIVE;
   if (c.ninst == 1) {
-    if (c.res_depth < 0) {
-      if (fp32) choose_solve<float, false>(c);
-      else if (weighted) choose_solve<double, true>(c);
-      else choose_solve<double, false>(c);
-    }
+    choose_solve(c);
     if (c.cluster_blocks > 0 && leaver < 0)    // (the failure-path check is of the waits of the others)
       return fp32 ? launch_cluster<float, false>(c, limit)
                   : weighted ? launch_cluster<double, true>(c, limit) : launch_cluster<double, false>(c, limit);
@@ -2686,6 +2704,14 @@ static cudaError_t launch_cg_upd(Ctx& c) {
   return cudaGetLastError();
 }
 
+cudaError_t launch_inner_iteration(Ctx& c) {
+  const bool fp32 = c.opts.precision == HF_PREC_MIXED;
+  cudaError_t e = fp32 ? launch_cg_pq<float>(c) : launch_cg_pq<double>(c);
+  if (e == cudaSuccess) e = launch_finalize(c, FIN_PQ, nullptr, 0, 0);
+  if (e == cudaSuccess) e = fp32 ? launch_cg_upd<float>(c) : launch_cg_upd<double>(c);
+  return e == cudaSuccess ? launch_finalize(c, FIN_UPD, nullptr, 0, 0) : e;
+}
+
 cudaError_t launch_graph_step_begin(Ctx& c, CtrlState* ctrl, int launches_per_step) {
   k_graph_step_begin<<<(unsigned)((c.ninst + 127) / 128), 128, 0, c.stream>>>(c.A, ctrl,
                                                                                launches_per_step);
@@ -2704,6 +2730,8 @@ cudaError_t launch_finalize(Ctx& c, int kind, CtrlState* ctrl, cudaGraphConditio
     case FIN_RHS_DIAG: k_finalize<FIN_RHS_DIAG><<<nb, 256, 0, c.stream>>>(c.A, ctrl, hw, graph); break;
     case FIN_RES_INIT: k_finalize<FIN_RES_INIT><<<nb, 256, 0, c.stream>>>(c.A, ctrl, hw, graph); break;
     case FIN_RES: k_finalize<FIN_RES><<<nb, 256, 0, c.stream>>>(c.A, ctrl, hw, graph); break;
+    case FIN_PQ: k_finalize<FIN_PQ><<<nb, 256, 0, c.stream>>>(c.A, ctrl, hw, graph); break;
+    case FIN_UPD: k_finalize<FIN_UPD><<<nb, 256, 0, c.stream>>>(c.A, ctrl, hw, graph); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();

@@ -189,6 +189,15 @@ class HeatFlow:
         self.opts = make_opts(**opts)
         self._check(self.lib.hf_set_opts(self.h, C.byref(self.opts)), "hf_set_opts")
 
+    def inner_solver(self, first=None) -> str:
+        """The kernel that runs the next step's inner CG solves: "cluster", "resident", "general" or
+        "launches".  `first` ("auto" or one of these): from now on, of these kernels in turn, only from
+        this one on.  The field's bits are the same on all of them."""
+        out = C.c_int32()
+        self._check(self.lib.hf_inner_solver(self.h, -1 if first is None else abi.INNER_NAMES.index(first),
+                                             C.byref(out)), "hf_inner_solver")
+        return abi.INNER_NAMES[out.value]
+
     # ---- state
     def set_state(self, tp, tpp):
         tp = np.ascontiguousarray(tp, np.float64)

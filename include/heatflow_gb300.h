@@ -95,7 +95,8 @@ typedef struct hf_solver_opts {
   double inner_tol;     /* mixed: relative reduction asked of each FP32 inner solve */
   int32_t inner_itmax;  /* mixed: max FP32 CG iterations per inner solve */
   int32_t max_refine;   /* mixed: max FP64 refinement sweeps per step */
-  int32_t check_every;  /* >= 1; without effect (inner solves run on the device to their end) */
+  int32_t check_every;  /* >= 1: iterations between the host's polls where every pass of an inner
+                           solve is a launch (hf_inner_solver); elsewhere without effect */
   int32_t use_graph;    /* hf_run's step loop: 0 = kernels launched by the host, which polls once
                            per refinement;
                            1 = the whole loop as one CUDA graph (a WHILE node around a step whose
@@ -284,6 +285,22 @@ enum {
  * first min(rounds, cap, 512) rounds, phases[r] = the phase instance 0 ran and round_us[r] = the
  * round's length in microseconds (device %globaltimer; round 0 counts from the kernel's start). */
 int hf_solve_profile(hf_ctx* ctx, int64_t cap, int64_t* rounds, int32_t* phases, double* round_us);
+
+/* Which kernel runs the inner CG solves.  No counterpart in the reference.  All give the same bits
+ * (a batch's, with task_depth = 0, where its tasks are cut as a single grid's).  A grid takes the
+ * first of these that it fits, from `from` on (< 0: as set before; HF_INNER_AUTO on creation);
+ * batches always take HF_INNER_GENERAL or HF_INNER_LAUNCHES.  The last one, whose kernels wait for
+ * nothing, serves use_graph = 0 (and stands in there where no persistent kernel can be resident);
+ * captured steps take HF_INNER_GENERAL in its place.  *kernel (or NULL): the one that the next step's
+ * inner solves run on. */
+enum {
+  HF_INNER_AUTO = 0,
+  HF_INNER_CLUSTER = 1,   /* one thread-block cluster, all state in its shared memory */
+  HF_INNER_RESIDENT = 2,  /* a task per block, all blocks resident, state in shared memory */
+  HF_INNER_GENERAL = 3,   /* persistent blocks, state in memory; batches: a queue of tasks */
+  HF_INNER_LAUNCHES = 4   /* a launch per pass, polled by the host every check_every iterations */
+};
+int hf_inner_solver(hf_ctx* ctx, int32_t from, int32_t* kernel);
 
 /* ---- index checks ------------------------------------------------------------------------------
  * No counterpart in the reference (the reference has no bounds-checked build; this stands in for a
