@@ -106,6 +106,13 @@ int dalloc(Ctx& c, T** p, size_t count) {
   return HF_OK;
 }
 
+// An executable graph, or null: a refused instantiation leaves no handle to destroy.
+cudaError_t instantiate(cudaGraphExec_t* exec, cudaGraph_t g) {
+  const cudaError_t e = cudaGraphInstantiate(exec, g, 0);
+  if (e != cudaSuccess) *exec = nullptr;
+  return e;
+}
+
 void drop_graph(Ctx& c) {
   if (c.graph_exec) cudaGraphExecDestroy(c.graph_exec);
   if (c.graph) cudaGraphDestroy(c.graph);
@@ -394,7 +401,7 @@ int run_solve(Ctx& c) {
       e = cudaStreamEndCapture(cs, &g);
     }
     cudaStreamDestroy(cs);
-    if (e == cudaSuccess && err.empty()) e = cudaGraphInstantiate(&c.solve_exec, g, 0);
+    if (e == cudaSuccess && err.empty()) e = instantiate(&c.solve_exec, g);
     if (e != cudaSuccess || !err.empty()) {
       if (g) cudaGraphDestroy(g);
       cudaGetLastError();
@@ -429,7 +436,7 @@ int build_graph_persistent(Ctx& c) {
     chk(launch_graph_step_end(c, c.d_ctrl, c.d_sctl), "step end");
     if (c.tempdep) chk(launch_tempdep(c), "properties");
     chk(cudaStreamEndCapture(cs, &g), "end capture");
-    if (err.empty()) chk(cudaGraphInstantiate(&c.graph_exec, g, 0), "instantiate");
+    if (err.empty()) chk(instantiate(&c.graph_exec, g), "instantiate");
   }
   c.stream = saved;
   cudaStreamDestroy(cs);
@@ -486,7 +493,7 @@ int build_loop_graph(Ctx& c) {
     if (c.tempdep) chk(launch_tempdep(c), "properties");
     cudaGraph_t tmp = nullptr;
     chk(cudaStreamEndCapture(cs, &tmp), "end capture");
-    if (err.empty()) chk(cudaGraphInstantiate(&c.loop_exec, g, 0), "instantiate");
+    if (err.empty()) chk(instantiate(&c.loop_exec, g), "instantiate");
   } while (0);
   c.stream = saved;
   cudaStreamDestroy(cs);
@@ -549,7 +556,7 @@ int build_post_graph(Ctx& c) {
       if (c.tempdep) chk(launch_tempdep(c), "properties");
       c.A.xout = nullptr;
       chk(cudaStreamEndCapture(cs, &g), "end capture");
-      if (err.empty()) chk(cudaGraphInstantiate(&c.post_exec[j], g, 0), "instantiate");
+      if (err.empty()) chk(instantiate(&c.post_exec[j], g), "instantiate");
     }
     c.post_graph[j] = g;
   }

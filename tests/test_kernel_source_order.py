@@ -33,3 +33,11 @@ def test_warp_votes_name_lanes_that_arrive():
     for unit in os.listdir(os.path.join(ROOT, "heatflow_gb300", "csrc")):
         text = open(os.path.join(ROOT, "heatflow_gb300", "csrc", unit)).read()
         assert "__activemask" not in text, unit
+
+
+def test_refused_instantiation_leaves_no_handle():
+    """A graph whose instantiation is refused has no executable: every instantiation goes through the one
+    place that says so, and none of the error paths destroys what was never made."""
+    text = open(os.path.join(ROOT, "heatflow_gb300", "csrc", "hf_abi.cu")).read()
+    assert text.count("cudaGraphInstantiate(") == 1
+    assert "nullptr" in _body("instantiate", "hf_abi.cu")
