@@ -2031,6 +2031,7 @@ int hf_get_rhs(hf_ctx* h, int64_t itime, double* B, double* Q, double* Qd, doubl
   if (!h) return set_err(HF_EARG, "null context");
   Ctx& c = h->c;
   if (!c.state_set) return set_err(HF_ESTATE, "hf_set_state must be called first");
+  if (int r_ = refuse_queued(c)) return r_;    // before anything is launched
   // scratch: the FP64 CG vectors are free outside a step (they start a solve as zeros in their
   // padding cells, so they are cleared afterwards)
   CU(launch_step_begin(c, itime, 0));
