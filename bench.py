@@ -102,7 +102,7 @@ def rhs_bytes(prob):
 
 
 def round_bytes_per_cell(rounds, precision):
-    """Algorithmic bytes per cell of each round of one persistent-solve launch (its round log)."""
+    """Algorithmic bytes per cell of each round of one solve (its round log)."""
     table = PHASE_BYTES[precision]
     out, first_cg, first_b, have_y, bx, passes = [], True, True, False, None, 0
     for ph, _ in rounds:
@@ -138,7 +138,7 @@ def round_bytes_per_cell(rounds, precision):
 
 
 def solve_bytes_per_cell(rounds, precision):
-    """Algorithmic bytes per cell of one persistent-solve launch from its round phases."""
+    """Algorithmic bytes per cell of one solve from its round phases."""
     return sum(round_bytes_per_cell(rounds, precision))
 
 
@@ -179,7 +179,7 @@ def solve_floor(rounds, precision, N, hbm_gbs, fp64_tflops):
 
 
 def phase_table(rounds, precision, N):
-    """Per phase of one persistent-solve launch: rounds, microseconds, upper GB/s (full bytes)."""
+    """Per phase of one solve: rounds, microseconds, upper GB/s (full bytes)."""
     out = {}
     for ph, us in rounds:
         e = out.setdefault(ph, {"rounds": 0, "us": 0.0})
@@ -444,7 +444,7 @@ def workload_config(args, prob):
         "step_loop": "host-polled kernels" if args.host_loop else
                      ("one CUDA graph launch per step" if args.per_step_graph else
                       "the whole loop as one CUDA graph (WHILE node)") +
-                     ": RHS + one persistent cooperative solve kernel per step",
+                     ": RHS, residual sweeps and a persistent kernel for the inner CG",
     }
 
 

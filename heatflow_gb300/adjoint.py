@@ -212,8 +212,7 @@ def _main(argv=None):
     ap.add_argument("--probes", type=int, default=64)
     ap.add_argument("--sources", type=int, default=8)
     ap.add_argument("--ckpt", type=int, default=25)
-    # per-step conditional graphs: at 64^3 (256 tasks) faster than the persistent solve, whose
-    # grid-wide rounds then wait on a few busy SMs
+    # a graph per step; the solves run in the same kernels with 1 and 3
     ap.add_argument("--use-graph", type=int, default=2)
     a = ap.parse_args(argv)
     # untimed warm-up on a small copy: the first use of each torch operation on the device may

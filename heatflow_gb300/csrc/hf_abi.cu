@@ -413,8 +413,7 @@ int run_solve(Ctx& c) {
   return HF_OK;
 }
 
-// Capture one step with the persistent solve: step begin, RHS and its finalize, the cooperative
-// solve kernel (zeroing its control block first), step end.  Five kernels per step.
+// Capture one step: step begin, RHS and its finalize, the solve (capture_solve), step end.
 int build_graph_persistent(Ctx& c) {
   if (int r = solve_grids(c)) return r;
   const bool split = c.split || c.opts.use_graph == 2;
@@ -452,7 +451,7 @@ int build_graph_persistent(Ctx& c) {
 }
 
 // The whole time loop as one graph: a WHILE conditional node whose body is one step (step begin,
-// RHS and its finalize, the persistent solve, step end).  k_graph_step_end sets the condition
+// RHS and its finalize, the solve, step end).  k_graph_step_end sets the condition
 // from the device step counter (CtrlState::itime < itime_end, and no failed solve), so a single
 // launch runs any number of steps and always ends.  Built once per options; not every runtime
 // accepts a cooperative kernel in a conditional body, and then hf_run launches the per-step graph
@@ -522,7 +521,7 @@ int build_graph(Ctx& c) {
   return HF_OK;
 }
 
-// The step after its RHS (RHS finalize, persistent solve, step end, property rebuild) as one
+// The step after its RHS (RHS finalize, solve, step end, property rebuild) as one
 // graph, for steps whose RHS runs chunk by chunk behind the host upload (hf_step_host_async).
 int build_post_graph(Ctx& c) {
   if (c.post_exec[0] && c.post_exec[1] && c.post_precision == c.opts.precision &&
@@ -691,12 +690,13 @@ int download_padded(Ctx& c, T* dst, const T* src) {
 }
 
 // Task depth of the option 0 (default): kZC planes, or fewer (halving down to kMinTaskDepth) while
-// the grids would give fewer than two tasks per block of a persistent solve (3 blocks per SM on
-// GB300's 152).  A round lasts as long as its slowest task, so on a small grid deep tasks leave
-// most SMs idle: a 64^3 grid has 32 tasks of 8192 cells at depth 32, 256 at depth 4; at 128^3
-// depth 8 (1024 tasks) solved faster than 16 (512) and 32.  A fixed count keeps the task table,
-// and so the bits, independent of the device.
-constexpr int64_t kDefaultMinTasks = 2 * 3 * 152;
+// the grids would give fewer than 912 tasks, six for each of GB300's 152 SMs: on a small grid deep tasks
+// leave most SMs idle (64^3, 32 tasks at depth 32, 256 at depth 4; ms a step of the mixed slab at
+// depths 4, 8, 16 and 32: 0.113, 0.119, 0.145 and 0.201).  The line was drawn when these tasks were the
+// inner solve's, too; its passes now have their own (cg_plan), and at 128^3, where the rule gives 8, the
+// depths 8, 16 and 32 measure 0.301, 0.281 and 0.282.  A fixed count keeps the task table, and so the
+// bits, independent of the device.
+constexpr int64_t kDefaultMinTasks = 912;
 int effective_depth(const Ctx& c, const hf_solver_opts& o) {
   if (o.task_depth > 0) return o.task_depth;
   for (int depth = kZC; depth > kMinTaskDepth; depth /= 2) {
@@ -724,8 +724,9 @@ int64_t inner_cells(const Ctx& c) {
 // many parts as make its longest chain of planes per block, over waves of kSolveBlocks blocks, shortest,
 // the halo counted as one plane per part; a count above one wave pays only where a wave could not be
 // filled.  Several grids: parts of one length for all, such that there are about kBatchWaves tasks per
-// block -- they are handed out one at a time, and each costs a few trips through L2 (64 uneven grids, 20
-// steps, with 2, 3, 4 and 5 per block: 56.2, 56.0, 58.0 and 64.6 ms).  The order of a grid's sums, and
+// block -- they are handed out one at a time, and each costs a few trips through L2 (ms a step with 2, 3 and 4
+// per block: 64 grids of 16 to 96 cells an edge mixed 2.70, 2.74, 2.83, FP64 5.94, 5.99, 6.05; 12 of 60 to 120 2.05,
+// 2.07, 2.11 and 4.60, 4.44, 4.57; 40 of 16 to 64 1.01, 1.10, 1.31 and 1.66, 1.67, 1.89).  The order of a grid's sums, and
 // with it its bits, then depends on the grids beside it.  Where the caller gives a task depth it does not:
 // every grid of a batch is cut as it would be alone, into tasks of no fewer cells than a cell task of
 // that depth has (the 64 grids at depths 8, 16, 32 and 64: 5.1, 3.7, 2.9 and 2.6 ms a step, 2.6 without).
@@ -826,7 +827,10 @@ int cg_plan(Ctx& c) {
 // passes want different registers and blocks per SM, and in one kernel the passes spill: at 256^3 the
 // SpMV pass took 242 us in the whole form and 115 in the split, the residual 407 and 274.  The split
 // costs about 10 us of launches per refinement; one grid still gains by it on 625 cells (0.86
-// against 0.92 ms a step), a batch of uneven grids only once its solve is longer than that.
+// against 0.92 ms a step).  Of batches the smaller ones keep one launch per solve; the line is a round
+// number, and batches of uneven grids on both sides of it gain by the split: ms a step, split and
+// whole, at 0.13, 0.62, 0.91, 1.2 and 12.3 million cells, mixed 0.51 0.57, 0.75 0.87, 0.90 1.16, 1.17 1.43,
+// 2.7 4.4, FP64 0.53 0.60, 1.10 1.27, 1.05 1.34, 1.09 1.31, 6.0 8.2.
 constexpr int64_t kSplitCells = 1000000;
 bool split_solve(const Ctx& c) {
   if (c.ninst == 1) return true;
@@ -1022,7 +1026,6 @@ int create_impl(const hf_problem* probs, int64_t count, const hf_solver_opts* op
   A.task_heat = d_task_heat;
   A.tasks = d_tasks;
   A.ntasks = c.ntasks;
-  ALLOC(A.counters, (size_t)count);
   ALLOC(c.d_bc, (size_t)count);
   A.inst = d_inst; A.scal = d_scal; A.tile_inst = d_tile_inst;
   ALLOC(A.diag, N); ALLOC(A.cx, N); ALLOC(A.cy, N); ALLOC(A.cz, N); ALLOC(A.sinv, N);
@@ -1050,7 +1053,6 @@ int create_impl(const hf_problem* probs, int64_t count, const hf_solver_opts* op
   c.h_flags = reinterpret_cast<int32_t*>(c.h_scal + count);
   auto fail = [&](int r) { free_all(c); delete h; return r; };
 #define CK(call) do { cudaError_t e_ = (call); if (e_ != cudaSuccess) return fail(set_err(HF_ECUDA, std::string(#call) + ": " + cudaGetErrorString(e_))); } while (0)
-  CK(cudaMemsetAsync(A.counters, 0, sizeof(unsigned) * count, c.stream));
   CK(cudaMemsetAsync(d_scal, 0, sizeof(InstScal) * count, c.stream));
   CK(cudaMemsetAsync(A.stamps, 0, sizeof(unsigned long long) * kStamps, c.stream));
   CK(cudaMemsetAsync(A.check, 0, sizeof(unsigned long long) * 4, c.stream));

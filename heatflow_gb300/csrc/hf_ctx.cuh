@@ -120,8 +120,8 @@ struct Ctx {
   std::vector<HostCall> async_calls;
   int64_t* d_check_call = nullptr;     // first call whose uploads differed from the device copy
   int64_t async_host_kernels = 0;      // host-copy kernels of the queued calls
-  // T^n moves in chunks of whole task z-slabs: each chunk's RHS tasks run as soon as its cells
-  // are placed, while later chunks are still on the link.  Cells [clo, chi) of the compact host
+  // T^n moves in chunks of whole groups of cell runs (Chunk): each chunk's RHS tasks run as soon as its
+  // cells are placed, while later chunks are still on the link.  Cells [clo, chi) of the compact host
   // layout, [glo, ghi) of the device layout, tasks [tlo, thi).
   struct HostChunk { int64_t clo, chi, glo, ghi, tlo, thi; };
   std::vector<HostChunk> host_chunks;

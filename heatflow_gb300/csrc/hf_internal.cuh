@@ -195,7 +195,6 @@ struct DevArrays {
   double* partials;       // partial sums of the tasks: value k of task t at [k * pcap + t]; two such
                           // tables of kNR values: the persistent solve of several grids uses the
                           // second for the inner solve's passes, whose tasks are numbered apart
-  unsigned int* counters; // per instance, last-block detection
   DevOpts opts;
   // static
   double *diag, *cx, *cy, *cz, *sinv, *a64x, *a64y, *a64z;

@@ -23,7 +23,7 @@
 //
 // The inner solve of one grid is one persistent kernel, of three (choose_solve): k_solve_cluster,
 // k_solve_res, k_solve_one.  Batches: k_solve_batch.  Residuals and x update are kernels of their own
-// but in small batches (split_solve).
+// but in small batches (split_solve).  launch_inner_iteration runs the same passes as plain launches.
 //
 // All solver state is per instance in device memory; tiles of instances that are not in the
 // phase a kernel serves return at once (per-instance convergence masks).
@@ -452,7 +452,6 @@ struct YEnd {
 template <typename TY>
 __device__ __forceinline__ void xupd_cells(const DevArrays& A, const Chunk& c, const InstScal& s) {
   constexpr bool F32 = sizeof(TY) == 4;
-  constexpr int U = 1;
   const InstDesc& d = *c.d;
   const double* XR = A.tbuf[s.role[2]] + d.off;
   double* XW = A.tbuf[s.role[3]] + d.off;
@@ -479,30 +478,17 @@ __device__ __forceinline__ void xupd_cells(const DevArrays& A, const Chunk& c, c
     return x;
   };
   auto cells = [&](auto with_tiny) {
-    for (unsigned l0 = c.first(); l0 < c.end; l0 += c.step * U) {
-      double2 xv[U];
-      decltype(ld_pair(sinv, 0, true)) yv[U], pv[U], sv[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const unsigned l = l0 + c.step * u;
-        yv[u] = pv[u] = sv[u] = pair_of(TY(0), TY(0));
-        if (l >= c.end) continue;
-        const bool two = l + 1 < c.end;
-        xv[u] = ld_pair(XR, HF_IXP(A, l, n, two), two);
-        if (use_y) {
-          if (ye.old) yv[u] = inner(Y, l, two);
-          if (ye.last) pv[u] = inner(P, l, two);
-          sv[u] = ld_pair(sinv, HF_IXP(A, l, n, two), two);
-        }
+    for (unsigned l = c.first(); l < c.end; l += c.step) {
+      const bool two = l + 1 < c.end;
+      decltype(ld_pair(sinv, 0, true)) y{}, p{}, si{};
+      const double2 x = ld_pair(XR, HF_IXP(A, l, n, two), two);
+      if (use_y) {
+        if (ye.old) y = inner(Y, l, two);
+        if (ye.last) p = inner(P, l, two);
+        si = ld_pair(sinv, HF_IXP(A, l, n, two), two);
       }
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const unsigned l = l0 + c.step * u;
-        if (l >= c.end) continue;
-        const double2 x = make_double2(cell(with_tiny, xv[u].x, ye(yv[u].x, pv[u].x), sv[u].x),
-                                       cell(with_tiny, xv[u].y, ye(yv[u].y, pv[u].y), sv[u].y));
-        st_pair(XW, HF_IXP(A, l, n, l + 1 < c.end), l + 1 < c.end, x);
-      }
+      st_pair(XW, HF_IXP(A, l, n, two), two,
+              make_double2(cell(with_tiny, x.x, ye(y.x, p.x), si.x), cell(with_tiny, x.y, ye(y.y, p.y), si.y)));
     }
   };
   if constexpr (F32) cells(std::false_type{});
@@ -1095,7 +1081,7 @@ __global__ void __launch_bounds__(kBlock) k_cg_upd(DevArrays A) {
 }
 
 // ---- summation of an instance's task partials ------------------------------------------------
-// One order for every path (finalize kernels, both persistent solves) and every batch composition:
+// One order for every path (finalize kernels, all persistent solves), for the tasks that the plan made:
 // thread c adds the partials of tasks c, c + kBlock, ... in turn, the eight threads of a lane are
 // added as tree8, the lanes as a shuffle tree.  The result is valid in thread 0.  Partials are read
 // through L2 (written by other blocks of the same persistent launch); the loads of a pass are
@@ -1439,12 +1425,12 @@ __global__ void k_graph_step_end(DevArrays A, CtrlState* ctrl, const SolveCtl* s
 }
 
 // ---- persistent solve ------------------------------------------------------------------------
-// One cooperative launch runs a step's whole refinement loop.  An instance goes through phases
-// (PH_*); in a phase every one of its tasks does the phase's work, writing its partial sums to its
-// fixed slot; then an epilogue sums the partials in the fixed order of instance_sum (the order the
-// finalize kernels use, so every path obtains the same bits) and updates the instance's scalars
-// (alpha, beta, convergence test, next phase).  One grid runs its phases in grid-wide rounds
-// (k_solve_one); the grids of a batch each at their own pace (k_solve_batch).
+// One cooperative launch runs the inner solves that are due, or in a small batch a step's whole
+// refinement loop.  An instance goes through phases (PH_*); in a phase every one of its tasks does the
+// phase's work, writing its partial sums to its fixed slot; then an epilogue sums the partials in the
+// fixed order of instance_sum (the order the finalize kernels use, so every path obtains the same bits)
+// and updates the instance's scalars (alpha, beta, convergence test, next phase).  One grid runs its
+// phases in grid-wide rounds (k_solve_one); the grids of a batch each at their own pace (k_solve_batch).
 //
 // Termination: every wait is bounded in time (wait_ns, 4 s by default) and in polls; a block that
 // gives up records SolveCtl::err and returns, and the blocks still waiting see the flag and return
@@ -1555,7 +1541,8 @@ __device__ __forceinline__ int32_t logged_phase(const InstScal& s) {
 // out next: a block that waits for its ticket's range to be published never holds up the others.
 // An instance's old range stays in its slot until the next replaces it; only blocks that hold one
 // of its tickets match it.
-// Blocks per SM: 3 (85 registers: the FP64 stencil and the FP32 vector pass need about that).
+// Two blocks per SM, by the passes' shared memory (99 KB each) and registers (114; the whole form, with the
+// FP64 sweeps in it, has 128 and spills, in 600 to 820 B of stores).
 // XOUT: the instance used by the graphs of host-buffer steps, whose residual sweeps also store x
 // into A.xout (a variant of its own, so the other solves carry none of it).
 constexpr int kSlotShift = 24;      // slot: first ticket << 24 | tasks << 1 | walk the tasks backwards

@@ -117,7 +117,7 @@ class HeatFlow:
         return ms.value
 
     def solve_profile(self, cap: int = 512):
-        """Rounds of the last persistent solve: [(phase name, microseconds), ...] and the total
+        """Rounds of the last captured solve: [(phase name, microseconds), ...] and the total
         number of rounds (the per-round list stops at 512)."""
         rounds = C.c_int64()
         ph = (C.c_int32 * cap)()
@@ -128,7 +128,7 @@ class HeatFlow:
 
     def step_timeline(self):
         """Microseconds of the latest step: step begin -> RHS, RHS -> its finalize, finalize ->
-        persistent solve, solve (to the end of its last round), -> step end (None where absent)."""
+        solve, solve (to the end of its last round), -> step end (None where absent)."""
         us = (C.c_double * 5)()
         self._check(self.lib.hf_step_timeline(self.h, us), "hf_step_timeline")
         keys = ("begin_to_rhs", "rhs", "finalize", "solve", "solve_to_end")

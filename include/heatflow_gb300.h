@@ -252,10 +252,9 @@ enum {
   HF_KERNEL_RESIDUAL_INIT = 8 /* the step-start residual sweep r = S - H (x0 + TINY) */
 };
 /* Timeline of the latest step, from %globaltimer stamps its kernels write when they start
- * (microseconds): us[0] step begin -> RHS, us[1] RHS -> RHS finalize, us[2] finalize -> persistent
- * solve, us[3] solve start -> end of its last round, us[4] -> step end.  -1 where the step had no
- * such kernel (the per-kernel solve paths, use_graph 0 and 2, have no persistent solve).  No
- * counterpart in the reference. */
+ * (microseconds): us[0] step begin -> RHS, us[1] RHS -> RHS finalize, us[2] finalize -> solve, us[3]
+ * solve start -> end of its last round, us[4] -> step end.  -1 where the step did not write them
+ * (use_graph 0 does not log its solve).  No counterpart in the reference. */
 int hf_step_timeline(hf_ctx* ctx, double* us);
 /* Launch one kernel `reps` times on the current state, each bracketed by CUDA events on the
  * context's stream, and return its mean duration in milliseconds.  Solver scalars are restored
@@ -280,7 +279,7 @@ enum {
   HF_PHASE_CG_BX = 10     /* inner CG update that also forms x += sigma S^-1 y: the iteration
                              predicted to end the inner solve (true-residual criterion) */
 };
-/* Round profile of the context's last solve (use_graph 1 or 3, or hf_time_kernel with
+/* Round profile of the context's last captured solve (use_graph 1, 2 or 3, or hf_time_kernel with
  * HF_KERNEL_SOLVE).  No counterpart in the reference.  *rounds = grid-wide rounds run; for the
  * first min(rounds, cap, 512) rounds, phases[r] = the phase instance 0 ran and round_us[r] = the
  * round's length in microseconds (device %globaltimer; round 0 counts from the kernel's start). */
@@ -345,8 +344,10 @@ int hf_subbox_async(hf_ctx* ctx, int64_t inst, const int64_t* lo, const int64_t*
 int hf_subbox_wait(hf_ctx* ctx, int64_t ticket);
 
 /* ---- failure-path check ------------------------------------------------------------------------
- * No counterpart in the reference.  Runs the next step's persistent solve once with one block
- * that leaves without arriving at the first grid barrier and a barrier time limit of wait_ms:
+ * No counterpart in the reference.  Runs the next step's persistent solve once (of one grid its inner
+ * solve, on the kernel that hf_inner_solver names, or HF_INNER_RESIDENT in place of the cluster, whose
+ * blocks wait in hardware) with one block that leaves without arriving at the end of the first
+ * round (a batch: with its first task) and a time limit of wait_ms:
  * the other blocks give up after wait_ms, record the failure and return, and *status receives the
  * code the step loop would report (HF_EDEVICE).  The temperature state and the scalars are
  * restored, so the context stays usable.  For tests of the bounded-wait path (no GPU fault). */
