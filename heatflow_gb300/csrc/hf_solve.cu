@@ -642,18 +642,22 @@ __device__ __forceinline__ Beyond beyond_of(const InstDesc& d, const CgPos& c) {
 
 // The sum of a pass over a task.  FP32 sums cover at most 8192 cells, 8 planes of the 4 cells of each
 // thread: a task of no more planes is added up in FP32, of a deeper one every 8 planes a warp's, and
-// these in FP64 (64 uneven grids 2.57 -> 2.60 ms a step, 256^3 1.400 -> 1.402).
+// these in FP64 (ms a step against sums in FP32 to the end: 64 uneven grids 2.56 -> 2.58, 256^3 1.402 -> 1.405).
 template <typename T>
 struct TaskSum {
   static constexpr int kPlanes = 8;
   T part = T(0);                              // of the present group of planes
   double whole = 0.0;                         // of those before it: the warp's
+  __device__ __forceinline__ T warp_part() const {
+    T v = part;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
+    return v;
+  }
   // a group of kPlanes ends, and not the task with it (all threads)
   __device__ __forceinline__ void group() {
     if constexpr (sizeof(T) == 4) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(kFull, part, o);
-      whole += f32_to_f64(part);
+      whole += f32_to_f64(warp_part());
       part = T(0);
     }
   }
@@ -663,16 +667,22 @@ struct TaskSum {
         task_store_f(slot, part);
         return;
       }
+      // a round waits for this: the FP64 adds by one warp, the last group's among them
       __shared__ double red[kBlock / 32];
-      group();
+      __shared__ float last[kBlock / 32];
+      const float v = warp_part();
       __syncthreads();
-      if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = whole;
+      if ((threadIdx.x & 31) == 0) {
+        red[threadIdx.x >> 5] = whole;
+        last[threadIdx.x >> 5] = v;
+      }
       __syncthreads();
-      if (threadIdx.x == 0) {
-        double u[8];
+      if (threadIdx.x < 32) {
+        const int w = threadIdx.x & (kBlock / 32 - 1);
+        double t = red[w] + f32_to_f64(last[w]);
 #pragma unroll
-        for (int w = 0; w < 8; ++w) u[w] = red[w];
-        *slot = tree8(u);
+        for (int o = kBlock / 64; o > 0; o >>= 1) t += __shfl_xor_sync(kFull, t, o);
+        if (threadIdx.x == 0) *slot = t;
       }
     } else {
       const double v[1] = {part};
