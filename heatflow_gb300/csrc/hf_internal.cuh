@@ -559,7 +559,7 @@ cudaError_t launch_subbox_gather(Ctx& c, int64_t inst, const int64_t* lo, const 
 // Temperature role buffer `which` of every instance <-> a compact device array, on `stream`;
 // host_in drops the stored products H T of an instance whose state it changes.
 cudaError_t launch_host_in(Ctx& c, const double* src, int which, cudaStream_t stream);
-// The same for the device cells [glo, ghi) (whole z-slabs of instances, padding skipped).
+// The same for the device cells [glo, ghi) (padding skipped).
 cudaError_t launch_host_in_range(Ctx& c, const double* src, int which, int64_t glo, int64_t ghi,
                                  cudaStream_t stream);
 cudaError_t launch_stage_fallback(Ctx& c);
